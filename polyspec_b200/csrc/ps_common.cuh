@@ -42,6 +42,10 @@ struct Plan {
   RingInfo* d_rings;        // [R]
   double* d_mnorm0;         // [mmax+1] spin-0 seed normalisation
   SeedNorm* d_seed[4];      // [mmax+1] per spin 1..3 (index 1..3), null if not in spin_mask
+  // FP64 plans: recurrence tables of the Legendre stage per spin (leg_tables_f64), null if not in spin_mask:
+  // c [nalm] (spin 0) or (c, d) [nalm][2], and gam [nalm]
+  double* d_leg_cd[4];
+  double* d_leg_g[4];
   double2* d_twiddle;       // [max_fft/2] e^{-2 pi i k / max_fft}
   double2* d_bs_spec;       // Bluestein spectra (FP64)
   float2* d_twiddle_f;      // FP32 copies for the mixed-precision ring transforms

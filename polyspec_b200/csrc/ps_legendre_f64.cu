@@ -3,32 +3,76 @@
 // Synthesis, per order m and ring pair (theta, pi - theta):
 //   spin 0:  F_m(theta) = sum_l lam_lm(theta) a_lm, split by the parity of l+m
 //            so that the mirror ring is  E - O  where the north ring is E + O.
-//   spin s:  the same with F+ = (+s lam + -s lam)/2 and F- = (+s lam - -s lam)/2
-//            against G and C (HEALPix conventions of polyspec/base.py:247-288).
-// Adjoint: a_lm = sum_rings lam_lm(theta_r) P_m(r) (and the spin analogue),
-// the exact adjoint under the m-weighted alm inner product of
+//   spin s:  with f = +s lam, g = -s lam (HEALPix conventions of
+//            polyspec/base.py:247-288) and a+- = G +- i C, the sums
+//            S+ = sum f a+, S- = sum g a- on the north ring and the same with
+//            f and g exchanged and the sign (-1)^(l+m) on its mirror; then
+//            Q = -(S+ + S-)/2, U = i (S+ - S-)/2 for even s, Q = -(S+ - S-)/2,
+//            U = i (S+ + S-)/2 for odd s.
+// Adjoint: the exact transpose, a_lm = sum_rings lam_lm(theta_r) P_m(r) (and the
+// spin analogue), under the m-weighted alm inner product of
 // polyspec/weighting.py:255, i.e. ducc0.sht.adjoint_synthesis.
 //
-// The recurrences (normalised associated Legendre functions for spin 0,
-// spin-weighted harmonics in the Goldberg/HEALPix convention for spin s) run in
-// FP64 with seeds scaled by 2^(800k) so that high m near the poles neither
-// underflows nor loses accuracy (Reinecke & Seljebotn 2013).
+// Recurrences: lam_l = gam_l mu_l with gam chosen so that the three-term
+// recurrence keeps the unit coefficient on its second term,
+//   mu_{l+1} = c_l x mu_l - mu_{l-1},   f_{l+1} = (c_l x + d_l) f_l - f_{l-1},
+//   g_{l+1} = (c_l x - d_l) g_l - g_{l-1}   (f, g scaled alike)
+// two FP64 instructions per l (four for f and g).  c, d and gam are tables of the
+// plan (leg_tables_f64); gam multiplies the alm once, outside the ring loops.
+// Seeds are scaled by 2^(800k) so that high m near the poles neither underflows
+// nor loses accuracy (Reinecke & Seljebotn 2013).
 //
-// Layouts: almT [nalm][B][ncomp] (m-major l within, map index and G/C
-// innermost), phase [R][mmax+1][B][ncomp] (ring-major, order m, then maps).
+// What bounds these kernels: the FP64 pipe (64 lanes per clock and SM; the FP64
+// MMA shares it, 37 TFLOP/s either way).  Per l and ring a map needs 2 (spin 0) or
+// 8 (spin s) FMAs, so for one map the recurrence is half (a third) of the work and
+// everything else has to stay off that pipe: range checks compare the exponent
+// bits as integers, values still below 2^-400 are not accumulated, and rings are
+// kept several to a thread so that one broadcast of c and the alm from shared
+// memory serves them all.
+//
+// Layouts: alm [B][ncomp][nalm] (m-major), phase [R][mmax+1][B][ncomp] (ring-major,
+// order m, then maps and Q/U).
+#include <algorithm>
+#include <type_traits>
+
 #include "ps_common.cuh"
 #include "ps_stats.cuh"
 
 namespace ps {
 
-constexpr int SYN_THREADS = 128;  // ring pairs per synthesis CTA
-constexpr int SYN_LCH = 64;       // l chunk staged in shared memory
-constexpr int ADJ_THREADS = 128;  // ring pairs per adjoint CTA (== ring tile)
-constexpr int ADJ_LCH = 16;       // l chunk of the adjoint's Legendre tile
+constexpr int SYN_THREADS = 128;  // threads per synthesis CTA
+constexpr int ADJ_LCH = 64;       // l chunk of the adjoint between two CTA barriers
 
 // ---------------------------------------------------------------- seeds
+// The products of ps_common.cuh's snorm / smul / spow on positive normal values,
+// with the exponent taken from the bits (frexp handles cases that do not occur here).
+__device__ __forceinline__ Scaled qnorm(double x) {
+  const int hi = __double2hiint(x);
+  Scaled r;
+  r.e = ((hi >> 20) & 0x7ff) - 1022;
+  r.v = __hiloint2double((hi & 0x000fffff) | 0x3fe00000, __double2loint(x));
+  return r;
+}
+__device__ __forceinline__ Scaled qmul(Scaled a, Scaled b) {
+  Scaled r = qnorm(a.v * b.v);
+  r.e += a.e + b.e;
+  return r;
+}
+__device__ __forceinline__ Scaled qpow(double x, int n) {
+  Scaled r;
+  r.v = 0.5;
+  r.e = 1;
+  Scaled b = qnorm(x);
+  while (n) {
+    if (n & 1) r = qmul(r, b);
+    b = qmul(b, b);
+    n >>= 1;
+  }
+  return r;
+}
+
 __device__ __forceinline__ void seed_spin0(int m, double sth, double mnorm, double& v, int& k) {
-  Scaled s = smul(spow(sth, m), snorm(mnorm));
+  Scaled s = qmul(qpow(sth, m), qnorm(mnorm));
   to_kscale(s, v, k);
   if (m & 1) v = -v;
 }
@@ -38,21 +82,15 @@ __device__ __forceinline__ void seed_spin0(int m, double sth, double mnorm, doub
 __device__ __forceinline__ void seed_spin(int m, int s, const RingInfo& g, SeedNorm nrm, double& f, double& gg,
                                           int& k) {
   const double sh = sqrt(0.5 * g.omz), ch = sqrt(0.5 * g.opz);
-  Scaled pf, pg;
-  double sgn_f, sgn_g;
-  if (m >= s) {
-    pf = smul(spow(sh, m + s), spow(ch, m - s));
-    pg = smul(spow(sh, m - s), spow(ch, m + s));
-    sgn_f = (m & 1) ? -1.0 : 1.0;
-    sgn_g = sgn_f;
-  } else {
-    pf = smul(spow(sh, s + m), spow(ch, s - m));
-    pg = smul(spow(sh, s - m), spow(ch, s + m));
-    sgn_f = (m & 1) ? -1.0 : 1.0;
-    sgn_g = (s & 1) ? -1.0 : 1.0;
-  }
-  Scaled n; n.v = nrm.v; n.e = nrm.e;
-  Scaled sf = smul(n, pf), sg = smul(n, pg);
+  const int lo = m < s ? m : s, hi = m < s ? s : m;
+  Scaled pf = qmul(qpow(sh, hi + lo), qpow(ch, hi - lo));
+  Scaled pg = qmul(qpow(sh, hi - lo), qpow(ch, hi + lo));
+  const double sgn_f = (m & 1) ? -1.0 : 1.0;
+  const double sgn_g = m >= s ? sgn_f : (s & 1) ? -1.0 : 1.0;
+  Scaled n;
+  n.v = nrm.v;
+  n.e = nrm.e;
+  Scaled sf = qmul(n, pf), sg = qmul(n, pg);
   Scaled big = (sf.e >= sg.e) ? sf : sg;
   double vb;
   to_kscale(big, vb, k);
@@ -61,17 +99,14 @@ __device__ __forceinline__ void seed_spin(int m, int s, const RingInfo& g, SeedN
   gg = ldexp(sg.v, max(sg.e - shift, -2000)) * sgn_g;
 }
 
-// spin-0 recurrence coefficients to step lam_{l-1} -> lam_l:
-//   lam_l = a_l x lam_{l-1} - b_l lam_{l-2},  a_l = sqrt((4l^2-1)/(l^2-m^2)), b_l = a_l/a_{l-1}
-__device__ __forceinline__ void coef_spin0(int l, int m, double& a, double& b) {
-  const double mm = double(m) * m;
-  a = sqrt((4.0 * l * l - 1.0) / (double(l) * l - mm));
-  b = 0.0;
-  if (l >= m + 2) b = a / sqrt((4.0 * (l - 1.0) * (l - 1.0) - 1.0) / ((l - 1.0) * (l - 1.0) - mm));
+// ---------------------------------------------------------------- recurrence tables
+// Three-term coefficients of the normalised functions:
+//   spin 0  lam_l = a_l x lam_{l-1} - (a_l / a_{l-1}) lam_{l-2},  a_l = sqrt((4l^2-1)/(l^2-m^2))
+//   spin s  f_{l+1} = (A x + D) f_l - C f_{l-1}  (g: -D),  l >= max(m, s)
+__device__ __forceinline__ double coef_a(int l, int m) {
+  const double ll = double(l) * l;
+  return sqrt((4.0 * ll - 1.0) / (ll - double(m) * m));
 }
-
-// spin-s coefficients to step l -> l+1 (l >= max(m, s)):
-//   f_{l+1} = (A x + D) f_l - C f_{l-1},  g_{l+1} = (A x - D) g_l - C g_{l-1}
 __device__ __forceinline__ void coef_spin(int l, int m, int s, double& A, double& D, double& C) {
   auto rho = [&](double L) {
     return sqrt(fmax(L * L - double(m) * m, 0.0) * fmax(L * L - double(s) * s, 0.0));
@@ -82,375 +117,629 @@ __device__ __forceinline__ void coef_spin(int l, int m, int s, double& A, double
   C = sqrt((2.0 * l + 3.0) / (2.0 * l - 1.0)) * (l + 1.0) * rho(double(l)) / (double(l) * r1);
 }
 
+// One thread per order m: gam_{l0} = gam_{l0+1} = 1 at l0 = max(m, s), gam_{l+1} = C_l gam_{l-1} and
+// c_l = A_l gam_l / gam_{l+1} (d alike).  spin 0: cd is c [nalm]; spin s: (c, d) pairs.  Entries with
+// l < s are zero.  Runs once per plan (0.2 ms at lmax 2048).
+__global__ void leg_tables_f64(int lmax, int mmax, int s, double* __restrict__ cd, double* __restrict__ gam) {
+  const int m = blockIdx.x * blockDim.x + threadIdx.x;
+  if (m > mmax) return;
+  const int l0 = max(m, s);
+  const int64_t o = alm_index(0, m, lmax);
+  for (int l = m; l < min(l0, lmax + 1); ++l) {
+    cd[2 * (o + l)] = cd[2 * (o + l) + 1] = 0.0;  // l < s only for spin s
+    gam[o + l] = 0.0;
+  }
+  double g0 = 1.0, gm = 1.0;  // gam_l, gam_{l-1}
+  double a0 = 0.0;
+  for (int l = l0; l <= lmax; ++l) {
+    if (s == 0) {
+      const double a1 = coef_a(l + 1, m);
+      const double g1 = l == l0 ? 1.0 : a1 / a0 * gm;
+      cd[o + l] = a1 * g0 / g1;
+      gam[o + l] = g0;
+      a0 = a1;
+      gm = g0;
+      g0 = g1;
+    } else {
+      double A, D, C;
+      coef_spin(l, m, s, A, D, C);
+      const double g1 = l == l0 ? 1.0 : C * gm;
+      cd[2 * (o + l)] = A * g0 / g1;
+      cd[2 * (o + l) + 1] = D * g0 / g1;
+      gam[o + l] = g0;
+      gm = g0;
+      g0 = g1;
+    }
+  }
+}
+
+// Size tests read the exponent bits: an FP64 compare would take a slot of the FP64 pipe.
+constexpr int HI_FTHRESH = (1023 + 400) << 20;
+__device__ __forceinline__ bool passed(double v) { return (__double2hiint(v) & 0x7fffffff) >= HI_FTHRESH; }
+__device__ __forceinline__ bool nonfinite(double v) { return (__double2hiint(v) & 0x7ff00000) == 0x7ff00000; }
+__device__ __forceinline__ bool nonfinite(double2 v) { return nonfinite(v.x) || nonfinite(v.y); }
+
+// Rings of a warp that is not all live are looked at every four l: c x stays below 2^8 per l, far from
+// overflow.  A value with k < 0 that has grown past 2^400 moves up by one scale.
+__device__ __forceinline__ void rescale(int& k, double& cur, double& prev) {
+  if (k < 0 && passed(cur)) {
+    cur *= PS_FSMALL;
+    prev *= PS_FSMALL;
+    ++k;
+  }
+}
+__device__ __forceinline__ void rescale(int& k, double& f, double& fp, double& g, double& gp) {
+  if (k < 0 && (passed(f) || passed(g))) {
+    f *= PS_FSMALL;
+    fp *= PS_FSMALL;
+    g *= PS_FSMALL;
+    gp *= PS_FSMALL;
+    ++k;
+  }
+}
+
+// How a warp takes the next few l: no ring of it above 2^-400 yet (recurrence only), some, or all.
+enum { LEG_DEAD = 0, LEG_MIXED = 1, LEG_LIVE = 2 };
+template <int RPT>
+__device__ __forceinline__ int leg_mode(const int (&k)[RPT], bool force) {
+  bool all = true, any = false;
+#pragma unroll
+  for (int i = 0; i < RPT; ++i) {
+    all = all && k[i] == 0;
+    any = any || k[i] == 0;
+  }
+  if (__all_sync(0xffffffffu, all)) return LEG_LIVE;
+  return (force || __any_sync(0xffffffffu, any)) ? LEG_MIXED : LEG_DEAD;
+}
+
 // =====================================================================
 // synthesis, spin 0
-// grid (ceil(Rh/SYN_THREADS), mmax+1, ceil(B/NB))
-template <int NB>
+// grid (ceil(Rh / (SYN_THREADS RPT)), mmax+1, ceil(B/NB)); a warp holds 32 RPT neighbouring ring pairs and
+// stages its alm (times gam) and c itself, 32 l at a time and one chunk ahead: the warps of a CTA run at
+// different speeds (fewer instructions while their rings are dead), so they share no barrier.
+// A non-finite alm reaches every ring (its product with a value that counts as zero is NaN): a chunk
+// that holds one takes the mixed steps on all warps.
+template <int NB, int RPT>
 __global__ void __launch_bounds__(SYN_THREADS) synth0_f64(const RingInfo* __restrict__ rings,
                                                            const double* __restrict__ mnorm,
-                                                           const double2* __restrict__ almT,
+                                                           const double* __restrict__ lc,
+                                                           const double* __restrict__ lg,
+                                                           const double2* __restrict__ alm,
                                                            double2* __restrict__ phase, int R, int Rh, int lmax,
-                                                           int mmax, int B) {
-  const int m = blockIdx.y;
-  const int rp = blockIdx.x * SYN_THREADS + threadIdx.x;
-  const int b0 = blockIdx.z * NB;
-  __shared__ double s_a[SYN_LCH], s_b[SYN_LCH];
-  __shared__ double2 s_alm[SYN_LCH][NB];
-  const bool active = rp < Rh;
-  const RingInfo g = rings[active ? rp : 0];
-  const double x = g.z;
-  double cur, prev = 0.0;
-  int k;
-  seed_spin0(m, g.sth, mnorm[m], cur, k);
-  double2 ae[NB], ao[NB];
-#pragma unroll
-  for (int i = 0; i < NB; ++i) { ae[i] = make_double2(0.0, 0.0); ao[i] = ae[i]; }
+                                                           int mmax, int B, int64_t nalm) {
+  const int m = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, b0 = blockIdx.z * NB;
+  const int wbase = (blockIdx.x * SYN_THREADS + (tid & ~31)) * RPT, r0 = wbase + lane;
+  if (wbase >= Rh) return;
+  __shared__ double s_c_[SYN_THREADS / 32][2][32];
+  __shared__ double2 s_alm_[SYN_THREADS / 32][2][32][NB];
+  double(*s_c)[32] = s_c_[warp];
+  double2(*s_alm)[32][NB] = s_alm_[warp];
   const int64_t base = alm_index(m, m, lmax);
-  for (int l0 = m; l0 <= lmax; l0 += SYN_LCH) {
-    const int n = min(SYN_LCH, lmax - l0 + 1);
-    for (int j = threadIdx.x; j < SYN_LCH; j += SYN_THREADS) {
-      double a = 0.0, b = 0.0;
-      const int l = l0 + j + 1;  // coefficients producing lam_{l0+j+1}
-      if (l <= lmax) coef_spin0(l, m, a, b);
-      s_a[j] = a; s_b[j] = b;
-    }
-    for (int t = threadIdx.x; t < n * NB; t += SYN_THREADS) {
-      const int j = t / NB, bi = t % NB;
-      s_alm[j][bi] = (b0 + bi < B) ? almT[(base + (l0 - m) + j) * B + b0 + bi] : make_double2(0.0, 0.0);
-    }
-    __syncthreads();
-    // l0 + m is even, so even j are parity 0 and odd j parity 1
-    auto step = [&](int j, double2* acc) {
-      const double val = (k == 0) ? cur : 0.0;
+
+  double2 pa[NB];
+  double pc;
+  auto fetch = [&](int l0) {  // the chunk's alm (times gam) and c, into registers
+    const int64_t idx = base + (l0 - m) + lane;
+    const bool in = l0 + lane <= lmax;
+    const double gm = in ? lg[idx] : 0.0;
+    pc = l0 + lane < lmax ? lc[idx] : 0.0;
 #pragma unroll
-      for (int i = 0; i < NB; ++i) acc[i] = cfma(val, s_alm[j][i], acc[i]);
-      const double nxt = s_a[j] * x * cur - s_b[j] * prev;
-      prev = cur;
-      cur = nxt;
-      if (k < 0 && fabs(cur) > PS_FTHRESH) { cur *= PS_FSMALL; prev *= PS_FSMALL; ++k; }
+    for (int b = 0; b < NB; ++b)
+      pa[b] = in && b0 + b < B ? cscale(alm[int64_t(b0 + b) * nalm + idx], gm) : make_double2(0.0, 0.0);
+  };
+  auto stage = [&](int buf) {  // registers -> shared memory; whether a value is not finite
+    bool bad = false;
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+      s_alm[buf][lane][b] = pa[b];
+      bad = bad || nonfinite(pa[b]);
+    }
+    s_c[buf][lane] = pc;
+    return __any_sync(0xffffffffu, bad);  // also orders the stores before the warp's reads
+  };
+
+  fetch(m);
+  double x[RPT], cur[RPT], prev[RPT];
+  int k[RPT];
+  const double mn = mnorm[m];
+#pragma unroll
+  for (int i = 0; i < RPT; ++i) {
+    const int rp = r0 + 32 * i;
+    const RingInfo& g = rings[rp < Rh ? rp : 0];
+    x[i] = g.z;
+    prev[i] = 0.0;
+    seed_spin0(m, g.sth, mn, cur[i], k[i]);
+    if (rp >= Rh) { cur[i] = 0.0; k[i] = 0; }
+  }
+  double2 ae[RPT][NB], ao[RPT][NB];
+#pragma unroll
+  for (int i = 0; i < RPT; ++i)
+#pragma unroll
+    for (int b = 0; b < NB; ++b) ae[i][b] = ao[i][b] = make_double2(0.0, 0.0);
+
+  int buf = 0;
+  for (int l0 = m; l0 <= lmax; l0 += 32, buf ^= 1) {
+    const bool force = stage(buf);
+    __syncwarp();
+    const int n = min(32, lmax - l0 + 1);
+    if (l0 + 32 <= lmax) fetch(l0 + 32);
+    auto step = [&](auto mode, int j, double2 (&acc)[RPT][NB]) {
+      constexpr int MODE = decltype(mode)::value;
+      const double c = s_c[buf][j];
+      double2 a[NB];
+      if (MODE != LEG_DEAD) {
+#pragma unroll
+        for (int b = 0; b < NB; ++b) a[b] = s_alm[buf][j][b];
+      }
+#pragma unroll
+      for (int i = 0; i < RPT; ++i) {
+        if (MODE != LEG_DEAD) {
+          const double v = (MODE == LEG_LIVE || k[i] == 0) ? cur[i] : 0.0;
+#pragma unroll
+          for (int b = 0; b < NB; ++b) acc[i][b] = cfma(v, a[b], acc[i][b]);
+        }
+        const double nxt = fma(c * x[i], cur[i], -prev[i]);
+        prev[i] = cur[i];
+        cur[i] = nxt;
+      }
+    };
+    auto four = [&](auto mode, int j) {  // l0 + m is even: even j have parity 0
+      step(mode, j, ae);
+      step(mode, j + 1, ao);
+      step(mode, j + 2, ae);
+      step(mode, j + 3, ao);
     };
     int j = 0;
-    for (; j + 1 < n; j += 2) { step(j, ae); step(j + 1, ao); }
-    if (j < n) step(j, ae);
-    __syncthreads();
-  }
-  if (!active) return;
-  const int rs = R - 1 - rp;
+    while (j + 4 <= n) {
+      const int mode = leg_mode<RPT>(k, force);
+      if (mode == LEG_LIVE) {
+        for (; j + 8 <= n; j += 8) {
+          four(std::integral_constant<int, LEG_LIVE>{}, j);
+          four(std::integral_constant<int, LEG_LIVE>{}, j + 4);
+        }
+        if (j + 4 <= n) { four(std::integral_constant<int, LEG_LIVE>{}, j); j += 4; }
+        break;
+      }
+      if (mode == LEG_DEAD) four(std::integral_constant<int, LEG_DEAD>{}, j);
+      else four(std::integral_constant<int, LEG_MIXED>{}, j);
+      j += 4;
 #pragma unroll
-  for (int i = 0; i < NB; ++i) {
-    if (b0 + i >= B) break;
-    phase[(int64_t(rp) * (mmax + 1) + m) * B + b0 + i] = cadd(ae[i], ao[i]);
-    if (rs != rp) phase[(int64_t(rs) * (mmax + 1) + m) * B + b0 + i] = csub(ae[i], ao[i]);
+      for (int i = 0; i < RPT; ++i) rescale(k[i], cur[i], prev[i]);
+    }
+    for (; j < n; ++j) {
+      if (j & 1) step(std::integral_constant<int, LEG_MIXED>{}, j, ao);
+      else step(std::integral_constant<int, LEG_MIXED>{}, j, ae);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < RPT; ++i) {
+    const int rp = r0 + 32 * i, rs = R - 1 - rp;
+    if (rp >= Rh) break;
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+      if (b0 + b >= B) break;
+      phase[(int64_t(rp) * (mmax + 1) + m) * B + b0 + b] = cadd(ae[i][b], ao[i][b]);
+      if (rs != rp) phase[(int64_t(rs) * (mmax + 1) + m) * B + b0 + b] = csub(ae[i][b], ao[i][b]);
+    }
   }
 }
 
 // =====================================================================
-// synthesis, spin s > 0.  almT [nalm][B][2] (G,C); phase [R][mmax+1][B][2] (Q,U)
-template <int NB>
+// synthesis, spin s > 0: alm [B][2][nalm] (G, C) -> phase [R][mmax+1][B][2] (Q, U)
+template <int NB, int RPT>
 __global__ void __launch_bounds__(SYN_THREADS) synthS_f64(const RingInfo* __restrict__ rings,
                                                            const SeedNorm* __restrict__ seednorm,
-                                                           const double2* __restrict__ almT,
+                                                           const double2* __restrict__ lcd,
+                                                           const double* __restrict__ lg,
+                                                           const double2* __restrict__ alm,
                                                            double2* __restrict__ phase, int R, int Rh, int lmax,
-                                                           int mmax, int B, int spin) {
-  const int m = blockIdx.y;
-  const int rp = blockIdx.x * SYN_THREADS + threadIdx.x;
-  const int b0 = blockIdx.z * NB;
-  __shared__ double s_A[SYN_LCH], s_D[SYN_LCH], s_C[SYN_LCH];
-  __shared__ double2 s_alm[SYN_LCH][NB][2];
-  const bool active = rp < Rh;
-  const RingInfo g = rings[active ? rp : 0];
-  const double x = g.z;
-  const int lmin = max(m, spin);
-  double sf, sg;
-  int k;
-  seed_spin(m, spin, g, seednorm[m], sf, sg, k);
-  double f = 0.0, gg = 0.0, fp = 0.0, gp = 0.0;
-  // accumulators [parity]: G*F+, G*F-, C*F+, C*F-
-  double2 GP[2][NB], GM[2][NB], CP[2][NB], CM[2][NB];
-#pragma unroll
-  for (int p = 0; p < 2; ++p)
-#pragma unroll
-    for (int i = 0; i < NB; ++i) {
-      GP[p][i] = make_double2(0.0, 0.0); GM[p][i] = GP[p][i]; CP[p][i] = GP[p][i]; CM[p][i] = GP[p][i];
-    }
+                                                           int mmax, int B, int64_t nalm, int spin) {
+  const int m = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, b0 = blockIdx.z * NB;
+  const int wbase = (blockIdx.x * SYN_THREADS + (tid & ~31)) * RPT, r0 = wbase + lane;
+  if (wbase >= Rh) return;
+  __shared__ double2 s_cd_[SYN_THREADS / 32][2][32];
+  __shared__ double2 s_alm_[SYN_THREADS / 32][2][32][NB][2];  // a+ = G + i C, a- = G - i C
+  double2(*s_cd)[32] = s_cd_[warp];
+  double2(*s_alm)[32][NB][2] = s_alm_[warp];
   const int64_t base = alm_index(m, m, lmax);
-  for (int l0 = m; l0 <= lmax; l0 += SYN_LCH) {
-    const int n = min(SYN_LCH, lmax - l0 + 1);
-    for (int j = threadIdx.x; j < SYN_LCH; j += SYN_THREADS) {
-      double A = 0.0, D = 0.0, C = 0.0;
-      const int l = l0 + j;  // step l -> l+1
-      if (l >= lmin && l < lmax) coef_spin(l, m, spin, A, D, C);
-      s_A[j] = A; s_D[j] = D; s_C[j] = C;
-    }
-    for (int t = threadIdx.x; t < n * NB; t += SYN_THREADS) {
-      const int j = t / NB, bi = t % NB;
-      const bool ok = b0 + bi < B;
-      const int64_t idx = ((base + (l0 - m) + j) * B + b0 + bi) * 2;
-      s_alm[j][bi][0] = ok ? almT[idx] : make_double2(0.0, 0.0);
-      s_alm[j][bi][1] = ok ? almT[idx + 1] : make_double2(0.0, 0.0);
-    }
-    __syncthreads();
-    auto step = [&](int j, int p) {
-      const int l = l0 + j;
-      if (l == lmin) { f = sf; gg = sg; fp = 0.0; gp = 0.0; }
-      const double vf = (k == 0) ? 0.5 * (f + gg) : 0.0;  // F+
-      const double vm = (k == 0) ? 0.5 * (f - gg) : 0.0;  // F-
+  const int lmin = max(m, spin);
+
+  double2 pp[NB], pm[NB], pc;
+  auto fetch = [&](int l0) {
+    const int64_t idx = base + (l0 - m) + lane;
+    const bool in = l0 + lane <= lmax;
+    const double gm = in ? lg[idx] : 0.0;
+    pc = l0 + lane < lmax ? lcd[idx] : make_double2(0.0, 0.0);
 #pragma unroll
-      for (int i = 0; i < NB; ++i) {
-        const double2 G = s_alm[j][i][0], C = s_alm[j][i][1];
-        GP[p][i] = cfma(vf, G, GP[p][i]);
-        GM[p][i] = cfma(vm, G, GM[p][i]);
-        CP[p][i] = cfma(vf, C, CP[p][i]);
-        CM[p][i] = cfma(vm, C, CM[p][i]);
+    for (int b = 0; b < NB; ++b) {
+      pp[b] = pm[b] = make_double2(0.0, 0.0);
+      if (in && b0 + b < B) {
+        const double2 G = cscale(alm[int64_t(b0 + b) * 2 * nalm + idx], gm);
+        const double2 C = cscale(alm[(int64_t(b0 + b) * 2 + 1) * nalm + idx], gm);
+        pp[b] = make_double2(G.x - C.y, G.y + C.x);
+        pm[b] = make_double2(G.x + C.y, G.y - C.x);
       }
-      const double ax = s_A[j] * x;
-      const double fn = (ax + s_D[j]) * f - s_C[j] * fp;
-      const double gn = (ax - s_D[j]) * gg - s_C[j] * gp;
-      fp = f; f = fn; gp = gg; gg = gn;
-      if (k < 0 && fmax(fabs(f), fabs(gg)) > PS_FTHRESH) {
-        f *= PS_FSMALL; fp *= PS_FSMALL; gg *= PS_FSMALL; gp *= PS_FSMALL; ++k;
+    }
+  };
+  auto stage = [&](int buf) {
+    bool bad = false;
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+      s_alm[buf][lane][b][0] = pp[b];
+      s_alm[buf][lane][b][1] = pm[b];
+      bad = bad || nonfinite(pp[b]) || nonfinite(pm[b]);
+    }
+    s_cd[buf][lane] = pc;
+    return __any_sync(0xffffffffu, bad);
+  };
+
+  fetch(lmin);
+  double x[RPT], f[RPT], fp[RPT], g[RPT], gp[RPT];
+  int k[RPT];
+  const SeedNorm sn = seednorm[m];
+#pragma unroll
+  for (int i = 0; i < RPT; ++i) {
+    const int rp = r0 + 32 * i;
+    const RingInfo& gi = rings[rp < Rh ? rp : 0];
+    x[i] = gi.z;
+    fp[i] = gp[i] = 0.0;
+    seed_spin(m, spin, gi, sn, f[i], g[i], k[i]);
+    if (rp >= Rh) { f[i] = g[i] = 0.0; k[i] = 0; }
+  }
+  // sums on the north ring and, with the sign of l - lmin, on its mirror
+  double2 PN[RPT][NB], MN[RPT][NB], PS[RPT][NB], MS[RPT][NB];
+#pragma unroll
+  for (int b = 0; b < NB; ++b) {
+    double2 z = make_double2(0.0, 0.0);
+    // alm with l < s do not enter, unless not finite (0 times them)
+    for (int l = m; l < min(spin, lmax + 1) && b0 + b < B; ++l)
+      for (int c = 0; c < 2; ++c) z = cfma(0.0, alm[(int64_t(b0 + b) * 2 + c) * nalm + base + (l - m)], z);
+#pragma unroll
+    for (int i = 0; i < RPT; ++i) PN[i][b] = MN[i][b] = PS[i][b] = MS[i][b] = z;
+  }
+
+  int buf = 0;
+  for (int l0 = lmin; l0 <= lmax; l0 += 32, buf ^= 1) {
+    const bool force = stage(buf);
+    __syncwarp();
+    const int n = min(32, lmax - l0 + 1);
+    if (l0 + 32 <= lmax) fetch(l0 + 32);
+    auto step = [&](auto mode, auto odd, int j) {
+      constexpr int MODE = decltype(mode)::value;
+      constexpr double SG = decltype(odd)::value ? -1.0 : 1.0;
+      const double2 cd = s_cd[buf][j];
+      double2 ap[NB], am[NB];
+      if (MODE != LEG_DEAD) {
+#pragma unroll
+        for (int b = 0; b < NB; ++b) { ap[b] = s_alm[buf][j][b][0]; am[b] = s_alm[buf][j][b][1]; }
+      }
+#pragma unroll
+      for (int i = 0; i < RPT; ++i) {
+        if (MODE != LEG_DEAD) {
+          const bool on = MODE == LEG_LIVE || k[i] == 0;
+          const double vf = on ? f[i] : 0.0, vg = on ? g[i] : 0.0;
+#pragma unroll
+          for (int b = 0; b < NB; ++b) {
+            PN[i][b] = cfma(vf, ap[b], PN[i][b]);
+            MN[i][b] = cfma(vg, am[b], MN[i][b]);
+            PS[i][b] = cfma(SG * vg, ap[b], PS[i][b]);
+            MS[i][b] = cfma(SG * vf, am[b], MS[i][b]);
+          }
+        }
+        const double fn = fma(fma(cd.x, x[i], cd.y), f[i], -fp[i]);
+        const double gn = fma(fma(cd.x, x[i], -cd.y), g[i], -gp[i]);
+        fp[i] = f[i]; f[i] = fn;
+        gp[i] = g[i]; g[i] = gn;
       }
     };
+    auto four = [&](auto mode, int j) {
+      step(mode, std::false_type{}, j);
+      step(mode, std::true_type{}, j + 1);
+      step(mode, std::false_type{}, j + 2);
+      step(mode, std::true_type{}, j + 3);
+    };
     int j = 0;
-    for (; j + 1 < n; j += 2) { step(j, 0); step(j + 1, 1); }
-    if (j < n) step(j, 0);
-    __syncthreads();
-  }
-  if (!active) return;
-  const int rs = R - 1 - rp;
-  const bool odd = spin & 1;
-#pragma unroll
-  for (int i = 0; i < NB; ++i) {
-    if (b0 + i >= B) break;
-    for (int side = 0; side < (rs != rp ? 2 : 1); ++side) {
-      // north: F+ and F- sums add; south: F+ -> (-1)^p, F- -> -(-1)^p
-      const double2 gps = side == 0 ? cadd(GP[0][i], GP[1][i]) : csub(GP[0][i], GP[1][i]);
-      const double2 gms = side == 0 ? cadd(GM[0][i], GM[1][i]) : csub(GM[1][i], GM[0][i]);
-      const double2 cps = side == 0 ? cadd(CP[0][i], CP[1][i]) : csub(CP[0][i], CP[1][i]);
-      const double2 cms = side == 0 ? cadd(CM[0][i], CM[1][i]) : csub(CM[1][i], CM[0][i]);
-      double2 q, u;
-      if (!odd) {  // Q = -(G F+ + i C F-),  U = i G F- - C F+
-        q = make_double2(-(gps.x - cms.y), -(gps.y + cms.x));
-        u = make_double2(-gms.y - cps.x, gms.x - cps.y);
-      } else {     // Q = -(G F- + i C F+),  U = i G F+ - C F-
-        q = make_double2(-(gms.x - cps.y), -(gms.y + cps.x));
-        u = make_double2(-gps.y - cms.x, gps.x - cms.y);
+    while (j + 4 <= n) {
+      const int mode = leg_mode<RPT>(k, force);
+      if (mode == LEG_LIVE) {
+        for (; j + 4 <= n; j += 4) four(std::integral_constant<int, LEG_LIVE>{}, j);
+        break;
       }
-      const int rr = side == 0 ? rp : rs;
-      const int64_t o = ((int64_t(rr) * (mmax + 1) + m) * B + b0 + i) * 2;
-      phase[o] = q;
-      phase[o + 1] = u;
+      if (mode == LEG_DEAD) four(std::integral_constant<int, LEG_DEAD>{}, j);
+      else four(std::integral_constant<int, LEG_MIXED>{}, j);
+      j += 4;
+#pragma unroll
+      for (int i = 0; i < RPT; ++i) rescale(k[i], f[i], fp[i], g[i], gp[i]);
+    }
+    for (; j < n; ++j) {
+      if (j & 1) step(std::integral_constant<int, LEG_MIXED>{}, std::true_type{}, j);
+      else step(std::integral_constant<int, LEG_MIXED>{}, std::false_type{}, j);
+    }
+  }
+  const bool odd = spin & 1;
+  const double ss = ((lmin + m) & 1) ? -0.5 : 0.5;
+#pragma unroll
+  for (int i = 0; i < RPT; ++i) {
+    const int rp = r0 + 32 * i, rs = R - 1 - rp;
+    if (rp >= Rh) break;
+#pragma unroll
+    for (int b = 0; b < NB; ++b) {
+      if (b0 + b >= B) break;
+      for (int side = 0; side < (rs != rp ? 2 : 1); ++side) {
+        const double h = side == 0 ? 0.5 : ss;
+        const double2 sp = cscale(side == 0 ? PN[i][b] : PS[i][b], h), sm = cscale(side == 0 ? MN[i][b] : MS[i][b], h);
+        const double2 sum = cadd(sp, sm), dif = csub(sp, sm);
+        const double2 q = odd ? dif : sum, u = odd ? sum : dif;
+        const int64_t o = ((int64_t(side == 0 ? rp : rs) * (mmax + 1) + m) * B + b0 + b) * 2;
+        phase[o] = make_double2(-q.x, -q.y);
+        phase[o + 1] = make_double2(-u.y, u.x);
+      }
     }
   }
 }
 
-// =====================================================================
-// adjoint, spin 0.  One CTA per (ring tile of ADJ_THREADS pairs, m, map chunk):
-// the tile's threads run the recurrence of their ring and drop lam into a
-// shared [ADJ_LCH][ADJ_THREADS] tile; then each thread reduces one l over a
-// strided subset of rings and the 8 subsets of a warp are combined by
-// shuffles.  Output: partial[tile][nalm][B] (summed by reduce_partials).
-//
-// reduction mapping (4 warps): warp w -> parity p = w & 1, jset = w >> 1;
-// lane -> jq = lane >> 3, seg = lane & 7; l offset j = p + 2 (4 jset + jq);
-// rings seg, seg+8, ..., seg+120.
-template <int NB>
-__global__ void __launch_bounds__(ADJ_THREADS) adj0_f64(const RingInfo* __restrict__ rings,
-                                                         const double* __restrict__ mnorm,
-                                                         const double2* __restrict__ phase,
-                                                         double2* __restrict__ partial, int R, int Rh, int lmax,
-                                                         int mmax, int B, int bofs, int Bc, int64_t nalm) {
-  const int m = blockIdx.y;
-  const int tile = blockIdx.x;
-  const int tid = threadIdx.x;
-  const int rp = tile * ADJ_THREADS + tid;
-  const int b0 = bofs + blockIdx.z * NB;
-  // ring-contiguous layouts (a warp's 8 ring segments read consecutive words)
-  __shared__ double s_lam[ADJ_LCH][ADJ_THREADS + 2];
-  __shared__ double2 s_P[2][NB][ADJ_THREADS];  // [even/odd][map][ring]
-  __shared__ double s_a[ADJ_LCH], s_b[ADJ_LCH];
-  const bool active = rp < Rh;
-  const RingInfo g = rings[active ? rp : 0];
-  const int rs = R - 1 - rp;
+// ---------------------------------------------------------------- adjoint
+// One CTA per (m, map): its threads keep RPT ring pairs each, with their phases and the recurrence in
+// registers, and sum over their own rings; 16 partial sums at a time (8 l of spin 0: re, im; 4 l of spin s:
+// T+, T-) are then summed over the warp by halving exchanges: one FP64 add per value and thread next to the
+// RPT FMAs.  In the first exchange (spin s: the first two) no selection is needed, because the lanes with bit 4
+// set hold re and im (with bit 3 set: T+ and T-) exchanged from the start, so that every lane keeps its first
+// half and sends its second.  The warps' sums meet in shared memory, in a fixed order, once per ADJ_LCH values
+// of l, and alm are written directly: no partial sums in memory.  Rings beyond one pass of the CTA are further
+// passes over l that add to the alm the CTA wrote before.
+template <int H>
+__device__ __forceinline__ void halve(double* v, int lane, int bit) {
+  const bool up = lane & bit;
 #pragma unroll
-  for (int i = 0; i < NB; ++i) {
-    double2 pn = make_double2(0.0, 0.0), ps = pn;
-    if (active && b0 + i < bofs + Bc) {
-      pn = phase[(int64_t(rp) * (mmax + 1) + m) * B + b0 + i];
-      if (rs != rp) ps = phase[(int64_t(rs) * (mmax + 1) + m) * B + b0 + i];
-    }
-    s_P[0][i][tid] = cadd(pn, ps);
-    s_P[1][i][tid] = csub(pn, ps);
-  }
-  const double x = g.z;
-  double cur, prev = 0.0;
-  int k;
-  seed_spin0(m, g.sth, mnorm[m], cur, k);
-  if (!active) { cur = 0.0; k = 0; }
-  const int warp = tid >> 5, lane = tid & 31;
-  const int p = warp & 1, jset = warp >> 1, jq = lane >> 3, seg = lane & 7;
-  const int jr = p + 2 * (4 * jset + jq);
-  const int64_t base = alm_index(m, m, lmax);
-  for (int l0 = m; l0 <= lmax; l0 += ADJ_LCH) {
-    const int n = min(ADJ_LCH, lmax - l0 + 1);
-    if (tid < ADJ_LCH) {
-      double a = 0.0, b = 0.0;
-      const int l = l0 + tid + 1;
-      if (l <= lmax) coef_spin0(l, m, a, b);
-      s_a[tid] = a; s_b[tid] = b;
-    }
-    __syncthreads();
-    for (int j = 0; j < ADJ_LCH; ++j) {
-      s_lam[j][tid] = (k == 0) ? cur : 0.0;
-      const double nxt = s_a[j] * x * cur - s_b[j] * prev;
-      prev = cur;
-      cur = nxt;
-      if (k < 0 && fabs(cur) > PS_FTHRESH) { cur *= PS_FSMALL; prev *= PS_FSMALL; ++k; }
-    }
-    __syncthreads();
-    double2 acc[NB];
-#pragma unroll
-    for (int i = 0; i < NB; ++i) acc[i] = make_double2(0.0, 0.0);
-#pragma unroll 4
-    for (int t = 0; t < ADJ_THREADS / 8; ++t) {
-      const int r = seg + 8 * t;
-      const double lam = s_lam[jr][r];
-#pragma unroll
-      for (int i = 0; i < NB; ++i) acc[i] = cfma(lam, s_P[p][i][r], acc[i]);
-    }
-#pragma unroll
-    for (int i = 0; i < NB; ++i) {
-#pragma unroll
-      for (int off = 1; off < 8; off <<= 1) {
-        acc[i].x += __shfl_xor_sync(0xffffffffu, acc[i].x, off);
-        acc[i].y += __shfl_xor_sync(0xffffffffu, acc[i].y, off);
-      }
-    }
-    if (seg == 0 && jr < n) {
-      const int64_t idx = base + (l0 - m) + jr;
-#pragma unroll
-      for (int i = 0; i < NB; ++i)
-        if (b0 + i < bofs + Bc) partial[(int64_t(tile) * nalm + idx) * Bc + (b0 - bofs) + i] = acc[i];
-    }
-    __syncthreads();
+  for (int i = 0; i < H; ++i) {
+    const double send = up ? v[i] : v[i + H], keep = up ? v[i + H] : v[i];
+    v[i] = keep + __shfl_xor_sync(0xffffffffu, send, bit);
   }
 }
 
-// =====================================================================
-// adjoint, spin s.  phase [R][mmax+1][B][2] (Q,U) -> partial[tile][nalm][B][2] (G,C)
-template <int NB>
-__global__ void __launch_bounds__(ADJ_THREADS) adjS_f64(const RingInfo* __restrict__ rings,
-                                                         const SeedNorm* __restrict__ seednorm,
-                                                         const double2* __restrict__ phase,
-                                                         double2* __restrict__ partial, int R, int Rh, int lmax,
-                                                         int mmax, int B, int bofs, int Bc, int64_t nalm, int spin) {
-  const int m = blockIdx.y;
-  const int tile = blockIdx.x;
-  const int tid = threadIdx.x;
-  const int rp = tile * ADJ_THREADS + tid;
-  const int b0 = bofs + blockIdx.z * NB;
-  __shared__ double s_fp[ADJ_LCH][ADJ_THREADS + 2];
-  __shared__ double s_fm[ADJ_LCH][ADJ_THREADS + 2];
-  __shared__ double2 s_Q[2][NB][ADJ_THREADS];  // [N+S, N-S][map][ring]
-  __shared__ double2 s_U[2][NB][ADJ_THREADS];
-  __shared__ double s_A[ADJ_LCH], s_D[ADJ_LCH], s_C[ADJ_LCH];
-  const bool active = rp < Rh;
-  const RingInfo g = rings[active ? rp : 0];
-  const int rs = R - 1 - rp;
-#pragma unroll
-  for (int i = 0; i < NB; ++i) {
-    double2 qn = make_double2(0.0, 0.0), qs = qn, un = qn, us = qn;
-    if (active && b0 + i < bofs + Bc) {
-      const int64_t o = ((int64_t(rp) * (mmax + 1) + m) * B + b0 + i) * 2;
-      qn = phase[o]; un = phase[o + 1];
-      if (rs != rp) {
-        const int64_t o2 = ((int64_t(rs) * (mmax + 1) + m) * B + b0 + i) * 2;
-        qs = phase[o2]; us = phase[o2 + 1];
-      }
-    }
-    s_Q[0][i][tid] = cadd(qn, qs); s_Q[1][i][tid] = csub(qn, qs);
-    s_U[0][i][tid] = cadd(un, us); s_U[1][i][tid] = csub(un, us);
-  }
-  const double x = g.z;
-  const int lmin = max(m, spin);
-  double sf, sg;
-  int k;
-  seed_spin(m, spin, g, seednorm[m], sf, sg, k);
-  if (!active) { sf = 0.0; sg = 0.0; k = 0; }
-  double f = 0.0, gg = 0.0, fpv = 0.0, gpv = 0.0;
-  const int warp = tid >> 5, lane = tid & 31;
-  const int p = warp & 1, jset = warp >> 1, jq = lane >> 3, seg = lane & 7;
-  const int jr = p + 2 * (4 * jset + jq);
-  // F+ multiplies (N + (-1)^p S), F- multiplies (N - (-1)^p S)
-  const int cplus = p, cminus = 1 - p;
-  const bool odd = spin & 1;
+// adjoint, spin 0: phase [R][mmax+1][B] -> alm [B][nalm].  grid (1, mmax+1, B)
+template <int RPT, int NW>
+__global__ void __launch_bounds__(32 * NW) adj0_f64(const RingInfo* __restrict__ rings,
+                                                    const double* __restrict__ mnorm, const double* __restrict__ lc,
+                                                    const double* __restrict__ lg, const double2* __restrict__ phase,
+                                                    double2* __restrict__ alm, int R, int Rh, int lmax, int mmax,
+                                                    int B, int bofs, int64_t nalm, double scale) {
+  const int m = blockIdx.y, b = bofs + blockIdx.z, tid = threadIdx.x, nt = blockDim.x;
+  const int warp = tid >> 5, lane = tid & 31, nw = nt >> 5;
+  __shared__ double2 s_red[2][NW][ADJ_LCH];
+  __shared__ double s_c[2][ADJ_LCH];
   const int64_t base = alm_index(m, m, lmax);
-  for (int l0 = m; l0 <= lmax; l0 += ADJ_LCH) {
-    const int n = min(ADJ_LCH, lmax - l0 + 1);
-    if (tid < ADJ_LCH) {
-      double A = 0.0, D = 0.0, C = 0.0;
-      const int l = l0 + tid;
-      if (l >= lmin && l < lmax) coef_spin(l, m, spin, A, D, C);
-      s_A[tid] = A; s_D[tid] = D; s_C[tid] = C;
+  double2* out = alm + int64_t(b) * nalm + base;
+  const double mn = mnorm[m];
+  const bool up16 = lane & 16;
+  int buf = 0;
+  for (int t0 = 0; t0 < Rh; t0 += nt * RPT) {
+    const int wbase = t0 + warp * 32 * RPT;
+    double x[RPT], cur[RPT], prev[RPT];
+    double2 E[RPT], O[RPT];
+    int k[RPT];
+    bool bad = false;
+#pragma unroll
+    for (int i = 0; i < RPT; ++i) {
+      const int rp = wbase + lane + 32 * i, rs = R - 1 - rp;
+      const RingInfo& g = rings[rp < Rh ? rp : 0];
+      double2 pn = make_double2(0.0, 0.0), ps = pn;
+      if (rp < Rh) {
+        pn = phase[(int64_t(rp) * (mmax + 1) + m) * B + b];
+        if (rs != rp) ps = phase[(int64_t(rs) * (mmax + 1) + m) * B + b];
+      }
+      E[i] = cadd(pn, ps);
+      O[i] = csub(pn, ps);
+      bad = bad || nonfinite(E[i]) || nonfinite(O[i]);
+      if (up16) { E[i] = make_double2(E[i].y, E[i].x); O[i] = make_double2(O[i].y, O[i].x); }
+      x[i] = g.z;
+      prev[i] = 0.0;
+      seed_spin0(m, g.sth, mn, cur[i], k[i]);
+      if (rp >= Rh) { cur[i] = 0.0; k[i] = 0; }
     }
+    // a phase that is not finite reaches every l (0 times it), as in the synthesis
+    const bool force = __any_sync(0xffffffffu, bad);
+    for (int t = tid; t < ADJ_LCH; t += nt) s_c[buf][t] = m + t < lmax ? lc[base + t] : 0.0;
     __syncthreads();
-    for (int j = 0; j < ADJ_LCH; ++j) {
-      if (l0 + j == lmin) { f = sf; gg = sg; fpv = 0.0; gpv = 0.0; }
-      s_fp[j][tid] = (k == 0) ? 0.5 * (f + gg) : 0.0;
-      s_fm[j][tid] = (k == 0) ? 0.5 * (f - gg) : 0.0;
-      const double ax = s_A[j] * x;
-      const double fn = (ax + s_D[j]) * f - s_C[j] * fpv;
-      const double gn = (ax - s_D[j]) * gg - s_C[j] * gpv;
-      fpv = f; f = fn; gpv = gg; gg = gn;
-      if (k < 0 && fmax(fabs(f), fabs(gg)) > PS_FTHRESH) {
-        f *= PS_FSMALL; fpv *= PS_FSMALL; gg *= PS_FSMALL; gpv *= PS_FSMALL; ++k;
-      }
-    }
-    __syncthreads();
-    // S1 = sum F+ Q+, S2 = sum F- U-, S3 = sum F- Q-, S4 = sum F+ U+
-    double2 S1[NB], S2[NB], S3[NB], S4[NB];
+    for (int l0 = m; l0 <= lmax; l0 += ADJ_LCH, buf ^= 1) {
+      const int n = min(ADJ_LCH, lmax - l0 + 1);
+      for (int t = tid; t < ADJ_LCH; t += nt)
+        s_c[buf ^ 1][t] = l0 + ADJ_LCH + t < lmax ? lc[base + (l0 - m) + ADJ_LCH + t] : 0.0;
+#pragma unroll 1
+      for (int j0 = 0; j0 < n; j0 += 8) {
+        double v[16];
+        auto block = [&](auto mode) {
+          constexpr int MODE = decltype(mode)::value;
 #pragma unroll
-    for (int i = 0; i < NB; ++i) {
-      S1[i] = make_double2(0.0, 0.0); S2[i] = S1[i]; S3[i] = S1[i]; S4[i] = S1[i];
-    }
-#pragma unroll 2
-    for (int t = 0; t < ADJ_THREADS / 8; ++t) {
-      const int r = seg + 8 * t;
-      const double vp = s_fp[jr][r], vm = s_fm[jr][r];
+          for (int j = 0; j < 8; ++j) {
+            const double c = s_c[buf][j0 + j];
+            double a0 = 0.0, a1 = 0.0;
 #pragma unroll
-      for (int i = 0; i < NB; ++i) {
-        S1[i] = cfma(vp, s_Q[cplus][i][r], S1[i]);
-        S2[i] = cfma(vm, s_U[cminus][i][r], S2[i]);
-        S3[i] = cfma(vm, s_Q[cminus][i][r], S3[i]);
-        S4[i] = cfma(vp, s_U[cplus][i][r], S4[i]);
-      }
-    }
+            for (int i = 0; i < RPT; ++i) {
+              if (MODE != LEG_DEAD) {
+                const double w = (MODE == LEG_LIVE || k[i] == 0) ? cur[i] : 0.0;
+                const double2 p = (j & 1) ? O[i] : E[i];
+                a0 = fma(w, p.x, a0);
+                a1 = fma(w, p.y, a1);
+              }
+              const double nxt = fma(c * x[i], cur[i], -prev[i]);
+              prev[i] = cur[i];
+              cur[i] = nxt;
+            }
+            if (MODE != LEG_DEAD) v[j] = a0 + __shfl_xor_sync(0xffffffffu, a1, 16);
+            if (MODE != LEG_LIVE && (j & 3) == 3) {
 #pragma unroll
-    for (int i = 0; i < NB; ++i) {
-#pragma unroll
-      for (int off = 1; off < 8; off <<= 1) {
-        S1[i].x += __shfl_xor_sync(0xffffffffu, S1[i].x, off); S1[i].y += __shfl_xor_sync(0xffffffffu, S1[i].y, off);
-        S2[i].x += __shfl_xor_sync(0xffffffffu, S2[i].x, off); S2[i].y += __shfl_xor_sync(0xffffffffu, S2[i].y, off);
-        S3[i].x += __shfl_xor_sync(0xffffffffu, S3[i].x, off); S3[i].y += __shfl_xor_sync(0xffffffffu, S3[i].y, off);
-        S4[i].x += __shfl_xor_sync(0xffffffffu, S4[i].x, off); S4[i].y += __shfl_xor_sync(0xffffffffu, S4[i].y, off);
-      }
-    }
-    if (seg == 0 && jr < n) {
-      const int64_t idx = base + (l0 - m) + jr;
-#pragma unroll
-      for (int i = 0; i < NB; ++i) {
-        if (b0 + i >= bofs + Bc) break;
-        double2 G, C;
-        if (!odd) {  // G = -S1 - i S2, C = i S3 - S4
-          G = make_double2(-S1[i].x + S2[i].y, -S1[i].y - S2[i].x);
-          C = make_double2(-S3[i].y - S4[i].x, S3[i].x - S4[i].y);
-        } else {     // G = -S3 - i S4, C = i S1 - S2
-          G = make_double2(-S3[i].x + S4[i].y, -S3[i].y - S4[i].x);
-          C = make_double2(-S1[i].y - S2[i].x, S1[i].x - S2[i].y);
+              for (int i = 0; i < RPT; ++i) rescale(k[i], cur[i], prev[i]);
+            }
+          }
+        };
+        const int mode = wbase < Rh ? leg_mode<RPT>(k, force) : LEG_DEAD;
+        double r = 0.0;
+        if (mode == LEG_DEAD) {
+          if (wbase < Rh) block(std::integral_constant<int, LEG_DEAD>{});
+        } else {
+          if (mode == LEG_LIVE) block(std::integral_constant<int, LEG_LIVE>{});
+          else block(std::integral_constant<int, LEG_MIXED>{});
+          halve<4>(v, lane, 8);
+          halve<2>(v, lane, 4);
+          halve<1>(v, lane, 2);
+          r = v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
         }
-        const int64_t o = ((int64_t(tile) * nalm + idx) * Bc + (b0 - bofs) + i) * 2;
-        partial[o] = G;
-        partial[o + 1] = C;
+        if (!(lane & 1)) (&s_red[buf][warp][j0 + ((lane >> 1) & 7)].x)[lane >> 4] = r;
+      }
+      __syncthreads();
+      for (int t = tid; t < n; t += nt) {
+        double2 a = make_double2(0.0, 0.0);
+        for (int w = 0; w < nw; ++w) a = cadd(a, s_red[buf][w][t]);
+        const int64_t o = l0 - m + t;
+        a = cscale(a, lg[base + o] * scale);
+        out[o] = t0 == 0 ? a : cadd(out[o], a);
+      }
+    }
+    __syncthreads();  // s_c of the next pass
+  }
+}
+
+// adjoint, spin s: phase [R][mmax+1][B][2] (Q, U) -> alm [B][2][nalm] (G, C).  With Z+- = Q +- i U,
+// T+ = sum f Z+(north) + (-1)^(l+m) g Z+(south), T- = sum g Z-(north) + (-1)^(l+m) f Z-(south):
+// G = -(T+ + T-)/2, C = i (T+ - T-)/2 for even s, G = -(T+ - T-)/2, C = i (T+ + T-)/2 for odd s.
+template <int RPT, int NW>
+__global__ void __launch_bounds__(32 * NW) adjS_f64(const RingInfo* __restrict__ rings,
+                                                    const SeedNorm* __restrict__ seednorm,
+                                                    const double2* __restrict__ lcd, const double* __restrict__ lg,
+                                                    const double2* __restrict__ phase, double2* __restrict__ alm,
+                                                    int R, int Rh, int lmax, int mmax, int B, int bofs, int64_t nalm,
+                                                    int spin, double scale) {
+  const int m = blockIdx.y, b = bofs + blockIdx.z, tid = threadIdx.x, nt = blockDim.x;
+  const int warp = tid >> 5, lane = tid & 31, nw = nt >> 5;
+  __shared__ double s_red[2][NW][4 * ADJ_LCH];
+  __shared__ double2 s_cd[2][ADJ_LCH];
+  const int64_t base = alm_index(m, m, lmax);
+  double2* outG = alm + int64_t(b) * 2 * nalm + base;
+  double2* outC = outG + nalm;
+  const int lmin = max(m, spin);
+  const double sgn0 = ((lmin + m) & 1) ? -1.0 : 1.0;
+  const SeedNorm sn = seednorm[m];
+  const bool odd = spin & 1, up16 = lane & 16, up8 = lane & 8;
+  const int dflip = up8 ? int(0x80000000) : 0;  // lanes with T+ and T- exchanged run g first: d changes sign
+  int buf = 0;
+  for (int t0 = 0; t0 < Rh; t0 += nt * RPT) {
+    const int wbase = t0 + warp * 32 * RPT;
+    double x[RPT], f[RPT], fp[RPT], g[RPT], gp[RPT];
+    double2 ZPN[RPT], ZPS[RPT], ZMN[RPT], ZMS[RPT];
+    int k[RPT];
+    bool bad = false;
+#pragma unroll
+    for (int i = 0; i < RPT; ++i) {
+      const int rp = wbase + lane + 32 * i, rs = R - 1 - rp;
+      const RingInfo& gi = rings[rp < Rh ? rp : 0];
+      double2 qn = make_double2(0.0, 0.0), un = qn, qs = qn, us = qn;
+      if (rp < Rh) {
+        const int64_t o = ((int64_t(rp) * (mmax + 1) + m) * B + b) * 2;
+        qn = phase[o];
+        un = phase[o + 1];
+        if (rs != rp) {
+          const int64_t o2 = ((int64_t(rs) * (mmax + 1) + m) * B + b) * 2;
+          qs = cscale(phase[o2], sgn0);
+          us = cscale(phase[o2 + 1], sgn0);
+        }
+      }
+      bad = bad || nonfinite(qn) || nonfinite(un) || nonfinite(qs) || nonfinite(us);
+      auto z = [&](double2 q, double2 u, bool plus) {  // Q + i U or Q - i U, re and im exchanged in the upper lanes
+        const double2 v = plus ? make_double2(q.x - u.y, q.y + u.x) : make_double2(q.x + u.y, q.y - u.x);
+        return up16 ? make_double2(v.y, v.x) : v;
+      };
+      ZPN[i] = z(qn, un, !up8);
+      ZMN[i] = z(qn, un, up8);
+      ZPS[i] = z(qs, us, !up8);
+      ZMS[i] = z(qs, us, up8);
+      x[i] = gi.z;
+      fp[i] = gp[i] = 0.0;
+      double sf, sg;
+      seed_spin(m, spin, gi, sn, sf, sg, k[i]);
+      f[i] = up8 ? sg : sf;
+      g[i] = up8 ? sf : sg;
+      if (rp >= Rh) { f[i] = g[i] = 0.0; k[i] = 0; }
+    }
+    const bool force = __any_sync(0xffffffffu, bad);
+    for (int t = tid; t < ADJ_LCH; t += nt)
+      s_cd[buf][t] = lmin + t < lmax ? lcd[base + (lmin - m) + t] : make_double2(0.0, 0.0);
+    const bool anybad = __syncthreads_or(bad);
+    if (m < spin && tid < spin - m && m + tid <= lmax) {  // l < s: zero, or 0 times a phase that is not finite
+      const double z = anybad ? __longlong_as_double(0x7ff8000000000000LL) : 0.0;
+      outG[tid] = t0 == 0 ? make_double2(z, z) : cadd(outG[tid], make_double2(z, z));
+      outC[tid] = t0 == 0 ? make_double2(z, z) : cadd(outC[tid], make_double2(z, z));
+    }
+    for (int l0 = lmin; l0 <= lmax; l0 += ADJ_LCH, buf ^= 1) {
+      const int n = min(ADJ_LCH, lmax - l0 + 1);
+      for (int t = tid; t < ADJ_LCH; t += nt)
+        s_cd[buf ^ 1][t] = l0 + ADJ_LCH + t < lmax ? lcd[base + (l0 - m) + ADJ_LCH + t] : make_double2(0.0, 0.0);
+#pragma unroll 1
+      for (int j0 = 0; j0 < n; j0 += 4) {
+        double v[4];
+        auto block = [&](auto mode) {
+          constexpr int MODE = decltype(mode)::value;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const double2 cd = s_cd[buf][j0 + j];
+            const double d = __hiloint2double(__double2hiint(cd.y) ^ dflip, __double2loint(cd.y));
+            double2 tp = make_double2(0.0, 0.0), tm = tp;
+#pragma unroll
+            for (int i = 0; i < RPT; ++i) {
+              if (MODE != LEG_DEAD) {
+                const bool on = MODE == LEG_LIVE || k[i] == 0;
+                const double vf = on ? f[i] : 0.0, vg = on ? g[i] : 0.0;
+                tp = cfma(vf, ZPN[i], tp);
+                tm = cfma(vg, ZMN[i], tm);
+                tp = cfma((j & 1) ? -vg : vg, ZPS[i], tp);
+                tm = cfma((j & 1) ? -vf : vf, ZMS[i], tm);
+              }
+              const double fn = fma(fma(cd.x, x[i], d), f[i], -fp[i]);
+              const double gn = fma(fma(cd.x, x[i], -d), g[i], -gp[i]);
+              fp[i] = f[i]; f[i] = fn;
+              gp[i] = g[i]; g[i] = gn;
+            }
+            if (MODE != LEG_DEAD) {
+              const double p = tp.x + __shfl_xor_sync(0xffffffffu, tp.y, 16);
+              const double q = tm.x + __shfl_xor_sync(0xffffffffu, tm.y, 16);
+              v[j] = p + __shfl_xor_sync(0xffffffffu, q, 8);
+            }
+          }
+          if (MODE != LEG_LIVE) {
+#pragma unroll
+            for (int i = 0; i < RPT; ++i) rescale(k[i], f[i], fp[i], g[i], gp[i]);
+          }
+        };
+        const int mode = wbase < Rh ? leg_mode<RPT>(k, force) : LEG_DEAD;
+        double r = 0.0;
+        if (mode == LEG_DEAD) {
+          if (wbase < Rh) block(std::integral_constant<int, LEG_DEAD>{});
+        } else {
+          if (mode == LEG_LIVE) block(std::integral_constant<int, LEG_LIVE>{});
+          else block(std::integral_constant<int, LEG_MIXED>{});
+          halve<2>(v, lane, 4);
+          halve<1>(v, lane, 2);
+          r = v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+        }
+        // value: l = j0 + bits 2, 1; T- in bit 3; im in bit 4
+        if (!(lane & 1)) s_red[buf][warp][4 * (j0 + ((lane >> 1) & 3)) + 2 * ((lane >> 3) & 1) + (lane >> 4)] = r;
+      }
+      __syncthreads();
+      for (int t = tid; t < n; t += nt) {
+        double2 tp = make_double2(0.0, 0.0), tm = tp;
+        for (int w = 0; w < nw; ++w) {
+          const double* r = &s_red[buf][w][4 * t];
+          tp = cadd(tp, make_double2(r[0], r[1]));
+          tm = cadd(tm, make_double2(r[2], r[3]));
+        }
+        const int64_t o = l0 - m + t;
+        const double h = 0.5 * lg[base + o] * scale;
+        const double2 sum = cscale(cadd(tp, tm), h), dif = cscale(csub(tp, tm), h);
+        double2 G = odd ? dif : sum, C = odd ? sum : dif;
+        G = make_double2(-G.x, -G.y);
+        C = make_double2(-C.y, C.x);
+        outG[o] = t0 == 0 ? G : cadd(outG[o], G);
+        outC[o] = t0 == 0 ? C : cadd(outC[o], C);
       }
     }
     __syncthreads();
@@ -471,20 +760,6 @@ __global__ void alm_to_T(const double2* __restrict__ alm, double2* __restrict__ 
   }
 }
 
-// sum_t partial[t][nalm][B][ncomp] * scale -> alm [B][ncomp][nalm]
-__global__ void reduce_partials(const double2* __restrict__ partial, double2* __restrict__ alm, int ntiles, int B,
-                                int ncomp, int64_t nalm, double scale, int bofs) {
-  const int64_t n = nalm * B * ncomp;
-  for (int64_t t = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; t < n; t += int64_t(gridDim.x) * blockDim.x) {
-    double2 s = make_double2(0.0, 0.0);
-    for (int i = 0; i < ntiles; ++i) s = cadd(s, partial[int64_t(i) * n + t]);
-    const int c = int(t % ncomp);
-    const int b = int((t / ncomp) % B);
-    const int64_t idx = t / (int64_t(ncomp) * B);
-    alm[(int64_t(bofs + b) * ncomp + c) * nalm + idx] = cscale(s, scale);
-  }
-}
-
 // ---------------------------------------------------------------- launchers
 // algorithmic Legendre work of one transform: 4 Rh nalm flops per spin-0 map,
 // 16 Rh nalm per spin-s (G, C) pair; bytes: alm in + per-ring phases out
@@ -496,59 +771,94 @@ static double leg_bytes(const Plan& P, int B, int spin) {
   return nf * 16.0 * (double(P.nalm) + double(P.R) * (P.mmax + 1));
 }
 
-int launch_legendre_synth_f64(const Plan& P, const double2* almT, double2* phase, int B, int spin,
-                              cudaStream_t st) {
+int launch_leg_tables_f64(const Plan& P, int spin, double* cd, double* gam, cudaStream_t st) {
+  leg_tables_f64<<<(P.mmax + 64) / 64, 64, 0, st>>>(P.lmax, P.mmax, spin, cd, gam);
+  PS_LAUNCH_CHECK();
+  return PS_OK;
+}
+
+template <int NB, int RPT>
+static void synth0_go(const Plan& P, const double2* alm, double2* phase, int B, cudaStream_t st) {
+  const dim3 grid((P.Rh + SYN_THREADS * RPT - 1) / (SYN_THREADS * RPT), P.mmax + 1, (B + NB - 1) / NB);
+  synth0_f64<NB, RPT><<<grid, SYN_THREADS, 0, st>>>(P.d_rings, P.d_mnorm0, P.d_leg_cd[0], P.d_leg_g[0], alm, phase,
+                                                    P.R, P.Rh, P.lmax, P.mmax, B, P.nalm);
+}
+template <int NB, int RPT>
+static void synthS_go(const Plan& P, const double2* alm, double2* phase, int B, int spin, cudaStream_t st) {
+  const dim3 grid((P.Rh + SYN_THREADS * RPT - 1) / (SYN_THREADS * RPT), P.mmax + 1, (B + NB - 1) / NB);
+  synthS_f64<NB, RPT><<<grid, SYN_THREADS, 0, st>>>(P.d_rings, P.d_seed[spin],
+                                                    reinterpret_cast<const double2*>(P.d_leg_cd[spin]),
+                                                    P.d_leg_g[spin], alm, phase, P.R, P.Rh, P.lmax, P.mmax, B, P.nalm,
+                                                    spin);
+}
+
+// Rings per thread of the synthesis: the rings of a thread share each shared-memory broadcast, fewer keep more
+// warps in flight where a plan has few rings.  Measured, one map, spin 0, one / two / four rings: Nside 1024,
+// lmax 2048 1661 / 1417 / 1353 us, Nside 512, lmax 1000 212 / 187 / 184 us, Nside 256, lmax 767 70 / 71 / 81 us;
+// spin 2 (whose eight sums per ring fill the registers) 4165 / 3880 / 3842 us at Nside 1024.
+int launch_legendre_synth_f64(const Plan& P, const double2* alm, double2* phase, int B, int spin, cudaStream_t st) {
   StatScope sc(PS_K_LEG_SYNTH, leg_flops(P, B, spin), leg_bytes(P, B, spin), st);
-  dim3 grid((P.Rh + SYN_THREADS - 1) / SYN_THREADS, P.mmax + 1, 1);
   const int t = P.tile[0][spin];
+  const bool two = P.Rh > 128;
   if (spin == 0) {
     if (t ? t == 4 : B >= 4) {
-      grid.z = (B + 3) / 4;
-      synth0_f64<4><<<grid, SYN_THREADS, 0, st>>>(P.d_rings, P.d_mnorm0, almT, phase, P.R, P.Rh, P.lmax, P.mmax, B);
+      two ? synth0_go<4, 2>(P, alm, phase, B, st) : synth0_go<4, 1>(P, alm, phase, B, st);
     } else {
-      grid.z = B;
-      synth0_f64<1><<<grid, SYN_THREADS, 0, st>>>(P.d_rings, P.d_mnorm0, almT, phase, P.R, P.Rh, P.lmax, P.mmax, B);
+      if (P.Rh >= 1024) synth0_go<1, 4>(P, alm, phase, B, st);
+      else two ? synth0_go<1, 2>(P, alm, phase, B, st) : synth0_go<1, 1>(P, alm, phase, B, st);
     }
   } else {
     if (!P.d_seed[spin]) return PS_ERR_INVALID;
     if (t ? t == 2 : B >= 2) {
-      grid.z = (B + 1) / 2;
-      synthS_f64<2><<<grid, SYN_THREADS, 0, st>>>(P.d_rings, P.d_seed[spin], almT, phase, P.R, P.Rh, P.lmax,
-                                                  P.mmax, B, spin);
+      two ? synthS_go<2, 2>(P, alm, phase, B, spin, st) : synthS_go<2, 1>(P, alm, phase, B, spin, st);
     } else {
-      grid.z = B;
-      synthS_f64<1><<<grid, SYN_THREADS, 0, st>>>(P.d_rings, P.d_seed[spin], almT, phase, P.R, P.Rh, P.lmax,
-                                                  P.mmax, B, spin);
+      two ? synthS_go<1, 2>(P, alm, phase, B, spin, st) : synthS_go<1, 1>(P, alm, phase, B, spin, st);
     }
   }
   PS_LAUNCH_CHECK();
   return PS_OK;
 }
 
-int adjoint_tiles(const Plan& P) { return (P.Rh + ADJ_THREADS - 1) / ADJ_THREADS; }
+constexpr int ADJ_BATCH = 65535;  // maps per launch (grid limit)
 
-// maps [bofs, bofs + Bc) of a batch of B; partial holds [tile][nalm][Bc][ncomp]
-int launch_legendre_adjoint_f64(const Plan& P, const double2* phase, double2* partial, int B, int bofs, int Bc,
-                                int spin, cudaStream_t st) {
-  StatScope sc(PS_K_LEG_ADJOINT, leg_flops(P, Bc, spin), leg_bytes(P, Bc, spin), st);
-  dim3 grid(adjoint_tiles(P), P.mmax + 1, 1);
-  const int t = P.tile[1][spin];
+template <int RPT, int NW>
+static void adj0_go(const Plan& P, const double2* phase, double2* alm, int B, double scale, cudaStream_t st) {
+  const int warps = std::min(NW, (P.Rh + 32 * RPT - 1) / (32 * RPT));
+  for (int b0 = 0; b0 < B; b0 += ADJ_BATCH)
+    adj0_f64<RPT, NW><<<dim3(1, P.mmax + 1, std::min(ADJ_BATCH, B - b0)), 32 * warps, 0, st>>>(
+        P.d_rings, P.d_mnorm0, P.d_leg_cd[0], P.d_leg_g[0], phase, alm, P.R, P.Rh, P.lmax, P.mmax, B, b0, P.nalm,
+        scale);
+}
+template <int RPT, int NW>
+static void adjS_go(const Plan& P, const double2* phase, double2* alm, int B, int spin, double scale,
+                    cudaStream_t st) {
+  const int warps = std::min(NW, (P.Rh + 32 * RPT - 1) / (32 * RPT));
+  for (int b0 = 0; b0 < B; b0 += ADJ_BATCH)
+    adjS_f64<RPT, NW><<<dim3(1, P.mmax + 1, std::min(ADJ_BATCH, B - b0)), 32 * warps, 0, st>>>(
+        P.d_rings, P.d_seed[spin], reinterpret_cast<const double2*>(P.d_leg_cd[spin]), P.d_leg_g[spin], phase, alm,
+        P.R, P.Rh, P.lmax, P.mmax, B, b0, P.nalm, spin, scale);
+}
+
+// Rings per thread and warps per CTA.  Four rings halve the share of the warp sums and are used wherever a
+// plan has enough rings for one warp of them per scheduler; a CTA of four warps passes several times over l at
+// Rh > 512 but more CTAs share an SM and hide each other's barriers, eight warps keep more of the chip busy when
+// there are few (m, map) pairs.  Measured, four against eight warps of four rings, one map: Nside 1024, lmax 2048
+// 1898 / 1957 us (spin 0), Nside 512, lmax 1000 298 / 259 us; spin 2, <4, 4> against <2, 8>: 5280 / 5720 us,
+// 706 / 759 us and, Nside 256, lmax 767, 259 / 240 us.
+int launch_legendre_adjoint_f64(const Plan& P, const double2* phase, double2* alm, int B, int spin, double scale,
+                                cudaStream_t st) {
+  StatScope sc(PS_K_LEG_ADJOINT, leg_flops(P, B, spin), leg_bytes(P, B, spin), st);
+  if (spin > 0 && !P.d_seed[spin]) return PS_ERR_INVALID;
+  const int64_t ctas = int64_t(P.mmax + 1) * B;
   if (spin == 0) {
-    if (t ? t == 4 : Bc >= 4) {
-      grid.z = (Bc + 3) / 4;
-      adj0_f64<4><<<grid, ADJ_THREADS, 0, st>>>(P.d_rings, P.d_mnorm0, phase, partial, P.R, P.Rh, P.lmax, P.mmax,
-                                                B, bofs, Bc, P.nalm);
-    } else {
-      grid.z = Bc;
-      adj0_f64<1><<<grid, ADJ_THREADS, 0, st>>>(P.d_rings, P.d_mnorm0, phase, partial, P.R, P.Rh, P.lmax, P.mmax,
-                                                B, bofs, Bc, P.nalm);
-    }
+    if (P.Rh > 256) ctas < 1500 ? adj0_go<4, 8>(P, phase, alm, B, scale, st) : adj0_go<4, 4>(P, phase, alm, B, scale, st);
+    else if (P.Rh > 64) adj0_go<2, 4>(P, phase, alm, B, scale, st);
+    else adj0_go<1, 2>(P, phase, alm, B, scale, st);
   } else {
-    if (!P.d_seed[spin]) return PS_ERR_INVALID;
-    // one map per CTA: two maps would exceed the 48 KB of static shared memory
-    grid.z = Bc;
-    adjS_f64<1><<<grid, ADJ_THREADS, 0, st>>>(P.d_rings, P.d_seed[spin], phase, partial, P.R, P.Rh, P.lmax,
-                                              P.mmax, B, bofs, Bc, P.nalm, spin);
+    if (P.Rh > 256 && ctas >= 900) adjS_go<4, 4>(P, phase, alm, B, spin, scale, st);
+    else if (P.Rh > 256) adjS_go<2, 8>(P, phase, alm, B, spin, scale, st);
+    else if (P.Rh > 64) adjS_go<2, 4>(P, phase, alm, B, spin, scale, st);
+    else adjS_go<1, 2>(P, phase, alm, B, spin, scale, st);
   }
   PS_LAUNCH_CHECK();
   return PS_OK;
@@ -560,17 +870,6 @@ int launch_alm_to_T(const double2* alm, double2* almT, int B, int ncomp, int64_t
   if (blocks < 1) blocks = 1;
   StatScope sc(PS_K_LAYOUT, 0.0, 32.0 * n, st);
   alm_to_T<<<blocks, 256, 0, st>>>(alm, almT, B, ncomp, nalm);
-  PS_LAUNCH_CHECK();
-  return PS_OK;
-}
-
-int launch_reduce_partials(const double2* partial, double2* alm, int ntiles, int B, int ncomp, int64_t nalm,
-                           double scale, int bofs, int sms, cudaStream_t st) {
-  const int64_t n = nalm * B * ncomp;
-  int blocks = (int)std::min<int64_t>((n + 255) / 256, int64_t(sms) * 8);
-  if (blocks < 1) blocks = 1;
-  StatScope sc(PS_K_LAYOUT, 0.0, 16.0 * n * (ntiles + 1), st);
-  reduce_partials<<<blocks, 256, 0, st>>>(partial, alm, ntiles, B, ncomp, nalm, scale, bofs);
   PS_LAUNCH_CHECK();
   return PS_OK;
 }

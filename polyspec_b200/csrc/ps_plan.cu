@@ -14,13 +14,11 @@
 #include "ps_common.cuh"
 
 namespace ps {
-int launch_legendre_synth_f64(const Plan& P, const double2* almT, double2* phase, int B, int spin, cudaStream_t st);
-int launch_legendre_adjoint_f64(const Plan& P, const double2* phase, double2* partial, int B, int bofs, int Bc,
-                                int spin, cudaStream_t st);
-int adjoint_tiles(const Plan& P);
+int launch_leg_tables_f64(const Plan& P, int spin, double* cd, double* gam, cudaStream_t st);
+int launch_legendre_synth_f64(const Plan& P, const double2* alm, double2* phase, int B, int spin, cudaStream_t st);
+int launch_legendre_adjoint_f64(const Plan& P, const double2* phase, double2* alm, int B, int spin, double scale,
+                                cudaStream_t st);
 int launch_alm_to_T(const double2* alm, double2* almT, int B, int ncomp, int64_t nalm, int sms, cudaStream_t st);
-int launch_reduce_partials(const double2* partial, double2* alm, int ntiles, int B, int ncomp, int64_t nalm,
-                           double scale, int bofs, int sms, cudaStream_t st);
 int launch_ring_synth_f64(const Plan& P, const int* d_list, int nrings, int work_len, const double2* phase,
                           double* map, int nf, int pack, cudaStream_t st);
 int launch_ring_adjoint_f64(const Plan& P, const int* d_list, int nrings, int work_len, const double* map,
@@ -98,6 +96,14 @@ int host_bitrev(int i, int logn) {
   int r = 0;
   for (int b = 0; b < logn; ++b) { r = (r << 1) | (i & 1); i >>= 1; }
   return r;
+}
+
+template <class T>
+T* dev_alloc(ps_plan* pl, size_t n, int& err) {
+  void* d = nullptr;
+  if (cudaMalloc(&d, n * sizeof(T)) != cudaSuccess) { cudaGetLastError(); err = PS_ERR_NOMEM; return nullptr; }
+  pl->owned.push_back(d);
+  return static_cast<T*>(d);
 }
 
 template <class T>
@@ -182,6 +188,7 @@ int ps_plan_create(int nside, int lmax, int mmax, int spin_mask, int prec, ps_pl
   P.R = 4 * nside - 1; P.Rh = 2 * nside;
   P.npix = 12 * int64_t(nside) * nside;
   P.nalm = int64_t(lmax + 1) * (lmax + 2) / 2;
+  for (int s = 0; s < 4; ++s) P.d_leg_cd[s] = P.d_leg_g[s] = nullptr;
   for (int s = 0; s < 4; ++s) { P.d_seed[s] = nullptr; P.d_tab[s] = nullptr; P.tab_fmt[s] = PS_TAB_TF32X3; }
   P.tab_fmt_build = PS_TAB_TF32X3;
   P.d_tab_off = nullptr;
@@ -370,6 +377,16 @@ int ps_plan_create(int nside, int lmax, int mmax, int spin_mask, int prec, ps_pl
     P.d_chirp_off = dev_upload(pl, chirp_off, err);
   }
   pl->d_ring_lists = dev_upload(pl, lists, err);
+  if (prec == PS_PREC_FP64) {
+    for (int s = 0; s < 4 && err == PS_OK; ++s) {
+      if (s > 0 && !P.d_seed[s]) continue;
+      P.d_leg_cd[s] = dev_alloc<double>(pl, size_t(P.nalm) * (s == 0 ? 1 : 2), err);
+      P.d_leg_g[s] = dev_alloc<double>(pl, size_t(P.nalm), err);
+      if (err == PS_OK) err = ps::launch_leg_tables_f64(P, s, P.d_leg_cd[s], P.d_leg_g[s], nullptr);
+    }
+    // the tables are read on the callers' streams
+    if (err == PS_OK && cudaStreamSynchronize(nullptr) != cudaSuccess) err = PS_ERR_CUDA;
+  }
   if (err != PS_OK) { ps_plan_destroy(pl); return err; }
   *out = pl;
   return PS_OK;
@@ -526,14 +543,12 @@ int ps_plan_info(const ps_plan* plan, int* nside, int* lmax, int64_t* npix, int6
   return PS_OK;
 }
 
-// maps per Legendre-adjoint pass: the per-ring-tile partial sums of one pass
-// bound the adjoint's workspace independently of the batch size (at most about
+// maps per pass of the mixed Legendre adjoint without a table: the per-ring-tile partial
+// sums of one pass bound its workspace independently of the batch size (at most about
 // 4 GiB of partials per pass, at least one map)
 static int adjoint_chunk(const ps::Plan& P, int batch, int spin) {
-  int c = (P.prec == PS_PREC_MIXED) ? (spin == 0 ? 16 : 8) : (spin == 0 ? 8 : 4);
-  const int tiles = (P.prec == PS_PREC_MIXED) ? ps::mx_adjoint_tiles(P) : ps::adjoint_tiles(P);
-  const double per_map = double(tiles) * double(P.nalm) * (spin == 0 ? 1 : 2) *
-                         (P.prec == PS_PREC_MIXED ? sizeof(float2) : sizeof(double2));
+  int c = spin == 0 ? 16 : 8;
+  const double per_map = double(ps::mx_adjoint_tiles(P)) * double(P.nalm) * (spin == 0 ? 1 : 2) * sizeof(float2);
   const int cap = int(4294967296.0 / per_map);
   if (c > cap) c = cap < 1 ? 1 : cap;
   return batch < c ? batch : c;
@@ -546,19 +561,15 @@ static size_t sht_ws_bytes(const ps_plan* plan, int batch, int spin, int adjoint
   const size_t phase = align256(size_t(P.R) * (P.mmax + 1) * nf * sizeof(double2));
   if (!adjoint) return align256(size_t(P.nalm) * nf * sizeof(double2)) + phase;
   TabRef tr;
-  if (table_for(plan, spin, tr)) return phase;  // the table adjoint writes alm directly
+  // the FP64 and the table adjoint write alm directly
+  if (P.prec == PS_PREC_FP64 || table_for(plan, spin, tr)) return phase;
   const size_t nfc = size_t(adjoint_chunk(P, batch, spin)) * ncomp;
-  return phase + align256(size_t(ps::adjoint_tiles(P)) * P.nalm * nfc * sizeof(double2));
+  return phase + align256(size_t(ps::mx_adjoint_tiles(P)) * P.nalm * nfc * sizeof(double2));
 }
 
 // Legendre stages alone (phase in and out in the caller's memory, complex128).
 // A mixed-precision plan runs its tensor-core synthesis / FP32 adjoint kernels
 // with the phases converted to complex64 in the workspace.
-static int fp64_adjoint_chunk(int batch, int spin) {
-  const int c = spin == 0 ? 8 : 4;
-  return batch < c ? batch : c;
-}
-
 namespace {
 __global__ void phase_f32_to_f64(const float2* __restrict__ in, double2* __restrict__ out, int64_t n) {
   for (int64_t i = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; i < n; i += int64_t(gridDim.x) * blockDim.x) {
@@ -584,15 +595,12 @@ static size_t leg_ws_bytes(const ps_plan* plan, int batch, int spin, int adjoint
   const size_t nf = size_t(batch) * ncomp;
   const bool mixed = P.prec == PS_PREC_MIXED;
   const size_t phase32 = mixed ? align256(size_t(P.R) * (P.mmax + 1) * nf * sizeof(float2)) : 0;
+  if (!mixed) return 256;  // the FP64 stages work between the caller's arrays
   if (!adjoint) return align256(size_t(P.nalm) * nf * sizeof(double2)) + phase32;
   TabRef tr;
   if (table_for(plan, spin, tr)) return phase32;
-  if (mixed) {
-    const size_t nfc = size_t(adjoint_chunk(P, batch, spin)) * ncomp;
-    return phase32 + align256(size_t(ps::mx_adjoint_tiles(P)) * P.nalm * nfc * sizeof(float2));
-  }
-  const size_t nfc = size_t(fp64_adjoint_chunk(batch, spin)) * ncomp;
-  return align256(size_t(ps::adjoint_tiles(P)) * P.nalm * nfc * sizeof(double2));
+  const size_t nfc = size_t(adjoint_chunk(P, batch, spin)) * ncomp;
+  return phase32 + align256(size_t(ps::mx_adjoint_tiles(P)) * P.nalm * nfc * sizeof(float2));
 }
 
 int ps_legendre_synthesis(const ps_plan* plan, const double* alm, double* phase, int batch, int spin,
@@ -604,10 +612,10 @@ int ps_legendre_synthesis(const ps_plan* plan, const double* alm, double* phase,
   if (spin > 0 && !P.d_seed[spin]) return PS_ERR_INVALID;
   if (workspace_bytes < leg_ws_bytes(plan, batch, spin, 0)) return PS_ERR_WORKSPACE;
   const int ncomp = spin == 0 ? 1 : 2;
-  double2* almT = static_cast<double2*>(workspace);
-  int rc = ps::launch_alm_to_T(reinterpret_cast<const double2*>(alm), almT, batch, ncomp, P.nalm, P.num_sms, stream);
-  if (rc) return rc;
   if (P.prec == PS_PREC_MIXED) {
+    double2* almT = static_cast<double2*>(workspace);
+    int rc = ps::launch_alm_to_T(reinterpret_cast<const double2*>(alm), almT, batch, ncomp, P.nalm, P.num_sms, stream);
+    if (rc) return rc;
     float2* ph32 = reinterpret_cast<float2*>(static_cast<char*>(workspace) +
                                              align256(size_t(P.nalm) * batch * ncomp * sizeof(double2)));
     TabRef tr;
@@ -622,7 +630,8 @@ int ps_legendre_synthesis(const ps_plan* plan, const double* alm, double* phase,
     PS_LAUNCH_CHECK();
     return PS_OK;
   }
-  return ps::launch_legendre_synth_f64(P, almT, reinterpret_cast<double2*>(phase), batch, spin, stream);
+  return ps::launch_legendre_synth_f64(P, reinterpret_cast<const double2*>(alm), reinterpret_cast<double2*>(phase),
+                                       batch, spin, stream);
 }
 
 int ps_legendre_adjoint(const ps_plan* plan, const double* phase, double* alm, int batch, int spin, double scale,
@@ -656,18 +665,8 @@ int ps_legendre_adjoint(const ps_plan* plan, const double* phase, double* alm, i
     }
     return PS_OK;
   }
-  double2* partial = static_cast<double2*>(workspace);
-  const int ch = fp64_adjoint_chunk(batch, spin);
-  for (int b0 = 0; b0 < batch; b0 += ch) {
-    const int bc = std::min(ch, batch - b0);
-    int rc = ps::launch_legendre_adjoint_f64(P, reinterpret_cast<const double2*>(phase), partial, batch, b0, bc,
-                                             spin, stream);
-    if (rc) return rc;
-    rc = ps::launch_reduce_partials(partial, reinterpret_cast<double2*>(alm), ps::adjoint_tiles(P), bc, ncomp,
-                                    P.nalm, scale, b0, P.num_sms, stream);
-    if (rc) return rc;
-  }
-  return PS_OK;
+  return ps::launch_legendre_adjoint_f64(P, reinterpret_cast<const double2*>(phase), reinterpret_cast<double2*>(alm),
+                                         batch, spin, scale, stream);
 }
 
 int ps_sht_workspace_bytes(const ps_plan* plan, int batch, int spin, int adjoint, size_t* bytes) {
@@ -691,13 +690,13 @@ int ps_synthesis(const ps_plan* plan, const double* alm, double* map, int batch,
   double2* almT = reinterpret_cast<double2*>(ws);
   char* phase_ptr = ws + align256(size_t(P.nalm) * nf * sizeof(double2));
   int rc;
-  if (nf == 1) {
-    almT = reinterpret_cast<double2*>(const_cast<double*>(alm));
-  } else {
-    rc = ps::launch_alm_to_T(reinterpret_cast<const double2*>(alm), almT, batch, ncomp, P.nalm, P.num_sms, stream);
-    if (rc) return rc;
-  }
   if (P.prec == PS_PREC_MIXED) {
+    if (nf == 1) {
+      almT = reinterpret_cast<double2*>(const_cast<double*>(alm));
+    } else {
+      rc = ps::launch_alm_to_T(reinterpret_cast<const double2*>(alm), almT, batch, ncomp, P.nalm, P.num_sms, stream);
+      if (rc) return rc;
+    }
     // tensor-core Legendre stage (TF32 x3, FP32 accumulation) and FP32 ring transforms
     float2* phase = reinterpret_cast<float2*>(phase_ptr);
     TabRef tr;
@@ -716,7 +715,7 @@ int ps_synthesis(const ps_plan* plan, const double* alm, double* map, int batch,
     return PS_OK;
   }
   double2* phase = reinterpret_cast<double2*>(phase_ptr);
-  rc = ps::launch_legendre_synth_f64(P, almT, phase, batch, spin, stream);
+  rc = ps::launch_legendre_synth_f64(P, reinterpret_cast<const double2*>(alm), phase, batch, spin, stream);
   if (rc) return rc;
   for (size_t c = 0; c < plan->cls_len.size(); ++c) {
     rc = ps::launch_ring_synth_f64(P, plan->d_ring_lists + (spin ? plan->cls_off[c] : plan->cls_off_n[c]),
@@ -768,23 +767,13 @@ int ps_adjoint(const ps_plan* plan, const double* map, double* alm, int batch, i
     return PS_OK;
   }
   double2* phase = reinterpret_cast<double2*>(ws);
-  double2* partial = reinterpret_cast<double2*>(ws + phase_bytes);
   for (size_t c = 0; c < plan->cls_len.size(); ++c) {
     rc = ps::launch_ring_adjoint_f64(P, plan->d_ring_lists + (spin ? plan->cls_off[c] : plan->cls_off_n[c]),
                                      spin ? plan->cls_cnt[c] : plan->cls_cnt_n[c], plan->cls_len[c], map, phase, nf,
                                      spin > 0, stream);
     if (rc) return rc;
   }
-  const int ch = adjoint_chunk(P, batch, spin);
-  for (int b0 = 0; b0 < batch; b0 += ch) {
-    const int bc = std::min(ch, batch - b0);
-    rc = ps::launch_legendre_adjoint_f64(P, phase, partial, batch, b0, bc, spin, stream);
-    if (rc) return rc;
-    rc = ps::launch_reduce_partials(partial, reinterpret_cast<double2*>(alm), ps::adjoint_tiles(P), bc, ncomp,
-                                    P.nalm, scale, b0, P.num_sms, stream);
-    if (rc) return rc;
-  }
-  return PS_OK;
+  return ps::launch_legendre_adjoint_f64(P, phase, reinterpret_cast<double2*>(alm), batch, spin, scale, stream);
 }
 
 }  // extern "C"
