@@ -51,20 +51,25 @@ __global__ void lm_matvec3_kernel(const double* __restrict__ S, const double* __
 
 constexpr int DOT_THREADS = 256;
 
-// partial[n][c]: CTA c's share of batch member n
+// partial[n][c]: CTA c's share of batch member n, the (l, m) of a contiguous range with their three fields: one
+// read of the weight per (l, m) and no remainder by nalm.  Chunks and order of the sums are those of the dot
+// products inside ps_cg_solve, so that both solvers take the same steps to the last bit.
 __global__ void lm_dot_stage1(const double2* __restrict__ x, const double2* __restrict__ y,
                               const double* __restrict__ w, int64_t nalm, int nchunks, double* __restrict__ partial) {
   const int n = blockIdx.y, c = blockIdx.x;
-  const int64_t len = 3 * nalm;
-  const int64_t per = (len + nchunks - 1) / nchunks;
-  const int64_t lo = int64_t(c) * per, hi = min(len, lo + per);
-  const double2* xn = x + int64_t(n) * len;
-  const double2* yn = y + int64_t(n) * len;
+  const int64_t per = (nalm + nchunks - 1) / nchunks;
+  const int64_t lo = int64_t(c) * per, hi = min(nalm, lo + per);
+  const double2* xn = x + int64_t(n) * 3 * nalm;
+  const double2* yn = y + int64_t(n) * 3 * nalm;
   double acc = 0.0;
-  for (int64_t k = lo + threadIdx.x; k < hi; k += DOT_THREADS) {
-    const int64_t i = k % nalm;
-    const double2 a = xn[k], b = yn[k];
-    acc += __ldg(w + i) * (a.x * b.x + a.y * b.y);
+  for (int64_t i = lo + threadIdx.x; i < hi; i += DOT_THREADS) {
+    double dot = 0.0;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      const double2 p = xn[int64_t(a) * nalm + i], q = yn[int64_t(a) * nalm + i];
+      dot += p.x * q.x + p.y * q.y;
+    }
+    acc = fma(__ldg(w + i), dot, acc);
   }
 #pragma unroll
   for (int off = 16; off > 0; off >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, off);
@@ -161,12 +166,12 @@ __global__ void cg_dir_kernel(double2* __restrict__ p, const double2* __restrict
     p[t] = cfma(beta[t / per], p[t], z[t]);
 }
 
+// about 4 CTAs per SM over the batch, at least 2048 (l, m) each (as ps_cg_solve)
 int dot_chunks(int B, int64_t nalm, int sms) {
-  int c = (sms * 4 + B - 1) / B;
-  const int64_t maxc = (3 * nalm + 8191) / 8192;
-  if (c > maxc) c = int(maxc);
-  if (c > 512) c = 512;
-  return c < 1 ? 1 : c;
+  int64_t c = (int64_t(sms) * 4 + B - 1) / B;
+  c = c < (nalm + 2047) / 2048 ? c : (nalm + 2047) / 2048;
+  c = c < 1024 ? c : 1024;
+  return c < 1 ? 1 : int(c);
 }
 
 int n_sms() {
