@@ -46,9 +46,13 @@ struct Plan {
   // c [nalm] (spin 0) or (c, d) [nalm][2], and gam [nalm]
   double* d_leg_cd[4];
   double* d_leg_g[4];
-  double2* d_twiddle;       // [max_fft/2] e^{-2 pi i k / max_fft}
-  double2* d_bs_spec;       // Bluestein spectra (FP64)
-  float2* d_twiddle_f;      // FP32 copies for the mixed-precision ring transforms
+  // FP64 plans: [max_fft/2] e^{-2 pi i k / max_fft}; Bluestein spectra; e^{i pi k / N}, k < N, of every ring
+  // length N = 4 i, i = 1 .. nside (at 2 i (i - 1)); the Bluestein chirps e^{-i pi j^2 / N}, j < N, of every slot
+  double2* d_twiddle;
+  double2* d_bs_spec;
+  double2* d_root;
+  double2* d_chirp;
+  float2* d_twiddle_f;      // mixed plans: the same in FP32
   float2* d_bs_spec_f;
   // mixed plans: e^{i m phi0} of every north ring (the mirror ring has the same phi0),
   // [Rh][mmax+1], and the Bluestein chirps e^{-i pi j^2 / N}, j < N, of every slot
@@ -73,6 +77,13 @@ struct Plan {
   // format of each built table (PS_TAB_TF32X3 or PS_TAB_BF16X3) and of the tables built next
   int tab_fmt[4];
   int tab_fmt_build;
+};
+
+// Rings of one FFT work length 2^logM, Bluestein rings (blue) and power-of-two rings apart, for the FP64 ring
+// transforms: all rings (spin s), or the north rings and the equator (spin 0, packed with their mirrors).
+struct RingClassList {
+  int logM, blue, count, count_n;
+  const int *rings, *rings_n;  // device
 };
 
 // ---------------------------------------------------------------------------

@@ -30,8 +30,9 @@
 // kept several to a thread so that one broadcast of c and the alm from shared
 // memory serves them all.
 //
-// Layouts: alm [B][ncomp][nalm] (m-major), phase [R][mmax+1][B][ncomp] (ring-major,
-// order m, then maps and Q/U).
+// Layouts: alm [B][ncomp][nalm] (m-major); phases ring-major, the value of order m and map b of a ring at
+// m ms + b bs (+ 1 for U): [R][B][mmax+1][ncomp] towards the ring transforms, [R][mmax+1][B][ncomp] in the calls of
+// the Legendre stage alone.
 #include <algorithm>
 #include <type_traits>
 
@@ -205,8 +206,8 @@ __global__ void __launch_bounds__(SYN_THREADS) synth0_f64(const RingInfo* __rest
                                                            const double* __restrict__ lc,
                                                            const double* __restrict__ lg,
                                                            const double2* __restrict__ alm,
-                                                           double2* __restrict__ phase, int R, int Rh, int lmax,
-                                                           int mmax, int B, int64_t nalm) {
+                                                           double2* __restrict__ phase, int64_t ms, int64_t bs,
+                                                           int R, int Rh, int lmax, int mmax, int B, int64_t nalm) {
   const int m = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, b0 = blockIdx.z * NB;
   const int wbase = (blockIdx.x * SYN_THREADS + (tid & ~31)) * RPT, r0 = wbase + lane;
   if (wbase >= Rh) return;
@@ -318,8 +319,9 @@ __global__ void __launch_bounds__(SYN_THREADS) synth0_f64(const RingInfo* __rest
 #pragma unroll
     for (int b = 0; b < NB; ++b) {
       if (b0 + b >= B) break;
-      phase[(int64_t(rp) * (mmax + 1) + m) * B + b0 + b] = cadd(ae[i][b], ao[i][b]);
-      if (rs != rp) phase[(int64_t(rs) * (mmax + 1) + m) * B + b0 + b] = csub(ae[i][b], ao[i][b]);
+      const int64_t o = m * ms + (b0 + b) * bs, ring = int64_t(mmax + 1) * B;
+      phase[rp * ring + o] = cadd(ae[i][b], ao[i][b]);
+      if (rs != rp) phase[rs * ring + o] = csub(ae[i][b], ao[i][b]);
     }
   }
 }
@@ -332,8 +334,9 @@ __global__ void __launch_bounds__(SYN_THREADS) synthS_f64(const RingInfo* __rest
                                                            const double2* __restrict__ lcd,
                                                            const double* __restrict__ lg,
                                                            const double2* __restrict__ alm,
-                                                           double2* __restrict__ phase, int R, int Rh, int lmax,
-                                                           int mmax, int B, int64_t nalm, int spin) {
+                                                           double2* __restrict__ phase, int64_t ms, int64_t bs,
+                                                           int R, int Rh, int lmax, int mmax, int B, int64_t nalm,
+                                                           int spin) {
   const int m = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, b0 = blockIdx.z * NB;
   const int wbase = (blockIdx.x * SYN_THREADS + (tid & ~31)) * RPT, r0 = wbase + lane;
   if (wbase >= Rh) return;
@@ -470,7 +473,7 @@ __global__ void __launch_bounds__(SYN_THREADS) synthS_f64(const RingInfo* __rest
         const double2 sp = cscale(side == 0 ? PN[i][b] : PS[i][b], h), sm = cscale(side == 0 ? MN[i][b] : MS[i][b], h);
         const double2 sum = cadd(sp, sm), dif = csub(sp, sm);
         const double2 q = odd ? dif : sum, u = odd ? sum : dif;
-        const int64_t o = ((int64_t(side == 0 ? rp : rs) * (mmax + 1) + m) * B + b0 + b) * 2;
+        const int64_t o = (side == 0 ? rp : rs) * (int64_t(mmax + 1) * B * 2) + m * ms + (b0 + b) * bs;
         phase[o] = make_double2(-q.x, -q.y);
         phase[o + 1] = make_double2(-u.y, u.x);
       }
@@ -502,8 +505,9 @@ template <int RPT, int NW>
 __global__ void __launch_bounds__(32 * NW) adj0_f64(const RingInfo* __restrict__ rings,
                                                     const double* __restrict__ mnorm, const double* __restrict__ lc,
                                                     const double* __restrict__ lg, const double2* __restrict__ phase,
-                                                    double2* __restrict__ alm, int R, int Rh, int lmax, int mmax,
-                                                    int B, int bofs, int64_t nalm, double scale) {
+                                                    int64_t ms, int64_t bs, double2* __restrict__ alm, int R, int Rh,
+                                                    int lmax, int mmax, int B, int bofs, int64_t nalm,
+                                                    double scale) {
   const int m = blockIdx.y, b = bofs + blockIdx.z, tid = threadIdx.x, nt = blockDim.x;
   const int warp = tid >> 5, lane = tid & 31, nw = nt >> 5;
   __shared__ double2 s_red[2][NW][ADJ_LCH];
@@ -525,8 +529,9 @@ __global__ void __launch_bounds__(32 * NW) adj0_f64(const RingInfo* __restrict__
       const RingInfo& g = rings[rp < Rh ? rp : 0];
       double2 pn = make_double2(0.0, 0.0), ps = pn;
       if (rp < Rh) {
-        pn = phase[(int64_t(rp) * (mmax + 1) + m) * B + b];
-        if (rs != rp) ps = phase[(int64_t(rs) * (mmax + 1) + m) * B + b];
+        const int64_t o = m * ms + b * bs, ring = int64_t(mmax + 1) * B;
+        pn = phase[rp * ring + o];
+        if (rs != rp) ps = phase[rs * ring + o];
       }
       E[i] = cadd(pn, ps);
       O[i] = csub(pn, ps);
@@ -607,9 +612,9 @@ template <int RPT, int NW>
 __global__ void __launch_bounds__(32 * NW) adjS_f64(const RingInfo* __restrict__ rings,
                                                     const SeedNorm* __restrict__ seednorm,
                                                     const double2* __restrict__ lcd, const double* __restrict__ lg,
-                                                    const double2* __restrict__ phase, double2* __restrict__ alm,
-                                                    int R, int Rh, int lmax, int mmax, int B, int bofs, int64_t nalm,
-                                                    int spin, double scale) {
+                                                    const double2* __restrict__ phase, int64_t ms, int64_t bs,
+                                                    double2* __restrict__ alm, int R, int Rh, int lmax, int mmax,
+                                                    int B, int bofs, int64_t nalm, int spin, double scale) {
   const int m = blockIdx.y, b = bofs + blockIdx.z, tid = threadIdx.x, nt = blockDim.x;
   const int warp = tid >> 5, lane = tid & 31, nw = nt >> 5;
   __shared__ double s_red[2][NW][4 * ADJ_LCH];
@@ -635,11 +640,11 @@ __global__ void __launch_bounds__(32 * NW) adjS_f64(const RingInfo* __restrict__
       const RingInfo& gi = rings[rp < Rh ? rp : 0];
       double2 qn = make_double2(0.0, 0.0), un = qn, qs = qn, us = qn;
       if (rp < Rh) {
-        const int64_t o = ((int64_t(rp) * (mmax + 1) + m) * B + b) * 2;
+        const int64_t ring = int64_t(mmax + 1) * B * 2, o = rp * ring + m * ms + b * bs;
         qn = phase[o];
         un = phase[o + 1];
         if (rs != rp) {
-          const int64_t o2 = ((int64_t(rs) * (mmax + 1) + m) * B + b) * 2;
+          const int64_t o2 = rs * ring + m * ms + b * bs;
           qs = cscale(phase[o2], sgn0);
           us = cscale(phase[o2 + 1], sgn0);
         }
@@ -778,41 +783,43 @@ int launch_leg_tables_f64(const Plan& P, int spin, double* cd, double* gam, cuda
 }
 
 template <int NB, int RPT>
-static void synth0_go(const Plan& P, const double2* alm, double2* phase, int B, cudaStream_t st) {
+static void synth0_go(const Plan& P, const double2* alm, double2* phase, int64_t ms, int64_t bs, int B, cudaStream_t st) {
   const dim3 grid((P.Rh + SYN_THREADS * RPT - 1) / (SYN_THREADS * RPT), P.mmax + 1, (B + NB - 1) / NB);
   synth0_f64<NB, RPT><<<grid, SYN_THREADS, 0, st>>>(P.d_rings, P.d_mnorm0, P.d_leg_cd[0], P.d_leg_g[0], alm, phase,
-                                                    P.R, P.Rh, P.lmax, P.mmax, B, P.nalm);
+                                                    ms, bs, P.R, P.Rh, P.lmax, P.mmax, B, P.nalm);
 }
 template <int NB, int RPT>
-static void synthS_go(const Plan& P, const double2* alm, double2* phase, int B, int spin, cudaStream_t st) {
+static void synthS_go(const Plan& P, const double2* alm, double2* phase, int64_t ms, int64_t bs, int B, int spin,
+                      cudaStream_t st) {
   const dim3 grid((P.Rh + SYN_THREADS * RPT - 1) / (SYN_THREADS * RPT), P.mmax + 1, (B + NB - 1) / NB);
   synthS_f64<NB, RPT><<<grid, SYN_THREADS, 0, st>>>(P.d_rings, P.d_seed[spin],
                                                     reinterpret_cast<const double2*>(P.d_leg_cd[spin]),
-                                                    P.d_leg_g[spin], alm, phase, P.R, P.Rh, P.lmax, P.mmax, B, P.nalm,
-                                                    spin);
+                                                    P.d_leg_g[spin], alm, phase, ms, bs, P.R, P.Rh, P.lmax, P.mmax, B,
+                                                    P.nalm, spin);
 }
 
 // Rings per thread of the synthesis: the rings of a thread share each shared-memory broadcast, fewer keep more
 // warps in flight where a plan has few rings.  Measured, one map, spin 0, one / two / four rings: Nside 1024,
 // lmax 2048 1661 / 1417 / 1353 us, Nside 512, lmax 1000 212 / 187 / 184 us, Nside 256, lmax 767 70 / 71 / 81 us;
 // spin 2 (whose eight sums per ring fill the registers) 4165 / 3880 / 3842 us at Nside 1024.
-int launch_legendre_synth_f64(const Plan& P, const double2* alm, double2* phase, int B, int spin, cudaStream_t st) {
+int launch_legendre_synth_f64(const Plan& P, const double2* alm, double2* phase, int64_t ms, int64_t bs, int B,
+                              int spin, cudaStream_t st) {
   StatScope sc(PS_K_LEG_SYNTH, leg_flops(P, B, spin), leg_bytes(P, B, spin), st);
   const int t = P.tile[0][spin];
   const bool two = P.Rh > 128;
   if (spin == 0) {
     if (t ? t == 4 : B >= 4) {
-      two ? synth0_go<4, 2>(P, alm, phase, B, st) : synth0_go<4, 1>(P, alm, phase, B, st);
+      two ? synth0_go<4, 2>(P, alm, phase, ms, bs, B, st) : synth0_go<4, 1>(P, alm, phase, ms, bs, B, st);
     } else {
-      if (P.Rh >= 1024) synth0_go<1, 4>(P, alm, phase, B, st);
-      else two ? synth0_go<1, 2>(P, alm, phase, B, st) : synth0_go<1, 1>(P, alm, phase, B, st);
+      if (P.Rh >= 1024) synth0_go<1, 4>(P, alm, phase, ms, bs, B, st);
+      else two ? synth0_go<1, 2>(P, alm, phase, ms, bs, B, st) : synth0_go<1, 1>(P, alm, phase, ms, bs, B, st);
     }
   } else {
     if (!P.d_seed[spin]) return PS_ERR_INVALID;
     if (t ? t == 2 : B >= 2) {
-      two ? synthS_go<2, 2>(P, alm, phase, B, spin, st) : synthS_go<2, 1>(P, alm, phase, B, spin, st);
+      two ? synthS_go<2, 2>(P, alm, phase, ms, bs, B, spin, st) : synthS_go<2, 1>(P, alm, phase, ms, bs, B, spin, st);
     } else {
-      two ? synthS_go<1, 2>(P, alm, phase, B, spin, st) : synthS_go<1, 1>(P, alm, phase, B, spin, st);
+      two ? synthS_go<1, 2>(P, alm, phase, ms, bs, B, spin, st) : synthS_go<1, 1>(P, alm, phase, ms, bs, B, spin, st);
     }
   }
   PS_LAUNCH_CHECK();
@@ -822,21 +829,22 @@ int launch_legendre_synth_f64(const Plan& P, const double2* alm, double2* phase,
 constexpr int ADJ_BATCH = 65535;  // maps per launch (grid limit)
 
 template <int RPT, int NW>
-static void adj0_go(const Plan& P, const double2* phase, double2* alm, int B, double scale, cudaStream_t st) {
-  const int warps = std::min(NW, (P.Rh + 32 * RPT - 1) / (32 * RPT));
-  for (int b0 = 0; b0 < B; b0 += ADJ_BATCH)
-    adj0_f64<RPT, NW><<<dim3(1, P.mmax + 1, std::min(ADJ_BATCH, B - b0)), 32 * warps, 0, st>>>(
-        P.d_rings, P.d_mnorm0, P.d_leg_cd[0], P.d_leg_g[0], phase, alm, P.R, P.Rh, P.lmax, P.mmax, B, b0, P.nalm,
-        scale);
-}
-template <int RPT, int NW>
-static void adjS_go(const Plan& P, const double2* phase, double2* alm, int B, int spin, double scale,
+static void adj0_go(const Plan& P, const double2* phase, int64_t ms, int64_t bs, double2* alm, int B, double scale,
                     cudaStream_t st) {
   const int warps = std::min(NW, (P.Rh + 32 * RPT - 1) / (32 * RPT));
   for (int b0 = 0; b0 < B; b0 += ADJ_BATCH)
+    adj0_f64<RPT, NW><<<dim3(1, P.mmax + 1, std::min(ADJ_BATCH, B - b0)), 32 * warps, 0, st>>>(
+        P.d_rings, P.d_mnorm0, P.d_leg_cd[0], P.d_leg_g[0], phase, ms, bs, alm, P.R, P.Rh, P.lmax, P.mmax, B, b0,
+        P.nalm, scale);
+}
+template <int RPT, int NW>
+static void adjS_go(const Plan& P, const double2* phase, int64_t ms, int64_t bs, double2* alm, int B, int spin,
+                    double scale, cudaStream_t st) {
+  const int warps = std::min(NW, (P.Rh + 32 * RPT - 1) / (32 * RPT));
+  for (int b0 = 0; b0 < B; b0 += ADJ_BATCH)
     adjS_f64<RPT, NW><<<dim3(1, P.mmax + 1, std::min(ADJ_BATCH, B - b0)), 32 * warps, 0, st>>>(
-        P.d_rings, P.d_seed[spin], reinterpret_cast<const double2*>(P.d_leg_cd[spin]), P.d_leg_g[spin], phase, alm,
-        P.R, P.Rh, P.lmax, P.mmax, B, b0, P.nalm, spin, scale);
+        P.d_rings, P.d_seed[spin], reinterpret_cast<const double2*>(P.d_leg_cd[spin]), P.d_leg_g[spin], phase, ms, bs,
+        alm, P.R, P.Rh, P.lmax, P.mmax, B, b0, P.nalm, spin, scale);
 }
 
 // Rings per thread and warps per CTA.  Four rings halve the share of the warp sums and are used wherever a
@@ -845,20 +853,20 @@ static void adjS_go(const Plan& P, const double2* phase, double2* alm, int B, in
 // there are few (m, map) pairs.  Measured, four against eight warps of four rings, one map: Nside 1024, lmax 2048
 // 1898 / 1957 us (spin 0), Nside 512, lmax 1000 298 / 259 us; spin 2, <4, 4> against <2, 8>: 5280 / 5720 us,
 // 706 / 759 us and, Nside 256, lmax 767, 259 / 240 us.
-int launch_legendre_adjoint_f64(const Plan& P, const double2* phase, double2* alm, int B, int spin, double scale,
-                                cudaStream_t st) {
+int launch_legendre_adjoint_f64(const Plan& P, const double2* phase, int64_t ms, int64_t bs, double2* alm, int B,
+                                int spin, double scale, cudaStream_t st) {
   StatScope sc(PS_K_LEG_ADJOINT, leg_flops(P, B, spin), leg_bytes(P, B, spin), st);
   if (spin > 0 && !P.d_seed[spin]) return PS_ERR_INVALID;
   const int64_t ctas = int64_t(P.mmax + 1) * B;
   if (spin == 0) {
-    if (P.Rh > 256) ctas < 1500 ? adj0_go<4, 8>(P, phase, alm, B, scale, st) : adj0_go<4, 4>(P, phase, alm, B, scale, st);
-    else if (P.Rh > 64) adj0_go<2, 4>(P, phase, alm, B, scale, st);
-    else adj0_go<1, 2>(P, phase, alm, B, scale, st);
+    if (P.Rh > 256) ctas < 1500 ? adj0_go<4, 8>(P, phase, ms, bs, alm, B, scale, st) : adj0_go<4, 4>(P, phase, ms, bs, alm, B, scale, st);
+    else if (P.Rh > 64) adj0_go<2, 4>(P, phase, ms, bs, alm, B, scale, st);
+    else adj0_go<1, 2>(P, phase, ms, bs, alm, B, scale, st);
   } else {
-    if (P.Rh > 256 && ctas >= 900) adjS_go<4, 4>(P, phase, alm, B, spin, scale, st);
-    else if (P.Rh > 256) adjS_go<2, 8>(P, phase, alm, B, spin, scale, st);
-    else if (P.Rh > 64) adjS_go<2, 4>(P, phase, alm, B, spin, scale, st);
-    else adjS_go<1, 2>(P, phase, alm, B, spin, scale, st);
+    if (P.Rh > 256 && ctas >= 900) adjS_go<4, 4>(P, phase, ms, bs, alm, B, spin, scale, st);
+    else if (P.Rh > 256) adjS_go<2, 8>(P, phase, ms, bs, alm, B, spin, scale, st);
+    else if (P.Rh > 64) adjS_go<2, 4>(P, phase, ms, bs, alm, B, spin, scale, st);
+    else adjS_go<1, 2>(P, phase, ms, bs, alm, B, spin, scale, st);
   }
   PS_LAUNCH_CHECK();
   return PS_OK;

@@ -15,14 +15,15 @@
 
 namespace ps {
 int launch_leg_tables_f64(const Plan& P, int spin, double* cd, double* gam, cudaStream_t st);
-int launch_legendre_synth_f64(const Plan& P, const double2* alm, double2* phase, int B, int spin, cudaStream_t st);
-int launch_legendre_adjoint_f64(const Plan& P, const double2* phase, double2* alm, int B, int spin, double scale,
-                                cudaStream_t st);
+int launch_legendre_synth_f64(const Plan& P, const double2* alm, double2* phase, int64_t ms, int64_t bs, int B,
+                              int spin, cudaStream_t st);
+int launch_legendre_adjoint_f64(const Plan& P, const double2* phase, int64_t ms, int64_t bs, double2* alm, int B,
+                                int spin, double scale, cudaStream_t st);
 int launch_alm_to_T(const double2* alm, double2* almT, int B, int ncomp, int64_t nalm, int sms, cudaStream_t st);
-int launch_ring_synth_f64(const Plan& P, const int* d_list, int nrings, int work_len, const double2* phase,
-                          double* map, int nf, int pack, cudaStream_t st);
-int launch_ring_adjoint_f64(const Plan& P, const int* d_list, int nrings, int work_len, const double* map,
-                            double2* phase, int nf, int pack, cudaStream_t st);
+int launch_ring_synth_f64(const Plan& P, const RingClassList* cls, int ncls, const double2* phase, double* map, int nf,
+                          int pack, cudaStream_t st);
+int launch_ring_adjoint_f64(const Plan& P, const RingClassList* cls, int ncls, const double* map, double2* phase,
+                            int nf, int pack, cudaStream_t st);
 int launch_ring_synth_f32(const Plan& P, const int* d_list, int nrings, int work_len, const float2* phase,
                           double* map, int nf, int pack, cudaStream_t st);
 int launch_ring_adjoint_f32(const Plan& P, const int* d_list, int nrings, int work_len, const double* map,
@@ -61,6 +62,7 @@ struct ps_plan {
   std::vector<int> cls_len, cls_off, cls_cnt;
   std::vector<int> cls_off_n, cls_cnt_n;  // the north rings (and the equator ring) of each class
   int* d_ring_lists = nullptr;
+  std::vector<ps::RingClassList> ring_cls;  // FP64 plans, longest work length first
   std::vector<void*> owned;  // device allocations to free
 };
 
@@ -70,8 +72,8 @@ bool is_pow2(int n) { return n > 0 && (n & (n - 1)) == 0; }
 int next_pow2(int n) { int m = 1; while (m < n) m <<= 1; return m; }
 
 // host radix-2 FFT (sign -1), natural order in and out; used once per plan to
-// build the Bluestein kernel spectra
-void host_fft(std::vector<std::complex<double>>& a) {
+// build the Bluestein kernel spectra.  tw[k] = e^{-2 pi i k / (2 tw.size())}
+void host_fft(std::vector<std::complex<double>>& a, const std::vector<double2>& tw) {
   const int n = (int)a.size();
   for (int i = 1, j = 0; i < n; ++i) {
     int bit = n >> 1;
@@ -80,9 +82,9 @@ void host_fft(std::vector<std::complex<double>>& a) {
     if (i < j) std::swap(a[i], a[j]);
   }
   for (int len = 2; len <= n; len <<= 1) {
+    const size_t step = 2 * tw.size() / size_t(len);
     for (int j = 0; j < len / 2; ++j) {
-      const double ang = -2.0 * M_PI * double(j) / double(len);
-      const std::complex<double> w(std::cos(ang), std::sin(ang));
+      const std::complex<double> w(tw[j * step].x, tw[j * step].y);
       for (int i = 0; i < n; i += len) {
         const std::complex<double> u = a[i + j], v = a[i + j + len / 2] * w;
         a[i + j] = u + v;
@@ -270,6 +272,25 @@ int ps_plan_create(int nside, int lmax, int mmax, int spin_mask, int prec, ps_pl
       if (ir <= P.R - 1 - ir) { lists.push_back(ir); ++n; }
     pl->cls_cnt_n.push_back(n);
   }
+  // FP64 plans: the same classes with the power-of-two rings apart
+  std::vector<std::vector<int>> ring_cls_rings;
+  if (prec == PS_PREC_FP64) {
+    for (auto kv = classes.rbegin(); kv != classes.rend(); ++kv)
+      for (int blue = 1; blue >= 0; --blue) {
+        std::vector<int> all, north;
+        for (int ir : kv->second)
+          if ((rings[ir].bs_slot >= 0) == (blue == 1)) {
+            all.push_back(ir);
+            if (ir <= P.R - 1 - ir) north.push_back(ir);
+          }
+        if (all.empty()) continue;
+        int logM = 0;
+        while ((1 << logM) < kv->first) ++logM;
+        pl->ring_cls.push_back({logM, blue, (int)all.size(), (int)north.size(), nullptr, nullptr});
+        ring_cls_rings.push_back(all);
+        ring_cls_rings.push_back(north);
+      }
+  }
   std::vector<double2> tw(max_fft / 2);
   for (int k = 0; k < max_fft / 2; ++k) {
     const double ang = -2.0 * M_PI * double(k) / double(max_fft);
@@ -289,7 +310,7 @@ int ps_plan_create(int nside, int lmax, int mmax, int spin_mask, int prec, ps_pl
       b[n] = v;
       if (n > 0) b[M - n] = v;
     }
-    host_fft(b);
+    host_fft(b, tw);
     bs_off.push_back((int64_t)bs_spec.size());
     const size_t o = bs_spec.size();
     bs_spec.resize(o + M);
@@ -335,21 +356,64 @@ int ps_plan_create(int nside, int lmax, int mmax, int spin_mask, int prec, ps_pl
   P.d_rings = dev_upload(pl, rings, err);
   P.d_mnorm0 = dev_upload(pl, mnorm, err);
   for (int s = 1; s <= 3; ++s) if (!seeds[s].empty()) P.d_seed[s] = dev_upload(pl, seeds[s], err);
-  P.d_twiddle = dev_upload(pl, tw, err);
-  P.d_bs_spec = dev_upload(pl, bs_spec, err);
-  {
+  P.d_twiddle = P.d_bs_spec = P.d_root = P.d_chirp = nullptr;
+  P.d_chirp_off = nullptr;
+  P.d_twiddle_f = P.d_bs_spec_f = nullptr;
+  if (prec == PS_PREC_FP64) {
+    // twiddles by level (see ps_fft_f64.cu), one level above the longest length
+    std::vector<double2> levels;
+    for (int64_t L = 8; L <= 2 * int64_t(std::max(max_fft, 4)); L *= 2)
+      for (int64_t p = 1; p <= 4; p *= 2)
+        for (int64_t j = 0; j < L / 8; ++j) {
+          const double a = -2.0 * M_PI * double(p * j) / double(L);
+          levels.push_back(make_double2(std::cos(a), std::sin(a)));
+        }
+    P.d_twiddle = dev_upload(pl, levels, err);
+    // Bluestein spectra as the middle pass reads them: [8][M/8], position 8 t + k at k M/8 + t
+    std::vector<double2> spec(bs_spec.size());
+    for (size_t slot = 0; slot < bs_n.size(); ++slot) {
+      const int64_t o = bs_off[slot], M = next_pow2(2 * bs_n[slot] - 1);
+      for (int64_t p = 0; p < M; ++p) spec[size_t(o + (p % 8) * (M / 8) + p / 8)] = bs_spec[size_t(o + p)];
+    }
+    P.d_bs_spec = dev_upload(pl, spec, err);
+    // ring rotations and Bluestein chirps from exact integer argument reduction
+    auto unit = [](int64_t q, int64_t den) {  // e^{i pi q / den}
+      const double a = M_PI * double(q % (2 * den)) / double(den);
+      return make_double2(std::cos(a), std::sin(a));
+    };
+    std::vector<double2> root, chirp;
+    std::vector<int64_t> chirp_off;
+    root.reserve(size_t(2) * nside * (nside + 1));
+    for (int64_t i = 1; i <= nside; ++i)
+      for (int64_t k = 0; k < 4 * i; ++k) root.push_back(unit(k, 4 * i));
+    for (int N : bs_n) {
+      chirp_off.push_back((int64_t)chirp.size());
+      for (int64_t j = 0; j < N; ++j) {
+        const double2 w = unit(j * j, N);
+        chirp.push_back(make_double2(w.x, -w.y));
+      }
+    }
+    P.d_root = dev_upload(pl, root, err);
+    P.d_chirp = dev_upload(pl, chirp, err);
+    P.d_chirp_off = dev_upload(pl, chirp_off, err);
+    for (size_t c = 0; c < pl->ring_cls.size(); ++c) {
+      pl->ring_cls[c].rings = dev_upload(pl, ring_cls_rings[2 * c], err);
+      pl->ring_cls[c].rings_n = dev_upload(pl, ring_cls_rings[2 * c + 1], err);
+    }
+  } else {
     std::vector<float2> twf(tw.size()), bsf(bs_spec.size());
     for (size_t i = 0; i < tw.size(); ++i) twf[i] = make_float2(float(tw[i].x), float(tw[i].y));
     for (size_t i = 0; i < bs_spec.size(); ++i) bsf[i] = make_float2(float(bs_spec[i].x), float(bs_spec[i].y));
     P.d_twiddle_f = dev_upload(pl, twf, err);
     P.d_bs_spec_f = dev_upload(pl, bsf, err);
+  }
+  {
     std::vector<int> zero(1, 0);
     P.d_err = dev_upload(pl, zero, err);
   }
   P.d_bs_off = dev_upload(pl, bs_off, err);
   P.d_rot_f = nullptr;
   P.d_chirp_f = nullptr;
-  P.d_chirp_off = nullptr;
   if (prec == PS_PREC_MIXED) {
     // ring rotations and Bluestein chirps of the FP32 ring transforms, from exact integer
     // argument reduction in FP64 (so the kernels evaluate no sincos)
@@ -631,7 +695,7 @@ int ps_legendre_synthesis(const ps_plan* plan, const double* alm, double* phase,
     return PS_OK;
   }
   return ps::launch_legendre_synth_f64(P, reinterpret_cast<const double2*>(alm), reinterpret_cast<double2*>(phase),
-                                       batch, spin, stream);
+                                       int64_t(batch) * ncomp, ncomp, batch, spin, stream);
 }
 
 int ps_legendre_adjoint(const ps_plan* plan, const double* phase, double* alm, int batch, int spin, double scale,
@@ -665,8 +729,8 @@ int ps_legendre_adjoint(const ps_plan* plan, const double* phase, double* alm, i
     }
     return PS_OK;
   }
-  return ps::launch_legendre_adjoint_f64(P, reinterpret_cast<const double2*>(phase), reinterpret_cast<double2*>(alm),
-                                         batch, spin, scale, stream);
+  return ps::launch_legendre_adjoint_f64(P, reinterpret_cast<const double2*>(phase), int64_t(batch) * ncomp, ncomp,
+                                         reinterpret_cast<double2*>(alm), batch, spin, scale, stream);
 }
 
 int ps_sht_workspace_bytes(const ps_plan* plan, int batch, int spin, int adjoint, size_t* bytes) {
@@ -715,15 +779,12 @@ int ps_synthesis(const ps_plan* plan, const double* alm, double* map, int batch,
     return PS_OK;
   }
   double2* phase = reinterpret_cast<double2*>(phase_ptr);
-  rc = ps::launch_legendre_synth_f64(P, reinterpret_cast<const double2*>(alm), phase, batch, spin, stream);
+  // between the two stages the phases are [R][batch][mmax+1][ncomp]
+  rc = ps::launch_legendre_synth_f64(P, reinterpret_cast<const double2*>(alm), phase, ncomp,
+                                     int64_t(P.mmax + 1) * ncomp, batch, spin, stream);
   if (rc) return rc;
-  for (size_t c = 0; c < plan->cls_len.size(); ++c) {
-    rc = ps::launch_ring_synth_f64(P, plan->d_ring_lists + (spin ? plan->cls_off[c] : plan->cls_off_n[c]),
-                                   spin ? plan->cls_cnt[c] : plan->cls_cnt_n[c], plan->cls_len[c], phase, map, nf,
-                                   spin > 0, stream);
-    if (rc) return rc;
-  }
-  return PS_OK;
+  return ps::launch_ring_synth_f64(P, plan->ring_cls.data(), int(plan->ring_cls.size()), phase, map, nf, spin > 0,
+                                   stream);
 }
 
 int ps_adjoint(const ps_plan* plan, const double* map, double* alm, int batch, int spin, double scale,
@@ -767,13 +828,11 @@ int ps_adjoint(const ps_plan* plan, const double* map, double* alm, int batch, i
     return PS_OK;
   }
   double2* phase = reinterpret_cast<double2*>(ws);
-  for (size_t c = 0; c < plan->cls_len.size(); ++c) {
-    rc = ps::launch_ring_adjoint_f64(P, plan->d_ring_lists + (spin ? plan->cls_off[c] : plan->cls_off_n[c]),
-                                     spin ? plan->cls_cnt[c] : plan->cls_cnt_n[c], plan->cls_len[c], map, phase, nf,
-                                     spin > 0, stream);
-    if (rc) return rc;
-  }
-  return ps::launch_legendre_adjoint_f64(P, phase, reinterpret_cast<double2*>(alm), batch, spin, scale, stream);
+  rc = ps::launch_ring_adjoint_f64(P, plan->ring_cls.data(), int(plan->ring_cls.size()), map, phase, nf, spin > 0,
+                                   stream);
+  if (rc) return rc;
+  return ps::launch_legendre_adjoint_f64(P, phase, ncomp, int64_t(P.mmax + 1) * ncomp, reinterpret_cast<double2*>(alm),
+                                         batch, spin, scale, stream);
 }
 
 }  // extern "C"
