@@ -402,11 +402,10 @@ struct SynthIn {
     }
   }
   __device__ __forceinline__ double2 combine(int k, double2 ca, double2 cb) const {
-    if (step < 0.0) {
-      const double2 e = __ldg(&root[k]);
-      ca = cmul(ca, e);
-      cb = cmul(cb, e);
-    }
+    // (also where the rotation is 1: a part that is not finite makes its complex product so)
+    const double2 e = step < 0.0 ? __ldg(&root[k]) : make_double2(1.0, 0.0);
+    ca = cmul(ca, e);
+    cb = cmul(cb, e);
     // a real field keeps only Re(c_0); it must not leak into the partner field of the pair
     if (k == 0) ca.y = cb.y = 0.0;
     const double2 v = make_double2(ca.x + cb.y, cb.x - ca.y);
@@ -565,12 +564,13 @@ __global__ void __launch_bounds__(NT, 512 / NT) ring_adjoint_f64(const __grid_co
     const double2 z = it.a[pad8(k)], z2 = cconj(it.a[pad8(k == 0 ? 0 : N - k)]);
     double2 xa = make_double2(0.5 * (z.x + z2.x), 0.5 * (z.y + z2.y));
     double2 xb = make_double2(0.5 * (z.y - z2.y), -0.5 * (z.x - z2.x));  // (z - z2) / (2i)
+    double2 e = make_double2(1.0, 0.0);
     if (it.turned) {
-      double2 e = cconj(__ldg(&it.root[k]));
+      e = cconj(__ldg(&it.root[k]));
       if (j & 1) e = make_double2(-e.x, -e.y);
-      xa = cmul(xa, e);
-      xb = cmul(xb, e);
     }
+    xa = cmul(xa, e);
+    xb = cmul(xb, e);
     pa[int64_t(m) * ms] = xa;
     if (it.vb) pb[int64_t(m) * ms] = xb;
   }

@@ -36,69 +36,13 @@
 #include <algorithm>
 #include <type_traits>
 
-#include "ps_common.cuh"
+#include "ps_legendre_f64.cuh"
 #include "ps_stats.cuh"
 
 namespace ps {
 
 constexpr int SYN_THREADS = 128;  // threads per synthesis CTA
 constexpr int ADJ_LCH = 64;       // l chunk of the adjoint between two CTA barriers
-
-// ---------------------------------------------------------------- seeds
-// The products of ps_common.cuh's snorm / smul / spow on positive normal values,
-// with the exponent taken from the bits (frexp handles cases that do not occur here).
-__device__ __forceinline__ Scaled qnorm(double x) {
-  const int hi = __double2hiint(x);
-  Scaled r;
-  r.e = ((hi >> 20) & 0x7ff) - 1022;
-  r.v = __hiloint2double((hi & 0x000fffff) | 0x3fe00000, __double2loint(x));
-  return r;
-}
-__device__ __forceinline__ Scaled qmul(Scaled a, Scaled b) {
-  Scaled r = qnorm(a.v * b.v);
-  r.e += a.e + b.e;
-  return r;
-}
-__device__ __forceinline__ Scaled qpow(double x, int n) {
-  Scaled r;
-  r.v = 0.5;
-  r.e = 1;
-  Scaled b = qnorm(x);
-  while (n) {
-    if (n & 1) r = qmul(r, b);
-    b = qmul(b, b);
-    n >>= 1;
-  }
-  return r;
-}
-
-__device__ __forceinline__ void seed_spin0(int m, double sth, double mnorm, double& v, int& k) {
-  Scaled s = qmul(qpow(sth, m), qnorm(mnorm));
-  to_kscale(s, v, k);
-  if (m & 1) v = -v;
-}
-
-// Seeds of +s lam and -s lam at l = max(m, s) (Goldberg et al. 1967 with a
-// single term left in the sum), with a common scale exponent k.
-__device__ __forceinline__ void seed_spin(int m, int s, const RingInfo& g, SeedNorm nrm, double& f, double& gg,
-                                          int& k) {
-  const double sh = sqrt(0.5 * g.omz), ch = sqrt(0.5 * g.opz);
-  const int lo = m < s ? m : s, hi = m < s ? s : m;
-  Scaled pf = qmul(qpow(sh, hi + lo), qpow(ch, hi - lo));
-  Scaled pg = qmul(qpow(sh, hi - lo), qpow(ch, hi + lo));
-  const double sgn_f = (m & 1) ? -1.0 : 1.0;
-  const double sgn_g = m >= s ? sgn_f : (s & 1) ? -1.0 : 1.0;
-  Scaled n;
-  n.v = nrm.v;
-  n.e = nrm.e;
-  Scaled sf = qmul(n, pf), sg = qmul(n, pg);
-  Scaled big = (sf.e >= sg.e) ? sf : sg;
-  double vb;
-  to_kscale(big, vb, k);
-  const int shift = k * SCALE_BITS;
-  f = ldexp(sf.v, max(sf.e - shift, -2000)) * sgn_f;
-  gg = ldexp(sg.v, max(sg.e - shift, -2000)) * sgn_g;
-}
 
 // ---------------------------------------------------------------- recurrence tables
 // Three-term coefficients of the normalised functions:
@@ -154,53 +98,14 @@ __global__ void leg_tables_f64(int lmax, int mmax, int s, double* __restrict__ c
   }
 }
 
-// Size tests read the exponent bits: an FP64 compare would take a slot of the FP64 pipe.
-constexpr int HI_FTHRESH = (1023 + 400) << 20;
-__device__ __forceinline__ bool passed(double v) { return (__double2hiint(v) & 0x7fffffff) >= HI_FTHRESH; }
-__device__ __forceinline__ bool nonfinite(double v) { return (__double2hiint(v) & 0x7ff00000) == 0x7ff00000; }
-__device__ __forceinline__ bool nonfinite(double2 v) { return nonfinite(v.x) || nonfinite(v.y); }
-
-// Rings of a warp that is not all live are looked at every four l: c x stays below 2^8 per l, far from
-// overflow.  A value with k < 0 that has grown past 2^400 moves up by one scale.
-__device__ __forceinline__ void rescale(int& k, double& cur, double& prev) {
-  if (k < 0 && passed(cur)) {
-    cur *= PS_FSMALL;
-    prev *= PS_FSMALL;
-    ++k;
-  }
-}
-__device__ __forceinline__ void rescale(int& k, double& f, double& fp, double& g, double& gp) {
-  if (k < 0 && (passed(f) || passed(g))) {
-    f *= PS_FSMALL;
-    fp *= PS_FSMALL;
-    g *= PS_FSMALL;
-    gp *= PS_FSMALL;
-    ++k;
-  }
-}
-
-// How a warp takes the next few l: no ring of it above 2^-400 yet (recurrence only), some, or all.
-enum { LEG_DEAD = 0, LEG_MIXED = 1, LEG_LIVE = 2 };
-template <int RPT>
-__device__ __forceinline__ int leg_mode(const int (&k)[RPT], bool force) {
-  bool all = true, any = false;
-#pragma unroll
-  for (int i = 0; i < RPT; ++i) {
-    all = all && k[i] == 0;
-    any = any || k[i] == 0;
-  }
-  if (__all_sync(0xffffffffu, all)) return LEG_LIVE;
-  return (force || __any_sync(0xffffffffu, any)) ? LEG_MIXED : LEG_DEAD;
-}
-
 // =====================================================================
 // synthesis, spin 0
-// grid (ceil(Rh / (SYN_THREADS RPT)), mmax+1, ceil(B/NB)); a warp holds 32 RPT neighbouring ring pairs and
+// grid (ceil(Rh / (SYN_THREADS RPT)), mmax+1, B); a warp holds 32 RPT neighbouring ring pairs and
 // stages its alm (times gam) and c itself, 32 l at a time and one chunk ahead: the warps of a CTA run at
 // different speeds (fewer instructions while their rings are dead), so they share no barrier.
 // A non-finite alm reaches every ring (its product with a value that counts as zero is NaN): a chunk
 // that holds one takes the mixed steps on all warps.
-template <int NB, int RPT>
+template <int RPT>
 __global__ void __launch_bounds__(SYN_THREADS) synth0_f64(const RingInfo* __restrict__ rings,
                                                            const double* __restrict__ mnorm,
                                                            const double* __restrict__ lc,
@@ -208,35 +113,28 @@ __global__ void __launch_bounds__(SYN_THREADS) synth0_f64(const RingInfo* __rest
                                                            const double2* __restrict__ alm,
                                                            double2* __restrict__ phase, int64_t ms, int64_t bs,
                                                            int R, int Rh, int lmax, int mmax, int B, int64_t nalm) {
-  const int m = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, b0 = blockIdx.z * NB;
+  const int m = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, b = blockIdx.z;
   const int wbase = (blockIdx.x * SYN_THREADS + (tid & ~31)) * RPT, r0 = wbase + lane;
   if (wbase >= Rh) return;
   __shared__ double s_c_[SYN_THREADS / 32][2][32];
-  __shared__ double2 s_alm_[SYN_THREADS / 32][2][32][NB];
+  __shared__ double2 s_alm_[SYN_THREADS / 32][2][32];
   double(*s_c)[32] = s_c_[warp];
-  double2(*s_alm)[32][NB] = s_alm_[warp];
+  double2(*s_alm)[32] = s_alm_[warp];
   const int64_t base = alm_index(m, m, lmax);
 
-  double2 pa[NB];
+  double2 pa;
   double pc;
   auto fetch = [&](int l0) {  // the chunk's alm (times gam) and c, into registers
     const int64_t idx = base + (l0 - m) + lane;
     const bool in = l0 + lane <= lmax;
     const double gm = in ? lg[idx] : 0.0;
     pc = l0 + lane < lmax ? lc[idx] : 0.0;
-#pragma unroll
-    for (int b = 0; b < NB; ++b)
-      pa[b] = in && b0 + b < B ? cscale(alm[int64_t(b0 + b) * nalm + idx], gm) : make_double2(0.0, 0.0);
+    pa = in ? cscale(alm[int64_t(b) * nalm + idx], gm) : make_double2(0.0, 0.0);
   };
   auto stage = [&](int buf) {  // registers -> shared memory; whether a value is not finite
-    bool bad = false;
-#pragma unroll
-    for (int b = 0; b < NB; ++b) {
-      s_alm[buf][lane][b] = pa[b];
-      bad = bad || nonfinite(pa[b]);
-    }
+    s_alm[buf][lane] = pa;
     s_c[buf][lane] = pc;
-    return __any_sync(0xffffffffu, bad);  // also orders the stores before the warp's reads
+    return __any_sync(0xffffffffu, nonfinite(pa));  // also orders the stores before the warp's reads
   };
 
   fetch(m);
@@ -252,11 +150,9 @@ __global__ void __launch_bounds__(SYN_THREADS) synth0_f64(const RingInfo* __rest
     seed_spin0(m, g.sth, mn, cur[i], k[i]);
     if (rp >= Rh) { cur[i] = 0.0; k[i] = 0; }
   }
-  double2 ae[RPT][NB], ao[RPT][NB];
+  double2 ae[RPT], ao[RPT];
 #pragma unroll
-  for (int i = 0; i < RPT; ++i)
-#pragma unroll
-    for (int b = 0; b < NB; ++b) ae[i][b] = ao[i][b] = make_double2(0.0, 0.0);
+  for (int i = 0; i < RPT; ++i) ae[i] = ao[i] = make_double2(0.0, 0.0);
 
   int buf = 0;
   for (int l0 = m; l0 <= lmax; l0 += 32, buf ^= 1) {
@@ -264,21 +160,13 @@ __global__ void __launch_bounds__(SYN_THREADS) synth0_f64(const RingInfo* __rest
     __syncwarp();
     const int n = min(32, lmax - l0 + 1);
     if (l0 + 32 <= lmax) fetch(l0 + 32);
-    auto step = [&](auto mode, int j, double2 (&acc)[RPT][NB]) {
+    auto step = [&](auto mode, int j, double2 (&acc)[RPT]) {
       constexpr int MODE = decltype(mode)::value;
       const double c = s_c[buf][j];
-      double2 a[NB];
-      if (MODE != LEG_DEAD) {
-#pragma unroll
-        for (int b = 0; b < NB; ++b) a[b] = s_alm[buf][j][b];
-      }
+      const double2 a = MODE != LEG_DEAD ? s_alm[buf][j] : make_double2(0.0, 0.0);
 #pragma unroll
       for (int i = 0; i < RPT; ++i) {
-        if (MODE != LEG_DEAD) {
-          const double v = (MODE == LEG_LIVE || k[i] == 0) ? cur[i] : 0.0;
-#pragma unroll
-          for (int b = 0; b < NB; ++b) acc[i][b] = cfma(v, a[b], acc[i][b]);
-        }
+        if (MODE != LEG_DEAD) acc[i] = cfma((MODE == LEG_LIVE || k[i] == 0) ? cur[i] : 0.0, a, acc[i]);
         const double nxt = fma(c * x[i], cur[i], -prev[i]);
         prev[i] = cur[i];
         cur[i] = nxt;
@@ -316,19 +204,15 @@ __global__ void __launch_bounds__(SYN_THREADS) synth0_f64(const RingInfo* __rest
   for (int i = 0; i < RPT; ++i) {
     const int rp = r0 + 32 * i, rs = R - 1 - rp;
     if (rp >= Rh) break;
-#pragma unroll
-    for (int b = 0; b < NB; ++b) {
-      if (b0 + b >= B) break;
-      const int64_t o = m * ms + (b0 + b) * bs, ring = int64_t(mmax + 1) * B;
-      phase[rp * ring + o] = cadd(ae[i][b], ao[i][b]);
-      if (rs != rp) phase[rs * ring + o] = csub(ae[i][b], ao[i][b]);
-    }
+    const int64_t o = m * ms + b * bs, ring = int64_t(mmax + 1) * B;
+    phase[rp * ring + o] = cadd(ae[i], ao[i]);
+    if (rs != rp) phase[rs * ring + o] = csub(ae[i], ao[i]);
   }
 }
 
 // =====================================================================
 // synthesis, spin s > 0: alm [B][2][nalm] (G, C) -> phase [R][mmax+1][B][2] (Q, U)
-template <int NB, int RPT>
+template <int RPT>
 __global__ void __launch_bounds__(SYN_THREADS) synthS_f64(const RingInfo* __restrict__ rings,
                                                            const SeedNorm* __restrict__ seednorm,
                                                            const double2* __restrict__ lcd,
@@ -337,43 +221,33 @@ __global__ void __launch_bounds__(SYN_THREADS) synthS_f64(const RingInfo* __rest
                                                            double2* __restrict__ phase, int64_t ms, int64_t bs,
                                                            int R, int Rh, int lmax, int mmax, int B, int64_t nalm,
                                                            int spin) {
-  const int m = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, b0 = blockIdx.z * NB;
+  const int m = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, b = blockIdx.z;
   const int wbase = (blockIdx.x * SYN_THREADS + (tid & ~31)) * RPT, r0 = wbase + lane;
   if (wbase >= Rh) return;
   __shared__ double2 s_cd_[SYN_THREADS / 32][2][32];
-  __shared__ double2 s_alm_[SYN_THREADS / 32][2][32][NB][2];  // a+ = G + i C, a- = G - i C
+  __shared__ double2 s_alm_[SYN_THREADS / 32][2][32][2];  // a+ = G + i C, a- = G - i C
   double2(*s_cd)[32] = s_cd_[warp];
-  double2(*s_alm)[32][NB][2] = s_alm_[warp];
+  double2(*s_alm)[32][2] = s_alm_[warp];
   const int64_t base = alm_index(m, m, lmax);
   const int lmin = max(m, spin);
 
-  double2 pp[NB], pm[NB], pc;
+  double2 pp, pm, pc;
   auto fetch = [&](int l0) {
     const int64_t idx = base + (l0 - m) + lane;
     const bool in = l0 + lane <= lmax;
     const double gm = in ? lg[idx] : 0.0;
     pc = l0 + lane < lmax ? lcd[idx] : make_double2(0.0, 0.0);
-#pragma unroll
-    for (int b = 0; b < NB; ++b) {
-      pp[b] = pm[b] = make_double2(0.0, 0.0);
-      if (in && b0 + b < B) {
-        const double2 G = cscale(alm[int64_t(b0 + b) * 2 * nalm + idx], gm);
-        const double2 C = cscale(alm[(int64_t(b0 + b) * 2 + 1) * nalm + idx], gm);
-        pp[b] = make_double2(G.x - C.y, G.y + C.x);
-        pm[b] = make_double2(G.x + C.y, G.y - C.x);
-      }
-    }
+    const double2 z = make_double2(0.0, 0.0);
+    const double2 G = in ? cscale(alm[int64_t(b) * 2 * nalm + idx], gm) : z;
+    const double2 C = in ? cscale(alm[(int64_t(b) * 2 + 1) * nalm + idx], gm) : z;
+    pp = make_double2(G.x - C.y, G.y + C.x);
+    pm = make_double2(G.x + C.y, G.y - C.x);
   };
   auto stage = [&](int buf) {
-    bool bad = false;
-#pragma unroll
-    for (int b = 0; b < NB; ++b) {
-      s_alm[buf][lane][b][0] = pp[b];
-      s_alm[buf][lane][b][1] = pm[b];
-      bad = bad || nonfinite(pp[b]) || nonfinite(pm[b]);
-    }
+    s_alm[buf][lane][0] = pp;
+    s_alm[buf][lane][1] = pm;
     s_cd[buf][lane] = pc;
-    return __any_sync(0xffffffffu, bad);
+    return __any_sync(0xffffffffu, nonfinite(pp) || nonfinite(pm));
   };
 
   fetch(lmin);
@@ -390,15 +264,14 @@ __global__ void __launch_bounds__(SYN_THREADS) synthS_f64(const RingInfo* __rest
     if (rp >= Rh) { f[i] = g[i] = 0.0; k[i] = 0; }
   }
   // sums on the north ring and, with the sign of l - lmin, on its mirror
-  double2 PN[RPT][NB], MN[RPT][NB], PS[RPT][NB], MS[RPT][NB];
-#pragma unroll
-  for (int b = 0; b < NB; ++b) {
+  double2 PN[RPT], MN[RPT], PS[RPT], MS[RPT];
+  {
     double2 z = make_double2(0.0, 0.0);
     // alm with l < s do not enter, unless not finite (0 times them)
-    for (int l = m; l < min(spin, lmax + 1) && b0 + b < B; ++l)
-      for (int c = 0; c < 2; ++c) z = cfma(0.0, alm[(int64_t(b0 + b) * 2 + c) * nalm + base + (l - m)], z);
+    for (int l = m; l < min(spin, lmax + 1); ++l)
+      for (int c = 0; c < 2; ++c) z = cfma(0.0, alm[(int64_t(b) * 2 + c) * nalm + base + (l - m)], z);
 #pragma unroll
-    for (int i = 0; i < RPT; ++i) PN[i][b] = MN[i][b] = PS[i][b] = MS[i][b] = z;
+    for (int i = 0; i < RPT; ++i) PN[i] = MN[i] = PS[i] = MS[i] = z;
   }
 
   int buf = 0;
@@ -411,23 +284,17 @@ __global__ void __launch_bounds__(SYN_THREADS) synthS_f64(const RingInfo* __rest
       constexpr int MODE = decltype(mode)::value;
       constexpr double SG = decltype(odd)::value ? -1.0 : 1.0;
       const double2 cd = s_cd[buf][j];
-      double2 ap[NB], am[NB];
-      if (MODE != LEG_DEAD) {
-#pragma unroll
-        for (int b = 0; b < NB; ++b) { ap[b] = s_alm[buf][j][b][0]; am[b] = s_alm[buf][j][b][1]; }
-      }
+      double2 ap = make_double2(0.0, 0.0), am = ap;
+      if (MODE != LEG_DEAD) { ap = s_alm[buf][j][0]; am = s_alm[buf][j][1]; }
 #pragma unroll
       for (int i = 0; i < RPT; ++i) {
         if (MODE != LEG_DEAD) {
           const bool on = MODE == LEG_LIVE || k[i] == 0;
           const double vf = on ? f[i] : 0.0, vg = on ? g[i] : 0.0;
-#pragma unroll
-          for (int b = 0; b < NB; ++b) {
-            PN[i][b] = cfma(vf, ap[b], PN[i][b]);
-            MN[i][b] = cfma(vg, am[b], MN[i][b]);
-            PS[i][b] = cfma(SG * vg, ap[b], PS[i][b]);
-            MS[i][b] = cfma(SG * vf, am[b], MS[i][b]);
-          }
+          PN[i] = cfma(vf, ap, PN[i]);
+          MN[i] = cfma(vg, am, MN[i]);
+          PS[i] = cfma(SG * vg, ap, PS[i]);
+          MS[i] = cfma(SG * vf, am, MS[i]);
         }
         const double fn = fma(fma(cd.x, x[i], cd.y), f[i], -fp[i]);
         const double gn = fma(fma(cd.x, x[i], -cd.y), g[i], -gp[i]);
@@ -465,18 +332,14 @@ __global__ void __launch_bounds__(SYN_THREADS) synthS_f64(const RingInfo* __rest
   for (int i = 0; i < RPT; ++i) {
     const int rp = r0 + 32 * i, rs = R - 1 - rp;
     if (rp >= Rh) break;
-#pragma unroll
-    for (int b = 0; b < NB; ++b) {
-      if (b0 + b >= B) break;
-      for (int side = 0; side < (rs != rp ? 2 : 1); ++side) {
-        const double h = side == 0 ? 0.5 : ss;
-        const double2 sp = cscale(side == 0 ? PN[i][b] : PS[i][b], h), sm = cscale(side == 0 ? MN[i][b] : MS[i][b], h);
-        const double2 sum = cadd(sp, sm), dif = csub(sp, sm);
-        const double2 q = odd ? dif : sum, u = odd ? sum : dif;
-        const int64_t o = (side == 0 ? rp : rs) * (int64_t(mmax + 1) * B * 2) + m * ms + (b0 + b) * bs;
-        phase[o] = make_double2(-q.x, -q.y);
-        phase[o + 1] = make_double2(-u.y, u.x);
-      }
+    for (int side = 0; side < (rs != rp ? 2 : 1); ++side) {
+      const double h = side == 0 ? 0.5 : ss;
+      const double2 sp = cscale(side == 0 ? PN[i] : PS[i], h), sm = cscale(side == 0 ? MN[i] : MS[i], h);
+      const double2 sum = cadd(sp, sm), dif = csub(sp, sm);
+      const double2 q = odd ? dif : sum, u = odd ? sum : dif;
+      const int64_t o = (side == 0 ? rp : rs) * (int64_t(mmax + 1) * B * 2) + m * ms + b * bs;
+      phase[o] = make_double2(-q.x, -q.y);
+      phase[o + 1] = make_double2(-u.y, u.x);
     }
   }
 }
@@ -776,64 +639,68 @@ static double leg_bytes(const Plan& P, int B, int spin) {
   return nf * 16.0 * (double(P.nalm) + double(P.R) * (P.mmax + 1));
 }
 
+int launch_synth_mma_f64(const Plan& P, const double2* alm, double2* phase, int64_t ms, int64_t bs, int B, int spin,
+                         cudaStream_t st);
+int launch_adjoint_mma_f64(const Plan& P, const double2* phase, int64_t ms, int64_t bs, double2* alm, int B, int spin,
+                           double scale, cudaStream_t st);
+
 int launch_leg_tables_f64(const Plan& P, int spin, double* cd, double* gam, cudaStream_t st) {
   leg_tables_f64<<<(P.mmax + 64) / 64, 64, 0, st>>>(P.lmax, P.mmax, spin, cd, gam);
   PS_LAUNCH_CHECK();
   return PS_OK;
 }
 
-template <int NB, int RPT>
+constexpr int MAX_GRID_Z = 65535;  // maps per launch
+
+template <int RPT>
 static void synth0_go(const Plan& P, const double2* alm, double2* phase, int64_t ms, int64_t bs, int B, cudaStream_t st) {
-  const dim3 grid((P.Rh + SYN_THREADS * RPT - 1) / (SYN_THREADS * RPT), P.mmax + 1, (B + NB - 1) / NB);
-  synth0_f64<NB, RPT><<<grid, SYN_THREADS, 0, st>>>(P.d_rings, P.d_mnorm0, P.d_leg_cd[0], P.d_leg_g[0], alm, phase,
-                                                    ms, bs, P.R, P.Rh, P.lmax, P.mmax, B, P.nalm);
+  const dim3 grid((P.Rh + SYN_THREADS * RPT - 1) / (SYN_THREADS * RPT), P.mmax + 1, B);
+  synth0_f64<RPT><<<grid, SYN_THREADS, 0, st>>>(P.d_rings, P.d_mnorm0, P.d_leg_cd[0], P.d_leg_g[0], alm, phase, ms, bs,
+                                                P.R, P.Rh, P.lmax, P.mmax, B, P.nalm);
 }
-template <int NB, int RPT>
+template <int RPT>
 static void synthS_go(const Plan& P, const double2* alm, double2* phase, int64_t ms, int64_t bs, int B, int spin,
                       cudaStream_t st) {
-  const dim3 grid((P.Rh + SYN_THREADS * RPT - 1) / (SYN_THREADS * RPT), P.mmax + 1, (B + NB - 1) / NB);
-  synthS_f64<NB, RPT><<<grid, SYN_THREADS, 0, st>>>(P.d_rings, P.d_seed[spin],
-                                                    reinterpret_cast<const double2*>(P.d_leg_cd[spin]),
-                                                    P.d_leg_g[spin], alm, phase, ms, bs, P.R, P.Rh, P.lmax, P.mmax, B,
-                                                    P.nalm, spin);
+  const dim3 grid((P.Rh + SYN_THREADS * RPT - 1) / (SYN_THREADS * RPT), P.mmax + 1, B);
+  synthS_f64<RPT><<<grid, SYN_THREADS, 0, st>>>(P.d_rings, P.d_seed[spin],
+                                                reinterpret_cast<const double2*>(P.d_leg_cd[spin]), P.d_leg_g[spin], alm,
+                                                phase, ms, bs, P.R, P.Rh, P.lmax, P.mmax, B, P.nalm, spin);
 }
 
-// Rings per thread of the synthesis: the rings of a thread share each shared-memory broadcast, fewer keep more
-// warps in flight where a plan has few rings.  Measured, one map, spin 0, one / two / four rings: Nside 1024,
-// lmax 2048 1661 / 1417 / 1353 us, Nside 512, lmax 1000 212 / 187 / 184 us, Nside 256, lmax 767 70 / 71 / 81 us;
-// spin 2 (whose eight sums per ring fill the registers) 4165 / 3880 / 3842 us at Nside 1024.
+// Batches run on the FP64 MMA, which takes maps four (spin 0) or two (spin s) at a time; fewer maps than most of a
+// tile run one by one.  Measured, FMA / MMA kernels: spin 0, Nside 512, lmax 1000: 2 maps 357 / 389 us, 4 maps 475 /
+// 397, 24 maps 2880 / 1916; Nside 256, lmax 500, 3 maps 93 / 60.  Spin 2, Nside 512: 2 maps 811 / 805, 24 maps 9646 /
+// 7208; Nside 256, lmax 500, 3 maps 227 / 184 us (the FMA kernels then took four and two maps per CTA).
+// Tile 1 forces single maps, tile 4 (spin s: 2) the MMA.
+//
+// Rings per thread of single maps: the rings of a thread share each shared-memory broadcast, fewer keep more warps
+// in flight where a plan has few rings.  Measured, one map, spin 0, one / two / four rings: Nside 1024, lmax 2048
+// 1661 / 1417 / 1353 us, Nside 512, lmax 1000 212 / 187 / 184 us, Nside 256, lmax 767 70 / 71 / 81 us; spin 2 (whose
+// eight sums per ring fill the registers) 4165 / 3880 / 3842 us at Nside 1024.
 int launch_legendre_synth_f64(const Plan& P, const double2* alm, double2* phase, int64_t ms, int64_t bs, int B,
                               int spin, cudaStream_t st) {
   StatScope sc(PS_K_LEG_SYNTH, leg_flops(P, B, spin), leg_bytes(P, B, spin), st);
+  if (spin > 0 && !P.d_seed[spin]) return PS_ERR_INVALID;
   const int t = P.tile[0][spin];
-  const bool two = P.Rh > 128;
+  if (t ? t > 1 : B >= 3) return launch_synth_mma_f64(P, alm, phase, ms, bs, B, spin, st);
   if (spin == 0) {
-    if (t ? t == 4 : B >= 4) {
-      two ? synth0_go<4, 2>(P, alm, phase, ms, bs, B, st) : synth0_go<4, 1>(P, alm, phase, ms, bs, B, st);
-    } else {
-      if (P.Rh >= 1024) synth0_go<1, 4>(P, alm, phase, ms, bs, B, st);
-      else two ? synth0_go<1, 2>(P, alm, phase, ms, bs, B, st) : synth0_go<1, 1>(P, alm, phase, ms, bs, B, st);
-    }
+    if (P.Rh >= 1024) synth0_go<4>(P, alm, phase, ms, bs, B, st);
+    else if (P.Rh > 128) synth0_go<2>(P, alm, phase, ms, bs, B, st);
+    else synth0_go<1>(P, alm, phase, ms, bs, B, st);
   } else {
-    if (!P.d_seed[spin]) return PS_ERR_INVALID;
-    if (t ? t == 2 : B >= 2) {
-      two ? synthS_go<2, 2>(P, alm, phase, ms, bs, B, spin, st) : synthS_go<2, 1>(P, alm, phase, ms, bs, B, spin, st);
-    } else {
-      two ? synthS_go<1, 2>(P, alm, phase, ms, bs, B, spin, st) : synthS_go<1, 1>(P, alm, phase, ms, bs, B, spin, st);
-    }
+    if (P.Rh > 128) synthS_go<2>(P, alm, phase, ms, bs, B, spin, st);
+    else synthS_go<1>(P, alm, phase, ms, bs, B, spin, st);
   }
   PS_LAUNCH_CHECK();
   return PS_OK;
 }
 
-constexpr int ADJ_BATCH = 65535;  // maps per launch (grid limit)
-
 template <int RPT, int NW>
 static void adj0_go(const Plan& P, const double2* phase, int64_t ms, int64_t bs, double2* alm, int B, double scale,
                     cudaStream_t st) {
   const int warps = std::min(NW, (P.Rh + 32 * RPT - 1) / (32 * RPT));
-  for (int b0 = 0; b0 < B; b0 += ADJ_BATCH)
-    adj0_f64<RPT, NW><<<dim3(1, P.mmax + 1, std::min(ADJ_BATCH, B - b0)), 32 * warps, 0, st>>>(
+  for (int b0 = 0; b0 < B; b0 += MAX_GRID_Z)
+    adj0_f64<RPT, NW><<<dim3(1, P.mmax + 1, std::min(MAX_GRID_Z, B - b0)), 32 * warps, 0, st>>>(
         P.d_rings, P.d_mnorm0, P.d_leg_cd[0], P.d_leg_g[0], phase, ms, bs, alm, P.R, P.Rh, P.lmax, P.mmax, B, b0,
         P.nalm, scale);
 }
@@ -841,8 +708,8 @@ template <int RPT, int NW>
 static void adjS_go(const Plan& P, const double2* phase, int64_t ms, int64_t bs, double2* alm, int B, int spin,
                     double scale, cudaStream_t st) {
   const int warps = std::min(NW, (P.Rh + 32 * RPT - 1) / (32 * RPT));
-  for (int b0 = 0; b0 < B; b0 += ADJ_BATCH)
-    adjS_f64<RPT, NW><<<dim3(1, P.mmax + 1, std::min(ADJ_BATCH, B - b0)), 32 * warps, 0, st>>>(
+  for (int b0 = 0; b0 < B; b0 += MAX_GRID_Z)
+    adjS_f64<RPT, NW><<<dim3(1, P.mmax + 1, std::min(MAX_GRID_Z, B - b0)), 32 * warps, 0, st>>>(
         P.d_rings, P.d_seed[spin], reinterpret_cast<const double2*>(P.d_leg_cd[spin]), P.d_leg_g[spin], phase, ms, bs,
         alm, P.R, P.Rh, P.lmax, P.mmax, B, b0, P.nalm, spin, scale);
 }
@@ -853,10 +720,17 @@ static void adjS_go(const Plan& P, const double2* phase, int64_t ms, int64_t bs,
 // there are few (m, map) pairs.  Measured, four against eight warps of four rings, one map: Nside 1024, lmax 2048
 // 1898 / 1957 us (spin 0), Nside 512, lmax 1000 298 / 259 us; spin 2, <4, 4> against <2, 8>: 5280 / 5720 us,
 // 706 / 759 us and, Nside 256, lmax 767, 259 / 240 us.
+//
+// Batches run on the FP64 MMA.  Measured, FMA / MMA kernels: spin 0, Nside 512, lmax 1000, 4 maps 1011 / 593 us, 24
+// maps 6002 / 2999; Nside 256, lmax 767, 2 maps 171 / 192, lmax 500, 3 maps 124 / 125.  Spin 2 (the sums of two
+// maps fill a tile): Nside 256, lmax 767, 2 maps 430 / 326, Nside 512, 24 maps 16359 / 9476; one map, half a tile,
+// 707 / 1054.  Tile 1 forces single maps of spin 0, tile 4 the MMA.
 int launch_legendre_adjoint_f64(const Plan& P, const double2* phase, int64_t ms, int64_t bs, double2* alm, int B,
                                 int spin, double scale, cudaStream_t st) {
   StatScope sc(PS_K_LEG_ADJOINT, leg_flops(P, B, spin), leg_bytes(P, B, spin), st);
   if (spin > 0 && !P.d_seed[spin]) return PS_ERR_INVALID;
+  const int t = P.tile[1][spin];
+  if (spin > 0 ? B >= 2 : t ? t > 1 : B >= 4) return launch_adjoint_mma_f64(P, phase, ms, bs, alm, B, spin, scale, st);
   const int64_t ctas = int64_t(P.mmax + 1) * B;
   if (spin == 0) {
     if (P.Rh > 256) ctas < 1500 ? adj0_go<4, 8>(P, phase, ms, bs, alm, B, scale, st) : adj0_go<4, 4>(P, phase, ms, bs, alm, B, scale, st);
