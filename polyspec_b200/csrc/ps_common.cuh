@@ -52,7 +52,8 @@ struct Plan {
   double2* d_bs_spec;
   double2* d_root;
   double2* d_chirp;
-  float2* d_twiddle_f;      // mixed plans: the same in FP32
+  // mixed plans, FP32: e^{-2 pi i j / 2^s}, j < 2^(s-1), level after level from s = 1; Bluestein spectra
+  float2* d_twiddle_f;
   float2* d_bs_spec_f;
   // mixed plans: e^{i m phi0} of every north ring (the mirror ring has the same phi0),
   // [Rh][mmax+1], and the Bluestein chirps e^{-i pi j^2 / N}, j < N, of every slot
@@ -79,8 +80,8 @@ struct Plan {
   int tab_fmt_build;
 };
 
-// Rings of one FFT work length 2^logM, Bluestein rings (blue) and power-of-two rings apart, for the FP64 ring
-// transforms: all rings (spin s), or the north rings and the equator (spin 0, packed with their mirrors).
+// Rings of one FFT work length 2^logM, Bluestein rings (blue) and power-of-two rings apart: all rings (spin s), or
+// the north rings and the equator (spin 0, packed with their mirrors).
 struct RingClassList {
   int logM, blue, count, count_n;
   const int *rings, *rings_n;  // device

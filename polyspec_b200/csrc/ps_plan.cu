@@ -24,10 +24,10 @@ int launch_ring_synth_f64(const Plan& P, const RingClassList* cls, int ncls, con
                           int pack, cudaStream_t st);
 int launch_ring_adjoint_f64(const Plan& P, const RingClassList* cls, int ncls, const double* map, double2* phase,
                             int nf, int pack, cudaStream_t st);
-int launch_ring_synth_f32(const Plan& P, const int* d_list, int nrings, int work_len, const float2* phase,
-                          double* map, int nf, int pack, cudaStream_t st);
-int launch_ring_adjoint_f32(const Plan& P, const int* d_list, int nrings, int work_len, const double* map,
-                            float2* phase, int nf, int pack, cudaStream_t st);
+int launch_ring_synth_f32(const Plan& P, const RingClassList* cls, int ncls, const float2* phase, double* map, int nf,
+                          int pack, cudaStream_t st);
+int launch_ring_adjoint_f32(const Plan& P, const RingClassList* cls, int ncls, const double* map, float2* phase,
+                            int nf, int pack, cudaStream_t st);
 int launch_legendre_synth_tc(const Plan& P, const double2* almT, float2* phase, int B, int spin, int* err_flag,
                              cudaStream_t st);
 int launch_legendre_adjoint_mx(const Plan& P, const float2* phase, float2* partial, int B, int bofs, int Bc,
@@ -58,11 +58,7 @@ struct ps_plan {
   // Legendre tables owned by this plan (ps_plan_build_table), per spin
   void* tab_alloc[4] = {nullptr, nullptr, nullptr, nullptr};
   void* tab_meta = nullptr;  // d_tab_off and d_tab_work in one allocation
-  // FFT length classes: rings with the same work length share a launch
-  std::vector<int> cls_len, cls_off, cls_cnt;
-  std::vector<int> cls_off_n, cls_cnt_n;  // the north rings (and the equator ring) of each class
-  int* d_ring_lists = nullptr;
-  std::vector<ps::RingClassList> ring_cls;  // FP64 plans, longest work length first
+  std::vector<ps::RingClassList> ring_cls;  // FFT length classes, longest work length first
   std::vector<void*> owned;  // device allocations to free
 };
 
@@ -257,40 +253,23 @@ int ps_plan_create(int nside, int lmax, int mmax, int spin_mask, int prec, ps_pl
     const size_t elem = (prec == PS_PREC_FP64) ? sizeof(double2) : sizeof(float2);
     if (size_t(max_fft) * elem > size_t(optin)) { delete pl; return PS_ERR_UNSUPPORTED; }
   }
-  std::vector<int> lists;
-  for (auto& kv : classes) {
-    pl->cls_len.push_back(kv.first);
-    pl->cls_off.push_back((int)lists.size());
-    pl->cls_cnt.push_back((int)kv.second.size());
-    // largest rings first inside a class does not matter: all have equal work
-    lists.insert(lists.end(), kv.second.begin(), kv.second.end());
-  }
-  for (auto& kv : classes) {
-    pl->cls_off_n.push_back((int)lists.size());
-    int n = 0;
-    for (int ir : kv.second)
-      if (ir <= P.R - 1 - ir) { lists.push_back(ir); ++n; }
-    pl->cls_cnt_n.push_back(n);
-  }
-  // FP64 plans: the same classes with the power-of-two rings apart
+  // rings of one work length, the power-of-two rings apart
   std::vector<std::vector<int>> ring_cls_rings;
-  if (prec == PS_PREC_FP64) {
-    for (auto kv = classes.rbegin(); kv != classes.rend(); ++kv)
-      for (int blue = 1; blue >= 0; --blue) {
-        std::vector<int> all, north;
-        for (int ir : kv->second)
-          if ((rings[ir].bs_slot >= 0) == (blue == 1)) {
-            all.push_back(ir);
-            if (ir <= P.R - 1 - ir) north.push_back(ir);
-          }
-        if (all.empty()) continue;
-        int logM = 0;
-        while ((1 << logM) < kv->first) ++logM;
-        pl->ring_cls.push_back({logM, blue, (int)all.size(), (int)north.size(), nullptr, nullptr});
-        ring_cls_rings.push_back(all);
-        ring_cls_rings.push_back(north);
-      }
-  }
+  for (auto kv = classes.rbegin(); kv != classes.rend(); ++kv)
+    for (int blue = 1; blue >= 0; --blue) {
+      std::vector<int> all, north;
+      for (int ir : kv->second)
+        if ((rings[ir].bs_slot >= 0) == (blue == 1)) {
+          all.push_back(ir);
+          if (ir <= P.R - 1 - ir) north.push_back(ir);
+        }
+      if (all.empty()) continue;
+      int logM = 0;
+      while ((1 << logM) < kv->first) ++logM;
+      pl->ring_cls.push_back({logM, blue, (int)all.size(), (int)north.size(), nullptr, nullptr});
+      ring_cls_rings.push_back(all);
+      ring_cls_rings.push_back(north);
+    }
   std::vector<double2> tw(max_fft / 2);
   for (int k = 0; k < max_fft / 2; ++k) {
     const double ang = -2.0 * M_PI * double(k) / double(max_fft);
@@ -396,16 +375,21 @@ int ps_plan_create(int nside, int lmax, int mmax, int spin_mask, int prec, ps_pl
     P.d_root = dev_upload(pl, root, err);
     P.d_chirp = dev_upload(pl, chirp, err);
     P.d_chirp_off = dev_upload(pl, chirp_off, err);
-    for (size_t c = 0; c < pl->ring_cls.size(); ++c) {
-      pl->ring_cls[c].rings = dev_upload(pl, ring_cls_rings[2 * c], err);
-      pl->ring_cls[c].rings_n = dev_upload(pl, ring_cls_rings[2 * c + 1], err);
-    }
   } else {
-    std::vector<float2> twf(tw.size()), bsf(bs_spec.size());
-    for (size_t i = 0; i < tw.size(); ++i) twf[i] = make_float2(float(tw[i].x), float(tw[i].y));
+    // twiddles e^{-2 pi i j / 2^s}, j < 2^(s-1), level after level from s = 1
+    std::vector<float2> twf, bsf(bs_spec.size());
+    for (size_t half = 1; half <= tw.size(); half *= 2)
+      for (size_t j = 0; j < half; ++j) {
+        const double2 w = tw[j * (tw.size() / half)];
+        twf.push_back(make_float2(float(w.x), float(w.y)));
+      }
     for (size_t i = 0; i < bs_spec.size(); ++i) bsf[i] = make_float2(float(bs_spec[i].x), float(bs_spec[i].y));
     P.d_twiddle_f = dev_upload(pl, twf, err);
     P.d_bs_spec_f = dev_upload(pl, bsf, err);
+  }
+  for (size_t c = 0; c < pl->ring_cls.size(); ++c) {
+    pl->ring_cls[c].rings = dev_upload(pl, ring_cls_rings[2 * c], err);
+    pl->ring_cls[c].rings_n = dev_upload(pl, ring_cls_rings[2 * c + 1], err);
   }
   {
     std::vector<int> zero(1, 0);
@@ -440,7 +424,6 @@ int ps_plan_create(int nside, int lmax, int mmax, int spin_mask, int prec, ps_pl
     P.d_chirp_f = dev_upload(pl, chirp, err);
     P.d_chirp_off = dev_upload(pl, chirp_off, err);
   }
-  pl->d_ring_lists = dev_upload(pl, lists, err);
   if (prec == PS_PREC_FP64) {
     for (int s = 0; s < 4 && err == PS_OK; ++s) {
       if (s > 0 && !P.d_seed[s]) continue;
@@ -770,13 +753,8 @@ int ps_synthesis(const ps_plan* plan, const double* alm, double* map, int batch,
     else
       rc = ps::launch_legendre_synth_tc(P, almT, phase, batch, spin, P.d_err, stream);
     if (rc) return rc;
-    for (size_t c = 0; c < plan->cls_len.size(); ++c) {
-      rc = ps::launch_ring_synth_f32(P, plan->d_ring_lists + (spin ? plan->cls_off[c] : plan->cls_off_n[c]),
-                                     spin ? plan->cls_cnt[c] : plan->cls_cnt_n[c], plan->cls_len[c], phase, map, nf,
-                                     spin > 0, stream);
-      if (rc) return rc;
-    }
-    return PS_OK;
+    return ps::launch_ring_synth_f32(P, plan->ring_cls.data(), int(plan->ring_cls.size()), phase, map, nf, spin > 0,
+                                     stream);
   }
   double2* phase = reinterpret_cast<double2*>(phase_ptr);
   // between the two stages the phases are [R][batch][mmax+1][ncomp]
@@ -805,12 +783,9 @@ int ps_adjoint(const ps_plan* plan, const double* map, double* alm, int batch, i
     // FP32 ring transforms, FP64 recurrences with FP32 contractions, FP64 cross-tile sums
     float2* phase = reinterpret_cast<float2*>(ws);
     float2* partial = reinterpret_cast<float2*>(ws + phase_bytes);
-    for (size_t c = 0; c < plan->cls_len.size(); ++c) {
-      rc = ps::launch_ring_adjoint_f32(P, plan->d_ring_lists + (spin ? plan->cls_off[c] : plan->cls_off_n[c]),
-                                       spin ? plan->cls_cnt[c] : plan->cls_cnt_n[c], plan->cls_len[c], map, phase,
-                                       nf, spin > 0, stream);
-      if (rc) return rc;
-    }
+    rc = ps::launch_ring_adjoint_f32(P, plan->ring_cls.data(), int(plan->ring_cls.size()), map, phase, nf, spin > 0,
+                                     stream);
+    if (rc) return rc;
     TabRef tr;
     if (table_for(plan, spin, tr))
       return ps::launch_tab_adj(P, tr.tab, tr.off, tr.work, tr.nwork, tr.Rh_table, tr.toff, phase,
@@ -847,12 +822,7 @@ struct RoundtripView {
   const int64_t* off;
   const int2* work;
   int nwork;
-  const int* ring_lists;
-  const int* cls_len;
-  const int* cls_off;
-  const int* cls_cnt;
-  const int* cls_off_n;
-  const int* cls_cnt_n;
+  const RingClassList* cls;
   int ncls;
   int fmt;
 };
@@ -866,13 +836,8 @@ int roundtrip_view(const ps_plan* plan, int spin, RoundtripView& v) {
   v.off = tr.off;
   v.work = tr.work;
   v.nwork = tr.nwork;
-  v.ring_lists = plan->d_ring_lists;
-  v.cls_len = plan->cls_len.data();
-  v.cls_off = plan->cls_off.data();
-  v.cls_cnt = plan->cls_cnt.data();
-  v.cls_off_n = plan->cls_off_n.data();
-  v.cls_cnt_n = plan->cls_cnt_n.data();
-  v.ncls = int(plan->cls_len.size());
+  v.cls = plan->ring_cls.data();
+  v.ncls = int(plan->ring_cls.size());
   v.fmt = tr.fmt;
   return PS_OK;
 }

@@ -4,9 +4,8 @@
 // lscale an optional per-(component, lm) factor (the beam).  For a mixed-precision
 // plan holding the Legendre table of the spin this runs as: strided gather of the
 // input alm with the factor (layout [nalm][batch][ncomp]) -> table synthesis
-// (tensor cores) -> one ring kernel per FFT length class that synthesises each
-// ring in shared memory, weights its pixels and transforms it back (the maps
-// never reach HBM) -> table adjoint writing the strided output with the factor.
+// (tensor cores) -> one ring kernel that synthesises each ring in shared memory,
+// weights its pixels and transforms it back (the maps never reach HBM) -> table adjoint writing the strided output with the factor.
 // Without the table the entry returns PS_ERR_UNSUPPORTED and the caller composes
 // ps_synthesis, the weighting and ps_adjoint itself.
 #include <algorithm>
@@ -22,8 +21,8 @@ int launch_tab_synth(const Plan& P, const float* table, const int64_t* d_blockof
 int launch_tab_adj(const Plan& P, const float* table, const int64_t* d_blockoff, const int2* d_work, int nwork,
                    int Rh_table, int toff, const float2* phase, double2* alm, int B, int spin, double scale,
                    int64_t out_stride, const double* lscale, int* err_flag, cudaStream_t st, int fmt);
-int launch_ring_roundtrip_f32(const Plan& P, const int* d_list, int nrings, int work_len, float2* phase,
-                              const double* weight, int nf, int pack, cudaStream_t st);
+int launch_ring_roundtrip_f32(const Plan& P, const RingClassList* cls, int ncls, float2* phase, const double* weight,
+                              int nf, int pack, cudaStream_t st);
 
 namespace {
 // alm (B maps at stride `stride` complex elements, ncomp components of nalm each) times
@@ -54,12 +53,7 @@ struct RoundtripView {
   const int64_t* off;
   const int2* work;
   int nwork;
-  const int* ring_lists;
-  const int* cls_len;
-  const int* cls_off;
-  const int* cls_cnt;
-  const int* cls_off_n;
-  const int* cls_cnt_n;
+  const RingClassList* cls;
   int ncls;
   int fmt;
 };
@@ -109,12 +103,8 @@ extern "C" int ps_sht_weighted_roundtrip(const ps_plan* plan, const double* alm_
   }
   rc = ps::launch_tab_synth(P, v.tab, v.off, P.Rh, 0, almT, phase, batch, spin, P.d_err, stream, v.fmt);
   if (rc) return rc;
-  for (int c = 0; c < v.ncls; ++c) {
-    rc = ps::launch_ring_roundtrip_f32(P, v.ring_lists + (spin ? v.cls_off[c] : v.cls_off_n[c]),
-                                       spin ? v.cls_cnt[c] : v.cls_cnt_n[c], v.cls_len[c], phase, weight, nf,
-                                       spin > 0, stream);
-    if (rc) return rc;
-  }
+  rc = ps::launch_ring_roundtrip_f32(P, v.cls, v.ncls, phase, weight, nf, spin > 0, stream);
+  if (rc) return rc;
   return ps::launch_tab_adj(P, v.tab, v.off, v.work, v.nwork, P.Rh, 0, phase, reinterpret_cast<double2*>(alm_out),
                             batch, spin, scale, alm_stride, lscale, P.d_err, stream, v.fmt);
 }
