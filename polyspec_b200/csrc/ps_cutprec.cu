@@ -30,6 +30,8 @@
 struct ps_plan;
 
 namespace ps {
+int launch_alm_to_T(const double2* alm, int64_t stride, const double* lscale, double2* almT, int B, int ncomp,
+                    int64_t nalm, cudaStream_t st);
 int launch_tab_synth(const Plan& P, const float* table, const int64_t* d_blockoff, int Rh_table, int toff,
                      const double2* almT, float2* phase, int B, int spin, int* err_flag, cudaStream_t st, int fmt);
 int launch_tab_adj(const Plan& P, const float* table, const int64_t* d_blockoff, const int2* d_work, int nwork,
@@ -303,19 +305,6 @@ __global__ void __launch_bounds__(CUT_THREADS, 1) cut_gemm(const uint16_t* __res
   if (warp == 0) tc::tmem_dealloc(tmem, tmem_cols);
 }
 
-// B s -> almT [nalm][B][ncomp] for components c0 .. c0 + ncomp of x [B][3][nalm]
-__global__ void cut_gather(const double2* __restrict__ x, const double* __restrict__ beam, int c0, int ncomp,
-                           double2* __restrict__ almT, int B, int64_t nalm) {
-  const int64_t total = nalm * B * ncomp;
-  for (int64_t t = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; t < total; t += int64_t(gridDim.x) * blockDim.x) {
-    const int c = int(t % ncomp);
-    const int b = int((t / ncomp) % B);
-    const int64_t idx = t / (int64_t(ncomp) * B);
-    const double2 v = x[(int64_t(b) * 3 + c0 + c) * nalm + idx];
-    almT[t] = cscale(v, beam[int64_t(c0 + c) * nalm + idx]);
-  }
-}
-
 // out[b][a][i] += Sum_c Sigma[a][c][i] a[b][c][i], with the imaginary part of the sum dropped at m = 0
 // (alm index i <= lmax)
 __global__ void cut_finish(const double* __restrict__ S, const double2* __restrict__ a, double2* __restrict__ out,
@@ -478,11 +467,9 @@ extern "C" int ps_cutprec_apply(const ps_cutprec* c, const double* r, double* ou
   for (int spin = 0; spin <= 2; spin += 2) {
     const int nc = spin ? 2 : 1;
     const BandView& v = spin ? v2 : v0;
-    {
-      StatScope sc(PS_K_LAYOUT, 0.0, 40.0 * double(nalm) * batch * nc, stream);
-      cut_gather<<<cut_grid(nalm * batch * nc), 256, 0, stream>>>(o, c->beam, spin ? 1 : 0, nc, almT, batch, nalm);
-      PS_LAUNCH_CHECK();
-    }
+    const int c0 = spin ? 1 : 0;
+    rc = launch_alm_to_T(o + c0 * nalm, 3 * nalm, c->beam + c0 * nalm, almT, batch, nc, nalm, stream);
+    if (rc != PS_OK) return rc;
     rc = launch_tab_synth(*v.P, v.tab, v.off, v.Rh_table, v.toff, almT, spin ? ph2 : ph0, batch, spin, err, stream,
                           v.fmt);
     if (rc != PS_OK) return rc;

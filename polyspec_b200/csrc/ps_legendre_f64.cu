@@ -614,20 +614,6 @@ __global__ void __launch_bounds__(32 * NW) adjS_f64(const RingInfo* __restrict__
   }
 }
 
-// =====================================================================
-// layout kernels
-// alm [B][ncomp][nalm] -> almT [nalm][B][ncomp]
-__global__ void alm_to_T(const double2* __restrict__ alm, double2* __restrict__ almT, int B, int ncomp,
-                         int64_t nalm) {
-  const int64_t n = nalm * B * ncomp;
-  for (int64_t t = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; t < n; t += int64_t(gridDim.x) * blockDim.x) {
-    const int c = int(t % ncomp);
-    const int b = int((t / ncomp) % B);
-    const int64_t idx = t / (int64_t(ncomp) * B);
-    almT[t] = alm[(int64_t(b) * ncomp + c) * nalm + idx];
-  }
-}
-
 // ---------------------------------------------------------------- launchers
 // algorithmic Legendre work of one transform: 4 Rh nalm flops per spin-0 map,
 // 16 Rh nalm per spin-s (G, C) pair; bytes: alm in + per-ring phases out
@@ -742,16 +728,6 @@ int launch_legendre_adjoint_f64(const Plan& P, const double2* phase, int64_t ms,
     else if (P.Rh > 64) adjS_go<2, 4>(P, phase, ms, bs, alm, B, spin, scale, st);
     else adjS_go<1, 2>(P, phase, ms, bs, alm, B, spin, scale, st);
   }
-  PS_LAUNCH_CHECK();
-  return PS_OK;
-}
-
-int launch_alm_to_T(const double2* alm, double2* almT, int B, int ncomp, int64_t nalm, int sms, cudaStream_t st) {
-  const int64_t n = nalm * B * ncomp;
-  int blocks = (int)std::min<int64_t>((n + 255) / 256, int64_t(sms) * 8);
-  if (blocks < 1) blocks = 1;
-  StatScope sc(PS_K_LAYOUT, 0.0, 32.0 * n, st);
-  alm_to_T<<<blocks, 256, 0, st>>>(alm, almT, B, ncomp, nalm);
   PS_LAUNCH_CHECK();
   return PS_OK;
 }

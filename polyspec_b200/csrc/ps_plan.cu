@@ -19,7 +19,8 @@ int launch_legendre_synth_f64(const Plan& P, const double2* alm, double2* phase,
                               int spin, cudaStream_t st);
 int launch_legendre_adjoint_f64(const Plan& P, const double2* phase, int64_t ms, int64_t bs, double2* alm, int B,
                                 int spin, double scale, cudaStream_t st);
-int launch_alm_to_T(const double2* alm, double2* almT, int B, int ncomp, int64_t nalm, int sms, cudaStream_t st);
+int launch_alm_to_T(const double2* alm, int64_t stride, const double* lscale, double2* almT, int B, int ncomp,
+                    int64_t nalm, cudaStream_t st);
 int launch_ring_synth_f64(const Plan& P, const RingClassList* cls, int ncls, const double2* phase, double* map, int nf,
                           int pack, cudaStream_t st);
 int launch_ring_adjoint_f64(const Plan& P, const RingClassList* cls, int ncls, const double* map, double2* phase,
@@ -661,7 +662,8 @@ int ps_legendre_synthesis(const ps_plan* plan, const double* alm, double* phase,
   const int ncomp = spin == 0 ? 1 : 2;
   if (P.prec == PS_PREC_MIXED) {
     double2* almT = static_cast<double2*>(workspace);
-    int rc = ps::launch_alm_to_T(reinterpret_cast<const double2*>(alm), almT, batch, ncomp, P.nalm, P.num_sms, stream);
+    int rc = ps::launch_alm_to_T(reinterpret_cast<const double2*>(alm), int64_t(ncomp) * P.nalm, nullptr, almT, batch, ncomp,
+                                 P.nalm, stream);
     if (rc) return rc;
     float2* ph32 = reinterpret_cast<float2*>(static_cast<char*>(workspace) +
                                              align256(size_t(P.nalm) * batch * ncomp * sizeof(double2)));
@@ -741,7 +743,8 @@ int ps_synthesis(const ps_plan* plan, const double* alm, double* map, int batch,
     if (nf == 1) {
       almT = reinterpret_cast<double2*>(const_cast<double*>(alm));
     } else {
-      rc = ps::launch_alm_to_T(reinterpret_cast<const double2*>(alm), almT, batch, ncomp, P.nalm, P.num_sms, stream);
+      rc = ps::launch_alm_to_T(reinterpret_cast<const double2*>(alm), int64_t(ncomp) * P.nalm, nullptr, almT, batch, ncomp,
+                                 P.nalm, stream);
       if (rc) return rc;
     }
     // tensor-core Legendre stage (TF32 x3, FP32 accumulation) and FP32 ring transforms

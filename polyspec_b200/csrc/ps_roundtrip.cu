@@ -16,6 +16,8 @@
 struct ps_plan;
 
 namespace ps {
+int launch_alm_to_T(const double2* alm, int64_t stride, const double* lscale, double2* almT, int B, int ncomp,
+                    int64_t nalm, cudaStream_t st);
 int launch_tab_synth(const Plan& P, const float* table, const int64_t* d_blockoff, int Rh_table, int toff,
                      const double2* almT, float2* phase, int B, int spin, int* err_flag, cudaStream_t st, int fmt);
 int launch_tab_adj(const Plan& P, const float* table, const int64_t* d_blockoff, const int2* d_work, int nwork,
@@ -25,24 +27,6 @@ int launch_ring_roundtrip_f32(const Plan& P, const RingClassList* cls, int ncls,
                               int nf, int pack, cudaStream_t st);
 
 namespace {
-// alm (B maps at stride `stride` complex elements, ncomp components of nalm each) times
-// lscale[comp][idx] (when given) -> almT [nalm][B][ncomp]
-__global__ void alm_gather_scaled(const double2* __restrict__ alm, int64_t stride, const double* __restrict__ lscale,
-                                  double2* __restrict__ almT, int B, int ncomp, int64_t nalm) {
-  const int64_t n = nalm * B * ncomp;
-  for (int64_t t = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; t < n; t += int64_t(gridDim.x) * blockDim.x) {
-    const int c = int(t % ncomp);
-    const int b = int((t / ncomp) % B);
-    const int64_t idx = t / (int64_t(ncomp) * B);
-    double2 v = alm[int64_t(b) * stride + int64_t(c) * nalm + idx];
-    if (lscale) {
-      const double f = lscale[int64_t(c) * nalm + idx];
-      v.x *= f;
-      v.y *= f;
-    }
-    almT[t] = v;
-  }
-}
 size_t al256(size_t x) { return (x + 255) & ~size_t(255); }
 }  // namespace
 
@@ -92,15 +76,9 @@ extern "C" int ps_sht_weighted_roundtrip(const ps_plan* plan, const double* alm_
   char* ws = static_cast<char*>(workspace);
   double2* almT = reinterpret_cast<double2*>(ws);
   float2* phase = reinterpret_cast<float2*>(ws + ps::al256(size_t(P.nalm) * nf * sizeof(double2)));
-  {
-    const int64_t n = P.nalm * int64_t(nf);
-    int blocks = int(std::min<int64_t>((n + 255) / 256, int64_t(P.num_sms) * 8));
-    if (blocks < 1) blocks = 1;
-    ps::StatScope sc(PS_K_LAYOUT, 0.0, 32.0 * n, stream);
-    ps::alm_gather_scaled<<<blocks, 256, 0, stream>>>(reinterpret_cast<const double2*>(alm_in), alm_stride, lscale,
-                                                      almT, batch, ncomp, P.nalm);
-    PS_LAUNCH_CHECK();
-  }
+  rc = ps::launch_alm_to_T(reinterpret_cast<const double2*>(alm_in), alm_stride, lscale, almT, batch, ncomp, P.nalm,
+                           stream);
+  if (rc) return rc;
   rc = ps::launch_tab_synth(P, v.tab, v.off, P.Rh, 0, almT, phase, batch, spin, P.d_err, stream, v.fmt);
   if (rc) return rc;
   rc = ps::launch_ring_roundtrip_f32(P, v.cls, v.ncls, phase, weight, nf, spin > 0, stream);
