@@ -117,6 +117,16 @@ int ps_synthesis(const ps_plan* plan, const double* alm, double* map, int batch,
 int ps_adjoint(const ps_plan* plan, const double* map, double* alm, int batch, int spin, double scale,
                void* workspace, size_t workspace_bytes, cudaStream_t stream);
 
+/* ps_synthesis / ps_adjoint on maps and alm that do not lie back to back: alm of map b at alm + b alm_stride
+ * (complex elements, at least ncomp nalm), its pixels at map + b map_stride (float64 elements, at least ncomp npix),
+ * components contiguous; a stride of 0 is the smallest.  With them the T and the (E, B) or (Q, U) parts of
+ * [batch][3][..] arrays are transformed in place of copies (polyspec/base.py:147-176). */
+int ps_synthesis_strided(const ps_plan* plan, const double* alm, int64_t alm_stride, double* map, int64_t map_stride,
+                         int batch, int spin, void* workspace, size_t workspace_bytes, cudaStream_t stream);
+int ps_adjoint_strided(const ps_plan* plan, const double* map, int64_t map_stride, double* alm, int64_t alm_stride,
+                       int batch, int spin, double scale, void* workspace, size_t workspace_bytes,
+                       cudaStream_t stream);
+
 /* Fused weighted round trip of the masked CG operator (no single reference call;
  * replaces, per spin, the pair to_map -> pixel weight -> to_lm inside
  * CGD._apply_A at polyspec/weighting.py:297-299):

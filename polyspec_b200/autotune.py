@@ -65,6 +65,7 @@ class Tuner:
         # tune separately
         self.prefix = "%s|kernels2|nside%d|lmax%d|%s" % (gpu, nside, lmax, "+".join(sorted(self.handles)))
         self.choices = {}
+        self.keys = {}
         self.disk = _load()
 
     @staticmethod
@@ -83,8 +84,12 @@ class Tuner:
         """Handle to run the transform with (its tile already set); `run(handle)` issues it.
         With `table` the mixed plan streams its Legendre table (ps_plan_build_table): its
         on-the-fly tile shapes do not apply, and the choice is cached under its own key."""
-        key = "%s|%s|spin%d|b%d%s" % (self.prefix, ("synthesis", "adjoint")[direction], spin, self.bucket(B),
-                                      "|tab" if table else "")
+        call = (direction, spin, self.bucket(B), table)
+        key = self.keys.get(call)
+        if key is None:
+            key = "%s|%s|spin%d|b%d%s" % (self.prefix, ("synthesis", "adjoint")[direction], spin, self.bucket(B),
+                                          "|tab" if table else "")
+            self.keys[call] = key
         choice = self.choices.get(key) or self.disk.get(key)
         if choice is None or choice.get("pipeline") not in self.handles:
             times = {}

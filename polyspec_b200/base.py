@@ -205,9 +205,7 @@ class PolySpec:
         B, nf = alm.shape[0], alm.shape[1]
         self.n_SHTs_reverse += B * (1 + (nf == 3))
         out = torch.empty((B, nf, self.Npix), dtype=torch.float64, device=self.device)
-        out[:, 0] = P.synthesis(alm[:, 0].contiguous(), 0)
-        if nf == 3:
-            out[:, 1:] = P.synthesis(alm[:, 1:].contiguous(), 2)
+        P.synthesis_fields(alm, out)
         return out
 
     def to_lm_batch(self, maps, lmax=None):
@@ -218,9 +216,7 @@ class PolySpec:
         self.n_SHTs_forward += B * (1 + (nf == 3))
         scale = np.pi / (3. * self.Nside ** 2)
         out = torch.empty((B, nf, P.nalm), dtype=torch.complex128, device=self.device)
-        out[:, 0] = P.adjoint(maps[:, 0].contiguous(), 0, scale)
-        if nf == 3:
-            out[:, 1:] = P.adjoint(maps[:, 1:].contiguous(), 2, scale)
+        P.adjoint_fields(maps, out, scale)
         return out
 
     # ------------------------------------------------------------------ SHT wrappers
@@ -237,8 +233,7 @@ class PolySpec:
         scale = np.pi / (3. * self.Nside ** 2)
         if len(m) == 3:
             out = torch.empty((3, P.nalm), dtype=torch.complex128, device=self.device)
-            out[0] = P.adjoint(m[0:1], 0, scale)[0]
-            out[1:] = P.adjoint(m[1:3].reshape(1, 2, -1), 2, scale)[0]
+            P.adjoint_fields(m.unsqueeze(0), out, scale)
         else:
             out = P.adjoint(m.reshape(1, -1), 0, scale)
         return self._out(out, as_torch)
@@ -255,8 +250,7 @@ class PolySpec:
         P = self.plan(lmax)
         if len(a) == 3:
             out = torch.empty((3, self.Npix), dtype=torch.float64, device=self.device)
-            out[0] = P.synthesis(a[0:1], 0)[0]
-            out[1:] = P.synthesis(a[1:3].reshape(1, 2, -1), 2)[0]
+            P.synthesis_fields(a.unsqueeze(0), out)
         else:
             out = P.synthesis(a.reshape(1, -1), 0)
         return self._out(out, as_torch)

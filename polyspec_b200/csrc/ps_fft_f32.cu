@@ -258,7 +258,7 @@ struct RingClassF {
 constexpr int RING_CLASSES_F = 28, RING_NT = 512;
 struct RingLaunchF {
   int n, units, pack, mmax, R;
-  int64_t nf, npix;
+  int64_t nf, npix, map_stride;  // map_stride: from one map to the next
   const RingInfo* rings;
   const float2 *tw, *spec, *rot, *chirp;
   const int64_t *spec_off, *chirp_off;
@@ -271,8 +271,7 @@ struct RingItemF {
   bool va, vb;
   const float2* rot;
   const float2 *chirp, *spec;
-  int64_t pa, pb, start_a, start_b;  // first phases; first pixels in map fa, fb
-  int fa, fb;
+  int64_t pa, pb, pix_a, pix_b, start_a, start_b;  // first phases; first pixels of the two rows, and in their maps
 };
 struct RingCtaF {  // what the transforms of a CTA share
   int M, logM, logT, T, G, item0, count, blue;
@@ -304,12 +303,12 @@ __device__ __forceinline__ RingItemF ring_item_f(const RingLaunchF& L, const Rin
   it.N = g.nphi;
   it.start_a = g.start;
   it.start_b = L.rings[irb].start;
-  it.fa = L.pack ? 2 * unit : unit;
-  it.fb = L.pack ? it.fa + 1 : unit;
-  it.vb = it.va && (L.pack ? it.fb < L.nf : irb != ira);
+  it.pix_a = unit * L.map_stride + it.start_a;
+  it.pix_b = unit * L.map_stride + (L.pack ? L.npix : 0) + it.start_b;
+  it.vb = it.va && (L.pack || irb != ira);
   const int64_t row = int64_t(L.mmax + 1) * L.nf;
-  it.pa = ira * row + it.fa;
-  it.pb = irb * row + it.fb;
+  it.pa = ira * row + (L.pack ? 2 * unit : unit);
+  it.pb = irb * row + (L.pack ? 2 * unit + 1 : unit);
   it.rot = L.rot + int64_t(min(ira, L.R - 1 - ira)) * (L.mmax + 1);  // e^{i m phi0} of this ring
   it.chirp = c.blue ? L.chirp + L.chirp_off[g.bs_slot] : nullptr;
   it.spec = c.blue ? L.spec + L.spec_off[g.bs_slot] : nullptr;
@@ -390,7 +389,7 @@ __device__ __forceinline__ float2 dechirp(float2 y, const float2* __restrict__ c
   return make_float2(v.x * s, v.y * s);
 }
 
-// synthesis: phase [R][mmax+1][nf] (complex64) -> map [nf][npix] (float64)
+// synthesis: phase [R][mmax+1][nf] (complex64) -> maps (float64)
 __global__ void __launch_bounds__(RING_NT, 2) ring_synth_f32(const __grid_constant__ RingLaunchF L,
                                                              const float2* __restrict__ phase,
                                                              double* __restrict__ map) {
@@ -401,8 +400,8 @@ __global__ void __launch_bounds__(RING_NT, 2) ring_synth_f32(const __grid_consta
   const int grp = threadIdx.x >> c.logT, u = threadIdx.x & (c.T - 1);
   const RingItemF it = ring_item_f(L, c, grp);
   float2* a = fbuf + grp * ring_smem_f(c);
-  double* oa = map + int64_t(it.fa) * L.npix + it.start_a;
-  double* ob = map + int64_t(it.fb) * L.npix + it.start_b;
+  double* oa = map + it.pix_a;
+  double* ob = map + it.pix_b;
   const float inv = 1.0f / float(c.M);
   auto out = [&](int j, float2 y) {
     if (c.blue) y = dechirp(y, it.chirp, j, inv);
@@ -432,7 +431,7 @@ struct MapIn {
   }
 };
 
-// adjoint: map [nf][npix] (float64) -> phase [R][mmax+1][nf] (complex64)
+// adjoint: maps (float64) -> phase [R][mmax+1][nf] (complex64)
 __global__ void __launch_bounds__(RING_NT, 2) ring_adjoint_f32(const __grid_constant__ RingLaunchF L,
                                                                const double* __restrict__ map,
                                                                float2* __restrict__ phase) {
@@ -441,7 +440,7 @@ __global__ void __launch_bounds__(RING_NT, 2) ring_adjoint_f32(const __grid_cons
   const int grp = threadIdx.x >> c.logT, u = threadIdx.x & (c.T - 1);
   const RingItemF it = ring_item_f(L, c, grp);
   float2* a = fbuf + grp * ring_smem_f(c);
-  const MapIn in{map + int64_t(it.fa) * L.npix + it.start_a, map + int64_t(it.fb) * L.npix + it.start_b,
+  const MapIn in{map + it.pix_a, map + it.pix_b,
                  it.chirp, it.N, it.va, it.vb, c.blue != 0};
   const float inv = 1.0f / float(c.M);
   auto out = [&](int k, float2 y) { a[fpad(k)] = c.blue ? dechirp(y, it.chirp, k, inv) : y; };
@@ -488,10 +487,11 @@ __global__ void __launch_bounds__(RING_NT, 2) ring_roundtrip_f32(const __grid_co
 
 // ------------------------------------------------------------------ launch
 template <class Launch>
-static int ring_launches_f(const Plan& P, const RingClassList* cls, int ncls, int nf, int pack, Launch go) {
+static int ring_launches_f(const Plan& P, const RingClassList* cls, int ncls, int64_t map_stride, int nf, int pack,
+                           Launch go) {
   RingLaunchF L;
   L.units = pack ? (nf + 1) / 2 : nf;
-  L.pack = pack; L.nf = nf; L.mmax = P.mmax; L.R = P.R; L.npix = P.npix; L.rings = P.d_rings;
+  L.pack = pack; L.nf = nf; L.mmax = P.mmax; L.R = P.R; L.npix = P.npix; L.map_stride = map_stride; L.rings = P.d_rings;
   L.tw = P.d_twiddle_f; L.spec = P.d_bs_spec_f; L.spec_off = P.d_bs_off;
   L.rot = P.d_rot_f; L.chirp = P.d_chirp_f; L.chirp_off = P.d_chirp_off;
   for (int big = 1; big >= 0; --big) {  // work length 16384 first, then all others, longest first
@@ -532,39 +532,42 @@ static bool ring_smem_ok(K kern, size_t smem) {
          cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess;
 }
 
-int launch_ring_synth_f32(const Plan& P, const RingClassList* cls, int ncls, const float2* phase, double* map, int nf,
-                          int pack, cudaStream_t st) {
-  return ring_launches_f(P, cls, ncls, nf, pack, [&](const RingLaunchF& L, int ctas, size_t smem, double) -> int {
+int launch_ring_synth_f32(const Plan& P, const RingClassList* cls, int ncls, const float2* phase, double* map,
+                          int64_t map_stride, int nf, int pack, cudaStream_t st) {
+  auto go = [&](const RingLaunchF& L, int ctas, size_t smem, double) -> int {
     if (!ring_smem_ok(ring_synth_f32, smem)) return PS_ERR_CUDA;
     StatScope sc(PS_K_FFT_SYNTH, 0.0, 0.0, st);
     ring_synth_f32<<<ctas, RING_NT, smem, st>>>(L, phase, map);
     PS_LAUNCH_CHECK();
     return PS_OK;
-  });
+  };
+  return ring_launches_f(P, cls, ncls, map_stride, nf, pack, go);
 }
 
-int launch_ring_adjoint_f32(const Plan& P, const RingClassList* cls, int ncls, const double* map, float2* phase,
-                            int nf, int pack, cudaStream_t st) {
-  return ring_launches_f(P, cls, ncls, nf, pack, [&](const RingLaunchF& L, int ctas, size_t smem, double) -> int {
+int launch_ring_adjoint_f32(const Plan& P, const RingClassList* cls, int ncls, const double* map,
+                            int64_t map_stride, float2* phase, int nf, int pack, cudaStream_t st) {
+  auto go = [&](const RingLaunchF& L, int ctas, size_t smem, double) -> int {
     if (!ring_smem_ok(ring_adjoint_f32, smem)) return PS_ERR_CUDA;
     StatScope sc(PS_K_FFT_ADJOINT, 0.0, 0.0, st);
     ring_adjoint_f32<<<ctas, RING_NT, smem, st>>>(L, map, phase);
     PS_LAUNCH_CHECK();
     return PS_OK;
-  });
+  };
+  return ring_launches_f(P, cls, ncls, map_stride, nf, pack, go);
 }
 
 int launch_ring_roundtrip_f32(const Plan& P, const RingClassList* cls, int ncls, float2* phase, const double* weight,
                               int nf, int pack, cudaStream_t st) {
   // the pixel weights and the phases, read and written once
   const double bytes = double(P.npix) * 8.0 * (pack ? 2.0 : 1.0) + 2.0 * 8.0 * P.R * (P.mmax + 1) * nf;
-  return ring_launches_f(P, cls, ncls, nf, pack, [&](const RingLaunchF& L, int ctas, size_t smem, double share) -> int {
+  auto go = [&](const RingLaunchF& L, int ctas, size_t smem, double share) -> int {
     if (!ring_smem_ok(ring_roundtrip_f32, smem)) return PS_ERR_CUDA;
     StatScope sc(PS_K_FFT_SYNTH, 0.0, bytes * share, st);
     ring_roundtrip_f32<<<ctas, RING_NT, smem, st>>>(L, weight, phase);
     PS_LAUNCH_CHECK();
     return PS_OK;
-  });
+  };
+  return ring_launches_f(P, cls, ncls, 0, nf, pack, go);
 }
 
 }  // namespace ps

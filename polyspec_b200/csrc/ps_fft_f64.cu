@@ -188,7 +188,8 @@ __device__ __forceinline__ void pass_dit8(double2* a, int M, int logq, const dou
   }
 }
 
-// Bluestein convolution: in.load<H>(x, t, q) gives the inputs at t + k q, k < H, already times the chirp and zero from N
+// Bluestein convolution: in.load<H>(x, t, q) gives the inputs at t + k q, k < H, already times the chirp and zero
+// from N
 // on; out(j, v), j < N <= M/2, takes M times the convolution, to be multiplied by the chirp / M.  M = R1 8^n, n >= 1;
 // spec is the kernel's spectrum as the middle pass reads it, [8][M/8].
 template <int R1, class In, class Out>
@@ -332,7 +333,7 @@ constexpr int RING_CLASSES = 28;
 struct RingLaunch {
   int n, units, pack, mmax, R;
   int64_t nf;
-  int64_t npix;
+  int64_t npix, map_stride;  // pixels; from one map to the next
   const RingInfo* rings;
   const double2 *tw, *spec, *root, *chirp;
   const int64_t *spec_off, *chirp_off;
@@ -345,7 +346,7 @@ struct RingItem {
   bool blue, va, vb, turned;  // turned: phi0 = pi / N
   const double2 *root, *chirp, *spec;
   int ira, irb;
-  int64_t start_a, start_b;
+  int64_t pix_a, pix_b;  // first pixels of the two rows
   double2* a;
 };
 __device__ __forceinline__ RingItem ring_item(const RingLaunch& L, double2* smem) {
@@ -366,8 +367,8 @@ __device__ __forceinline__ RingItem ring_item(const RingLaunch& L, double2* smem
   it.irb = L.pack ? it.ira : L.R - 1 - it.ira;
   const RingInfo g = L.rings[it.ira];
   it.N = g.nphi;
-  it.start_a = g.start;
-  it.start_b = L.rings[it.irb].start;
+  it.pix_a = unit * L.map_stride + g.start;
+  it.pix_b = unit * L.map_stride + (L.pack ? L.npix : 0) + L.rings[it.irb].start;
   it.turned = g.phi_num != 0;
   it.fa = L.pack ? 2 * unit : unit;
   it.fb = L.pack ? it.fa + 1 : unit;
@@ -458,7 +459,7 @@ struct SynthIn {
       }
     };
 
-// synthesis: phase -> map [nf][npix]
+// synthesis: phase -> maps
 template <int NT>
 __global__ void __launch_bounds__(NT, 512 / NT) ring_synth_f64(const __grid_constant__ RingLaunch L,
                                                                const double2* __restrict__ phase,
@@ -478,8 +479,8 @@ __global__ void __launch_bounds__(NT, 512 / NT) ring_synth_f64(const __grid_cons
   in.va = it.va;
   in.vb = it.vb;
   in.blue = it.blue;
-  double* oa = map + int64_t(it.fa) * L.npix + it.start_a;
-  double* ob = map + int64_t(it.fb) * L.npix + it.start_b;
+  double* oa = map + it.pix_a;
+  double* ob = map + it.pix_b;
   const double inv = 1.0 / double(it.M);
   auto out = [&](int j, double2 y) {
     if (it.blue) y = cscale(cmul(y, __ldg(&it.chirp[j])), inv);
@@ -538,7 +539,7 @@ struct AdjointIn {
   }
 };
 
-// adjoint: map [nf][npix] -> phase
+// adjoint: maps -> phase
 template <int NT>
 __global__ void __launch_bounds__(NT, 512 / NT) ring_adjoint_f64(const __grid_constant__ RingLaunch L,
                                                                  const double* __restrict__ map,
@@ -546,7 +547,7 @@ __global__ void __launch_bounds__(NT, 512 / NT) ring_adjoint_f64(const __grid_co
   extern __shared__ double2 smem[];
   const RingItem it = ring_item(L, smem);
   const int N = it.N, mmax = L.mmax, T = it.T, u = it.u;
-  const AdjointIn in{map + int64_t(it.fa) * L.npix + it.start_a, map + int64_t(it.fb) * L.npix + it.start_b,
+  const AdjointIn in{map + it.pix_a, map + it.pix_b,
                      it.chirp, N, it.va, it.vb, it.blue};
   const double inv = 1.0 / double(it.M);
   auto out = [&](int k, double2 y) {
@@ -586,10 +587,11 @@ static int ring_logT(int logM, int mmax, int nt) {
 }
 
 template <class Launch>
-static int ring_launches(const Plan& P, const RingClassList* cls, int ncls, int nf, int pack, Launch go) {
+static int ring_launches(const Plan& P, const RingClassList* cls, int ncls, int64_t map_stride, int nf, int pack,
+                         Launch go) {
   RingLaunch L;
   L.units = pack ? (nf + 1) / 2 : nf;
-  L.pack = pack; L.nf = nf; L.mmax = P.mmax; L.R = P.R; L.npix = P.npix; L.rings = P.d_rings;
+  L.pack = pack; L.nf = nf; L.mmax = P.mmax; L.R = P.R; L.npix = P.npix; L.map_stride = map_stride; L.rings = P.d_rings;
   L.tw = P.d_twiddle; L.spec = P.d_bs_spec; L.spec_off = P.d_bs_off;
   L.root = P.d_root; L.chirp = P.d_chirp; L.chirp_off = P.d_chirp_off;
   for (int big = 1; big >= 0; --big) {  // work length 8192 first, then all others, longest first
@@ -623,9 +625,9 @@ static int ring_launches(const Plan& P, const RingClassList* cls, int ncls, int 
   return PS_OK;
 }
 
-int launch_ring_synth_f64(const Plan& P, const RingClassList* cls, int ncls, const double2* phase, double* map, int nf,
-                          int pack, cudaStream_t st) {
-  return ring_launches(P, cls, ncls, nf, pack, [&](const RingLaunch& L, int nt, int ctas, size_t smem) -> int {
+int launch_ring_synth_f64(const Plan& P, const RingClassList* cls, int ncls, const double2* phase, double* map,
+                          int64_t map_stride, int nf, int pack, cudaStream_t st) {
+  auto go = [&](const RingLaunch& L, int nt, int ctas, size_t smem) -> int {
     const auto kern = nt == 512 ? ring_synth_f64<512> : ring_synth_f64<256>;
     if (smem > 48 * 1024 &&
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
@@ -634,12 +636,13 @@ int launch_ring_synth_f64(const Plan& P, const RingClassList* cls, int ncls, con
     kern<<<ctas, nt, smem, st>>>(L, phase, map);
     PS_LAUNCH_CHECK();
     return PS_OK;
-  });
+  };
+  return ring_launches(P, cls, ncls, map_stride, nf, pack, go);
 }
 
-int launch_ring_adjoint_f64(const Plan& P, const RingClassList* cls, int ncls, const double* map, double2* phase,
-                            int nf, int pack, cudaStream_t st) {
-  return ring_launches(P, cls, ncls, nf, pack, [&](const RingLaunch& L, int nt, int ctas, size_t smem) -> int {
+int launch_ring_adjoint_f64(const Plan& P, const RingClassList* cls, int ncls, const double* map,
+                            int64_t map_stride, double2* phase, int nf, int pack, cudaStream_t st) {
+  auto go = [&](const RingLaunch& L, int nt, int ctas, size_t smem) -> int {
     const auto kern = nt == 512 ? ring_adjoint_f64<512> : ring_adjoint_f64<256>;
     if (smem > 48 * 1024 &&
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
@@ -648,7 +651,8 @@ int launch_ring_adjoint_f64(const Plan& P, const RingClassList* cls, int ncls, c
     kern<<<ctas, nt, smem, st>>>(L, map, phase);
     PS_LAUNCH_CHECK();
     return PS_OK;
-  });
+  };
+  return ring_launches(P, cls, ncls, map_stride, nf, pack, go);
 }
 
 }  // namespace ps

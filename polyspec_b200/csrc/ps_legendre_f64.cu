@@ -30,9 +30,9 @@
 // kept several to a thread so that one broadcast of c and the alm from shared
 // memory serves them all.
 //
-// Layouts: alm [B][ncomp][nalm] (m-major); phases ring-major, the value of order m and map b of a ring at
-// m ms + b bs (+ 1 for U): [R][B][mmax+1][ncomp] towards the ring transforms, [R][mmax+1][B][ncomp] in the calls of
-// the Legendre stage alone.
+// Layouts: alm [ncomp][nalm] (m-major) per map, `as` elements from one map to the next; phases ring-major, the value
+// of order m and map b of a ring at m ms + b bs (+ 1 for U): [R][B][mmax+1][ncomp] towards the ring transforms,
+// [R][mmax+1][B][ncomp] in the calls of the Legendre stage alone.
 #include <algorithm>
 #include <type_traits>
 
@@ -110,9 +110,9 @@ __global__ void __launch_bounds__(SYN_THREADS) synth0_f64(const RingInfo* __rest
                                                            const double* __restrict__ mnorm,
                                                            const double* __restrict__ lc,
                                                            const double* __restrict__ lg,
-                                                           const double2* __restrict__ alm,
+                                                           const double2* __restrict__ alm, int64_t as,
                                                            double2* __restrict__ phase, int64_t ms, int64_t bs,
-                                                           int R, int Rh, int lmax, int mmax, int B, int64_t nalm) {
+                                                           int R, int Rh, int lmax, int mmax, int B) {
   const int m = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, b = blockIdx.z;
   const int wbase = (blockIdx.x * SYN_THREADS + (tid & ~31)) * RPT, r0 = wbase + lane;
   if (wbase >= Rh) return;
@@ -129,7 +129,7 @@ __global__ void __launch_bounds__(SYN_THREADS) synth0_f64(const RingInfo* __rest
     const bool in = l0 + lane <= lmax;
     const double gm = in ? lg[idx] : 0.0;
     pc = l0 + lane < lmax ? lc[idx] : 0.0;
-    pa = in ? cscale(alm[int64_t(b) * nalm + idx], gm) : make_double2(0.0, 0.0);
+    pa = in ? cscale(alm[b * as + idx], gm) : make_double2(0.0, 0.0);
   };
   auto stage = [&](int buf) {  // registers -> shared memory; whether a value is not finite
     s_alm[buf][lane] = pa;
@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(SYN_THREADS) synthS_f64(const RingInfo* __rest
                                                            const SeedNorm* __restrict__ seednorm,
                                                            const double2* __restrict__ lcd,
                                                            const double* __restrict__ lg,
-                                                           const double2* __restrict__ alm,
+                                                           const double2* __restrict__ alm, int64_t as,
                                                            double2* __restrict__ phase, int64_t ms, int64_t bs,
                                                            int R, int Rh, int lmax, int mmax, int B, int64_t nalm,
                                                            int spin) {
@@ -238,8 +238,8 @@ __global__ void __launch_bounds__(SYN_THREADS) synthS_f64(const RingInfo* __rest
     const double gm = in ? lg[idx] : 0.0;
     pc = l0 + lane < lmax ? lcd[idx] : make_double2(0.0, 0.0);
     const double2 z = make_double2(0.0, 0.0);
-    const double2 G = in ? cscale(alm[int64_t(b) * 2 * nalm + idx], gm) : z;
-    const double2 C = in ? cscale(alm[(int64_t(b) * 2 + 1) * nalm + idx], gm) : z;
+    const double2 G = in ? cscale(alm[b * as + idx], gm) : z;
+    const double2 C = in ? cscale(alm[b * as + nalm + idx], gm) : z;
     pp = make_double2(G.x - C.y, G.y + C.x);
     pm = make_double2(G.x + C.y, G.y - C.x);
   };
@@ -269,7 +269,7 @@ __global__ void __launch_bounds__(SYN_THREADS) synthS_f64(const RingInfo* __rest
     double2 z = make_double2(0.0, 0.0);
     // alm with l < s do not enter, unless not finite (0 times them)
     for (int l = m; l < min(spin, lmax + 1); ++l)
-      for (int c = 0; c < 2; ++c) z = cfma(0.0, alm[(int64_t(b) * 2 + c) * nalm + base + (l - m)], z);
+      for (int c = 0; c < 2; ++c) z = cfma(0.0, alm[b * as + c * nalm + base + (l - m)], z);
 #pragma unroll
     for (int i = 0; i < RPT; ++i) PN[i] = MN[i] = PS[i] = MS[i] = z;
   }
@@ -368,15 +368,14 @@ template <int RPT, int NW>
 __global__ void __launch_bounds__(32 * NW) adj0_f64(const RingInfo* __restrict__ rings,
                                                     const double* __restrict__ mnorm, const double* __restrict__ lc,
                                                     const double* __restrict__ lg, const double2* __restrict__ phase,
-                                                    int64_t ms, int64_t bs, double2* __restrict__ alm, int R, int Rh,
-                                                    int lmax, int mmax, int B, int bofs, int64_t nalm,
-                                                    double scale) {
+                                                    int64_t ms, int64_t bs, double2* __restrict__ alm, int64_t as,
+                                                    int R, int Rh, int lmax, int mmax, int B, int bofs, double scale) {
   const int m = blockIdx.y, b = bofs + blockIdx.z, tid = threadIdx.x, nt = blockDim.x;
   const int warp = tid >> 5, lane = tid & 31, nw = nt >> 5;
   __shared__ double2 s_red[2][NW][ADJ_LCH];
   __shared__ double s_c[2][ADJ_LCH];
   const int64_t base = alm_index(m, m, lmax);
-  double2* out = alm + int64_t(b) * nalm + base;
+  double2* out = alm + b * as + base;
   const double mn = mnorm[m];
   const bool up16 = lane & 16;
   int buf = 0;
@@ -476,14 +475,15 @@ __global__ void __launch_bounds__(32 * NW) adjS_f64(const RingInfo* __restrict__
                                                     const SeedNorm* __restrict__ seednorm,
                                                     const double2* __restrict__ lcd, const double* __restrict__ lg,
                                                     const double2* __restrict__ phase, int64_t ms, int64_t bs,
-                                                    double2* __restrict__ alm, int R, int Rh, int lmax, int mmax,
+                                                    double2* __restrict__ alm, int64_t as, int R, int Rh, int lmax,
+                                                    int mmax,
                                                     int B, int bofs, int64_t nalm, int spin, double scale) {
   const int m = blockIdx.y, b = bofs + blockIdx.z, tid = threadIdx.x, nt = blockDim.x;
   const int warp = tid >> 5, lane = tid & 31, nw = nt >> 5;
   __shared__ double s_red[2][NW][4 * ADJ_LCH];
   __shared__ double2 s_cd[2][ADJ_LCH];
   const int64_t base = alm_index(m, m, lmax);
-  double2* outG = alm + int64_t(b) * 2 * nalm + base;
+  double2* outG = alm + b * as + base;
   double2* outC = outG + nalm;
   const int lmin = max(m, spin);
   const double sgn0 = ((lmin + m) & 1) ? -1.0 : 1.0;
@@ -625,10 +625,10 @@ static double leg_bytes(const Plan& P, int B, int spin) {
   return nf * 16.0 * (double(P.nalm) + double(P.R) * (P.mmax + 1));
 }
 
-int launch_synth_mma_f64(const Plan& P, const double2* alm, double2* phase, int64_t ms, int64_t bs, int B, int spin,
-                         cudaStream_t st);
-int launch_adjoint_mma_f64(const Plan& P, const double2* phase, int64_t ms, int64_t bs, double2* alm, int B, int spin,
-                           double scale, cudaStream_t st);
+int launch_synth_mma_f64(const Plan& P, const double2* alm, int64_t as, double2* phase, int64_t ms, int64_t bs, int B,
+                         int spin, cudaStream_t st);
+int launch_adjoint_mma_f64(const Plan& P, const double2* phase, int64_t ms, int64_t bs, double2* alm, int64_t as, int B,
+                           int spin, double scale, cudaStream_t st);
 
 int launch_leg_tables_f64(const Plan& P, int spin, double* cd, double* gam, cudaStream_t st) {
   leg_tables_f64<<<(P.mmax + 64) / 64, 64, 0, st>>>(P.lmax, P.mmax, spin, cd, gam);
@@ -639,18 +639,19 @@ int launch_leg_tables_f64(const Plan& P, int spin, double* cd, double* gam, cuda
 constexpr int MAX_GRID_Z = 65535;  // maps per launch
 
 template <int RPT>
-static void synth0_go(const Plan& P, const double2* alm, double2* phase, int64_t ms, int64_t bs, int B, cudaStream_t st) {
-  const dim3 grid((P.Rh + SYN_THREADS * RPT - 1) / (SYN_THREADS * RPT), P.mmax + 1, B);
-  synth0_f64<RPT><<<grid, SYN_THREADS, 0, st>>>(P.d_rings, P.d_mnorm0, P.d_leg_cd[0], P.d_leg_g[0], alm, phase, ms, bs,
-                                                P.R, P.Rh, P.lmax, P.mmax, B, P.nalm);
-}
-template <int RPT>
-static void synthS_go(const Plan& P, const double2* alm, double2* phase, int64_t ms, int64_t bs, int B, int spin,
+static void synth0_go(const Plan& P, const double2* alm, int64_t as, double2* phase, int64_t ms, int64_t bs, int B,
                       cudaStream_t st) {
   const dim3 grid((P.Rh + SYN_THREADS * RPT - 1) / (SYN_THREADS * RPT), P.mmax + 1, B);
+  synth0_f64<RPT><<<grid, SYN_THREADS, 0, st>>>(P.d_rings, P.d_mnorm0, P.d_leg_cd[0], P.d_leg_g[0], alm, as, phase,
+                                                ms, bs, P.R, P.Rh, P.lmax, P.mmax, B);
+}
+template <int RPT>
+static void synthS_go(const Plan& P, const double2* alm, int64_t as, double2* phase, int64_t ms, int64_t bs, int B,
+                      int spin, cudaStream_t st) {
+  const dim3 grid((P.Rh + SYN_THREADS * RPT - 1) / (SYN_THREADS * RPT), P.mmax + 1, B);
   synthS_f64<RPT><<<grid, SYN_THREADS, 0, st>>>(P.d_rings, P.d_seed[spin],
-                                                reinterpret_cast<const double2*>(P.d_leg_cd[spin]), P.d_leg_g[spin], alm,
-                                                phase, ms, bs, P.R, P.Rh, P.lmax, P.mmax, B, P.nalm, spin);
+                                                reinterpret_cast<const double2*>(P.d_leg_cd[spin]), P.d_leg_g[spin],
+                                                alm, as, phase, ms, bs, P.R, P.Rh, P.lmax, P.mmax, B, P.nalm, spin);
 }
 
 // Batches run on the FP64 MMA, which takes maps four (spin 0) or two (spin s) at a time; fewer maps than most of a
@@ -663,41 +664,41 @@ static void synthS_go(const Plan& P, const double2* alm, double2* phase, int64_t
 // in flight where a plan has few rings.  Measured, one map, spin 0, one / two / four rings: Nside 1024, lmax 2048
 // 1661 / 1417 / 1353 us, Nside 512, lmax 1000 212 / 187 / 184 us, Nside 256, lmax 767 70 / 71 / 81 us; spin 2 (whose
 // eight sums per ring fill the registers) 4165 / 3880 / 3842 us at Nside 1024.
-int launch_legendre_synth_f64(const Plan& P, const double2* alm, double2* phase, int64_t ms, int64_t bs, int B,
-                              int spin, cudaStream_t st) {
+int launch_legendre_synth_f64(const Plan& P, const double2* alm, int64_t as, double2* phase, int64_t ms, int64_t bs,
+                              int B, int spin, cudaStream_t st) {
   StatScope sc(PS_K_LEG_SYNTH, leg_flops(P, B, spin), leg_bytes(P, B, spin), st);
   if (spin > 0 && !P.d_seed[spin]) return PS_ERR_INVALID;
   const int t = P.tile[0][spin];
-  if (t ? t > 1 : B >= 3) return launch_synth_mma_f64(P, alm, phase, ms, bs, B, spin, st);
+  if (t ? t > 1 : B >= 3) return launch_synth_mma_f64(P, alm, as, phase, ms, bs, B, spin, st);
   if (spin == 0) {
-    if (P.Rh >= 1024) synth0_go<4>(P, alm, phase, ms, bs, B, st);
-    else if (P.Rh > 128) synth0_go<2>(P, alm, phase, ms, bs, B, st);
-    else synth0_go<1>(P, alm, phase, ms, bs, B, st);
+    if (P.Rh >= 1024) synth0_go<4>(P, alm, as, phase, ms, bs, B, st);
+    else if (P.Rh > 128) synth0_go<2>(P, alm, as, phase, ms, bs, B, st);
+    else synth0_go<1>(P, alm, as, phase, ms, bs, B, st);
   } else {
-    if (P.Rh > 128) synthS_go<2>(P, alm, phase, ms, bs, B, spin, st);
-    else synthS_go<1>(P, alm, phase, ms, bs, B, spin, st);
+    if (P.Rh > 128) synthS_go<2>(P, alm, as, phase, ms, bs, B, spin, st);
+    else synthS_go<1>(P, alm, as, phase, ms, bs, B, spin, st);
   }
   PS_LAUNCH_CHECK();
   return PS_OK;
 }
 
 template <int RPT, int NW>
-static void adj0_go(const Plan& P, const double2* phase, int64_t ms, int64_t bs, double2* alm, int B, double scale,
-                    cudaStream_t st) {
+static void adj0_go(const Plan& P, const double2* phase, int64_t ms, int64_t bs, double2* alm, int64_t as, int B,
+                    double scale, cudaStream_t st) {
   const int warps = std::min(NW, (P.Rh + 32 * RPT - 1) / (32 * RPT));
   for (int b0 = 0; b0 < B; b0 += MAX_GRID_Z)
     adj0_f64<RPT, NW><<<dim3(1, P.mmax + 1, std::min(MAX_GRID_Z, B - b0)), 32 * warps, 0, st>>>(
-        P.d_rings, P.d_mnorm0, P.d_leg_cd[0], P.d_leg_g[0], phase, ms, bs, alm, P.R, P.Rh, P.lmax, P.mmax, B, b0,
-        P.nalm, scale);
+        P.d_rings, P.d_mnorm0, P.d_leg_cd[0], P.d_leg_g[0], phase, ms, bs, alm, as, P.R, P.Rh, P.lmax, P.mmax, B, b0,
+        scale);
 }
 template <int RPT, int NW>
-static void adjS_go(const Plan& P, const double2* phase, int64_t ms, int64_t bs, double2* alm, int B, int spin,
-                    double scale, cudaStream_t st) {
+static void adjS_go(const Plan& P, const double2* phase, int64_t ms, int64_t bs, double2* alm, int64_t as, int B,
+                    int spin, double scale, cudaStream_t st) {
   const int warps = std::min(NW, (P.Rh + 32 * RPT - 1) / (32 * RPT));
   for (int b0 = 0; b0 < B; b0 += MAX_GRID_Z)
     adjS_f64<RPT, NW><<<dim3(1, P.mmax + 1, std::min(MAX_GRID_Z, B - b0)), 32 * warps, 0, st>>>(
         P.d_rings, P.d_seed[spin], reinterpret_cast<const double2*>(P.d_leg_cd[spin]), P.d_leg_g[spin], phase, ms, bs,
-        alm, P.R, P.Rh, P.lmax, P.mmax, B, b0, P.nalm, spin, scale);
+        alm, as, P.R, P.Rh, P.lmax, P.mmax, B, b0, P.nalm, spin, scale);
 }
 
 // Rings per thread and warps per CTA.  Four rings halve the share of the warp sums and are used wherever a
@@ -711,22 +712,24 @@ static void adjS_go(const Plan& P, const double2* phase, int64_t ms, int64_t bs,
 // maps 6002 / 2999; Nside 256, lmax 767, 2 maps 171 / 192, lmax 500, 3 maps 124 / 125.  Spin 2 (the sums of two
 // maps fill a tile): Nside 256, lmax 767, 2 maps 430 / 326, Nside 512, 24 maps 16359 / 9476; one map, half a tile,
 // 707 / 1054.  Tile 1 forces single maps of spin 0, tile 4 the MMA.
-int launch_legendre_adjoint_f64(const Plan& P, const double2* phase, int64_t ms, int64_t bs, double2* alm, int B,
-                                int spin, double scale, cudaStream_t st) {
+int launch_legendre_adjoint_f64(const Plan& P, const double2* phase, int64_t ms, int64_t bs, double2* alm, int64_t as,
+                                int B, int spin, double scale, cudaStream_t st) {
   StatScope sc(PS_K_LEG_ADJOINT, leg_flops(P, B, spin), leg_bytes(P, B, spin), st);
   if (spin > 0 && !P.d_seed[spin]) return PS_ERR_INVALID;
   const int t = P.tile[1][spin];
-  if (spin > 0 ? B >= 2 : t ? t > 1 : B >= 4) return launch_adjoint_mma_f64(P, phase, ms, bs, alm, B, spin, scale, st);
+  if (spin > 0 ? B >= 2 : t ? t > 1 : B >= 4)
+    return launch_adjoint_mma_f64(P, phase, ms, bs, alm, as, B, spin, scale, st);
   const int64_t ctas = int64_t(P.mmax + 1) * B;
   if (spin == 0) {
-    if (P.Rh > 256) ctas < 1500 ? adj0_go<4, 8>(P, phase, ms, bs, alm, B, scale, st) : adj0_go<4, 4>(P, phase, ms, bs, alm, B, scale, st);
-    else if (P.Rh > 64) adj0_go<2, 4>(P, phase, ms, bs, alm, B, scale, st);
-    else adj0_go<1, 2>(P, phase, ms, bs, alm, B, scale, st);
+    if (P.Rh > 256 && ctas < 1500) adj0_go<4, 8>(P, phase, ms, bs, alm, as, B, scale, st);
+    else if (P.Rh > 256) adj0_go<4, 4>(P, phase, ms, bs, alm, as, B, scale, st);
+    else if (P.Rh > 64) adj0_go<2, 4>(P, phase, ms, bs, alm, as, B, scale, st);
+    else adj0_go<1, 2>(P, phase, ms, bs, alm, as, B, scale, st);
   } else {
-    if (P.Rh > 256 && ctas >= 900) adjS_go<4, 4>(P, phase, ms, bs, alm, B, spin, scale, st);
-    else if (P.Rh > 256) adjS_go<2, 8>(P, phase, ms, bs, alm, B, spin, scale, st);
-    else if (P.Rh > 64) adjS_go<2, 4>(P, phase, ms, bs, alm, B, spin, scale, st);
-    else adjS_go<1, 2>(P, phase, ms, bs, alm, B, spin, scale, st);
+    if (P.Rh > 256 && ctas >= 900) adjS_go<4, 4>(P, phase, ms, bs, alm, as, B, spin, scale, st);
+    else if (P.Rh > 256) adjS_go<2, 8>(P, phase, ms, bs, alm, as, B, spin, scale, st);
+    else if (P.Rh > 64) adjS_go<2, 4>(P, phase, ms, bs, alm, as, B, spin, scale, st);
+    else adjS_go<1, 2>(P, phase, ms, bs, alm, as, B, spin, scale, st);
   }
   PS_LAUNCH_CHECK();
   return PS_OK;

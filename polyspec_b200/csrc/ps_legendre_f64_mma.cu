@@ -8,7 +8,8 @@
 //
 // A warp owns 32 ring pairs.  Every lane runs the recurrence of its ring for 16 l (spin 0) or 8 l (spin s: f and
 // (-1)^l g) and drops the values into the warp's shared tile, 16 rows of 32 rings, whose columns are ordered so that
-// one 16-byte read gives a lane the elements of two A operands, 8 rings x 4 l (synthesis) or 8 l x 4 rings (adjoint).  Rows 0-7 hold the l of parity 0 (f), rows 8-15 those of parity 1 ((-1)^l g):
+// one 16-byte read gives a lane the elements of two A operands, 8 rings x 4 l (synthesis) or
+// 8 l x 4 rings (adjoint).  Rows 0-7 hold the l of parity 0 (f), rows 8-15 those of parity 1 ((-1)^l g):
 //   synthesis spin 0: B = alm; E, O = even and odd sums, north = E + O, south = E - O.
 //   synthesis spin s: B = (a+, (-1)^l a-) for f and, the same columns exchanged, for (-1)^l g; the
 //                     accumulators are the north and south sums of ps_legendre_f64.cu.
@@ -105,8 +106,9 @@ __device__ __forceinline__ int warp_mode(int k, bool force) {
 template <bool SPIN, int NT>
 __global__ void __launch_bounds__(32 * SYN_WARPS) synth_mma_f64(
     const RingInfo* __restrict__ rings, const double* __restrict__ mnorm, const SeedNorm* __restrict__ seednorm,
-    const double* __restrict__ lcd, const double* __restrict__ lg, const double2* __restrict__ alm,
-    double2* __restrict__ phase, int64_t ms, int64_t bs, int R, int Rh, int lmax, int mmax, int B, int per, int64_t nalm,
+    const double* __restrict__ lcd, const double* __restrict__ lg, const double2* __restrict__ alm, int64_t as,
+    double2* __restrict__ phase, int64_t ms, int64_t bs, int R, int Rh, int lmax, int mmax, int B, int per,
+    int64_t nalm,
     int spin) {
   constexpr int MAPS = SPIN ? 2 * NT : 4 * NT, CH = 32, BLK = SPIN ? 8 : 16;
   constexpr int AROW = 8 * NT + (SPIN ? 4 : 2);  // B-operand rows l, l + 1, .. (spin 0: l, l + 2, ..) in distinct banks
@@ -133,13 +135,13 @@ __global__ void __launch_bounds__(32 * SYN_WARPS) synth_mma_f64(
       const bool on = in && b < nb;
       if constexpr (SPIN) {
         const double2 z = make_double2(0.0, 0.0);
-        const double2 G = on ? cscale(alm[int64_t(b0 + b) * 2 * nalm + idx], gm) : z;
-        const double2 C = on ? cscale(alm[(int64_t(b0 + b) * 2 + 1) * nalm + idx], gm) : z;
+        const double2 G = on ? cscale(alm[(b0 + b) * as + idx], gm) : z;
+        const double2 C = on ? cscale(alm[(b0 + b) * as + nalm + idx], gm) : z;
         pa[i][0] = make_double2(G.x - C.y, G.y + C.x);
         const double2 am = make_double2(G.x + C.y, G.y - C.x);
         pa[i][1] = (lane & 1) ? make_double2(-am.x, -am.y) : am;  // l - lmin has the parity of lane
       } else {
-        pa[i][0] = on ? cscale(alm[int64_t(b0 + b) * nalm + idx], gm) : make_double2(0.0, 0.0);
+        pa[i][0] = on ? cscale(alm[(b0 + b) * as + idx], gm) : make_double2(0.0, 0.0);
       }
     }
     pc = make_double2(0.0, 0.0);
@@ -231,7 +233,7 @@ __global__ void __launch_bounds__(32 * SYN_WARPS) synth_mma_f64(
         if (b >= nb || (south && rs == rp)) continue;
         double2 z = make_double2(0.0, 0.0);  // alm with l < s enter only if not finite
         for (int l = m; l < min(spin, lmax + 1); ++l)
-          for (int c = 0; c < 2; ++c) z = cfma(0.0, alm[(int64_t(b0 + b) * 2 + c) * nalm + base + (l - m)], z);
+          for (int c = 0; c < 2; ++c) z = cfma(0.0, alm[(b0 + b) * as + c * nalm + base + (l - m)], z);
         const double h = south && ((lmin + m) & 1) ? -0.5 : 0.5;
         const double2 sp = cadd(z, cscale(south ? acc[1][r][t] : acc[0][r][t], h));
         const double2 sm = cadd(z, cscale(south ? acc[0][r][t] : acc[1][r][t], h));
@@ -265,7 +267,8 @@ template <bool SPIN, int NT>
 __global__ void __launch_bounds__(32 * ADJ_MMA_WARPS, 3) adj_mma_f64(
     const RingInfo* __restrict__ rings, const double* __restrict__ mnorm, const SeedNorm* __restrict__ seednorm,
     const double* __restrict__ lcd, const double* __restrict__ lg, const double2* __restrict__ phase, int64_t ms,
-    int64_t bs, double2* __restrict__ alm, int R, int Rh, int lmax, int mmax, int B, int bofs, int per, int64_t nalm,
+    int64_t bs, double2* __restrict__ alm, int64_t as, int R, int Rh, int lmax, int mmax, int B, int bofs, int per,
+    int64_t nalm,
     int spin, double scale) {
   constexpr int CH = 16, MAPS = SPIN ? 2 * NT : 4 * NT, ITEMS = (MAPS + ADJ_MMA_WARPS - 1) / ADJ_MMA_WARPS;
   extern __shared__ __align__(16) unsigned char adj_smem[];
@@ -344,7 +347,7 @@ __global__ void __launch_bounds__(32 * ADJ_MMA_WARPS, 3) adj_mma_f64(
         for (int w = 0; w < ADJ_MMA_WARPS; ++w) any |= S.bad[w];
         const double z = (any >> b) & 1 ? __longlong_as_double(0x7ff8000000000000LL) : 0.0;
         for (int c = 0; c < 2; ++c) {
-          double2& o = alm[(int64_t(b0 + b) * 2 + c) * nalm + base + j];
+          double2& o = alm[(b0 + b) * as + c * nalm + base + j];
           o = t0 == 0 ? make_double2(z, z) : cadd(o, make_double2(z, z));
         }
       }
@@ -364,10 +367,10 @@ __global__ void __launch_bounds__(32 * ADJ_MMA_WARPS, 3) adj_mma_f64(
           const int b = warp + ADJ_MMA_WARPS * i;
           const bool on = ins && b < nb;
           if constexpr (SPIN) {
-            old[i][0] = on ? (&alm[int64_t(b0 + b) * 2 * nalm + os].x)[cs] : 0.0;
-            old[i][1] = on ? (&alm[(int64_t(b0 + b) * 2 + 1) * nalm + os].x)[cs ^ 1] : 0.0;
+            old[i][0] = on ? (&alm[(b0 + b) * as + os].x)[cs] : 0.0;
+            old[i][1] = on ? (&alm[(b0 + b) * as + nalm + os].x)[cs ^ 1] : 0.0;
           } else {
-            old[i][0] = on ? (&alm[int64_t(b0 + b) * nalm + os].x)[cs] : 0.0;
+            old[i][0] = on ? (&alm[(b0 + b) * as + os].x)[cs] : 0.0;
           }
         }
       } else {
@@ -429,13 +432,13 @@ __global__ void __launch_bounds__(32 * ADJ_MMA_WARPS, 3) adj_mma_f64(
           const double sum = 0.5 * h * (tp + tm), dif = 0.5 * h * (tp - tm);
           // G = -(..); C = i (..): the real parts' sum is C's imaginary part, the imaginary ones', negated, its real
           const double G = (spin & 1) ? -dif : -sum, C = (spin & 1) ? sum : dif;
-          (&alm[int64_t(b0 + bm) * 2 * nalm + os].x)[cs] = old[i][0] + G;
-          (&alm[(int64_t(b0 + bm) * 2 + 1) * nalm + os].x)[cs ^ 1] = old[i][1] + (cs ? -C : C);
+          (&alm[(b0 + bm) * as + os].x)[cs] = old[i][0] + G;
+          (&alm[(b0 + bm) * as + nalm + os].x)[cs ^ 1] = old[i][1] + (cs ? -C : C);
         } else {
           double v = 0.0;
 #pragma unroll
           for (int w = 0; w < ADJ_MMA_WARPS; ++w) v += (&S.red[buf][w][ls][bm].x)[cs];
-          (&alm[int64_t(b0 + bm) * nalm + os].x)[cs] = old[i][0] + v * h;
+          (&alm[(b0 + bm) * as + os].x)[cs] = old[i][0] + v * h;
         }
       }
     }
@@ -444,18 +447,18 @@ __global__ void __launch_bounds__(32 * ADJ_MMA_WARPS, 3) adj_mma_f64(
 }
 
 template <bool SPIN, int NT>
-int synth_go(const Plan& P, const double2* alm, double2* phase, int64_t ms, int64_t bs, int B, int per, int spin,
-             cudaStream_t st) {
+int synth_go(const Plan& P, const double2* alm, int64_t as, double2* phase, int64_t ms, int64_t bs, int B, int per,
+             int spin, cudaStream_t st) {
   const dim3 grid((P.Rh + 32 * SYN_WARPS - 1) / (32 * SYN_WARPS), P.mmax + 1, (B + per - 1) / per);
   synth_mma_f64<SPIN, NT><<<grid, 32 * SYN_WARPS, 0, st>>>(P.d_rings, P.d_mnorm0, P.d_seed[spin], P.d_leg_cd[spin],
-                                                           P.d_leg_g[spin], alm, phase, ms, bs, P.R, P.Rh, P.lmax,
+                                                           P.d_leg_g[spin], alm, as, phase, ms, bs, P.R, P.Rh, P.lmax,
                                                            P.mmax, B, per, P.nalm, spin);
   PS_LAUNCH_CHECK();
   return PS_OK;
 }
 template <bool SPIN, int NT>
-int adj_go(const Plan& P, const double2* phase, int64_t ms, int64_t bs, double2* alm, int B, int per, int spin,
-           double scale, cudaStream_t st) {
+int adj_go(const Plan& P, const double2* phase, int64_t ms, int64_t bs, double2* alm, int64_t as, int B, int per,
+           int spin, double scale, cudaStream_t st) {
   const size_t smem = sizeof(AdjShared<SPIN, NT>);
   if (cudaFuncSetAttribute(adj_mma_f64<SPIN, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) !=
       cudaSuccess)
@@ -464,8 +467,8 @@ int adj_go(const Plan& P, const double2* phase, int64_t ms, int64_t bs, double2*
   for (int bofs = 0; bofs < B; bofs += step) {
     const int z = (std::min(step, B - bofs) + per - 1) / per;
     adj_mma_f64<SPIN, NT><<<dim3(1, P.mmax + 1, z), 32 * ADJ_MMA_WARPS, smem, st>>>(
-        P.d_rings, P.d_mnorm0, P.d_seed[spin], P.d_leg_cd[spin], P.d_leg_g[spin], phase, ms, bs, alm, P.R, P.Rh, P.lmax,
-        P.mmax, B, bofs, per, P.nalm, spin, scale);
+        P.d_rings, P.d_mnorm0, P.d_seed[spin], P.d_leg_cd[spin], P.d_leg_g[spin], phase, ms, bs, alm, as, P.R, P.Rh,
+        P.lmax, P.mmax, B, bofs, per, P.nalm, spin, scale);
     PS_LAUNCH_CHECK();
   }
   return PS_OK;
@@ -482,28 +485,28 @@ static int group_maps(int B, int most) {
   return (B + groups - 1) / groups;
 }
 
-int launch_synth_mma_f64(const Plan& P, const double2* alm, double2* phase, int64_t ms, int64_t bs, int B, int spin,
-                         cudaStream_t st) {
+int launch_synth_mma_f64(const Plan& P, const double2* alm, int64_t as, double2* phase, int64_t ms, int64_t bs, int B,
+                         int spin, cudaStream_t st) {
   const int per = group_maps(B, spin == 0 ? 12 : 6), nt = (per * (spin == 0 ? 2 : 4) + 7) / 8;
   if (spin == 0)
-    return nt == 1   ? synth_go<false, 1>(P, alm, phase, ms, bs, B, per, 0, st)
-           : nt == 2 ? synth_go<false, 2>(P, alm, phase, ms, bs, B, per, 0, st)
-                     : synth_go<false, 3>(P, alm, phase, ms, bs, B, per, 0, st);
-  return nt == 1   ? synth_go<true, 1>(P, alm, phase, ms, bs, B, per, spin, st)
-         : nt == 2 ? synth_go<true, 2>(P, alm, phase, ms, bs, B, per, spin, st)
-                   : synth_go<true, 3>(P, alm, phase, ms, bs, B, per, spin, st);
+    return nt == 1   ? synth_go<false, 1>(P, alm, as, phase, ms, bs, B, per, 0, st)
+           : nt == 2 ? synth_go<false, 2>(P, alm, as, phase, ms, bs, B, per, 0, st)
+                     : synth_go<false, 3>(P, alm, as, phase, ms, bs, B, per, 0, st);
+  return nt == 1   ? synth_go<true, 1>(P, alm, as, phase, ms, bs, B, per, spin, st)
+         : nt == 2 ? synth_go<true, 2>(P, alm, as, phase, ms, bs, B, per, spin, st)
+                   : synth_go<true, 3>(P, alm, as, phase, ms, bs, B, per, spin, st);
 }
 
-int launch_adjoint_mma_f64(const Plan& P, const double2* phase, int64_t ms, int64_t bs, double2* alm, int B, int spin,
-                           double scale, cudaStream_t st) {
+int launch_adjoint_mma_f64(const Plan& P, const double2* phase, int64_t ms, int64_t bs, double2* alm, int64_t as, int B,
+                           int spin, double scale, cudaStream_t st) {
   const int per = group_maps(B, spin == 0 ? 12 : 6), nt = (per * (spin == 0 ? 2 : 4) + 7) / 8;
   if (spin == 0)
-    return nt == 1   ? adj_go<false, 1>(P, phase, ms, bs, alm, B, per, 0, scale, st)
-           : nt == 2 ? adj_go<false, 2>(P, phase, ms, bs, alm, B, per, 0, scale, st)
-                     : adj_go<false, 3>(P, phase, ms, bs, alm, B, per, 0, scale, st);
-  return nt == 1   ? adj_go<true, 1>(P, phase, ms, bs, alm, B, per, spin, scale, st)
-         : nt == 2 ? adj_go<true, 2>(P, phase, ms, bs, alm, B, per, spin, scale, st)
-                   : adj_go<true, 3>(P, phase, ms, bs, alm, B, per, spin, scale, st);
+    return nt == 1   ? adj_go<false, 1>(P, phase, ms, bs, alm, as, B, per, 0, scale, st)
+           : nt == 2 ? adj_go<false, 2>(P, phase, ms, bs, alm, as, B, per, 0, scale, st)
+                     : adj_go<false, 3>(P, phase, ms, bs, alm, as, B, per, 0, scale, st);
+  return nt == 1   ? adj_go<true, 1>(P, phase, ms, bs, alm, as, B, per, spin, scale, st)
+         : nt == 2 ? adj_go<true, 2>(P, phase, ms, bs, alm, as, B, per, spin, scale, st)
+                   : adj_go<true, 3>(P, phase, ms, bs, alm, as, B, per, spin, scale, st);
 }
 
 }  // namespace ps

@@ -315,7 +315,7 @@ __global__ void __launch_bounds__(MX_THREADS) adjS_mx(const RingInfo* __restrict
 
 // sum_t partial[t][nalm][B][ncomp] (FP32) in FP64, times scale -> alm [B][ncomp][nalm] (FP64)
 __global__ void reduce_partials_f32(const float2* __restrict__ partial, double2* __restrict__ alm, int ntiles,
-                                    int B, int ncomp, int64_t nalm, double scale, int bofs) {
+                                    int B, int ncomp, int64_t nalm, int64_t as, double scale, int bofs) {
   const int64_t n = nalm * B * ncomp;
   for (int64_t t = blockIdx.x * int64_t(blockDim.x) + threadIdx.x; t < n; t += int64_t(gridDim.x) * blockDim.x) {
     double sx = 0.0, sy = 0.0;
@@ -327,7 +327,7 @@ __global__ void reduce_partials_f32(const float2* __restrict__ partial, double2*
     const int c = int(t % ncomp);
     const int b = int((t / ncomp) % B);
     const int64_t idx = t / (int64_t(ncomp) * B);
-    alm[(int64_t(bofs + b) * ncomp + c) * nalm + idx] = make_double2(sx * scale, sy * scale);
+    alm[(bofs + b) * as + c * nalm + idx] = make_double2(sx * scale, sy * scale);
   }
 }
 
@@ -378,13 +378,13 @@ int launch_legendre_adjoint_mx(const Plan& P, const float2* phase, float2* parti
   return PS_OK;
 }
 
-int launch_reduce_partials_f32(const float2* partial, double2* alm, int ntiles, int B, int ncomp, int64_t nalm,
-                               double scale, int bofs, int sms, cudaStream_t st) {
+int launch_reduce_partials_f32(const float2* partial, double2* alm, int64_t as, int ntiles, int B, int ncomp,
+                               int64_t nalm, double scale, int bofs, int sms, cudaStream_t st) {
   const int64_t n = nalm * B * ncomp;
   int blocks = (int)std::min<int64_t>((n + 255) / 256, int64_t(sms) * 8);
   if (blocks < 1) blocks = 1;
   StatScope sc(PS_K_LAYOUT, 0.0, 8.0 * n * ntiles + 16.0 * n, st);
-  reduce_partials_f32<<<blocks, 256, 0, st>>>(partial, alm, ntiles, B, ncomp, nalm, scale, bofs);
+  reduce_partials_f32<<<blocks, 256, 0, st>>>(partial, alm, ntiles, B, ncomp, nalm, as, scale, bofs);
   PS_LAUNCH_CHECK();
   return PS_OK;
 }

@@ -15,27 +15,27 @@
 
 namespace ps {
 int launch_leg_tables_f64(const Plan& P, int spin, double* cd, double* gam, cudaStream_t st);
-int launch_legendre_synth_f64(const Plan& P, const double2* alm, double2* phase, int64_t ms, int64_t bs, int B,
-                              int spin, cudaStream_t st);
-int launch_legendre_adjoint_f64(const Plan& P, const double2* phase, int64_t ms, int64_t bs, double2* alm, int B,
-                                int spin, double scale, cudaStream_t st);
+int launch_legendre_synth_f64(const Plan& P, const double2* alm, int64_t as, double2* phase, int64_t ms, int64_t bs,
+                              int B, int spin, cudaStream_t st);
+int launch_legendre_adjoint_f64(const Plan& P, const double2* phase, int64_t ms, int64_t bs, double2* alm,
+                                int64_t as, int B, int spin, double scale, cudaStream_t st);
 int launch_alm_to_T(const double2* alm, int64_t stride, const double* lscale, double2* almT, int B, int ncomp,
                     int64_t nalm, cudaStream_t st);
-int launch_ring_synth_f64(const Plan& P, const RingClassList* cls, int ncls, const double2* phase, double* map, int nf,
-                          int pack, cudaStream_t st);
-int launch_ring_adjoint_f64(const Plan& P, const RingClassList* cls, int ncls, const double* map, double2* phase,
-                            int nf, int pack, cudaStream_t st);
-int launch_ring_synth_f32(const Plan& P, const RingClassList* cls, int ncls, const float2* phase, double* map, int nf,
-                          int pack, cudaStream_t st);
-int launch_ring_adjoint_f32(const Plan& P, const RingClassList* cls, int ncls, const double* map, float2* phase,
-                            int nf, int pack, cudaStream_t st);
+int launch_ring_synth_f64(const Plan& P, const RingClassList* cls, int ncls, const double2* phase, double* map,
+                          int64_t map_stride, int nf, int pack, cudaStream_t st);
+int launch_ring_adjoint_f64(const Plan& P, const RingClassList* cls, int ncls, const double* map,
+                            int64_t map_stride, double2* phase, int nf, int pack, cudaStream_t st);
+int launch_ring_synth_f32(const Plan& P, const RingClassList* cls, int ncls, const float2* phase, double* map,
+                          int64_t map_stride, int nf, int pack, cudaStream_t st);
+int launch_ring_adjoint_f32(const Plan& P, const RingClassList* cls, int ncls, const double* map,
+                            int64_t map_stride, float2* phase, int nf, int pack, cudaStream_t st);
 int launch_legendre_synth_tc(const Plan& P, const double2* almT, float2* phase, int B, int spin, int* err_flag,
                              cudaStream_t st);
 int launch_legendre_adjoint_mx(const Plan& P, const float2* phase, float2* partial, int B, int bofs, int Bc,
                                int spin, cudaStream_t st);
 int mx_adjoint_tiles(const Plan& P);
-int launch_reduce_partials_f32(const float2* partial, double2* alm, int ntiles, int B, int ncomp, int64_t nalm,
-                               double scale, int bofs, int sms, cudaStream_t st);
+int launch_reduce_partials_f32(const float2* partial, double2* alm, int64_t as, int ntiles, int B, int ncomp,
+                               int64_t nalm, double scale, int bofs, int sms, cudaStream_t st);
 size_t tab_bytes(int Rh, int lmax, int mmax, int spin);
 size_t tab3_bytes(int Rh, int lmax, int mmax, int spin);
 int launch_tab3_gen(const Plan& P, int spin, const int64_t* d_blockoff, uint16_t* table, cudaStream_t st);
@@ -662,8 +662,8 @@ int ps_legendre_synthesis(const ps_plan* plan, const double* alm, double* phase,
   const int ncomp = spin == 0 ? 1 : 2;
   if (P.prec == PS_PREC_MIXED) {
     double2* almT = static_cast<double2*>(workspace);
-    int rc = ps::launch_alm_to_T(reinterpret_cast<const double2*>(alm), int64_t(ncomp) * P.nalm, nullptr, almT, batch, ncomp,
-                                 P.nalm, stream);
+    int rc = ps::launch_alm_to_T(reinterpret_cast<const double2*>(alm), int64_t(ncomp) * P.nalm, nullptr, almT, batch,
+                                 ncomp, P.nalm, stream);
     if (rc) return rc;
     float2* ph32 = reinterpret_cast<float2*>(static_cast<char*>(workspace) +
                                              align256(size_t(P.nalm) * batch * ncomp * sizeof(double2)));
@@ -679,8 +679,9 @@ int ps_legendre_synthesis(const ps_plan* plan, const double* alm, double* phase,
     PS_LAUNCH_CHECK();
     return PS_OK;
   }
-  return ps::launch_legendre_synth_f64(P, reinterpret_cast<const double2*>(alm), reinterpret_cast<double2*>(phase),
-                                       int64_t(batch) * ncomp, ncomp, batch, spin, stream);
+  return ps::launch_legendre_synth_f64(P, reinterpret_cast<const double2*>(alm), ncomp * P.nalm,
+                                       reinterpret_cast<double2*>(phase), int64_t(batch) * ncomp, ncomp, batch, spin,
+                                       stream);
 }
 
 int ps_legendre_adjoint(const ps_plan* plan, const double* phase, double* alm, int batch, int spin, double scale,
@@ -708,14 +709,14 @@ int ps_legendre_adjoint(const ps_plan* plan, const double* phase, double* alm, i
       const int bc = std::min(ch, batch - b0);
       int rc = ps::launch_legendre_adjoint_mx(P, ph32, partial, batch, b0, bc, spin, stream);
       if (rc) return rc;
-      rc = ps::launch_reduce_partials_f32(partial, reinterpret_cast<double2*>(alm), ps::mx_adjoint_tiles(P), bc, ncomp,
-                                          P.nalm, scale, b0, P.num_sms, stream);
+      rc = ps::launch_reduce_partials_f32(partial, reinterpret_cast<double2*>(alm), ncomp * P.nalm,
+                                          ps::mx_adjoint_tiles(P), bc, ncomp, P.nalm, scale, b0, P.num_sms, stream);
       if (rc) return rc;
     }
     return PS_OK;
   }
   return ps::launch_legendre_adjoint_f64(P, reinterpret_cast<const double2*>(phase), int64_t(batch) * ncomp, ncomp,
-                                         reinterpret_cast<double2*>(alm), batch, spin, scale, stream);
+                                         reinterpret_cast<double2*>(alm), ncomp * P.nalm, batch, spin, scale, stream);
 }
 
 int ps_sht_workspace_bytes(const ps_plan* plan, int batch, int spin, int adjoint, size_t* bytes) {
@@ -726,6 +727,11 @@ int ps_sht_workspace_bytes(const ps_plan* plan, int batch, int spin, int adjoint
 
 int ps_synthesis(const ps_plan* plan, const double* alm, double* map, int batch, int spin, void* workspace,
                  size_t workspace_bytes, cudaStream_t stream) {
+  return ps_synthesis_strided(plan, alm, 0, map, 0, batch, spin, workspace, workspace_bytes, stream);
+}
+
+int ps_synthesis_strided(const ps_plan* plan, const double* alm, int64_t alm_stride, double* map, int64_t map_stride,
+                         int batch, int spin, void* workspace, size_t workspace_bytes, cudaStream_t stream) {
   if (!plan || batch < 0 || spin < 0 || spin > 3) return PS_ERR_INVALID;
   if (plan->is_band) return PS_ERR_UNSUPPORTED;
   if (batch == 0) return PS_OK;
@@ -734,6 +740,9 @@ int ps_synthesis(const ps_plan* plan, const double* alm, double* map, int batch,
   if (spin > 0 && !P.d_seed[spin]) return PS_ERR_INVALID;
   if (workspace_bytes < sht_ws_bytes(plan, batch, spin, 0)) return PS_ERR_WORKSPACE;
   const int ncomp = spin == 0 ? 1 : 2;
+  if (alm_stride == 0) alm_stride = ncomp * P.nalm;
+  if (map_stride == 0) map_stride = ncomp * P.npix;
+  if (alm_stride < ncomp * P.nalm || map_stride < ncomp * P.npix) return PS_ERR_INVALID;
   const int nf = batch * ncomp;
   char* ws = static_cast<char*>(workspace);
   double2* almT = reinterpret_cast<double2*>(ws);
@@ -743,8 +752,8 @@ int ps_synthesis(const ps_plan* plan, const double* alm, double* map, int batch,
     if (nf == 1) {
       almT = reinterpret_cast<double2*>(const_cast<double*>(alm));
     } else {
-      rc = ps::launch_alm_to_T(reinterpret_cast<const double2*>(alm), int64_t(ncomp) * P.nalm, nullptr, almT, batch, ncomp,
-                                 P.nalm, stream);
+      rc = ps::launch_alm_to_T(reinterpret_cast<const double2*>(alm), alm_stride, nullptr, almT, batch, ncomp, P.nalm,
+                               stream);
       if (rc) return rc;
     }
     // tensor-core Legendre stage (TF32 x3, FP32 accumulation) and FP32 ring transforms
@@ -756,20 +765,26 @@ int ps_synthesis(const ps_plan* plan, const double* alm, double* map, int batch,
     else
       rc = ps::launch_legendre_synth_tc(P, almT, phase, batch, spin, P.d_err, stream);
     if (rc) return rc;
-    return ps::launch_ring_synth_f32(P, plan->ring_cls.data(), int(plan->ring_cls.size()), phase, map, nf, spin > 0,
-                                     stream);
+    return ps::launch_ring_synth_f32(P, plan->ring_cls.data(), int(plan->ring_cls.size()), phase, map,
+                                     map_stride, nf, spin > 0, stream);
   }
   double2* phase = reinterpret_cast<double2*>(phase_ptr);
   // between the two stages the phases are [R][batch][mmax+1][ncomp]
-  rc = ps::launch_legendre_synth_f64(P, reinterpret_cast<const double2*>(alm), phase, ncomp,
+  rc = ps::launch_legendre_synth_f64(P, reinterpret_cast<const double2*>(alm), alm_stride, phase, ncomp,
                                      int64_t(P.mmax + 1) * ncomp, batch, spin, stream);
   if (rc) return rc;
-  return ps::launch_ring_synth_f64(P, plan->ring_cls.data(), int(plan->ring_cls.size()), phase, map, nf, spin > 0,
-                                   stream);
+  return ps::launch_ring_synth_f64(P, plan->ring_cls.data(), int(plan->ring_cls.size()), phase, map,
+                                   map_stride, nf, spin > 0, stream);
 }
 
 int ps_adjoint(const ps_plan* plan, const double* map, double* alm, int batch, int spin, double scale,
                void* workspace, size_t workspace_bytes, cudaStream_t stream) {
+  return ps_adjoint_strided(plan, map, 0, alm, 0, batch, spin, scale, workspace, workspace_bytes, stream);
+}
+
+int ps_adjoint_strided(const ps_plan* plan, const double* map, int64_t map_stride, double* alm, int64_t alm_stride,
+                       int batch, int spin, double scale, void* workspace, size_t workspace_bytes,
+                       cudaStream_t stream) {
   if (!plan || batch < 0 || spin < 0 || spin > 3) return PS_ERR_INVALID;
   if (plan->is_band) return PS_ERR_UNSUPPORTED;
   if (batch == 0) return PS_OK;
@@ -778,6 +793,9 @@ int ps_adjoint(const ps_plan* plan, const double* map, double* alm, int batch, i
   if (spin > 0 && !P.d_seed[spin]) return PS_ERR_INVALID;
   if (workspace_bytes < sht_ws_bytes(plan, batch, spin, 1)) return PS_ERR_WORKSPACE;
   const int ncomp = spin == 0 ? 1 : 2;
+  if (alm_stride == 0) alm_stride = ncomp * P.nalm;
+  if (map_stride == 0) map_stride = ncomp * P.npix;
+  if (alm_stride < ncomp * P.nalm || map_stride < ncomp * P.npix) return PS_ERR_INVALID;
   const int nf = batch * ncomp;
   char* ws = static_cast<char*>(workspace);
   const size_t phase_bytes = align256(size_t(P.R) * (P.mmax + 1) * nf * sizeof(double2));
@@ -786,31 +804,31 @@ int ps_adjoint(const ps_plan* plan, const double* map, double* alm, int batch, i
     // FP32 ring transforms, FP64 recurrences with FP32 contractions, FP64 cross-tile sums
     float2* phase = reinterpret_cast<float2*>(ws);
     float2* partial = reinterpret_cast<float2*>(ws + phase_bytes);
-    rc = ps::launch_ring_adjoint_f32(P, plan->ring_cls.data(), int(plan->ring_cls.size()), map, phase, nf, spin > 0,
-                                     stream);
+    rc = ps::launch_ring_adjoint_f32(P, plan->ring_cls.data(), int(plan->ring_cls.size()), map, map_stride,
+                                     phase, nf, spin > 0, stream);
     if (rc) return rc;
     TabRef tr;
     if (table_for(plan, spin, tr))
       return ps::launch_tab_adj(P, tr.tab, tr.off, tr.work, tr.nwork, tr.Rh_table, tr.toff, phase,
-                                reinterpret_cast<double2*>(alm), batch, spin, scale, int64_t(ncomp) * P.nalm, nullptr,
+                                reinterpret_cast<double2*>(alm), batch, spin, scale, alm_stride, nullptr,
                                 P.d_err, stream, tr.fmt);
     const int ch = adjoint_chunk(P, batch, spin);
     for (int b0 = 0; b0 < batch; b0 += ch) {
       const int bc = std::min(ch, batch - b0);
       rc = ps::launch_legendre_adjoint_mx(P, phase, partial, batch, b0, bc, spin, stream);
       if (rc) return rc;
-      rc = ps::launch_reduce_partials_f32(partial, reinterpret_cast<double2*>(alm), ps::mx_adjoint_tiles(P), bc,
-                                          ncomp, P.nalm, scale, b0, P.num_sms, stream);
+      rc = ps::launch_reduce_partials_f32(partial, reinterpret_cast<double2*>(alm), alm_stride, ps::mx_adjoint_tiles(P),
+                                          bc, ncomp, P.nalm, scale, b0, P.num_sms, stream);
       if (rc) return rc;
     }
     return PS_OK;
   }
   double2* phase = reinterpret_cast<double2*>(ws);
-  rc = ps::launch_ring_adjoint_f64(P, plan->ring_cls.data(), int(plan->ring_cls.size()), map, phase, nf, spin > 0,
-                                   stream);
+  rc = ps::launch_ring_adjoint_f64(P, plan->ring_cls.data(), int(plan->ring_cls.size()), map, map_stride,
+                                   phase, nf, spin > 0, stream);
   if (rc) return rc;
   return ps::launch_legendre_adjoint_f64(P, phase, ncomp, int64_t(P.mmax + 1) * ncomp, reinterpret_cast<double2*>(alm),
-                                         batch, spin, scale, stream);
+                                         alm_stride, batch, spin, scale, stream);
 }
 
 }  // extern "C"

@@ -59,6 +59,7 @@ class SHTPlan:
                       _lib.PS_PREC_FP64 if prec == "fp64" else _lib.PS_PREC_MIXED, ctypes.byref(h))
         self._h = h
         self._ws = None
+        self._ws_need = {}  # (batch, spin, adjoint) -> bytes; they depend on the tables
         # Legendre table format of a mixed plan: 'tf32x3' (FP32 values, split by the kernels) or
         # 'bf16x3' (BF16 hi + mid + lo planes in the tensor core's operand layout, 1.5x the bytes)
         if table_format is None:
@@ -131,10 +132,12 @@ class SHTPlan:
             if rc == _lib.PS_ERR_NOMEM and not force:
                 return False
             _lib.check("ps_plan_build_table", rc)
+        self._ws_need.clear()
         return True
 
     def drop_tables(self):
         _lib.call("ps_plan_drop_tables", self._h)
+        self._ws_need.clear()
         self._tab_tried.clear()
 
     def _maybe_table(self, spin):
@@ -169,20 +172,25 @@ class SHTPlan:
 
     # ------------------------------------------------------------ workspace
     def workspace(self, batch, spin, adjoint):
-        need = 0
-        for h in (self._h, self._h64):
-            if h is None:
-                continue
-            n = ctypes.c_size_t()
-            _lib.call("ps_sht_workspace_bytes", h, int(batch), int(spin), int(adjoint), ctypes.byref(n))
-            need = max(need, int(n.value))
+        key = (int(batch), int(spin), int(adjoint))
+        need = self._ws_need.get(key)
+        if need is None:
+            need = 0
+            for h in (self._h, self._h64):
+                if h is None:
+                    continue
+                n = ctypes.c_size_t()
+                _lib.call("ps_sht_workspace_bytes", h, *key, ctypes.byref(n))
+                need = max(need, int(n.value))
+            self._ws_need[key] = need
         if self._ws is None or self._ws.numel() < need:
             self._ws = torch.empty(max(need, 256), dtype=torch.uint8, device=self.device)
         return self._ws, need
 
     @staticmethod
     def _stream():
-        return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+        # the current stream's handle, without building a torch.cuda.Stream (4 us a call)
+        return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
     def _check_alm(self, alm, spin):
         ncomp = 1 if spin == 0 else 2
@@ -198,23 +206,64 @@ class SHTPlan:
             B *= int(d)
         return lead, B, ncomp
 
-    def synthesis(self, alm, spin=0):
-        spin = int(spin)
-        lead, B, ncomp = self._check_alm(alm, spin)
-        alm = alm.contiguous()
-        shape = tuple(lead) + ((2,) if spin > 0 else ()) + (self.npix,)
-        out = torch.empty(shape, dtype=torch.float64, device=alm.device)
-        if B == 0:
-            return out
+    @staticmethod
+    def _maps_in(t, nf, n):
+        """(tensor, stride) of an input [..., n] (nf = 1) or [..., nf, n] for the strided entry points: read
+        in place where each map's fields are contiguous and the maps lie at one stride, else copied."""
+        if t.is_conj():
+            t = t.resolve_conj()
+        if t.is_neg():
+            t = t.resolve_neg()
+        if t.is_contiguous():
+            return t, nf * n
+        if (t.dim() == (2 if nf == 1 else 3) and t.stride(-1) == 1 and (nf == 1 or t.stride(-2) == n)
+                and t.stride(0) >= nf * n):
+            return t, t.stride(0)
+        return t.contiguous(), nf * n
+
+    def _issue_synthesis(self, spin, B, alm, alm_stride, out, map_stride):
+        """Synthesis of B maps at the addresses and strides of ps_synthesis_strided."""
         self._maybe_table(spin)
         ws, nbytes = self.workspace(B, spin, 0)
 
         def run(h):
-            _lib.call("ps_synthesis", h, ctypes.c_void_p(alm.data_ptr()), ctypes.c_void_p(out.data_ptr()),
-                      B, spin, ctypes.c_void_p(ws.data_ptr()), nbytes, self._stream())
+            _lib.call("ps_synthesis_strided", h, alm, alm_stride, out, map_stride, B, spin, ws.data_ptr(), nbytes,
+                      self._stream())
         run(self._pick(("synthesis", spin, B), run))
         self.n_synthesis += B
+
+    def _issue_adjoint(self, spin, B, map, map_stride, out, alm_stride, scale):
+        """Adjoint of B maps at the addresses and strides of ps_adjoint_strided."""
+        self._maybe_table(spin)
+        ws, nbytes = self.workspace(B, spin, 1)
+
+        def run(h):
+            _lib.call("ps_adjoint_strided", h, map, map_stride, out, alm_stride, B, spin, float(scale), ws.data_ptr(),
+                      nbytes, self._stream())
+        run(self._pick(("adjoint", spin, B), run))
+        self.n_adjoint += B
+
+    def synthesis(self, alm, spin=0):
+        spin = int(spin)
+        lead, B, ncomp = self._check_alm(alm, spin)
+        alm, stride = self._maps_in(alm, ncomp, self.nalm)
+        shape = tuple(lead) + ((2,) if spin > 0 else ()) + (self.npix,)
+        out = torch.empty(shape, dtype=torch.float64, device=alm.device)
+        if B > 0:
+            self._issue_synthesis(spin, B, alm.data_ptr(), stride, out.data_ptr(), 0)
         return out
+
+    def synthesis_fields(self, alm, out):
+        """alm [B, nf, nalm] -> out [B, nf, npix]: T (spin 0) and, of three fields, (E, B) -> (Q, U), read
+        and written where they lie."""
+        self._check_alm(alm, 0)
+        B, nf = alm.shape[0], alm.shape[1]
+        alm, stride = self._maps_in(alm, nf, self.nalm)
+        if B > 0:
+            a, o = alm.data_ptr(), out.data_ptr()
+            self._issue_synthesis(0, B, a, stride, o, nf * self.npix)
+            if nf == 3:
+                self._issue_synthesis(2, B, a + 16 * self.nalm, stride, o + 8 * self.npix, nf * self.npix)
 
     def weighted_roundtrip(self, alm, weight, lscale=None, scale=1.0, out=None):
         """Fused  out = scale * lscale * Y^H W Y (lscale * alm)  for every field of alm [B, nf, nalm]
@@ -250,8 +299,7 @@ class SHTPlan:
         self.n_adjoint += B * len(spins)
         return out
 
-    def adjoint(self, map, spin=0, scale=1.0):
-        spin = int(spin)
+    def _check_map(self, map, spin):
         if map.dtype != torch.float64 or not map.is_cuda:
             raise TypeError("map must be a float64 CUDA tensor")
         if map.shape[-1] != self.npix:
@@ -262,17 +310,26 @@ class SHTPlan:
         B = 1
         for d in lead:
             B *= int(d)
-        map = map.contiguous()
+        return lead, B, 1 if spin == 0 else 2
+
+    def adjoint(self, map, spin=0, scale=1.0):
+        spin = int(spin)
+        lead, B, ncomp = self._check_map(map, spin)
+        map, stride = self._maps_in(map, ncomp, self.npix)
         shape = tuple(lead) + ((2,) if spin > 0 else ()) + (self.nalm,)
         out = torch.empty(shape, dtype=torch.complex128, device=map.device)
-        if B == 0:
-            return out
-        self._maybe_table(spin)
-        ws, nbytes = self.workspace(B, spin, 1)
-
-        def run(h):
-            _lib.call("ps_adjoint", h, ctypes.c_void_p(map.data_ptr()), ctypes.c_void_p(out.data_ptr()),
-                      B, spin, float(scale), ctypes.c_void_p(ws.data_ptr()), nbytes, self._stream())
-        run(self._pick(("adjoint", spin, B), run))
-        self.n_adjoint += B
+        if B > 0:
+            self._issue_adjoint(spin, B, map.data_ptr(), stride, out.data_ptr(), 0, scale)
         return out
+
+    def adjoint_fields(self, maps, out, scale=1.0):
+        """maps [B, nf, npix] -> out [B, nf, nalm]: T (spin 0) and, of three fields, (Q, U) -> (E, B), read
+        and written where they lie."""
+        self._check_map(maps, 0)
+        B, nf = maps.shape[0], maps.shape[1]
+        maps, stride = self._maps_in(maps, nf, self.npix)
+        if B > 0:
+            m, o = maps.data_ptr(), out.data_ptr()
+            self._issue_adjoint(0, B, m, stride, o, nf * self.nalm, scale)
+            if nf == 3:
+                self._issue_adjoint(2, B, m + 8 * self.npix, stride, o + 16 * self.nalm, nf * self.nalm, scale)
