@@ -127,6 +127,19 @@ int ps_adjoint_strided(const ps_plan* plan, const double* map, int64_t map_strid
                        int batch, int spin, double scale, void* workspace, size_t workspace_bytes,
                        cudaStream_t stream);
 
+/* Spin-s transforms between scalar alm and complex maps (polyspec/base.py:179-232), spin >= 1.
+ * ps_synthesis_pm: alm [batch][nalm] -> plus = Q + iU and minus = Q - iU, [batch][npix] complex128 each, of the
+ * spin-s maps of (G, C) = (-alm, 0).
+ * ps_adjoint_pm: complex maps plus, minus [batch][npix], of which Q = Re (plus + minus) / 2 and U = Im (plus -
+ * minus) / 2 enter, -> alm_plus = -(G + iC), alm_minus = -(-1)^s (G - iC), [batch][nalm] each; gc [batch][2][nalm]
+ * is scratch and ends as (G, C).  Workspace: ps_sht_workspace_bytes of the same batch, spin and direction.
+ * All arrays 16-byte aligned. */
+int ps_synthesis_pm(const ps_plan* plan, const double* alm, double* plus, double* minus, int batch, int spin,
+                    void* workspace, size_t workspace_bytes, cudaStream_t stream);
+int ps_adjoint_pm(const ps_plan* plan, const double* plus, const double* minus, double* gc, double* alm_plus,
+                  double* alm_minus, int batch, int spin, double scale, void* workspace, size_t workspace_bytes,
+                  cudaStream_t stream);
+
 /* Fused weighted round trip of the masked CG operator (no single reference call;
  * replaces, per spin, the pair to_map -> pixel weight -> to_lm inside
  * CGD._apply_A at polyspec/weighting.py:297-299):

@@ -39,6 +39,10 @@ SIGNATURES = {
                                       _c_size_t, _c_void_p]),
     "ps_adjoint_strided": (_c_int, [_c_void_p, _c_void_p, _c_int64, _c_void_p, _c_int64, _c_int, _c_int, _c_double,
                                     _c_void_p, _c_size_t, _c_void_p]),
+    "ps_synthesis_pm": (_c_int, [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_void_p, _c_size_t,
+                                 _c_void_p]),
+    "ps_adjoint_pm": (_c_int, [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int,
+                               _c_double, _c_void_p, _c_size_t, _c_void_p]),
     "ps_synthesis_noalloc": (_c_int, [_c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_void_p]),
     "ps_plan_band": (_c_int, [_c_void_p, _c_int, ctypes.POINTER(_c_void_p)]),
     "ps_plan_set_tile": (_c_int, [_c_void_p, _c_int, _c_int, _c_int]),

@@ -270,9 +270,7 @@ class PolySpec:
         assert spin > 0, "Spin must be positive!"
         assert len(input_vec) == 2, "Must input both +s and -s maps"
         v, as_torch = self._in(input_vec, torch.complex128)
-        map_inputs = _to_real_imag(v[0], v[1])  # [n, 2, npix]
-        lm = P.adjoint(map_inputs.contiguous(), int(spin), scale)
-        return self._out(_to_plus_minus_complex(lm, spin), as_torch)
+        return self._out(P.adjoint_pm(v[0], v[1], int(spin), scale), as_torch)
 
     @timer_func
     def to_map_vec(self, input_lm_vec, output_spin=0, lmax=None):
@@ -286,9 +284,7 @@ class PolySpec:
         P = self.plan(lmax)
         if output_spin == 0:
             return self._out(P.synthesis(a, 0), as_torch)
-        inp = torch.stack([-a, torch.zeros_like(a)], dim=1)
-        out = P.synthesis(inp, int(output_spin))
-        return self._out(_to_plus_minus(out), as_torch)
+        return self._out(P.synthesis_pm(a, int(output_spin)), as_torch)
 
     @timer_func
     def to_lm_spin(self, input_map_plus, input_map_minus, spin, lmax=None):

@@ -30,7 +30,7 @@
 struct ps_plan;
 
 namespace ps {
-int launch_alm_to_T(const double2* alm, int64_t stride, const double* lscale, double2* almT, int B, int ncomp,
+int launch_alm_to_T(const double2* alm, int64_t stride, const double* lscale, bool grad, double2* almT, int B, int ncomp,
                     int64_t nalm, cudaStream_t st);
 int launch_tab_synth(const Plan& P, const float* table, const int64_t* d_blockoff, int Rh_table, int toff,
                      const double2* almT, float2* phase, int B, int spin, int* err_flag, cudaStream_t st, int fmt);
@@ -468,7 +468,8 @@ extern "C" int ps_cutprec_apply(const ps_cutprec* c, const double* r, double* ou
     const int nc = spin ? 2 : 1;
     const BandView& v = spin ? v2 : v0;
     const int c0 = spin ? 1 : 0;
-    rc = launch_alm_to_T(o + c0 * nalm, 3 * nalm, c->beam + c0 * nalm, almT, batch, nc, nalm, stream);
+    rc = launch_alm_to_T(o + c0 * nalm, 3 * nalm, c->beam + c0 * nalm, false, almT, batch, nc,
+                         nalm, stream);
     if (rc != PS_OK) return rc;
     rc = launch_tab_synth(*v.P, v.tab, v.off, v.Rh_table, v.toff, almT, spin ? ph2 : ph0, batch, spin, err, stream,
                           v.fmt);

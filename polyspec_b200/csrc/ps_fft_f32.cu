@@ -389,10 +389,12 @@ __device__ __forceinline__ float2 dechirp(float2 y, const float2* __restrict__ c
   return make_float2(v.x * s, v.y * s);
 }
 
-// synthesis: phase [R][mmax+1][nf] (complex64) -> maps (float64)
+// synthesis: phase [R][mmax+1][nf] (complex64) -> maps (float64), or (PAIR, packed) complex maps Q + iU at map and
+// Q - iU at minus (complex128)
+template <bool PAIR>
 __global__ void __launch_bounds__(RING_NT, 2) ring_synth_f32(const __grid_constant__ RingLaunchF L,
                                                              const float2* __restrict__ phase,
-                                                             double* __restrict__ map) {
+                                                             double* __restrict__ map, double2* __restrict__ minus) {
   extern __shared__ float2 fbuf[];
   const RingCtaF c = ring_cta_f(L);
   fold_phases(L, c, phase, fbuf);
@@ -402,17 +404,28 @@ __global__ void __launch_bounds__(RING_NT, 2) ring_synth_f32(const __grid_consta
   float2* a = fbuf + grp * ring_smem_f(c);
   double* oa = map + it.pix_a;
   double* ob = map + it.pix_b;
+  double2* op = reinterpret_cast<double2*>(map) + it.pix_a;
+  double2* om = minus + it.pix_a;
   const float inv = 1.0f / float(c.M);
   auto out = [&](int j, float2 y) {
     if (c.blue) y = dechirp(y, it.chirp, j, inv);
-    if (it.va) oa[j] = double(y.x);
-    if (it.vb) ob[j] = double(y.y);
+    if constexpr (PAIR) {
+      if (it.va) {
+        op[j] = make_double2(y.x, y.y);
+        om[j] = make_double2(y.x, -y.y);
+      }
+    } else {
+      if (it.va) oa[j] = double(y.x);
+      if (it.vb) ob[j] = double(y.y);
+    }
   };
   ring_dft_f<true>(c.blue, a, it.N, c.M, c.logM, it.spec, L.tw, u, c.T, LocalIn{a}, out);
 }
 
+template <bool PAIR>
 struct MapIn {
   const double *ia, *ib;
+  const double2 *ip, *im;
   const float2* chirp;
   int N;
   bool va, vb, blue;
@@ -421,7 +434,12 @@ struct MapIn {
 #pragma unroll
     for (int i = 0; i < K; ++i) {
       const int j = t + i * q;
-      x[i] = make_float2(va && j < N ? float(ia[j]) : 0.f, vb && j < N ? float(ib[j]) : 0.f);
+      if constexpr (PAIR) {
+        const double2 z = make_double2(0.0, 0.0), p = va && j < N ? ip[j] : z, n = va && j < N ? im[j] : z;
+        x[i] = make_float2(float(0.5 * (p.x + n.x)), float(0.5 * (p.y - n.y)));
+      } else {
+        x[i] = make_float2(va && j < N ? float(ia[j]) : 0.f, vb && j < N ? float(ib[j]) : 0.f);
+      }
     }
     if (blue) {
 #pragma unroll
@@ -431,17 +449,20 @@ struct MapIn {
   }
 };
 
-// adjoint: maps (float64) -> phase [R][mmax+1][nf] (complex64)
+// adjoint: maps (float64), or (PAIR, packed) Q = Re (p + n) / 2, U = Im (p - n) / 2 of the complex maps p and
+// n = minus -> phase [R][mmax+1][nf] (complex64)
+template <bool PAIR>
 __global__ void __launch_bounds__(RING_NT, 2) ring_adjoint_f32(const __grid_constant__ RingLaunchF L,
                                                                const double* __restrict__ map,
+                                                               const double2* __restrict__ minus,
                                                                float2* __restrict__ phase) {
   extern __shared__ float2 fbuf[];
   const RingCtaF c = ring_cta_f(L);
   const int grp = threadIdx.x >> c.logT, u = threadIdx.x & (c.T - 1);
   const RingItemF it = ring_item_f(L, c, grp);
   float2* a = fbuf + grp * ring_smem_f(c);
-  const MapIn in{map + it.pix_a, map + it.pix_b,
-                 it.chirp, it.N, it.va, it.vb, c.blue != 0};
+  const MapIn<PAIR> in{map + it.pix_a, map + it.pix_b, reinterpret_cast<const double2*>(map) + it.pix_a,
+                       minus + it.pix_a, it.chirp, it.N, it.va, it.vb, c.blue != 0};
   const float inv = 1.0f / float(c.M);
   auto out = [&](int k, float2 y) { a[fpad(k)] = c.blue ? dechirp(y, it.chirp, k, inv) : y; };
   ring_dft_f<false>(c.blue, a, it.N, c.M, c.logM, it.spec, L.tw, u, c.T, in, out);
@@ -533,11 +554,12 @@ static bool ring_smem_ok(K kern, size_t smem) {
 }
 
 int launch_ring_synth_f32(const Plan& P, const RingClassList* cls, int ncls, const float2* phase, double* map,
-                          int64_t map_stride, int nf, int pack, cudaStream_t st) {
+                          double2* minus, int64_t map_stride, int nf, int pack, cudaStream_t st) {
   auto go = [&](const RingLaunchF& L, int ctas, size_t smem, double) -> int {
-    if (!ring_smem_ok(ring_synth_f32, smem)) return PS_ERR_CUDA;
+    const auto kern = minus ? ring_synth_f32<true> : ring_synth_f32<false>;
+    if (!ring_smem_ok(kern, smem)) return PS_ERR_CUDA;
     StatScope sc(PS_K_FFT_SYNTH, 0.0, 0.0, st);
-    ring_synth_f32<<<ctas, RING_NT, smem, st>>>(L, phase, map);
+    kern<<<ctas, RING_NT, smem, st>>>(L, phase, map, minus);
     PS_LAUNCH_CHECK();
     return PS_OK;
   };
@@ -545,11 +567,12 @@ int launch_ring_synth_f32(const Plan& P, const RingClassList* cls, int ncls, con
 }
 
 int launch_ring_adjoint_f32(const Plan& P, const RingClassList* cls, int ncls, const double* map,
-                            int64_t map_stride, float2* phase, int nf, int pack, cudaStream_t st) {
+                            const double2* minus, int64_t map_stride, float2* phase, int nf, int pack, cudaStream_t st) {
   auto go = [&](const RingLaunchF& L, int ctas, size_t smem, double) -> int {
-    if (!ring_smem_ok(ring_adjoint_f32, smem)) return PS_ERR_CUDA;
+    const auto kern = minus ? ring_adjoint_f32<true> : ring_adjoint_f32<false>;
+    if (!ring_smem_ok(kern, smem)) return PS_ERR_CUDA;
     StatScope sc(PS_K_FFT_ADJOINT, 0.0, 0.0, st);
-    ring_adjoint_f32<<<ctas, RING_NT, smem, st>>>(L, map, phase);
+    kern<<<ctas, RING_NT, smem, st>>>(L, map, minus, phase);
     PS_LAUNCH_CHECK();
     return PS_OK;
   };

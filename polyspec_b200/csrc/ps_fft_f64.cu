@@ -459,11 +459,11 @@ struct SynthIn {
       }
     };
 
-// synthesis: phase -> maps
-template <int NT>
+// synthesis: phase -> maps, or (PAIR, packed) complex maps Q + iU at map and Q - iU at minus
+template <int NT, bool PAIR>
 __global__ void __launch_bounds__(NT, 512 / NT) ring_synth_f64(const __grid_constant__ RingLaunch L,
                                                                const double2* __restrict__ phase,
-                                                               double* __restrict__ map) {
+                                                               double* __restrict__ map, double2* __restrict__ minus) {
   extern __shared__ double2 smem[];
   const RingItem it = ring_item(L, smem);
   const int N = it.N, T = it.T, u = it.u;
@@ -481,11 +481,20 @@ __global__ void __launch_bounds__(NT, 512 / NT) ring_synth_f64(const __grid_cons
   in.blue = it.blue;
   double* oa = map + it.pix_a;
   double* ob = map + it.pix_b;
+  double2* op = reinterpret_cast<double2*>(map) + it.pix_a;
+  double2* om = minus + it.pix_a;
   const double inv = 1.0 / double(it.M);
   auto out = [&](int j, double2 y) {
     if (it.blue) y = cscale(cmul(y, __ldg(&it.chirp[j])), inv);
-    if (it.va) oa[j] = y.x;
-    if (it.vb) ob[j] = y.y;
+    if constexpr (PAIR) {
+      if (it.va) {
+        op[j] = y;
+        om[j] = cconj(y);
+      }
+    } else {
+      if (it.va) oa[j] = y.x;
+      if (it.vb) ob[j] = y.y;
+    }
   };
   if (T >= (it.blue ? it.M / 2 : it.M)) {
     // short rings (every ring of the class has at most T pixels): the aliases of each index are shared by
@@ -519,8 +528,10 @@ __global__ void __launch_bounds__(NT, 512 / NT) ring_synth_f64(const __grid_cons
   }
 }
 
+template <bool PAIR>
 struct AdjointIn {
   const double *ia, *ib;
+  const double2 *ip, *im;
   const double2* chirp;
   int N;
   bool va, vb, blue;
@@ -529,7 +540,12 @@ struct AdjointIn {
 #pragma unroll
     for (int i = 0; i < K; ++i) {
       const int j = t + i * q;
-      x[i] = make_double2(va && j < N ? ia[j] : 0.0, vb && j < N ? ib[j] : 0.0);
+      if constexpr (PAIR) {
+        const double2 z = make_double2(0.0, 0.0), p = va && j < N ? ip[j] : z, n = va && j < N ? im[j] : z;
+        x[i] = make_double2(0.5 * (p.x + n.x), 0.5 * (p.y - n.y));
+      } else {
+        x[i] = make_double2(va && j < N ? ia[j] : 0.0, vb && j < N ? ib[j] : 0.0);
+      }
     }
     if (blue) {
 #pragma unroll
@@ -539,16 +555,17 @@ struct AdjointIn {
   }
 };
 
-// adjoint: maps -> phase
-template <int NT>
+// adjoint: maps, or (PAIR, packed) Q = Re (p + n) / 2, U = Im (p - n) / 2 of the complex maps p and n = minus -> phase
+template <int NT, bool PAIR>
 __global__ void __launch_bounds__(NT, 512 / NT) ring_adjoint_f64(const __grid_constant__ RingLaunch L,
                                                                  const double* __restrict__ map,
+                                                                 const double2* __restrict__ minus,
                                                                  double2* __restrict__ phase) {
   extern __shared__ double2 smem[];
   const RingItem it = ring_item(L, smem);
   const int N = it.N, mmax = L.mmax, T = it.T, u = it.u;
-  const AdjointIn in{map + it.pix_a, map + it.pix_b,
-                     it.chirp, N, it.va, it.vb, it.blue};
+  const AdjointIn<PAIR> in{map + it.pix_a, map + it.pix_b, reinterpret_cast<const double2*>(map) + it.pix_a,
+                           minus + it.pix_a, it.chirp, N, it.va, it.vb, it.blue};
   const double inv = 1.0 / double(it.M);
   auto out = [&](int k, double2 y) {
     if (it.blue) y = cscale(cmul(y, __ldg(&it.chirp[k])), inv);
@@ -626,14 +643,15 @@ static int ring_launches(const Plan& P, const RingClassList* cls, int ncls, int6
 }
 
 int launch_ring_synth_f64(const Plan& P, const RingClassList* cls, int ncls, const double2* phase, double* map,
-                          int64_t map_stride, int nf, int pack, cudaStream_t st) {
+                          double2* minus, int64_t map_stride, int nf, int pack, cudaStream_t st) {
   auto go = [&](const RingLaunch& L, int nt, int ctas, size_t smem) -> int {
-    const auto kern = nt == 512 ? ring_synth_f64<512> : ring_synth_f64<256>;
+    const auto kern = minus ? (nt == 512 ? ring_synth_f64<512, true> : ring_synth_f64<256, true>)
+                            : (nt == 512 ? ring_synth_f64<512, false> : ring_synth_f64<256, false>);
     if (smem > 48 * 1024 &&
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
       return PS_ERR_CUDA;
     StatScope sc(PS_K_FFT_SYNTH, 0.0, 0.0, st);
-    kern<<<ctas, nt, smem, st>>>(L, phase, map);
+    kern<<<ctas, nt, smem, st>>>(L, phase, map, minus);
     PS_LAUNCH_CHECK();
     return PS_OK;
   };
@@ -641,14 +659,15 @@ int launch_ring_synth_f64(const Plan& P, const RingClassList* cls, int ncls, con
 }
 
 int launch_ring_adjoint_f64(const Plan& P, const RingClassList* cls, int ncls, const double* map,
-                            int64_t map_stride, double2* phase, int nf, int pack, cudaStream_t st) {
+                            const double2* minus, int64_t map_stride, double2* phase, int nf, int pack, cudaStream_t st) {
   auto go = [&](const RingLaunch& L, int nt, int ctas, size_t smem) -> int {
-    const auto kern = nt == 512 ? ring_adjoint_f64<512> : ring_adjoint_f64<256>;
+    const auto kern = minus ? (nt == 512 ? ring_adjoint_f64<512, true> : ring_adjoint_f64<256, true>)
+                            : (nt == 512 ? ring_adjoint_f64<512, false> : ring_adjoint_f64<256, false>);
     if (smem > 48 * 1024 &&
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
       return PS_ERR_CUDA;
     StatScope sc(PS_K_FFT_ADJOINT, 0.0, 0.0, st);
-    kern<<<ctas, nt, smem, st>>>(L, map, phase);
+    kern<<<ctas, nt, smem, st>>>(L, map, minus, phase);
     PS_LAUNCH_CHECK();
     return PS_OK;
   };

@@ -212,7 +212,9 @@ __global__ void __launch_bounds__(SYN_THREADS) synth0_f64(const RingInfo* __rest
 
 // =====================================================================
 // synthesis, spin s > 0: alm [B][2][nalm] (G, C) -> phase [R][mmax+1][B][2] (Q, U)
-template <int RPT>
+// GRAD: alm [B][nalm], G = -alm, C = 0.  Then a+ = a- and the sums of both hemispheres follow from those over even and
+// over odd l: four FMAs per l and ring instead of eight, in the same registers.
+template <int RPT, bool GRAD>
 __global__ void __launch_bounds__(SYN_THREADS) synthS_f64(const RingInfo* __restrict__ rings,
                                                            const SeedNorm* __restrict__ seednorm,
                                                            const double2* __restrict__ lcd,
@@ -239,13 +241,17 @@ __global__ void __launch_bounds__(SYN_THREADS) synthS_f64(const RingInfo* __rest
     pc = l0 + lane < lmax ? lcd[idx] : make_double2(0.0, 0.0);
     const double2 z = make_double2(0.0, 0.0);
     const double2 G = in ? cscale(alm[b * as + idx], gm) : z;
-    const double2 C = in ? cscale(alm[b * as + nalm + idx], gm) : z;
-    pp = make_double2(G.x - C.y, G.y + C.x);
-    pm = make_double2(G.x + C.y, G.y - C.x);
+    if constexpr (GRAD) {
+      pp = pm = G;
+    } else {
+      const double2 C = in ? cscale(alm[b * as + nalm + idx], gm) : z;
+      pp = make_double2(G.x - C.y, G.y + C.x);
+      pm = make_double2(G.x + C.y, G.y - C.x);
+    }
   };
   auto stage = [&](int buf) {
     s_alm[buf][lane][0] = pp;
-    s_alm[buf][lane][1] = pm;
+    if (!GRAD) s_alm[buf][lane][1] = pm;
     s_cd[buf][lane] = pc;
     return __any_sync(0xffffffffu, nonfinite(pp) || nonfinite(pm));
   };
@@ -263,13 +269,13 @@ __global__ void __launch_bounds__(SYN_THREADS) synthS_f64(const RingInfo* __rest
     seed_spin(m, spin, gi, sn, f[i], g[i], k[i]);
     if (rp >= Rh) { f[i] = g[i] = 0.0; k[i] = 0; }
   }
-  // sums on the north ring and, with the sign of l - lmin, on its mirror
+  // sums on the north ring and, with the sign of l - lmin, on its mirror (GRAD: f and g over even, g and f over odd l)
   double2 PN[RPT], MN[RPT], PS[RPT], MS[RPT];
   {
     double2 z = make_double2(0.0, 0.0);
     // alm with l < s do not enter, unless not finite (0 times them)
     for (int l = m; l < min(spin, lmax + 1); ++l)
-      for (int c = 0; c < 2; ++c) z = cfma(0.0, alm[b * as + c * nalm + base + (l - m)], z);
+      for (int c = 0; c < (GRAD ? 1 : 2); ++c) z = cfma(0.0, alm[b * as + c * nalm + base + (l - m)], z);
 #pragma unroll
     for (int i = 0; i < RPT; ++i) PN[i] = MN[i] = PS[i] = MS[i] = z;
   }
@@ -285,16 +291,20 @@ __global__ void __launch_bounds__(SYN_THREADS) synthS_f64(const RingInfo* __rest
       constexpr double SG = decltype(odd)::value ? -1.0 : 1.0;
       const double2 cd = s_cd[buf][j];
       double2 ap = make_double2(0.0, 0.0), am = ap;
-      if (MODE != LEG_DEAD) { ap = s_alm[buf][j][0]; am = s_alm[buf][j][1]; }
+      if (MODE != LEG_DEAD) { ap = s_alm[buf][j][0]; am = GRAD ? ap : s_alm[buf][j][1]; }
 #pragma unroll
       for (int i = 0; i < RPT; ++i) {
         if (MODE != LEG_DEAD) {
           const bool on = MODE == LEG_LIVE || k[i] == 0;
           const double vf = on ? f[i] : 0.0, vg = on ? g[i] : 0.0;
-          PN[i] = cfma(vf, ap, PN[i]);
-          MN[i] = cfma(vg, am, MN[i]);
-          PS[i] = cfma(SG * vg, ap, PS[i]);
-          MS[i] = cfma(SG * vf, am, MS[i]);
+          if constexpr (!GRAD || !decltype(odd)::value) {
+            PN[i] = cfma(vf, ap, PN[i]);
+            MN[i] = cfma(vg, am, MN[i]);
+          }
+          if constexpr (!GRAD || decltype(odd)::value) {
+            PS[i] = cfma(GRAD ? vg : SG * vg, ap, PS[i]);
+            MS[i] = cfma(GRAD ? vf : SG * vf, am, MS[i]);
+          }
         }
         const double fn = fma(fma(cd.x, x[i], cd.y), f[i], -fp[i]);
         const double gn = fma(fma(cd.x, x[i], -cd.y), g[i], -gp[i]);
@@ -332,14 +342,21 @@ __global__ void __launch_bounds__(SYN_THREADS) synthS_f64(const RingInfo* __rest
   for (int i = 0; i < RPT; ++i) {
     const int rp = r0 + 32 * i, rs = R - 1 - rp;
     if (rp >= Rh) break;
+    if constexpr (GRAD) {
+      const double2 fe = PN[i], ge = MN[i], go = PS[i], fo = MS[i];
+      PN[i] = cadd(fe, fo);
+      MN[i] = cadd(ge, go);
+      PS[i] = csub(ge, go);
+      MS[i] = csub(fe, fo);
+    }
     for (int side = 0; side < (rs != rp ? 2 : 1); ++side) {
       const double h = side == 0 ? 0.5 : ss;
       const double2 sp = cscale(side == 0 ? PN[i] : PS[i], h), sm = cscale(side == 0 ? MN[i] : MS[i], h);
       const double2 sum = cadd(sp, sm), dif = csub(sp, sm);
       const double2 q = odd ? dif : sum, u = odd ? sum : dif;
       const int64_t o = (side == 0 ? rp : rs) * (int64_t(mmax + 1) * B * 2) + m * ms + b * bs;
-      phase[o] = make_double2(-q.x, -q.y);
-      phase[o + 1] = make_double2(-u.y, u.x);
+      phase[o] = GRAD ? q : make_double2(-q.x, -q.y);
+      phase[o + 1] = GRAD ? make_double2(u.y, -u.x) : make_double2(-u.y, u.x);
     }
   }
 }
@@ -626,7 +643,7 @@ static double leg_bytes(const Plan& P, int B, int spin) {
 }
 
 int launch_synth_mma_f64(const Plan& P, const double2* alm, int64_t as, double2* phase, int64_t ms, int64_t bs, int B,
-                         int spin, cudaStream_t st);
+                         int spin, bool grad, cudaStream_t st);
 int launch_adjoint_mma_f64(const Plan& P, const double2* phase, int64_t ms, int64_t bs, double2* alm, int64_t as, int B,
                            int spin, double scale, cudaStream_t st);
 
@@ -645,11 +662,11 @@ static void synth0_go(const Plan& P, const double2* alm, int64_t as, double2* ph
   synth0_f64<RPT><<<grid, SYN_THREADS, 0, st>>>(P.d_rings, P.d_mnorm0, P.d_leg_cd[0], P.d_leg_g[0], alm, as, phase,
                                                 ms, bs, P.R, P.Rh, P.lmax, P.mmax, B);
 }
-template <int RPT>
+template <int RPT, bool GRAD>
 static void synthS_go(const Plan& P, const double2* alm, int64_t as, double2* phase, int64_t ms, int64_t bs, int B,
                       int spin, cudaStream_t st) {
   const dim3 grid((P.Rh + SYN_THREADS * RPT - 1) / (SYN_THREADS * RPT), P.mmax + 1, B);
-  synthS_f64<RPT><<<grid, SYN_THREADS, 0, st>>>(P.d_rings, P.d_seed[spin],
+  synthS_f64<RPT, GRAD><<<grid, SYN_THREADS, 0, st>>>(P.d_rings, P.d_seed[spin],
                                                 reinterpret_cast<const double2*>(P.d_leg_cd[spin]), P.d_leg_g[spin],
                                                 alm, as, phase, ms, bs, P.R, P.Rh, P.lmax, P.mmax, B, P.nalm, spin);
 }
@@ -658,25 +675,30 @@ static void synthS_go(const Plan& P, const double2* alm, int64_t as, double2* ph
 // tile run one by one.  Measured, FMA / MMA kernels: spin 0, Nside 512, lmax 1000: 2 maps 357 / 389 us, 4 maps 475 /
 // 397, 24 maps 2880 / 1916; Nside 256, lmax 500, 3 maps 93 / 60.  Spin 2, Nside 512: 2 maps 811 / 805, 24 maps 9646 /
 // 7208; Nside 256, lmax 500, 3 maps 227 / 184 us (the FMA kernels then took four and two maps per CTA).
-// Tile 1 forces single maps, tile 4 (spin s: 2) the MMA.
+// Tile 1 forces single maps, tile 4 (spin s: 2) the MMA.  grad (C = 0), spin 2: Nside 512, lmax 1000 one map 387 us (508
+// with C), 2 maps 761 / 830, 3 maps 1130 / 845; Nside 256, lmax 500 one map 64 (82), 2 maps 124 / 127, 3 maps
+// 178 / 131: the same line, whatever the tile.
 //
 // Rings per thread of single maps: the rings of a thread share each shared-memory broadcast, fewer keep more warps
 // in flight where a plan has few rings.  Measured, one map, spin 0, one / two / four rings: Nside 1024, lmax 2048
 // 1661 / 1417 / 1353 us, Nside 512, lmax 1000 212 / 187 / 184 us, Nside 256, lmax 767 70 / 71 / 81 us; spin 2 (whose
 // eight sums per ring fill the registers) 4165 / 3880 / 3842 us at Nside 1024.
 int launch_legendre_synth_f64(const Plan& P, const double2* alm, int64_t as, double2* phase, int64_t ms, int64_t bs,
-                              int B, int spin, cudaStream_t st) {
+                              int B, int spin, bool grad, cudaStream_t st) {
   StatScope sc(PS_K_LEG_SYNTH, leg_flops(P, B, spin), leg_bytes(P, B, spin), st);
   if (spin > 0 && !P.d_seed[spin]) return PS_ERR_INVALID;
   const int t = P.tile[0][spin];
-  if (t ? t > 1 : B >= 3) return launch_synth_mma_f64(P, alm, as, phase, ms, bs, B, spin, st);
+  if (t && !grad ? t > 1 : B >= 3) return launch_synth_mma_f64(P, alm, as, phase, ms, bs, B, spin, grad, st);
   if (spin == 0) {
     if (P.Rh >= 1024) synth0_go<4>(P, alm, as, phase, ms, bs, B, st);
     else if (P.Rh > 128) synth0_go<2>(P, alm, as, phase, ms, bs, B, st);
     else synth0_go<1>(P, alm, as, phase, ms, bs, B, st);
+  } else if (grad) {
+    if (P.Rh > 128) synthS_go<2, true>(P, alm, as, phase, ms, bs, B, spin, st);
+    else synthS_go<1, true>(P, alm, as, phase, ms, bs, B, spin, st);
   } else {
-    if (P.Rh > 128) synthS_go<2>(P, alm, as, phase, ms, bs, B, spin, st);
-    else synthS_go<1>(P, alm, as, phase, ms, bs, B, spin, st);
+    if (P.Rh > 128) synthS_go<2, false>(P, alm, as, phase, ms, bs, B, spin, st);
+    else synthS_go<1, false>(P, alm, as, phase, ms, bs, B, spin, st);
   }
   PS_LAUNCH_CHECK();
   return PS_OK;

@@ -40,7 +40,7 @@ __device__ __forceinline__ void dmma(double2& d, double a, double b) {
                : "d"(a), "d"(b));
 }
 // The recurrence of one ring pair, and the next values into column `lane` of the warp's tile.
-template <bool SPIN>
+template <bool SPIN, bool GRAD = false>
 struct Ring {
   double x, f, fp, g, gp;
   int k;
@@ -65,8 +65,9 @@ struct Ring {
         if constexpr (MODE != LEG_DEAD) {
           const bool on = MODE == LEG_LIVE || k == 0;
           if constexpr (SPIN) {
-            tile[j][col] = on ? f : 0.0;
-            tile[8 + j][col] = on ? ((j & 1) ? -g : g) : 0.0;
+            const int row = GRAD ? (j >> 1) + 4 * (j & 1) : j;
+            tile[row][col] = on ? f : 0.0;
+            tile[8 + row][col] = on ? ((j & 1) && !GRAD ? -g : g) : 0.0;
           } else {
             tile[8 * h + (j >> 1)][col] = on ? f : 0.0;
           }
@@ -102,16 +103,21 @@ __device__ __forceinline__ int warp_mode(int k, bool force) {
 }
 
 // ------------------------------------------------------------------ synthesis
-// grid (ceil(Rh / 128), mmax+1, groups of `per` maps); per <= 4 NT (spin 0), 2 NT (spin s)
-template <bool SPIN, int NT>
+// grid (ceil(Rh / 128), mmax+1, groups of `per` maps); per <= 4 NT (spin 0 and GRAD), 2 NT (spin s)
+//
+// GRAD: spin s with alm [B][nalm], G = -alm, C = 0.  Then a+ = a- and the sums of both hemispheres follow from those over
+// even and over odd l, a map takes two columns as for spin 0, and half the MMAs remain; the tile's rows are f even, f
+// odd, g even, g odd.
+template <bool SPIN, int NT, bool GRAD = false>
 __global__ void __launch_bounds__(32 * SYN_WARPS) synth_mma_f64(
     const RingInfo* __restrict__ rings, const double* __restrict__ mnorm, const SeedNorm* __restrict__ seednorm,
     const double* __restrict__ lcd, const double* __restrict__ lg, const double2* __restrict__ alm, int64_t as,
     double2* __restrict__ phase, int64_t ms, int64_t bs, int R, int Rh, int lmax, int mmax, int B, int per,
     int64_t nalm,
     int spin) {
-  constexpr int MAPS = SPIN ? 2 * NT : 4 * NT, CH = 32, BLK = SPIN ? 8 : 16;
-  constexpr int AROW = 8 * NT + (SPIN ? 4 : 2);  // B-operand rows l, l + 1, .. (spin 0: l, l + 2, ..) in distinct banks
+  constexpr bool FULL = SPIN && !GRAD;  // four columns per map
+  constexpr int MAPS = FULL ? 2 * NT : 4 * NT, CH = 32, BLK = SPIN ? 8 : 16;
+  constexpr int AROW = 8 * NT + (FULL ? 4 : 2);  // B-operand rows l, l + 1, .. (else l, l + 2, ..) in distinct banks
   const int m = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int b0 = blockIdx.z * per, nb = min(per, B - b0);
   __shared__ __align__(16) double s_lam_[SYN_WARPS][16][SYN_ROW];
@@ -124,7 +130,7 @@ __global__ void __launch_bounds__(32 * SYN_WARPS) synth_mma_f64(
 
   // the chunk's alm: thread -> l = l0 + lane of maps warp, warp + 4, ..
   constexpr int PER = (MAPS + SYN_WARPS - 1) / SYN_WARPS;
-  double2 pa[PER][SPIN ? 2 : 1], pc;
+  double2 pa[PER][FULL ? 2 : 1], pc;
   auto fetch = [&](int l0) {
     const int64_t idx = base + (l0 - m) + lane;
     const bool in = l0 + lane <= lmax;
@@ -133,7 +139,7 @@ __global__ void __launch_bounds__(32 * SYN_WARPS) synth_mma_f64(
     for (int i = 0; i < PER; ++i) {
       const int b = warp + SYN_WARPS * i;
       const bool on = in && b < nb;
-      if constexpr (SPIN) {
+      if constexpr (FULL) {
         const double2 z = make_double2(0.0, 0.0);
         const double2 G = on ? cscale(alm[(b0 + b) * as + idx], gm) : z;
         const double2 C = on ? cscale(alm[(b0 + b) * as + nalm + idx], gm) : z;
@@ -157,8 +163,8 @@ __global__ void __launch_bounds__(32 * SYN_WARPS) synth_mma_f64(
       const int b = warp + SYN_WARPS * i;
       if (b < MAPS) {
 #pragma unroll
-        for (int c = 0; c < (SPIN ? 2 : 1); ++c) {
-          *reinterpret_cast<double2*>(&s_a[buf][lane][b * (SPIN ? 4 : 2) + 2 * c]) = pa[i][c];
+        for (int c = 0; c < (FULL ? 2 : 1); ++c) {
+          *reinterpret_cast<double2*>(&s_a[buf][lane][b * (FULL ? 4 : 2) + 2 * c]) = pa[i][c];
           bad = bad || nonfinite(pa[i][c]);
         }
       }
@@ -171,11 +177,11 @@ __global__ void __launch_bounds__(32 * SYN_WARPS) synth_mma_f64(
   };
 
   fetch(lmin);
-  Ring<SPIN> ring;
+  Ring<SPIN, GRAD> ring;
   ring.seed(rings, wbase + lane, Rh, m, spin, mnorm, seednorm);
-  double2 acc[2][4][NT];
+  double2 acc[GRAD ? 4 : 2][4][NT];  // GRAD: [f, g][even, odd]
 #pragma unroll
-  for (int a = 0; a < 2; ++a)
+  for (int a = 0; a < (GRAD ? 4 : 2); ++a)
 #pragma unroll
     for (int r = 0; r < 4; ++r)
 #pragma unroll
@@ -205,13 +211,13 @@ __global__ void __launch_bounds__(32 * SYN_WARPS) synth_mma_f64(
               fa[r] = v.x;
               fa[r + 1] = v.y;
             }
-            const double* brow = s_a[buf][j0 + (SPIN ? kr : 2 * kr + a)];
+            const double* brow = s_a[buf][j0 + (FULL ? kr : GRAD ? 2 * (lane & 3) + q : 2 * kr + a)];
 #pragma unroll
-            for (int t = 0; t < NT; ++t) fb[t] = brow[8 * t + (SPIN ? ((lane >> 2) ^ (2 * a)) : (lane >> 2))];
+            for (int t = 0; t < NT; ++t) fb[t] = brow[8 * t + (FULL ? ((lane >> 2) ^ (2 * a)) : (lane >> 2))];
 #pragma unroll
             for (int t = 0; t < NT; ++t)
 #pragma unroll
-              for (int r = 0; r < 4; ++r) dmma(acc[a][r][t], fa[r], fb[t]);
+              for (int r = 0; r < 4; ++r) dmma(acc[GRAD ? 2 * a + q : a][r][t], fa[r], fb[t]);
           }
         __syncwarp();
       }
@@ -226,7 +232,23 @@ __global__ void __launch_bounds__(32 * SYN_WARPS) synth_mma_f64(
     if (rp >= Rh) continue;
 #pragma unroll
     for (int t = 0; t < NT; ++t) {
-      if constexpr (SPIN) {
+      if constexpr (GRAD) {
+        const int b = 4 * t + (lane & 3);
+        if (b >= nb) continue;
+        double2 z = make_double2(0.0, 0.0);  // alm with l < s enter only if not finite
+        for (int l = m; l < min(spin, lmax + 1); ++l) z = cfma(0.0, alm[(b0 + b) * as + base + (l - m)], z);
+        const double2 fe = cadd(z, acc[0][r][t]), fo = acc[1][r][t], ge = cadd(z, acc[2][r][t]), go = acc[3][r][t];
+        for (int south = 0; south < (rs != rp ? 2 : 1); ++south) {
+          const double h = south && ((lmin + m) & 1) ? -0.5 : 0.5;
+          const double2 sp = cscale(south ? csub(ge, go) : cadd(fe, fo), h);
+          const double2 sm = cscale(south ? csub(fe, fo) : cadd(ge, go), h);
+          const double2 sum = cadd(sp, sm), dif = csub(sp, sm);
+          const double2 u = (spin & 1) ? sum : dif;
+          const int64_t o = (south ? rs : rp) * row + m * ms + (b0 + b) * bs;
+          phase[o] = (spin & 1) ? dif : sum;
+          phase[o + 1] = make_double2(u.y, -u.x);
+        }
+      } else if constexpr (SPIN) {
         // even lanes: S+ and S- of the north ring, odd lanes those of its mirror (S- in the first tile)
         const int b = 2 * t + ((lane & 3) >> 1);
         const bool south = lane & 1;
@@ -446,11 +468,11 @@ __global__ void __launch_bounds__(32 * ADJ_MMA_WARPS, 3) adj_mma_f64(
   }
 }
 
-template <bool SPIN, int NT>
+template <bool SPIN, int NT, bool GRAD = false>
 int synth_go(const Plan& P, const double2* alm, int64_t as, double2* phase, int64_t ms, int64_t bs, int B, int per,
              int spin, cudaStream_t st) {
   const dim3 grid((P.Rh + 32 * SYN_WARPS - 1) / (32 * SYN_WARPS), P.mmax + 1, (B + per - 1) / per);
-  synth_mma_f64<SPIN, NT><<<grid, 32 * SYN_WARPS, 0, st>>>(P.d_rings, P.d_mnorm0, P.d_seed[spin], P.d_leg_cd[spin],
+  synth_mma_f64<SPIN, NT, GRAD><<<grid, 32 * SYN_WARPS, 0, st>>>(P.d_rings, P.d_mnorm0, P.d_seed[spin], P.d_leg_cd[spin],
                                                            P.d_leg_g[spin], alm, as, phase, ms, bs, P.R, P.Rh, P.lmax,
                                                            P.mmax, B, per, P.nalm, spin);
   PS_LAUNCH_CHECK();
@@ -486,7 +508,12 @@ static int group_maps(int B, int most) {
 }
 
 int launch_synth_mma_f64(const Plan& P, const double2* alm, int64_t as, double2* phase, int64_t ms, int64_t bs, int B,
-                         int spin, cudaStream_t st) {
+                         int spin, bool grad, cudaStream_t st) {
+  if (grad) {
+    const int per = group_maps(B, 8);  // 24 maps, Nside 512, lmax 1000: 5457 us, with C 7318
+    return per <= 4 ? synth_go<true, 1, true>(P, alm, as, phase, ms, bs, B, per, spin, st)
+                    : synth_go<true, 2, true>(P, alm, as, phase, ms, bs, B, per, spin, st);
+  }
   const int per = group_maps(B, spin == 0 ? 12 : 6), nt = (per * (spin == 0 ? 2 : 4) + 7) / 8;
   if (spin == 0)
     return nt == 1   ? synth_go<false, 1>(P, alm, as, phase, ms, bs, B, per, 0, st)

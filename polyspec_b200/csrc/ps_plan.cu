@@ -16,19 +16,20 @@
 namespace ps {
 int launch_leg_tables_f64(const Plan& P, int spin, double* cd, double* gam, cudaStream_t st);
 int launch_legendre_synth_f64(const Plan& P, const double2* alm, int64_t as, double2* phase, int64_t ms, int64_t bs,
-                              int B, int spin, cudaStream_t st);
+                              int B, int spin, bool grad, cudaStream_t st);
+int launch_gc_to_pm(const double2* gc, double2* plus, double2* minus, int B, int64_t nalm, int spin, cudaStream_t st);
 int launch_legendre_adjoint_f64(const Plan& P, const double2* phase, int64_t ms, int64_t bs, double2* alm,
                                 int64_t as, int B, int spin, double scale, cudaStream_t st);
-int launch_alm_to_T(const double2* alm, int64_t stride, const double* lscale, double2* almT, int B, int ncomp,
+int launch_alm_to_T(const double2* alm, int64_t stride, const double* lscale, bool grad, double2* almT, int B, int ncomp,
                     int64_t nalm, cudaStream_t st);
 int launch_ring_synth_f64(const Plan& P, const RingClassList* cls, int ncls, const double2* phase, double* map,
-                          int64_t map_stride, int nf, int pack, cudaStream_t st);
+                          double2* minus, int64_t map_stride, int nf, int pack, cudaStream_t st);
 int launch_ring_adjoint_f64(const Plan& P, const RingClassList* cls, int ncls, const double* map,
-                            int64_t map_stride, double2* phase, int nf, int pack, cudaStream_t st);
+                            const double2* minus, int64_t map_stride, double2* phase, int nf, int pack, cudaStream_t st);
 int launch_ring_synth_f32(const Plan& P, const RingClassList* cls, int ncls, const float2* phase, double* map,
-                          int64_t map_stride, int nf, int pack, cudaStream_t st);
+                          double2* minus, int64_t map_stride, int nf, int pack, cudaStream_t st);
 int launch_ring_adjoint_f32(const Plan& P, const RingClassList* cls, int ncls, const double* map,
-                            int64_t map_stride, float2* phase, int nf, int pack, cudaStream_t st);
+                            const double2* minus, int64_t map_stride, float2* phase, int nf, int pack, cudaStream_t st);
 int launch_legendre_synth_tc(const Plan& P, const double2* almT, float2* phase, int B, int spin, int* err_flag,
                              cudaStream_t st);
 int launch_legendre_adjoint_mx(const Plan& P, const float2* phase, float2* partial, int B, int bofs, int Bc,
@@ -662,8 +663,8 @@ int ps_legendre_synthesis(const ps_plan* plan, const double* alm, double* phase,
   const int ncomp = spin == 0 ? 1 : 2;
   if (P.prec == PS_PREC_MIXED) {
     double2* almT = static_cast<double2*>(workspace);
-    int rc = ps::launch_alm_to_T(reinterpret_cast<const double2*>(alm), int64_t(ncomp) * P.nalm, nullptr, almT, batch,
-                                 ncomp, P.nalm, stream);
+    int rc = ps::launch_alm_to_T(reinterpret_cast<const double2*>(alm), int64_t(ncomp) * P.nalm, nullptr, false, almT,
+                                 batch, ncomp, P.nalm, stream);
     if (rc) return rc;
     float2* ph32 = reinterpret_cast<float2*>(static_cast<char*>(workspace) +
                                              align256(size_t(P.nalm) * batch * ncomp * sizeof(double2)));
@@ -681,7 +682,7 @@ int ps_legendre_synthesis(const ps_plan* plan, const double* alm, double* phase,
   }
   return ps::launch_legendre_synth_f64(P, reinterpret_cast<const double2*>(alm), ncomp * P.nalm,
                                        reinterpret_cast<double2*>(phase), int64_t(batch) * ncomp, ncomp, batch, spin,
-                                       stream);
+                                       false, stream);
 }
 
 int ps_legendre_adjoint(const ps_plan* plan, const double* phase, double* alm, int batch, int spin, double scale,
@@ -725,13 +726,13 @@ int ps_sht_workspace_bytes(const ps_plan* plan, int batch, int spin, int adjoint
   return PS_OK;
 }
 
-int ps_synthesis(const ps_plan* plan, const double* alm, double* map, int batch, int spin, void* workspace,
-                 size_t workspace_bytes, cudaStream_t stream) {
-  return ps_synthesis_strided(plan, alm, 0, map, 0, batch, spin, workspace, workspace_bytes, stream);
-}
+}  // extern "C"
 
-int ps_synthesis_strided(const ps_plan* plan, const double* alm, int64_t alm_stride, double* map, int64_t map_stride,
-                         int batch, int spin, void* workspace, size_t workspace_bytes, cudaStream_t stream) {
+// minus null: maps (or (Q, U)) of alm (or (G, C)); else complex maps Q + iU at map and Q - iU at minus of
+// (G, C) = (-alm, 0)
+static int synthesis(const ps_plan* plan, const double* alm, int64_t alm_stride, double* map, double* minus,
+                     int64_t map_stride, int batch, int spin, void* workspace, size_t workspace_bytes,
+                     cudaStream_t stream) {
   if (!plan || batch < 0 || spin < 0 || spin > 3) return PS_ERR_INVALID;
   if (plan->is_band) return PS_ERR_UNSUPPORTED;
   if (batch == 0) return PS_OK;
@@ -740,9 +741,11 @@ int ps_synthesis_strided(const ps_plan* plan, const double* alm, int64_t alm_str
   if (spin > 0 && !P.d_seed[spin]) return PS_ERR_INVALID;
   if (workspace_bytes < sht_ws_bytes(plan, batch, spin, 0)) return PS_ERR_WORKSPACE;
   const int ncomp = spin == 0 ? 1 : 2;
-  if (alm_stride == 0) alm_stride = ncomp * P.nalm;
-  if (map_stride == 0) map_stride = ncomp * P.npix;
-  if (alm_stride < ncomp * P.nalm || map_stride < ncomp * P.npix) return PS_ERR_INVALID;
+  const int nc = minus ? 1 : ncomp;
+  if (alm_stride == 0) alm_stride = nc * P.nalm;
+  if (map_stride == 0) map_stride = nc * P.npix;
+  if (alm_stride < nc * P.nalm || map_stride < nc * P.npix) return PS_ERR_INVALID;
+  double2* mc = reinterpret_cast<double2*>(minus);
   const int nf = batch * ncomp;
   char* ws = static_cast<char*>(workspace);
   double2* almT = reinterpret_cast<double2*>(ws);
@@ -752,8 +755,8 @@ int ps_synthesis_strided(const ps_plan* plan, const double* alm, int64_t alm_str
     if (nf == 1) {
       almT = reinterpret_cast<double2*>(const_cast<double*>(alm));
     } else {
-      rc = ps::launch_alm_to_T(reinterpret_cast<const double2*>(alm), alm_stride, nullptr, almT, batch, ncomp, P.nalm,
-                               stream);
+      rc = ps::launch_alm_to_T(reinterpret_cast<const double2*>(alm), alm_stride, nullptr, minus != nullptr, almT, batch,
+                               ncomp, P.nalm, stream);
       if (rc) return rc;
     }
     // tensor-core Legendre stage (TF32 x3, FP32 accumulation) and FP32 ring transforms
@@ -765,26 +768,22 @@ int ps_synthesis_strided(const ps_plan* plan, const double* alm, int64_t alm_str
     else
       rc = ps::launch_legendre_synth_tc(P, almT, phase, batch, spin, P.d_err, stream);
     if (rc) return rc;
-    return ps::launch_ring_synth_f32(P, plan->ring_cls.data(), int(plan->ring_cls.size()), phase, map,
+    return ps::launch_ring_synth_f32(P, plan->ring_cls.data(), int(plan->ring_cls.size()), phase, map, mc,
                                      map_stride, nf, spin > 0, stream);
   }
   double2* phase = reinterpret_cast<double2*>(phase_ptr);
   // between the two stages the phases are [R][batch][mmax+1][ncomp]
   rc = ps::launch_legendre_synth_f64(P, reinterpret_cast<const double2*>(alm), alm_stride, phase, ncomp,
-                                     int64_t(P.mmax + 1) * ncomp, batch, spin, stream);
+                                     int64_t(P.mmax + 1) * ncomp, batch, spin, minus != nullptr, stream);
   if (rc) return rc;
-  return ps::launch_ring_synth_f64(P, plan->ring_cls.data(), int(plan->ring_cls.size()), phase, map,
+  return ps::launch_ring_synth_f64(P, plan->ring_cls.data(), int(plan->ring_cls.size()), phase, map, mc,
                                    map_stride, nf, spin > 0, stream);
 }
 
-int ps_adjoint(const ps_plan* plan, const double* map, double* alm, int batch, int spin, double scale,
-               void* workspace, size_t workspace_bytes, cudaStream_t stream) {
-  return ps_adjoint_strided(plan, map, 0, alm, 0, batch, spin, scale, workspace, workspace_bytes, stream);
-}
-
-int ps_adjoint_strided(const ps_plan* plan, const double* map, int64_t map_stride, double* alm, int64_t alm_stride,
-                       int batch, int spin, double scale, void* workspace, size_t workspace_bytes,
-                       cudaStream_t stream) {
+// minus null: of maps (or (Q, U)); else of Q = Re (map + minus) / 2, U = Im (map - minus) / 2 of complex maps
+static int adjoint(const ps_plan* plan, const double* map, const double* minus, int64_t map_stride, double* alm,
+                   int64_t alm_stride, int batch, int spin, double scale, void* workspace, size_t workspace_bytes,
+                   cudaStream_t stream) {
   if (!plan || batch < 0 || spin < 0 || spin > 3) return PS_ERR_INVALID;
   if (plan->is_band) return PS_ERR_UNSUPPORTED;
   if (batch == 0) return PS_OK;
@@ -794,8 +793,10 @@ int ps_adjoint_strided(const ps_plan* plan, const double* map, int64_t map_strid
   if (workspace_bytes < sht_ws_bytes(plan, batch, spin, 1)) return PS_ERR_WORKSPACE;
   const int ncomp = spin == 0 ? 1 : 2;
   if (alm_stride == 0) alm_stride = ncomp * P.nalm;
-  if (map_stride == 0) map_stride = ncomp * P.npix;
-  if (alm_stride < ncomp * P.nalm || map_stride < ncomp * P.npix) return PS_ERR_INVALID;
+  const int nc = minus ? 1 : ncomp;
+  if (map_stride == 0) map_stride = nc * P.npix;
+  if (alm_stride < ncomp * P.nalm || map_stride < nc * P.npix) return PS_ERR_INVALID;
+  const double2* mc = reinterpret_cast<const double2*>(minus);
   const int nf = batch * ncomp;
   char* ws = static_cast<char*>(workspace);
   const size_t phase_bytes = align256(size_t(P.R) * (P.mmax + 1) * nf * sizeof(double2));
@@ -804,7 +805,7 @@ int ps_adjoint_strided(const ps_plan* plan, const double* map, int64_t map_strid
     // FP32 ring transforms, FP64 recurrences with FP32 contractions, FP64 cross-tile sums
     float2* phase = reinterpret_cast<float2*>(ws);
     float2* partial = reinterpret_cast<float2*>(ws + phase_bytes);
-    rc = ps::launch_ring_adjoint_f32(P, plan->ring_cls.data(), int(plan->ring_cls.size()), map, map_stride,
+    rc = ps::launch_ring_adjoint_f32(P, plan->ring_cls.data(), int(plan->ring_cls.size()), map, mc, map_stride,
                                      phase, nf, spin > 0, stream);
     if (rc) return rc;
     TabRef tr;
@@ -824,11 +825,51 @@ int ps_adjoint_strided(const ps_plan* plan, const double* map, int64_t map_strid
     return PS_OK;
   }
   double2* phase = reinterpret_cast<double2*>(ws);
-  rc = ps::launch_ring_adjoint_f64(P, plan->ring_cls.data(), int(plan->ring_cls.size()), map, map_stride,
+  rc = ps::launch_ring_adjoint_f64(P, plan->ring_cls.data(), int(plan->ring_cls.size()), map, mc, map_stride,
                                    phase, nf, spin > 0, stream);
   if (rc) return rc;
   return ps::launch_legendre_adjoint_f64(P, phase, ncomp, int64_t(P.mmax + 1) * ncomp, reinterpret_cast<double2*>(alm),
                                          alm_stride, batch, spin, scale, stream);
+}
+
+extern "C" {
+
+int ps_synthesis(const ps_plan* plan, const double* alm, double* map, int batch, int spin, void* workspace,
+                 size_t workspace_bytes, cudaStream_t stream) {
+  return synthesis(plan, alm, 0, map, nullptr, 0, batch, spin, workspace, workspace_bytes, stream);
+}
+
+int ps_synthesis_strided(const ps_plan* plan, const double* alm, int64_t alm_stride, double* map, int64_t map_stride,
+                         int batch, int spin, void* workspace, size_t workspace_bytes, cudaStream_t stream) {
+  return synthesis(plan, alm, alm_stride, map, nullptr, map_stride, batch, spin, workspace, workspace_bytes, stream);
+}
+
+int ps_synthesis_pm(const ps_plan* plan, const double* alm, double* plus, double* minus, int batch, int spin,
+                    void* workspace, size_t workspace_bytes, cudaStream_t stream) {
+  if (spin < 1 || (batch > 0 && !minus)) return PS_ERR_INVALID;
+  return synthesis(plan, alm, 0, plus, minus, 0, batch, spin, workspace, workspace_bytes, stream);
+}
+
+int ps_adjoint(const ps_plan* plan, const double* map, double* alm, int batch, int spin, double scale,
+               void* workspace, size_t workspace_bytes, cudaStream_t stream) {
+  return adjoint(plan, map, nullptr, 0, alm, 0, batch, spin, scale, workspace, workspace_bytes, stream);
+}
+
+int ps_adjoint_strided(const ps_plan* plan, const double* map, int64_t map_stride, double* alm, int64_t alm_stride,
+                       int batch, int spin, double scale, void* workspace, size_t workspace_bytes,
+                       cudaStream_t stream) {
+  return adjoint(plan, map, nullptr, map_stride, alm, alm_stride, batch, spin, scale, workspace, workspace_bytes,
+                 stream);
+}
+
+int ps_adjoint_pm(const ps_plan* plan, const double* plus, const double* minus, double* gc, double* alm_plus,
+                  double* alm_minus, int batch, int spin, double scale, void* workspace, size_t workspace_bytes,
+                  cudaStream_t stream) {
+  if (spin < 1 || (batch > 0 && (!minus || !alm_plus || !alm_minus))) return PS_ERR_INVALID;
+  const int rc = adjoint(plan, plus, minus, 0, gc, 0, batch, spin, scale, workspace, workspace_bytes, stream);
+  if (rc != PS_OK || batch == 0) return rc;
+  return ps::launch_gc_to_pm(reinterpret_cast<const double2*>(gc), reinterpret_cast<double2*>(alm_plus),
+                             reinterpret_cast<double2*>(alm_minus), batch, plan->p.nalm, spin, stream);
 }
 
 }  // extern "C"

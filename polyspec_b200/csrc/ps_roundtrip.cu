@@ -16,7 +16,7 @@
 struct ps_plan;
 
 namespace ps {
-int launch_alm_to_T(const double2* alm, int64_t stride, const double* lscale, double2* almT, int B, int ncomp,
+int launch_alm_to_T(const double2* alm, int64_t stride, const double* lscale, bool grad, double2* almT, int B, int ncomp,
                     int64_t nalm, cudaStream_t st);
 int launch_tab_synth(const Plan& P, const float* table, const int64_t* d_blockoff, int Rh_table, int toff,
                      const double2* almT, float2* phase, int B, int spin, int* err_flag, cudaStream_t st, int fmt);
@@ -76,7 +76,7 @@ extern "C" int ps_sht_weighted_roundtrip(const ps_plan* plan, const double* alm_
   char* ws = static_cast<char*>(workspace);
   double2* almT = reinterpret_cast<double2*>(ws);
   float2* phase = reinterpret_cast<float2*>(ws + ps::al256(size_t(P.nalm) * nf * sizeof(double2)));
-  rc = ps::launch_alm_to_T(reinterpret_cast<const double2*>(alm_in), alm_stride, lscale, almT, batch, ncomp, P.nalm,
+  rc = ps::launch_alm_to_T(reinterpret_cast<const double2*>(alm_in), alm_stride, lscale, false, almT, batch, ncomp, P.nalm,
                            stream);
   if (rc) return rc;
   rc = ps::launch_tab_synth(P, v.tab, v.off, P.Rh, 0, almT, phase, batch, spin, P.d_err, stream, v.fmt);

@@ -265,6 +265,27 @@ class SHTPlan:
             if nf == 3:
                 self._issue_synthesis(2, B, a + 16 * self.nalm, stride, o + 8 * self.npix, nf * self.npix)
 
+    def synthesis_pm(self, alm, spin):
+        """(+s, -s) maps [2, n, npix] (complex128) of the spin-s transform of (G, C) = (-alm, 0), alm [n, nalm]."""
+        spin = int(spin)
+        self._check_alm(alm, 0)
+        if alm.dim() != 2:
+            raise ValueError("alm must be [n, nalm]")
+        alm, _ = self._maps_in(alm.contiguous(), 1, self.nalm)
+        B = alm.shape[0]
+        out = torch.empty((2, B, self.npix), dtype=torch.complex128, device=alm.device)
+        if B > 0:
+            self._maybe_table(spin)
+            ws, nbytes = self.workspace(B, spin, 0)
+
+            def run(h):
+                _lib.call("ps_synthesis_pm", h, alm.data_ptr(), out.data_ptr(), out.data_ptr() + 16 * B * self.npix, B,
+                          spin, ws.data_ptr(), nbytes, self._stream())
+            # the FP64 kernels follow a rule of their own here, a mixed plan has two pipelines to choose from
+            run(self._h if self.prec == "fp64" else self._pick(("synthesis", spin, B), run))
+            self.n_synthesis += B
+        return out
+
     def weighted_roundtrip(self, alm, weight, lscale=None, scale=1.0, out=None):
         """Fused  out = scale * lscale * Y^H W Y (lscale * alm)  for every field of alm [B, nf, nalm]
         (nf = 1: T, spin 0; nf = 3: T spin 0 and (E, B) spin 2), weight [nf, npix] float64,
@@ -333,3 +354,28 @@ class SHTPlan:
             self._issue_adjoint(0, B, m, stride, o, nf * self.nalm, scale)
             if nf == 3:
                 self._issue_adjoint(2, B, m + 8 * self.npix, stride, o + 16 * self.nalm, nf * self.nalm, scale)
+
+    def adjoint_pm(self, plus, minus, spin, scale=1.0):
+        """(+s, -s) harmonics [2, n, nalm] of the complex maps plus, minus [n, npix] (ps_adjoint_pm)."""
+        spin = int(spin)
+        for t in (plus, minus):
+            if t.dtype != torch.complex128 or not t.is_cuda:
+                raise TypeError("maps must be complex128 CUDA tensors")
+            if t.dim() != 2 or t.shape[-1] != self.npix or t.shape != plus.shape:
+                raise ValueError("maps of shape %s, expected [n, %d] twice" % (tuple(t.shape), self.npix))
+        plus, _ = self._maps_in(plus.contiguous(), 1, self.npix)
+        minus, _ = self._maps_in(minus.contiguous(), 1, self.npix)
+        B = plus.shape[0]
+        out = torch.empty((2, B, self.nalm), dtype=torch.complex128, device=plus.device)
+        if B > 0:
+            self._maybe_table(spin)
+            ws, nbytes = self.workspace(B, spin, 1)
+            gc = torch.empty_like(out)
+
+            def run(h):
+                _lib.call("ps_adjoint_pm", h, plus.data_ptr(), minus.data_ptr(), gc.data_ptr(), out.data_ptr(),
+                          out.data_ptr() + 16 * B * self.nalm, B, spin, float(scale), ws.data_ptr(), nbytes,
+                          self._stream())
+            run(self._pick(("adjoint", spin, B), run))
+            self.n_adjoint += B
+        return out
