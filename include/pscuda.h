@@ -360,6 +360,25 @@ int ps_cg_xr_update(double* x, const int64_t* slot, const double* alpha, const d
                     int batch, int64_t per, cudaStream_t stream);
 int ps_cg_direction(double* p, const double* z, const double* beta, int batch, int64_t per, cudaStream_t stream);
 
+/* One step of the CG of a single system without its transforms (polyspec/weighting.py:326-339), the scalars left on
+ * the device.  Vectors [nf][nalm] complex128 (nf 1 or 3), matrices [nf][nf][nalm], beam [nf][nalm] and w [nalm] float64;
+ * scal: 4 float64 on the device, scal[0] = r^T z before the first step.
+ * ps_cgd_apply: y = beam y + S p in place (p is not y), scal[1] = Sum w Re(p conj(y));
+ * ps_cgd_update: alpha = scal[0] / scal[1]; x += alpha p, r -= alpha q; with Sigma also z = Sigma r and then as
+ * ps_cgd_rz: scal[2] = t / scal[0], scal[0] = t, t = Sum w Re(r conj(z));
+ * ps_cgd_direction: p = z + scal[2] p, beam_p = beam p.
+ * The workspace (zeroed once) belongs to one solve on one stream. */
+int ps_cgd_workspace_bytes(size_t* bytes);
+int ps_cgd_apply(const double* S, const double* beam, const double* w, const double* p, double* y, int nf,
+                 int64_t nalm, double* scal, void* workspace, size_t workspace_bytes, cudaStream_t stream);
+int ps_cgd_update(const double* Sigma, const double* w, const double* p, const double* q, double* x, double* r,
+                  double* z, int nf, int64_t nalm, double* scal, void* workspace, size_t workspace_bytes,
+                  cudaStream_t stream);
+int ps_cgd_rz(const double* w, const double* r, const double* z, int nf, int64_t nalm, double* scal, void* workspace,
+              size_t workspace_bytes, cudaStream_t stream);
+int ps_cgd_direction(const double* beam, const double* z, double* p, double* beam_p, int nf, int64_t nalm,
+                     const double* scal, cudaStream_t stream);
+
 /* ------------------------------------------------ masked-band CG preconditioner
  * M r = Sigma r + Sigma B L^H Om^1/2 K_m^-1 Om^1/2 L B Sigma r (per order m; the m = 0 part
  * of the correction real), L the Legendre synthesis stage on a band plan (ps_plan_band) of

@@ -165,6 +165,15 @@ SIGNATURES = {
     "ps_cg_xr_update": (_c_int, [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int64,
                                  _c_void_p]),
     "ps_cg_direction": (_c_int, [_c_void_p, _c_void_p, _c_void_p, _c_int, _c_int64, _c_void_p]),
+    "ps_cgd_workspace_bytes": (_c_int, [ctypes.POINTER(_c_size_t)]),
+    "ps_cgd_apply": (_c_int, [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int64, _c_void_p,
+                              _c_void_p, _c_size_t, _c_void_p]),
+    "ps_cgd_update": (_c_int, [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int,
+                               _c_int64, _c_void_p, _c_void_p, _c_size_t, _c_void_p]),
+    "ps_cgd_rz": (_c_int, [_c_void_p, _c_void_p, _c_void_p, _c_int, _c_int64, _c_void_p, _c_void_p, _c_size_t,
+                           _c_void_p]),
+    "ps_cgd_direction": (_c_int, [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int64, _c_void_p,
+                                  _c_void_p]),
     "ps_cutprec_create": (_c_int, [_c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_void_p, _c_void_p, _c_void_p,
                                    _c_void_p, ctypes.POINTER(_c_void_p)]),
     "ps_cutprec_destroy": (_c_int, [_c_void_p]),

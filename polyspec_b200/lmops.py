@@ -93,3 +93,40 @@ def direction(p, z, beta):
         raise ValueError("direction needs contiguous complex128 tensors")
     beta = beta.to(torch.float64).contiguous()
     _lib.call("ps_cg_direction", _vp(p), _vp(z), _vp(beta), B, per, _stream())
+
+
+class StepScalars:
+    """The scalars and the reduction workspace of one single-system CG (ps_cgd_*): vectors [nf, nlm] complex128
+    contiguous, nf 1 or 3; S, Sigma float64 [nf, nf, nlm], beam float64 [nf, nlm], w float64 [nlm]."""
+
+    def __init__(self, rz, device):
+        n = ctypes.c_size_t()
+        _lib.call("ps_cgd_workspace_bytes", ctypes.byref(n))
+        self.nbytes = int(n.value)
+        self.ws = torch.zeros(self.nbytes, dtype=torch.uint8, device=device)
+        self.t = torch.zeros(4, dtype=torch.float64, device=device)
+        self.t[0] = rz
+
+    def apply(self, S, beam, w, p, y):
+        """y = beam y + S p in place; p^T y kept."""
+        _lib.call("ps_cgd_apply", _vp(S), _vp(beam), _vp(w), _vp(p), _vp(y), p.shape[0], p.shape[1], _vp(self.t),
+                  _vp(self.ws), self.nbytes, _stream())
+
+    def update(self, Sigma, w, p, q, x, r, z):
+        """x += alpha p, r -= alpha q; with Sigma z = Sigma r and the next r^T z."""
+        _lib.call("ps_cgd_update", _vp(Sigma), _vp(w), _vp(p), _vp(q), _vp(x), _vp(r), _vp(z), p.shape[0], p.shape[1],
+                  _vp(self.t), _vp(self.ws), self.nbytes, _stream())
+
+    def next_rz(self, w, r, z):
+        """The next r^T z and beta."""
+        _lib.call("ps_cgd_rz", _vp(w), _vp(r), _vp(z), r.shape[0], r.shape[1], _vp(self.t), _vp(self.ws), self.nbytes,
+                  _stream())
+
+    def direction(self, beam, z, p, beam_p):
+        """p = z + beta p, beam_p = beam p."""
+        _lib.call("ps_cgd_direction", _vp(beam), _vp(z), _vp(p), _vp(beam_p), p.shape[0], p.shape[1], _vp(self.t),
+                  _stream())
+
+    def rz_pq(self):
+        """(the next r^T z, p^T A p) of the step (waits for them)."""
+        return tuple(self.t[:2].tolist())

@@ -506,9 +506,17 @@ class CGD:
         z = self._apply_M(self.r)
         self.rz = self.dot(self.r, z)
         self.rz0 = float(self.dot(b0, self._apply_M(b0)))
-        self.p = z
+        self.p = z.contiguous()
         self.i = 0
         self.err = self.rz / self.rz0
+        # operands of the fused step (ps_cgd_*), which works on contiguous complex128 vectors of its own
+        self.x, self.r = self.x.contiguous(), self.r.contiguous()
+        W, base = weightings, self.base
+        self.d_Cinv, self.d_Sigma = lmops.real3(W.d_inv_Cl), lmops.real3(W.d_Sigma)
+        self.d_beam = base.dev('beam_lm').expand(self.r.shape).contiguous()
+        self.d_weight = W.d_WNW / W.pixel_area
+        self.scal = lmops.StepScalars(self.rz, base.device)
+        self.beam_p = self._apply_beam(self.p).contiguous()
 
     def dot(self, a, b):
         """m-weighted real inner product sum a b^* (1 + [m > 0]) (polyspec/weighting.py:255)."""
@@ -559,17 +567,23 @@ class CGD:
             raise Exception("Unknown preconditioner %s specified!" % self.preconditioner)
 
     def step(self):
-        Ap = self._apply_A(self.p)
-        alpha = self.rz / self.dot(self.p, Ap)
-        self.x += alpha * self.p
-        self.r -= alpha * Ap
-        del Ap
-        z = self._apply_M(self.r)
-        next_rz = self.dot(self.r, z)
-        self.err = next_rz / self.rz0
-        beta = next_rz / self.rz
-        self.rz = next_rz
-        self.p = z + beta * self.p
+        # A p = C^-1 p + B Y^dagger W N^-1 W Y B p
+        Ap = self.base.to_lm(self.base.to_map(self.beam_p) * self.d_weight)
+        sc = self.scal
+        sc.apply(self.d_Cinv, self.d_beam, self.w, self.p, Ap)
+        if self.preconditioner == 'harmonic':
+            z = torch.empty_like(self.r)
+            sc.update(self.d_Sigma, self.w, self.p, Ap, self.x, self.r, z)
+        else:
+            sc.update(None, self.w, self.p, Ap, self.x, self.r, None)
+            z = self._apply_M(self.r).contiguous()
+            sc.next_rz(self.w, self.r, z)
+        sc.direction(self.d_beam, z, self.p, self.beam_p)
+        rz, pq = sc.rz_pq()
+        if self.rz == 0 or pq == 0:
+            raise ZeroDivisionError("CGD step from a zero residual or direction")
+        self.rz = rz
+        self.err = self.rz / self.rz0
         self.i += 1
 
     def run(self, nstep=10, thresh=1e-6):
