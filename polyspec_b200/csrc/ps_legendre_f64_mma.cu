@@ -6,10 +6,10 @@
 // MMA.  What it needs is eight columns: four maps of spin 0 (re, im) or two of spin s (four sums each).  So this
 // file takes batches and ps_legendre_f64.cu single maps; the rule and both sides' times stand at its launchers.
 //
-// A warp owns 32 ring pairs.  Every lane runs the recurrence of its ring for 16 l (spin 0) or 8 l (spin s: f and
-// (-1)^l g) and drops the values into the warp's shared tile, 16 rows of 32 rings, whose columns are ordered so that
-// one 16-byte read gives a lane the elements of two A operands, 8 rings x 4 l (synthesis) or
-// 8 l x 4 rings (adjoint).  Rows 0-7 hold the l of parity 0 (f), rows 8-15 those of parity 1 ((-1)^l g):
+// A warp owns 32 ring pairs (spin-s synthesis: 16).  Every lane runs the recurrence of its ring for 16 l (spin 0) or
+// 8 l (spin s: f and (-1)^l g) and drops the values into the warp's shared tile, 16 rows of 32 rings, whose columns are
+// ordered so that one 16-byte read gives a lane the elements of two A operands, 8 rings x 4 l (synthesis) or 8 l x 4
+// rings (adjoint).  Rows 0-7 hold the l of parity 0 (f), rows 8-15 those of parity 1 ((-1)^l g):
 //   synthesis spin 0: B = alm; E, O = even and odd sums, north = E + O, south = E - O.
 //   synthesis spin s: B = (a+, (-1)^l a-) for f and, the same columns exchanged, for (-1)^l g; the
 //                     accumulators are the north and south sums of ps_legendre_f64.cu.
@@ -40,7 +40,7 @@ __device__ __forceinline__ void dmma(double2& d, double a, double b) {
                : "d"(a), "d"(b));
 }
 // The recurrence of one ring pair, and the next values into column `lane` of the warp's tile.
-template <bool SPIN, bool GRAD = false>
+template <bool SPIN>
 struct Ring {
   double x, f, fp, g, gp;
   int k;
@@ -65,9 +65,8 @@ struct Ring {
         if constexpr (MODE != LEG_DEAD) {
           const bool on = MODE == LEG_LIVE || k == 0;
           if constexpr (SPIN) {
-            const int row = GRAD ? (j >> 1) + 4 * (j & 1) : j;
-            tile[row][col] = on ? f : 0.0;
-            tile[8 + row][col] = on ? ((j & 1) && !GRAD ? -g : g) : 0.0;
+            tile[j][col] = on ? f : 0.0;
+            tile[8 + j][col] = on ? ((j & 1) ? -g : g) : 0.0;
           } else {
             tile[8 * h + (j >> 1)][col] = on ? f : 0.0;
           }
@@ -102,35 +101,28 @@ __device__ __forceinline__ int warp_mode(int k, bool force) {
   return leg_mode<1>(ks, force);
 }
 
-// ------------------------------------------------------------------ synthesis
-// grid (ceil(Rh / 128), mmax+1, groups of `per` maps); per <= 4 NT (spin 0 and GRAD), 2 NT (spin s)
-//
-// GRAD: spin s with alm [B][nalm], G = -alm, C = 0.  Then a+ = a- and the sums of both hemispheres follow from those over
-// even and over odd l, a map takes two columns as for spin 0, and half the MMAs remain; the tile's rows are f even, f
-// odd, g even, g odd.
-template <bool SPIN, int NT, bool GRAD = false>
-__global__ void __launch_bounds__(32 * SYN_WARPS) synth_mma_f64(
-    const RingInfo* __restrict__ rings, const double* __restrict__ mnorm, const SeedNorm* __restrict__ seednorm,
-    const double* __restrict__ lcd, const double* __restrict__ lg, const double2* __restrict__ alm, int64_t as,
-    double2* __restrict__ phase, int64_t ms, int64_t bs, int R, int Rh, int lmax, int mmax, int B, int per,
-    int64_t nalm,
-    int spin) {
-  constexpr bool FULL = SPIN && !GRAD;  // four columns per map
-  constexpr int MAPS = FULL ? 2 * NT : 4 * NT, CH = 32, BLK = SPIN ? 8 : 16;
-  constexpr int AROW = 8 * NT + (FULL ? 4 : 2);  // B-operand rows l, l + 1, .. (else l, l + 2, ..) in distinct banks
+// ------------------------------------------------------------------ synthesis, spin 0
+// grid (ceil(Rh / 128), mmax+1, groups of `per` maps); per <= 4 NT
+template <int NT>
+__global__ void __launch_bounds__(32 * SYN_WARPS) synth0_mma_f64(
+    const RingInfo* __restrict__ rings, const double* __restrict__ mnorm, const double* __restrict__ lc,
+    const double* __restrict__ lg, const double2* __restrict__ alm, int64_t as, double2* __restrict__ phase, int64_t ms,
+    int64_t bs, int R, int Rh, int lmax, int mmax, int B, int per) {
+  constexpr int MAPS = 4 * NT, CH = 32;
+  constexpr int AROW = 8 * NT + 2;  // B-operand rows l, l + 2, .. in distinct banks
   const int m = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int b0 = blockIdx.z * per, nb = min(per, B - b0);
   __shared__ __align__(16) double s_lam_[SYN_WARPS][16][SYN_ROW];
-  __shared__ __align__(16) double s_cd[2][CH * (SPIN ? 2 : 1)];
+  __shared__ __align__(16) double s_cd[2][CH];
   __shared__ __align__(16) double s_a[2][CH][AROW];
   double(*s_lam)[SYN_ROW] = s_lam_[warp];
   const int wbase = (blockIdx.x * SYN_WARPS + warp) * 32;
   const int64_t base = alm_index(m, m, lmax);
-  const int lmin = SPIN ? max(m, spin) : m;
 
   // the chunk's alm: thread -> l = l0 + lane of maps warp, warp + 4, ..
   constexpr int PER = (MAPS + SYN_WARPS - 1) / SYN_WARPS;
-  double2 pa[PER][FULL ? 2 : 1], pc;
+  double2 pa[PER];
+  double pc;
   auto fetch = [&](int l0) {
     const int64_t idx = base + (l0 - m) + lane;
     const bool in = l0 + lane <= lmax;
@@ -138,23 +130,9 @@ __global__ void __launch_bounds__(32 * SYN_WARPS) synth_mma_f64(
 #pragma unroll
     for (int i = 0; i < PER; ++i) {
       const int b = warp + SYN_WARPS * i;
-      const bool on = in && b < nb;
-      if constexpr (FULL) {
-        const double2 z = make_double2(0.0, 0.0);
-        const double2 G = on ? cscale(alm[(b0 + b) * as + idx], gm) : z;
-        const double2 C = on ? cscale(alm[(b0 + b) * as + nalm + idx], gm) : z;
-        pa[i][0] = make_double2(G.x - C.y, G.y + C.x);
-        const double2 am = make_double2(G.x + C.y, G.y - C.x);
-        pa[i][1] = (lane & 1) ? make_double2(-am.x, -am.y) : am;  // l - lmin has the parity of lane
-      } else {
-        pa[i][0] = on ? cscale(alm[(b0 + b) * as + idx], gm) : make_double2(0.0, 0.0);
-      }
+      pa[i] = in && b < nb ? cscale(alm[(b0 + b) * as + idx], gm) : make_double2(0.0, 0.0);
     }
-    pc = make_double2(0.0, 0.0);
-    if (warp == 0 && l0 + lane < lmax) {
-      if constexpr (SPIN) pc = reinterpret_cast<const double2*>(lcd)[idx];
-      else pc.x = lcd[idx];
-    }
+    pc = warp == 0 && l0 + lane < lmax ? lc[idx] : 0.0;
   };
   auto stage = [&](int buf) {
     bool bad = false;
@@ -162,41 +140,35 @@ __global__ void __launch_bounds__(32 * SYN_WARPS) synth_mma_f64(
     for (int i = 0; i < PER; ++i) {
       const int b = warp + SYN_WARPS * i;
       if (b < MAPS) {
-#pragma unroll
-        for (int c = 0; c < (FULL ? 2 : 1); ++c) {
-          *reinterpret_cast<double2*>(&s_a[buf][lane][b * (FULL ? 4 : 2) + 2 * c]) = pa[i][c];
-          bad = bad || nonfinite(pa[i][c]);
-        }
+        *reinterpret_cast<double2*>(&s_a[buf][lane][2 * b]) = pa[i];
+        bad = bad || nonfinite(pa[i]);
       }
     }
-    if (warp == 0) {
-      if constexpr (SPIN) *reinterpret_cast<double2*>(&s_cd[buf][2 * lane]) = pc;
-      else s_cd[buf][lane] = pc.x;
-    }
+    if (warp == 0) s_cd[buf][lane] = pc;
     return bad;
   };
 
-  fetch(lmin);
-  Ring<SPIN, GRAD> ring;
-  ring.seed(rings, wbase + lane, Rh, m, spin, mnorm, seednorm);
-  double2 acc[GRAD ? 4 : 2][4][NT];  // GRAD: [f, g][even, odd]
+  fetch(m);
+  Ring<false> ring;
+  ring.seed(rings, wbase + lane, Rh, m, 0, mnorm, nullptr);
+  double2 acc[2][4][NT];  // even, odd l
 #pragma unroll
-  for (int a = 0; a < (GRAD ? 4 : 2); ++a)
+  for (int a = 0; a < 2; ++a)
 #pragma unroll
     for (int r = 0; r < 4; ++r)
 #pragma unroll
       for (int t = 0; t < NT; ++t) acc[a][r][t] = make_double2(0.0, 0.0);
   bool force = __syncthreads_or(stage(0));
   int buf = 0;
-  for (int l0 = lmin; l0 <= lmax; l0 += CH, buf ^= 1) {
+  for (int l0 = m; l0 <= lmax; l0 += CH, buf ^= 1) {
     const bool more = l0 + CH <= lmax;
     if (more) fetch(l0 + CH);
     if (wbase < Rh) {
 #pragma unroll 1
-      for (int j0 = 0; j0 < CH && l0 + j0 <= lmax; j0 += BLK) {
+      for (int j0 = 0; j0 < CH && l0 + j0 <= lmax; j0 += 16) {
         const int mode = warp_mode(ring.k, force);
         // ring 16 h + 8 b + c in column 16 h + 2 c + b
-        ring.block(&s_cd[buf][j0 * (SPIN ? 2 : 1)], s_lam, (lane & 16) + 2 * (lane & 7) + ((lane >> 3) & 1), mode);
+        ring.block(&s_cd[buf][j0], s_lam, (lane & 16) + 2 * (lane & 7) + ((lane >> 3) & 1), mode);
         if (mode == LEG_DEAD) continue;
         __syncwarp();
 #pragma unroll
@@ -211,13 +183,13 @@ __global__ void __launch_bounds__(32 * SYN_WARPS) synth_mma_f64(
               fa[r] = v.x;
               fa[r + 1] = v.y;
             }
-            const double* brow = s_a[buf][j0 + (FULL ? kr : GRAD ? 2 * (lane & 3) + q : 2 * kr + a)];
+            const double* brow = s_a[buf][j0 + 2 * kr + a];
 #pragma unroll
-            for (int t = 0; t < NT; ++t) fb[t] = brow[8 * t + (FULL ? ((lane >> 2) ^ (2 * a)) : (lane >> 2))];
+            for (int t = 0; t < NT; ++t) fb[t] = brow[8 * t + (lane >> 2)];
 #pragma unroll
             for (int t = 0; t < NT; ++t)
 #pragma unroll
-              for (int r = 0; r < 4; ++r) dmma(acc[GRAD ? 2 * a + q : a][r][t], fa[r], fb[t]);
+              for (int r = 0; r < 4; ++r) dmma(acc[a][r][t], fa[r], fb[t]);
           }
         __syncwarp();
       }
@@ -225,52 +197,197 @@ __global__ void __launch_bounds__(32 * SYN_WARPS) synth_mma_f64(
     if (more) force = __syncthreads_or(stage(buf ^ 1));
   }
   // lane: ring 8 r + lane / 4, columns 2 (lane & 3) and the next one
-  const int64_t row = int64_t(mmax + 1) * B * (SPIN ? 2 : 1);
+  const int64_t row = int64_t(mmax + 1) * B;
 #pragma unroll
   for (int r = 0; r < 4; ++r) {
     const int rp = wbase + 8 * r + (lane >> 2), rs = R - 1 - rp;
     if (rp >= Rh) continue;
 #pragma unroll
     for (int t = 0; t < NT; ++t) {
+      const int b = 4 * t + (lane & 3);
+      if (b >= nb) continue;
+      const double2 e = acc[0][r][t], d = acc[1][r][t];
+      const int64_t o = m * ms + (b0 + b) * bs;
+      phase[rp * row + o] = cadd(e, d);
+      if (rs != rp) phase[rs * row + o] = csub(e, d);
+    }
+  }
+}
+
+// ------------------------------------------------------------------ synthesis, spin s
+// grid (ceil(Rh / 64), mmax+1, groups of `per` maps).  A warp owns 16 ring pairs: lanes 0-15 run f, lanes 16-31
+// (-1)^l g, which obeys the same recurrence at -x, each with its own scale, so that all lanes do the same.
+//
+// Full: four columns per map, per <= 2 NT.  GRAD: alm [B][nalm], G = -alm, C = 0; then a+ = a- and the sums of both
+// hemispheres follow from those over even and over odd l: two columns per map as for spin 0, per <= 4 NT, half the
+// MMAs; the tile's rows are f even, f odd, g even, g odd.
+//
+// Sixteen rings and twelve maps fill the same accumulators as 32 rings and six maps, with half the recurrences and
+// half the A operands per MMA.  24 maps, Nside 512, lmax 1000: full 7318 us before, now 6893, GRAD 5457 and 4247.
+constexpr int SYNS_ROW = 20;  // row stride of the tile (doubles): as SYN_ROW
+template <int NT, bool GRAD>
+__global__ void __launch_bounds__(32 * SYN_WARPS) synthS_mma_f64(
+    const RingInfo* __restrict__ rings, const SeedNorm* __restrict__ seednorm, const double2* __restrict__ lcd,
+    const double* __restrict__ lg, const double2* __restrict__ alm, int64_t as, double2* __restrict__ phase, int64_t ms,
+    int64_t bs, int R, int Rh, int lmax, int mmax, int B, int per, int64_t nalm, int spin) {
+  constexpr int MAPS = GRAD ? 4 * NT : 2 * NT, CH = 32, NC = GRAD ? 1 : 2, NA = GRAD ? 4 : 2, BLK = 16;
+  constexpr int AROW = 8 * NT + (GRAD ? 2 : 4);  // rows l, l + 1, .. (GRAD: l, l + 2, ..) in distinct banks
+  const int m = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int b0 = blockIdx.z * per, nb = min(per, B - b0);
+  __shared__ __align__(16) double s_lam_[SYN_WARPS][2 * BLK][SYNS_ROW];
+  __shared__ __align__(16) double2 s_cd[2][CH];
+  __shared__ __align__(16) double s_a[2][CH][AROW];
+  double(*s_lam)[SYNS_ROW] = s_lam_[warp];
+  const int wbase = (blockIdx.x * SYN_WARPS + warp) * 16;
+  const int64_t base = alm_index(m, m, lmax);
+  const int lmin = max(m, spin);
+
+  // the chunk's alm: thread -> l = l0 + lane of maps warp, warp + 4, ..
+  constexpr int PER = (MAPS + SYN_WARPS - 1) / SYN_WARPS;
+  double2 pa[PER][NC], pc;
+  auto fetch = [&](int l0) {
+    const int64_t idx = base + (l0 - m) + lane;
+    const bool in = l0 + lane <= lmax;
+    const double gm = in ? lg[idx] : 0.0;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+      const int b = warp + SYN_WARPS * i;
+      const bool on = in && b < nb;
+      const double2 z = make_double2(0.0, 0.0), G = on ? cscale(alm[(b0 + b) * as + idx], gm) : z;
       if constexpr (GRAD) {
-        const int b = 4 * t + (lane & 3);
-        if (b >= nb) continue;
-        double2 z = make_double2(0.0, 0.0);  // alm with l < s enter only if not finite
-        for (int l = m; l < min(spin, lmax + 1); ++l) z = cfma(0.0, alm[(b0 + b) * as + base + (l - m)], z);
-        const double2 fe = cadd(z, acc[0][r][t]), fo = acc[1][r][t], ge = cadd(z, acc[2][r][t]), go = acc[3][r][t];
-        for (int south = 0; south < (rs != rp ? 2 : 1); ++south) {
-          const double h = south && ((lmin + m) & 1) ? -0.5 : 0.5;
-          const double2 sp = cscale(south ? csub(ge, go) : cadd(fe, fo), h);
-          const double2 sm = cscale(south ? csub(fe, fo) : cadd(ge, go), h);
-          const double2 sum = cadd(sp, sm), dif = csub(sp, sm);
-          const double2 u = (spin & 1) ? sum : dif;
-          const int64_t o = (south ? rs : rp) * row + m * ms + (b0 + b) * bs;
-          phase[o] = (spin & 1) ? dif : sum;
-          phase[o + 1] = make_double2(u.y, -u.x);
-        }
-      } else if constexpr (SPIN) {
-        // even lanes: S+ and S- of the north ring, odd lanes those of its mirror (S- in the first tile)
-        const int b = 2 * t + ((lane & 3) >> 1);
-        const bool south = lane & 1;
-        if (b >= nb || (south && rs == rp)) continue;
-        double2 z = make_double2(0.0, 0.0);  // alm with l < s enter only if not finite
-        for (int l = m; l < min(spin, lmax + 1); ++l)
-          for (int c = 0; c < 2; ++c) z = cfma(0.0, alm[(b0 + b) * as + c * nalm + base + (l - m)], z);
-        const double h = south && ((lmin + m) & 1) ? -0.5 : 0.5;
-        const double2 sp = cadd(z, cscale(south ? acc[1][r][t] : acc[0][r][t], h));
-        const double2 sm = cadd(z, cscale(south ? acc[0][r][t] : acc[1][r][t], h));
-        const double2 sum = cadd(sp, sm), dif = csub(sp, sm);
-        const double2 q = (spin & 1) ? dif : sum, u = (spin & 1) ? sum : dif;
-        const int64_t o = (south ? rs : rp) * row + m * ms + (b0 + b) * bs;
-        phase[o] = make_double2(-q.x, -q.y);
-        phase[o + 1] = make_double2(-u.y, u.x);
+        pa[i][0] = G;
       } else {
-        const int b = 4 * t + (lane & 3);
-        if (b >= nb) continue;
-        const double2 e = acc[0][r][t], d = acc[1][r][t];
-        const int64_t o = m * ms + (b0 + b) * bs;
-        phase[rp * row + o] = cadd(e, d);
-        if (rs != rp) phase[rs * row + o] = csub(e, d);
+        const double2 C = on ? cscale(alm[(b0 + b) * as + nalm + idx], gm) : z;
+        pa[i][0] = make_double2(G.x - C.y, G.y + C.x);
+        const double2 am = make_double2(G.x + C.y, G.y - C.x);
+        pa[i][1] = (lane & 1) ? make_double2(-am.x, -am.y) : am;  // l - lmin has the parity of lane
+      }
+    }
+    pc = warp == 0 && l0 + lane < lmax ? lcd[idx] : make_double2(0.0, 0.0);
+  };
+  auto stage = [&](int buf) {
+    bool bad = false;
+#pragma unroll
+    for (int i = 0; i < PER; ++i) {
+      const int b = warp + SYN_WARPS * i;
+      if (b < MAPS) {
+#pragma unroll
+        for (int c = 0; c < NC; ++c) {
+          *reinterpret_cast<double2*>(&s_a[buf][lane][2 * (b * NC + c)]) = pa[i][c];
+          bad = bad || nonfinite(pa[i][c]);
+        }
+      }
+    }
+    if (warp == 0) s_cd[buf][lane] = pc;
+    return bad;
+  };
+
+  fetch(lmin);
+  const int half = lane >> 4, rl = wbase + (lane & 15);
+  const RingInfo& ri = rings[rl < Rh ? rl : 0];
+  double x = ri.z, v, vp = 0.0;
+  int k;
+  {
+    double f, g;
+    seed_spin(m, spin, ri, seednorm[m], f, g, k);
+    v = half ? g : f;
+    if (half) x = -x;
+    if (rl >= Rh) { v = 0.0; k = 0; }
+  }
+  double2 acc[NA][2][NT];  // GRAD: [f, g][even, odd]
+#pragma unroll
+  for (int a = 0; a < NA; ++a)
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+#pragma unroll
+      for (int t = 0; t < NT; ++t) acc[a][r][t] = make_double2(0.0, 0.0);
+  // the values of 16 l into the lane's column: ring 8 b + c in column 2 c + b
+  double* col = &s_lam[BLK * half][2 * (lane & 7) + ((lane >> 3) & 1)];
+  auto steps = [&](auto mode_, const double2* cd) {
+    constexpr int MODE = decltype(mode_)::value;
+#pragma unroll
+    for (int j = 0; j < BLK; ++j) {
+      const double2 c = cd[j];
+      if constexpr (MODE != LEG_DEAD)
+        col[(GRAD ? (j >> 1) + BLK / 2 * (j & 1) : j) * SYNS_ROW] = MODE == LEG_LIVE || k == 0 ? v : 0.0;
+      const double vn = fma(fma(c.x, x, c.y), v, -vp);
+      vp = v;
+      v = vn;
+      if constexpr (MODE != LEG_LIVE) {
+        if ((j & 3) == 3) rescale(k, v, vp);
+      }
+    }
+  };
+  bool force = __syncthreads_or(stage(0));
+  int buf = 0;
+  for (int l0 = lmin; l0 <= lmax; l0 += CH, buf ^= 1) {
+    const bool more = l0 + CH <= lmax;
+    if (more) fetch(l0 + CH);
+    if (wbase < Rh) {
+#pragma unroll 1
+      for (int j0 = 0; j0 < CH && l0 + j0 <= lmax; j0 += BLK) {
+        const int mode = warp_mode(k, force);
+        const double2* cd = &s_cd[buf][j0];
+        if (mode == LEG_LIVE) steps(std::integral_constant<int, LEG_LIVE>{}, cd);
+        else if (mode == LEG_MIXED) steps(std::integral_constant<int, LEG_MIXED>{}, cd);
+        else steps(std::integral_constant<int, LEG_DEAD>{}, cd);
+        if (mode == LEG_DEAD) continue;
+        __syncwarp();
+#pragma unroll
+        for (int a = 0; a < 2; ++a)
+#pragma unroll
+          for (int q = 0; q < BLK / 4; ++q) {
+            const int kr = 4 * q + (lane & 3), odd = GRAD ? q / (BLK / 8) : 0;  // row of the tile's half a
+            const double2 fa = *reinterpret_cast<const double2*>(&s_lam[a * BLK + kr][2 * (lane >> 2)]);
+            const double* brow = s_a[buf][j0 + (GRAD ? 2 * (kr - odd * BLK / 2) + odd : kr)];
+            double fb[NT];
+#pragma unroll
+            for (int t = 0; t < NT; ++t) fb[t] = brow[8 * t + (GRAD ? (lane >> 2) : ((lane >> 2) ^ (2 * a)))];
+#pragma unroll
+            for (int t = 0; t < NT; ++t) {
+              dmma(acc[GRAD ? 2 * a + odd : a][0][t], fa.x, fb[t]);
+              dmma(acc[GRAD ? 2 * a + odd : a][1][t], fa.y, fb[t]);
+            }
+          }
+        __syncwarp();
+      }
+    }
+    if (more) force = __syncthreads_or(stage(buf ^ 1));
+  }
+  // lane: ring 8 r + lane / 4, columns 2 (lane & 3) and the next one
+  const int64_t row = int64_t(mmax + 1) * B * 2;
+  auto put = [&](int ring, int b, double h, double2 sp, double2 sm) {  // sums S+, S- of G + iC, G - iC
+    sp = cscale(sp, h);
+    sm = cscale(sm, h);
+    const double2 sum = cadd(sp, sm), dif = csub(sp, sm);
+    const double2 q = (spin & 1) ? dif : sum, u = (spin & 1) ? sum : dif;
+    const int64_t o = ring * row + m * ms + (b0 + b) * bs;
+    phase[o] = GRAD ? q : make_double2(-q.x, -q.y);
+    phase[o + 1] = GRAD ? make_double2(u.y, -u.x) : make_double2(-u.y, u.x);
+  };
+  const double hs = ((lmin + m) & 1) ? -0.5 : 0.5;
+#pragma unroll
+  for (int r = 0; r < 2; ++r) {
+    const int rp = wbase + 8 * r + (lane >> 2), rs = R - 1 - rp;
+    if (rp >= Rh) continue;
+#pragma unroll
+    for (int t = 0; t < NT; ++t) {
+      // GRAD: both hemispheres in one lane; else even lanes S+ and S- of the north ring, odd lanes those of its
+      // mirror (S- in the first tile)
+      const int b = GRAD ? 4 * t + (lane & 3) : 2 * t + ((lane & 3) >> 1);
+      const bool south = !GRAD && (lane & 1);
+      if (b >= nb || (south && rs == rp)) continue;
+      double2 z = make_double2(0.0, 0.0);  // alm with l < s enter only if not finite
+      for (int l = m; l < min(spin, lmax + 1); ++l)
+        for (int c = 0; c < NC; ++c) z = cfma(0.0, alm[(b0 + b) * as + c * nalm + base + (l - m)], z);
+      if constexpr (GRAD) {
+        const double2 fe = cadd(z, acc[0][r][t]), fo = acc[1][r][t], ge = cadd(z, acc[2][r][t]), go = acc[3][r][t];
+        put(rp, b, 0.5, cadd(fe, fo), csub(ge, go));
+        if (rs != rp) put(rs, b, hs, cadd(ge, go), csub(fe, fo));
+      } else {
+        const double2 s0 = cadd(z, acc[0][r][t]), s1 = cadd(z, acc[1][r][t]);
+        if (south) put(rs, b, hs, s1, s0);
+        else put(rp, b, 0.5, s0, s1);
       }
     }
   }
@@ -468,13 +585,22 @@ __global__ void __launch_bounds__(32 * ADJ_MMA_WARPS, 3) adj_mma_f64(
   }
 }
 
-template <bool SPIN, int NT, bool GRAD = false>
+template <int NT>
 int synth_go(const Plan& P, const double2* alm, int64_t as, double2* phase, int64_t ms, int64_t bs, int B, int per,
-             int spin, cudaStream_t st) {
+             cudaStream_t st) {
   const dim3 grid((P.Rh + 32 * SYN_WARPS - 1) / (32 * SYN_WARPS), P.mmax + 1, (B + per - 1) / per);
-  synth_mma_f64<SPIN, NT, GRAD><<<grid, 32 * SYN_WARPS, 0, st>>>(P.d_rings, P.d_mnorm0, P.d_seed[spin], P.d_leg_cd[spin],
-                                                           P.d_leg_g[spin], alm, as, phase, ms, bs, P.R, P.Rh, P.lmax,
-                                                           P.mmax, B, per, P.nalm, spin);
+  synth0_mma_f64<NT><<<grid, 32 * SYN_WARPS, 0, st>>>(P.d_rings, P.d_mnorm0, P.d_leg_cd[0], P.d_leg_g[0], alm, as, phase,
+                                                      ms, bs, P.R, P.Rh, P.lmax, P.mmax, B, per);
+  PS_LAUNCH_CHECK();
+  return PS_OK;
+}
+template <int NT, bool GRAD>
+int synthS_go(const Plan& P, const double2* alm, int64_t as, double2* phase, int64_t ms, int64_t bs, int B, int per,
+              int spin, cudaStream_t st) {
+  const dim3 grid((P.Rh + 16 * SYN_WARPS - 1) / (16 * SYN_WARPS), P.mmax + 1, (B + per - 1) / per);
+  synthS_mma_f64<NT, GRAD><<<grid, 32 * SYN_WARPS, 0, st>>>(
+      P.d_rings, P.d_seed[spin], reinterpret_cast<const double2*>(P.d_leg_cd[spin]), P.d_leg_g[spin], alm, as, phase, ms,
+      bs, P.R, P.Rh, P.lmax, P.mmax, B, per, P.nalm, spin);
   PS_LAUNCH_CHECK();
   return PS_OK;
 }
@@ -498,7 +624,7 @@ int adj_go(const Plan& P, const double2* phase, int64_t ms, int64_t bs, double2*
 
 }  // namespace
 
-// Maps per group: as few groups as possible, evenly filled; at most 12 (spin 0) or 6 (spin s), the most whose
+// Maps per group: as few groups as possible, evenly filled; at most 12 (adjoint of spin s: 6), the most whose
 // accumulators (synthesis) or B operands (adjoint) leave the registers of three CTAs an SM.  A value computed by the
 // recurrence crosses shared memory twice (16 bytes) for the FMAs of all its maps, which the shared-memory path
 // feeds at about half the MMA's rate for one tile of eight columns and at full rate from three on.
@@ -509,19 +635,23 @@ static int group_maps(int B, int most) {
 
 int launch_synth_mma_f64(const Plan& P, const double2* alm, int64_t as, double2* phase, int64_t ms, int64_t bs, int B,
                          int spin, bool grad, cudaStream_t st) {
-  if (grad) {
-    const int per = group_maps(B, 8);  // 24 maps, Nside 512, lmax 1000: 5457 us, with C 7318
-    return per <= 4 ? synth_go<true, 1, true>(P, alm, as, phase, ms, bs, B, per, spin, st)
-                    : synth_go<true, 2, true>(P, alm, as, phase, ms, bs, B, per, spin, st);
-  }
-  const int per = group_maps(B, spin == 0 ? 12 : 6), nt = (per * (spin == 0 ? 2 : 4) + 7) / 8;
+  const int per = group_maps(B, 12);
   if (spin == 0)
-    return nt == 1   ? synth_go<false, 1>(P, alm, as, phase, ms, bs, B, per, 0, st)
-           : nt == 2 ? synth_go<false, 2>(P, alm, as, phase, ms, bs, B, per, 0, st)
-                     : synth_go<false, 3>(P, alm, as, phase, ms, bs, B, per, 0, st);
-  return nt == 1   ? synth_go<true, 1>(P, alm, as, phase, ms, bs, B, per, spin, st)
-         : nt == 2 ? synth_go<true, 2>(P, alm, as, phase, ms, bs, B, per, spin, st)
-                   : synth_go<true, 3>(P, alm, as, phase, ms, bs, B, per, spin, st);
+    return per <= 4   ? synth_go<1>(P, alm, as, phase, ms, bs, B, per, st)
+           : per <= 8 ? synth_go<2>(P, alm, as, phase, ms, bs, B, per, st)
+                      : synth_go<3>(P, alm, as, phase, ms, bs, B, per, st);
+  if (grad)
+    return per <= 4   ? synthS_go<1, true>(P, alm, as, phase, ms, bs, B, per, spin, st)
+           : per <= 8 ? synthS_go<2, true>(P, alm, as, phase, ms, bs, B, per, spin, st)
+                      : synthS_go<3, true>(P, alm, as, phase, ms, bs, B, per, spin, st);
+  switch ((per + 1) / 2) {
+    case 1: return synthS_go<1, false>(P, alm, as, phase, ms, bs, B, per, spin, st);
+    case 2: return synthS_go<2, false>(P, alm, as, phase, ms, bs, B, per, spin, st);
+    case 3: return synthS_go<3, false>(P, alm, as, phase, ms, bs, B, per, spin, st);
+    case 4: return synthS_go<4, false>(P, alm, as, phase, ms, bs, B, per, spin, st);
+    case 5: return synthS_go<5, false>(P, alm, as, phase, ms, bs, B, per, spin, st);
+    default: return synthS_go<6, false>(P, alm, as, phase, ms, bs, B, per, spin, st);
+  }
 }
 
 int launch_adjoint_mma_f64(const Plan& P, const double2* phase, int64_t ms, int64_t bs, double2* alm, int64_t as, int B,
