@@ -731,7 +731,7 @@ static void adjS_go(const Plan& P, const double2* phase, int64_t ms, int64_t bs,
 // 706 / 759 us and, Nside 256, lmax 767, 259 / 240 us.
 //
 // Batches run on the FP64 MMA.  Measured, FMA / MMA kernels: spin 0, Nside 512, lmax 1000, 4 maps 1011 / 593 us, 24
-// maps 6002 / 2999; Nside 256, lmax 767, 2 maps 171 / 192, lmax 500, 3 maps 124 / 125.  Spin 2 (the sums of two
+// maps 6002 / 2597; Nside 256, lmax 767, 2 maps 171 / 192, lmax 500, 3 maps 124 / 125.  Spin 2 (the sums of two
 // maps fill a tile): Nside 256, lmax 767, 2 maps 430 / 326, Nside 512, 24 maps 16359 / 9476; one map, half a tile,
 // 707 / 1054.  Tile 1 forces single maps of spin 0, tile 4 the MMA.
 int launch_legendre_adjoint_f64(const Plan& P, const double2* phase, int64_t ms, int64_t bs, double2* alm, int64_t as,

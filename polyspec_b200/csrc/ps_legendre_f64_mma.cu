@@ -18,8 +18,11 @@
 //                     for both: columns T+ and (-1)^l T-.
 // Synthesis: accumulators of the warp's rings stay in registers over all l; the alm of 32 l are staged for the CTA's
 // four warps.  Adjoint: the B operand (phases) stays in registers over all l; per 16 l the warps' sums meet in
-// shared memory and are added up in a fixed order.
+// shared memory and are added up in a fixed order.  What bounds it is the latency of twelve warps an SM (the B
+// operand takes their registers): the MMA pipe is busy 41 % of the time.  Running the next tile's recurrence between
+// one tile's MMAs (two tiles a warp) was slower, 2806 us for 2667: it spills, and its FMAs queue behind the MMAs.
 #include <algorithm>
+#include <climits>
 #include <type_traits>
 
 #include "ps_legendre_f64.cuh"
@@ -398,9 +401,16 @@ __global__ void __launch_bounds__(32 * SYN_WARPS) synthS_mma_f64(
 template <bool SPIN, int NT>
 struct AdjShared {
   double lam[ADJ_MMA_WARPS][16][ADJ_ROW];
-  double2 red[2][ADJ_MMA_WARPS][16][4 * NT];  // [l][column pair]
+  // Column pairs of 16 l, as rows of l (spin s) or of the even and then the odd l (spin 0).  Rows are 16 banks apart
+  // and the pairs of a row exchanged, so that neither the MMAs' layout (two rows of four pairs an access phase) nor the
+  // sums' (one pair of eight rows) meets a bank twice.
+  // 24 maps, Nside 512, lmax 1000, spin 0: 2950 us with plain rows (eight lanes of the sums on a bank), 2667 so.
+  double2 red[2][ADJ_MMA_WARPS][16][4 * (NT | 1)];
+  __device__ static int row(int l) { return SPIN ? l : 8 * (l & 1) + (l >> 1); }
+  __device__ static int pair(int row, int p) { return p ^ (SPIN ? (row >> 1) & 3 : ((row >> 1) & 1) | ((row >> 2) & 2)); }
   double2 cd[2][SPIN ? 16 : 8];
   unsigned bad[ADJ_MMA_WARPS];  // maps with a phase that is not finite
+  int start[ADJ_MMA_WARPS];     // first l with a value of the warp's rings above 2^-400
 };
 template <bool SPIN, int NT>
 __global__ void __launch_bounds__(32 * ADJ_MMA_WARPS, 3) adj_mma_f64(
@@ -463,21 +473,42 @@ __global__ void __launch_bounds__(32 * ADJ_MMA_WARPS, 3) adj_mma_f64(
     bad = __reduce_or_sync(0xffffffffu, bad);
     const bool force = bad != 0;
     if (lane == 0) S.bad[warp] = bad;
-    auto coef = [&](int l) {  // of l, by thread l - l0
+    auto coef = [&](int l) {
       double2 c = make_double2(0.0, 0.0);
-      if (tid < CH && l < lmax) {
+      if (l < lmax) {
         if constexpr (SPIN) c = reinterpret_cast<const double2*>(lcd)[base + (l - m)];
         else c.x = lcd[base + (l - m)];
       }
       return c;
     };
-    auto put_coef = [&](int bu, double2 c) {
+    auto put_coef = [&](double2* cd, double2 c) {  // of l, by thread l - l0
       if (tid < CH) {
-        if constexpr (SPIN) S.cd[bu][tid] = c;
-        else (&S.cd[bu][0].x)[tid] = c.x;
+        if constexpr (SPIN) cd[tid] = c;
+        else (&cd[0].x)[tid] = c.x;
       }
     };
-    put_coef(buf, coef(lmin + tid));
+    // The recurrence alone, without the other warps, up to the first 16 l in which the warp has something to add: a
+    // third of all (l, m, ring) lie before, and each 16 l of them took a barrier, sums of zeros and a read and write of
+    // alm.  24 maps, Nside 512, lmax 1000, spin 0: 2667 us without, 2597 with it.
+    int first = INT_MAX;
+    if (wbase < Rh) {
+      double* st = &s_lam[0][0];
+      first = lmin;
+      double2 c = coef(first + (lane & 15));
+      while (first <= lmax && warp_mode(ring.k, force) == LEG_DEAD) {
+        if (lane < CH) {
+          if constexpr (SPIN) reinterpret_cast<double2*>(st)[lane] = c;
+          else st[lane] = c.x;
+        }
+        __syncwarp();
+        c = coef(first + CH + (lane & 15));
+#pragma unroll
+        for (int i = 0; i < (SPIN ? 2 : 1); ++i) ring.template steps<LEG_DEAD>(st + 16 * i, s_lam, 0);
+        __syncwarp();
+        first += CH;
+      }
+    }
+    if (lane == 0) S.start[warp] = first;
     __syncthreads();
     if (SPIN && m < spin && tid < (spin - m) * nb) {  // l < s: zero, or 0 times a phase that is not finite
       const int b = tid / (spin - m), j = tid - b * (spin - m);
@@ -491,11 +522,24 @@ __global__ void __launch_bounds__(32 * ADJ_MMA_WARPS, 3) adj_mma_f64(
         }
       }
     }
-    for (int l0 = lmin; l0 <= lmax; l0 += CH, buf ^= 1) {
+    int start = lmax + 1;
+#pragma unroll
+    for (int w = 0; w < ADJ_MMA_WARPS; ++w) start = min(start, S.start[w]);
+    if (t0 == 0) {
+      for (int b = 0; b < nb; ++b)
+        for (int l = lmin + tid; l < start; l += 32 * ADJ_MMA_WARPS) {
+          alm[(b0 + b) * as + base + (l - m)] = make_double2(0.0, 0.0);
+          if constexpr (SPIN) alm[(b0 + b) * as + nalm + base + (l - m)] = make_double2(0.0, 0.0);
+        }
+    }
+    put_coef(S.cd[buf], coef(start + (tid & 15)));
+    __syncthreads();
+    for (int l0 = start; l0 <= lmax; l0 += CH, buf ^= 1) {
       const int n = min(CH, lmax - l0 + 1);
-      const double2 cnext = coef(l0 + CH + tid);
+      double2 cnext = make_double2(0.0, 0.0);
+      if (tid < CH) cnext = coef(l0 + CH + tid);
       // thread -> l, re / im and maps warp, warp + 4, ..; what the sums below need from memory is fetched now
-      const int ls = lane >> 1, cs = lane & 1;
+      const int ls = lane >> 1, cs = lane & 1, rs = S.row(ls);
       const int64_t os = base + (l0 - m) + ls;
       const bool ins = ls < n;
       const double gm = ins ? lg[os] : 0.0;
@@ -525,11 +569,10 @@ __global__ void __launch_bounds__(32 * ADJ_MMA_WARPS, 3) adj_mma_f64(
         for (int a = 0; a < (SPIN ? 1 : 2); ++a)
 #pragma unroll
           for (int t = 0; t < NT; ++t) d[a][t] = make_double2(0.0, 0.0);
-        const int mode = wbase < Rh ? warp_mode(ring.k, force) : int(LEG_DEAD);
-        // ring 8 h + 4 b + c in column 8 h + 2 c + b
-        if (wbase < Rh)
-          ring.block(&S.cd[buf][j0].x, s_lam, (lane & 24) + 2 * (lane & 3) + ((lane >> 2) & 1), mode);
-        if (mode != LEG_DEAD) {
+        if (l0 >= first) {
+          // ring 8 h + 4 b + c in column 8 h + 2 c + b
+          ring.block(&S.cd[buf][j0].x, s_lam, (lane & 24) + 2 * (lane & 3) + ((lane >> 2) & 1),
+                     warp_mode(ring.k, force));
           __syncwarp();
 #pragma unroll
           for (int a = 0; a < 2; ++a) {
@@ -550,10 +593,12 @@ __global__ void __launch_bounds__(32 * ADJ_MMA_WARPS, 3) adj_mma_f64(
 #pragma unroll
         for (int a = 0; a < (SPIN ? 1 : 2); ++a)
 #pragma unroll
-          for (int t = 0; t < NT; ++t)
-            S.red[buf][warp][SPIN ? j0 + (lane >> 2) : 2 * (lane >> 2) + a][4 * t + (lane & 3)] = d[a][t];
+          for (int t = 0; t < NT; ++t) {
+            const int r = (SPIN ? j0 : 8 * a) + (lane >> 2);
+            S.red[buf][warp][r][S.pair(r, 4 * t + (lane & 3))] = d[a][t];
+          }
       }
-      put_coef(buf ^ 1, cnext);
+      put_coef(S.cd[buf ^ 1], cnext);
       __syncthreads();
       const double h = gm * scale;
 #pragma unroll
@@ -564,8 +609,8 @@ __global__ void __launch_bounds__(32 * ADJ_MMA_WARPS, 3) adj_mma_f64(
           double tp = 0.0, tm = 0.0;
 #pragma unroll
           for (int w = 0; w < ADJ_MMA_WARPS; ++w) {
-            tp += (&S.red[buf][w][ls][2 * bm].x)[cs];
-            tm += (&S.red[buf][w][ls][2 * bm + 1].x)[cs];
+            tp += (&S.red[buf][w][rs][S.pair(rs, 2 * bm)].x)[cs];
+            tm += (&S.red[buf][w][rs][S.pair(rs, 2 * bm + 1)].x)[cs];
           }
           if (ls & 1) tm = -tm;
           const double sum = 0.5 * h * (tp + tm), dif = 0.5 * h * (tp - tm);
@@ -576,7 +621,7 @@ __global__ void __launch_bounds__(32 * ADJ_MMA_WARPS, 3) adj_mma_f64(
         } else {
           double v = 0.0;
 #pragma unroll
-          for (int w = 0; w < ADJ_MMA_WARPS; ++w) v += (&S.red[buf][w][ls][bm].x)[cs];
+          for (int w = 0; w < ADJ_MMA_WARPS; ++w) v += (&S.red[buf][w][rs][S.pair(rs, bm)].x)[cs];
           (&alm[(b0 + bm) * as + os].x)[cs] = old[i][0] + v * h;
         }
       }
