@@ -127,6 +127,15 @@ int ps_adjoint_strided(const ps_plan* plan, const double* map, int64_t map_strid
                        int batch, int spin, double scale, void* workspace, size_t workspace_bytes,
                        cudaStream_t stream);
 
+/* The three fields of [batch][3][..] arrays of an FP64 plan (spins 0 and 2) in one call: T, E, B alm -> T, Q, U maps
+ * and back (polyspec/base.py:147-176).  As two calls of the strided transforms, but the rings of T and of (Q, U) share a
+ * launch.  Strides as there, at least 3 nalm and 3 npix; PS_ERR_UNSUPPORTED for mixed and band plans. */
+int ps_fields_workspace_bytes(const ps_plan* plan, int batch, size_t* bytes);
+int ps_synthesis_fields(const ps_plan* plan, const double* alm, int64_t alm_stride, double* map, int64_t map_stride,
+                        int batch, void* workspace, size_t workspace_bytes, cudaStream_t stream);
+int ps_adjoint_fields(const ps_plan* plan, const double* map, int64_t map_stride, double* alm, int64_t alm_stride,
+                      int batch, double scale, void* workspace, size_t workspace_bytes, cudaStream_t stream);
+
 /* Spin-s transforms between scalar alm and complex maps (polyspec/base.py:179-232), spin >= 1.
  * ps_synthesis_pm: alm [batch][nalm] -> plus = Q + iU and minus = Q - iU, [batch][npix] complex128 each, of the
  * spin-s maps of (G, C) = (-alm, 0).

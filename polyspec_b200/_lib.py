@@ -39,6 +39,11 @@ SIGNATURES = {
                                       _c_size_t, _c_void_p]),
     "ps_adjoint_strided": (_c_int, [_c_void_p, _c_void_p, _c_int64, _c_void_p, _c_int64, _c_int, _c_int, _c_double,
                                     _c_void_p, _c_size_t, _c_void_p]),
+    "ps_fields_workspace_bytes": (_c_int, [_c_void_p, _c_int, ctypes.POINTER(_c_size_t)]),
+    "ps_synthesis_fields": (_c_int, [_c_void_p, _c_void_p, _c_int64, _c_void_p, _c_int64, _c_int, _c_void_p, _c_size_t,
+                                     _c_void_p]),
+    "ps_adjoint_fields": (_c_int, [_c_void_p, _c_void_p, _c_int64, _c_void_p, _c_int64, _c_int, _c_double, _c_void_p,
+                                   _c_size_t, _c_void_p]),
     "ps_synthesis_pm": (_c_int, [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int, _c_void_p, _c_size_t,
                                  _c_void_p]),
     "ps_adjoint_pm": (_c_int, [_c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_void_p, _c_int, _c_int,

@@ -20,7 +20,10 @@
 // transforms of it, items ordered ring by ring with the fields fastest, so that the CTAs of all
 // maps of a ring share in L2 the sectors of its phases (stored map-innermost).  One launch per
 // class left the chip to a handful of CTAs in most of them: 10 launches of 3 to 40 us for one
-// Nside 256 map.
+// Nside 256 map.  The rings of T and of (Q, U) of the same maps share a launch too: a launch of
+// one map lasts as long as its longest chain of passes, so that two of them side by side take
+// little longer than one.  T, Q, U synthesis, two launches and one: Nside 16 18 and 9.5 us, 128
+// 39 and 20 us, 256 94 and 78 us.
 //
 // The transforms are radix 8 in registers between shared-memory exchanges (one element of
 // padding per eight: the stride-8 accesses are then free of bank conflicts), with a first pass of
@@ -326,14 +329,21 @@ __device__ __forceinline__ void ring_dft(bool blue, double2* a, int N, int M, in
 // ------------------------------------------------------------------ kernels
 // One length class of a launch: CTAs [cta0, next class's cta0) run its `count` items, G to a CTA.
 struct RingClass {
-  int cta0, count, logM, logT, blue;
+  int cta0, count, logM, logT, blue, part;
   const int* rings;
 };
-constexpr int RING_CLASSES = 28;
-struct RingLaunch {
-  int n, units, pack, mmax, R;
+// The fields of one spin: nf of them, of units spin-0 maps or (packed) spin-s maps.
+struct RingPart {
+  int units, pack;
   int64_t nf;
+  double2* phase;
+  double* map;
+};
+constexpr int RING_CLASSES = 56;
+struct RingLaunch {
+  int n, mmax, R;
   int64_t npix, map_stride;  // pixels; from one map to the next
+  RingPart part[2];
   const RingInfo* rings;
   const double2 *tw, *spec, *root, *chirp;
   const int64_t *spec_off, *chirp_off;
@@ -342,8 +352,11 @@ struct RingLaunch {
 
 // What a group of T threads works on: item -> (ring, unit) -> the two packed rows of phases and pixels.
 struct RingItem {
-  int N, M, logM, T, u, fa, fb;
+  int N, M, logM, T, u, fa, fb, pack;
   bool blue, va, vb, turned;  // turned: phi0 = pi / N
+  int64_t nf;
+  double2* phase;
+  double* map;
   const double2 *root, *chirp, *spec;
   int ira, irb;
   int64_t pix_a, pix_b;  // first pixels of the two rows
@@ -362,17 +375,22 @@ __device__ __forceinline__ RingItem ring_item(const RingLaunch& L, double2* smem
   it.M = 1 << c.logM;
   it.blue = c.blue;
   it.va = item < c.count;
-  const int ring = it.va ? item / L.units : 0, unit = it.va ? item - ring * L.units : 0;
+  const RingPart& p = L.part[c.part];
+  it.pack = p.pack;
+  it.nf = p.nf;
+  it.phase = p.phase;
+  it.map = p.map;
+  const int ring = it.va ? item / p.units : 0, unit = it.va ? item - ring * p.units : 0;
   it.ira = c.rings[ring];
-  it.irb = L.pack ? it.ira : L.R - 1 - it.ira;
+  it.irb = it.pack ? it.ira : L.R - 1 - it.ira;
   const RingInfo g = L.rings[it.ira];
   it.N = g.nphi;
   it.pix_a = unit * L.map_stride + g.start;
-  it.pix_b = unit * L.map_stride + (L.pack ? L.npix : 0) + L.rings[it.irb].start;
+  it.pix_b = unit * L.map_stride + (it.pack ? L.npix : 0) + L.rings[it.irb].start;
   it.turned = g.phi_num != 0;
-  it.fa = L.pack ? 2 * unit : unit;
-  it.fb = L.pack ? it.fa + 1 : unit;
-  it.vb = it.va && (L.pack || it.irb != it.ira);
+  it.fa = it.pack ? 2 * unit : unit;
+  it.fb = it.pack ? it.fa + 1 : unit;
+  it.vb = it.va && (it.pack || it.irb != it.ira);
   const int i = it.N / 4;
   it.root = L.root + int64_t(2) * i * (i - 1);
   it.chirp = it.blue ? L.chirp + L.chirp_off[g.bs_slot] : nullptr;
@@ -383,8 +401,8 @@ __device__ __forceinline__ RingItem ring_item(const RingLaunch& L, double2* smem
 
 // Phases are [R][B][mmax+1][ncomp] (ncomp 2 when packed): one transform's run contiguously in m.
 __device__ __forceinline__ int64_t phase_row(const RingLaunch& L, const RingItem& it, int ring, bool second) {
-  const int64_t row = int64_t(L.mmax + 1) * (L.pack ? 2 : 1);
-  return (int64_t(ring) * (L.mmax + 1)) * L.nf + (L.pack ? it.fa / 2 : it.fa) * row + (L.pack && second ? 1 : 0);
+  const int64_t row = int64_t(L.mmax + 1) * (it.pack ? 2 : 1);
+  return (int64_t(ring) * (L.mmax + 1)) * it.nf + (it.pack ? it.fa / 2 : it.fa) * row + (it.pack && second ? 1 : 0);
 }
 
 // What a transform of the synthesis reads at index k: conj(c_a) + i conj(c_b) with
@@ -398,8 +416,8 @@ struct SynthIn {
   // sums over the aliases m0, m0 + dm, ... of ds^j F_m, times sg
   __device__ __forceinline__ void sum(int m0, int dm, double sg, double ds, double2& sa, double2& sb) const {
     for (int m = m0; m <= mmax; m += dm, sg *= ds) {
-      sa = cfma(sg, pa[int64_t(m) * ms], sa);
-      if (vb) sb = cfma(sg, pb[int64_t(m) * ms], sb);
+      sa = cfma(sg, __ldg(&pa[int64_t(m) * ms]), sa);
+      if (vb) sb = cfma(sg, __ldg(&pb[int64_t(m) * ms]), sb);
     }
   }
   __device__ __forceinline__ double2 combine(int k, double2 ca, double2 cb) const {
@@ -425,10 +443,10 @@ struct SynthIn {
       for (int i = 0; i < C; ++i) {
         const int k = t + (c + i) * q, k2 = k == 0 ? N : N - k;
         const bool on = va && k < N, h1 = on && k <= mmax, h2 = on && k2 <= mmax;
-        a1[i] = h1 ? pa[int64_t(k) * ms] : z;
-        b1[i] = h1 && vb ? pb[int64_t(k) * ms] : z;
-        a2[i] = h2 ? pa[int64_t(k2) * ms] : z;
-        b2[i] = h2 && vb ? pb[int64_t(k2) * ms] : z;
+        a1[i] = h1 ? __ldg(&pa[int64_t(k) * ms]) : z;
+        b1[i] = h1 && vb ? __ldg(&pb[int64_t(k) * ms]) : z;
+        a2[i] = h2 ? __ldg(&pa[int64_t(k2) * ms]) : z;
+        b2[i] = h2 && vb ? __ldg(&pb[int64_t(k2) * ms]) : z;
       }
       if (mmax >= N) {
 #pragma unroll
@@ -449,28 +467,27 @@ struct SynthIn {
 };
 
 // inputs already folded, in shared memory
-    struct PartIn {
-      const double2* part;
-      int N;
-      template <int K>
-      __device__ __forceinline__ void load(double2* x, int t, int q) const {
+struct PartIn {
+  const double2* part;
+  int N;
+  template <int K>
+  __device__ __forceinline__ void load(double2* x, int t, int q) const {
 #pragma unroll
-        for (int i = 0; i < K; ++i) x[i] = t + i * q < N ? part[t + i * q] : make_double2(0.0, 0.0);
-      }
-    };
+    for (int i = 0; i < K; ++i) x[i] = t + i * q < N ? part[t + i * q] : make_double2(0.0, 0.0);
+  }
+};
 
 // synthesis: phase -> maps, or (PAIR, packed) complex maps Q + iU at map and Q - iU at minus
 template <int NT, bool PAIR>
 __global__ void __launch_bounds__(NT, 512 / NT) ring_synth_f64(const __grid_constant__ RingLaunch L,
-                                                               const double2* __restrict__ phase,
-                                                               double* __restrict__ map, double2* __restrict__ minus) {
+                                                               double2* __restrict__ minus) {
   extern __shared__ double2 smem[];
   const RingItem it = ring_item(L, smem);
   const int N = it.N, T = it.T, u = it.u;
   SynthIn in;
-  in.pa = phase + phase_row(L, it, it.ira, false);
-  in.pb = phase + phase_row(L, it, it.irb, true);
-  in.ms = L.pack ? 2 : 1;
+  in.pa = it.phase + phase_row(L, it, it.ira, false);
+  in.pb = it.phase + phase_row(L, it, it.irb, true);
+  in.ms = it.pack ? 2 : 1;
   in.root = it.root;
   in.chirp = it.chirp;
   in.N = N;
@@ -479,9 +496,9 @@ __global__ void __launch_bounds__(NT, 512 / NT) ring_synth_f64(const __grid_cons
   in.va = it.va;
   in.vb = it.vb;
   in.blue = it.blue;
-  double* oa = map + it.pix_a;
-  double* ob = map + it.pix_b;
-  double2* op = reinterpret_cast<double2*>(map) + it.pix_a;
+  double* oa = it.map + it.pix_a;
+  double* ob = it.map + it.pix_b;
+  double2* op = reinterpret_cast<double2*>(it.map) + it.pix_a;
   double2* om = minus + it.pix_a;
   const double inv = 1.0 / double(it.M);
   auto out = [&](int j, double2 y) {
@@ -541,10 +558,10 @@ struct AdjointIn {
     for (int i = 0; i < K; ++i) {
       const int j = t + i * q;
       if constexpr (PAIR) {
-        const double2 z = make_double2(0.0, 0.0), p = va && j < N ? ip[j] : z, n = va && j < N ? im[j] : z;
+        const double2 z = make_double2(0.0, 0.0), p = va && j < N ? __ldg(&ip[j]) : z, n = va && j < N ? __ldg(&im[j]) : z;
         x[i] = make_double2(0.5 * (p.x + n.x), 0.5 * (p.y - n.y));
       } else {
-        x[i] = make_double2(va && j < N ? ia[j] : 0.0, vb && j < N ? ib[j] : 0.0);
+        x[i] = make_double2(va && j < N ? __ldg(&ia[j]) : 0.0, vb && j < N ? __ldg(&ib[j]) : 0.0);
       }
     }
     if (blue) {
@@ -558,13 +575,11 @@ struct AdjointIn {
 // adjoint: maps, or (PAIR, packed) Q = Re (p + n) / 2, U = Im (p - n) / 2 of the complex maps p and n = minus -> phase
 template <int NT, bool PAIR>
 __global__ void __launch_bounds__(NT, 512 / NT) ring_adjoint_f64(const __grid_constant__ RingLaunch L,
-                                                                 const double* __restrict__ map,
-                                                                 const double2* __restrict__ minus,
-                                                                 double2* __restrict__ phase) {
+                                                                 const double2* __restrict__ minus) {
   extern __shared__ double2 smem[];
   const RingItem it = ring_item(L, smem);
   const int N = it.N, mmax = L.mmax, T = it.T, u = it.u;
-  const AdjointIn<PAIR> in{map + it.pix_a, map + it.pix_b, reinterpret_cast<const double2*>(map) + it.pix_a,
+  const AdjointIn<PAIR> in{it.map + it.pix_a, it.map + it.pix_b, reinterpret_cast<const double2*>(it.map) + it.pix_a,
                            minus + it.pix_a, it.chirp, N, it.va, it.vb, it.blue};
   const double inv = 1.0 / double(it.M);
   auto out = [&](int k, double2 y) {
@@ -574,9 +589,9 @@ __global__ void __launch_bounds__(NT, 512 / NT) ring_adjoint_f64(const __grid_co
   ring_dft(it.blue, it.a, N, it.M, it.logM, it.spec, L.tw, u, T, in, out);
   __syncthreads();
   if (!it.va) return;
-  const int ms = L.pack ? 2 : 1;
-  double2* pa = phase + phase_row(L, it, it.ira, false);
-  double2* pb = phase + phase_row(L, it, it.irb, true);
+  const int ms = it.pack ? 2 : 1;
+  double2* pa = it.phase + phase_row(L, it, it.ira, false);
+  double2* pb = it.phase + phase_row(L, it, it.irb, true);
   for (int m = u; m <= mmax; m += T) {
     const int j = m < N ? 0 : m / N, k = m - j * N;
     const double2 z = it.a[pad8(k)], z2 = cconj(it.a[pad8(k == 0 ? 0 : N - k)]);
@@ -604,13 +619,13 @@ static int ring_logT(int logM, int mmax, int nt) {
 }
 
 template <class Launch>
-static int ring_launches(const Plan& P, const RingClassList* cls, int ncls, int64_t map_stride, int nf, int pack,
-                         Launch go) {
+static int ring_launches(const Plan& P, const RingClassList* cls, int ncls, int64_t map_stride, const RingPart* part,
+                         int nparts, Launch go) {
   RingLaunch L;
-  L.units = pack ? (nf + 1) / 2 : nf;
-  L.pack = pack; L.nf = nf; L.mmax = P.mmax; L.R = P.R; L.npix = P.npix; L.map_stride = map_stride; L.rings = P.d_rings;
+  L.mmax = P.mmax; L.R = P.R; L.npix = P.npix; L.map_stride = map_stride; L.rings = P.d_rings;
   L.tw = P.d_twiddle; L.spec = P.d_bs_spec; L.spec_off = P.d_bs_off;
   L.root = P.d_root; L.chirp = P.d_chirp; L.chirp_off = P.d_chirp_off;
+  for (int p = 0; p < nparts; ++p) L.part[p] = part[p];
   for (int big = 1; big >= 0; --big) {  // work length 8192 first, then all others, longest first
     const int nt = big ? 512 : 256;
     size_t smem = 0;
@@ -618,21 +633,25 @@ static int ring_launches(const Plan& P, const RingClassList* cls, int ncls, int6
     L.n = 0;
     for (int i = 0; i < ncls; ++i) {
       const RingClassList& c = cls[i];
-      const int count = pack ? c.count : c.count_n;
-      if ((c.logM > 12) != (big == 1) || count == 0) continue;
-      if (L.n == RING_CLASSES) return PS_ERR_UNSUPPORTED;
-      RingClass& r = L.c[L.n++];
-      r.cta0 = int(ctas);
-      r.logM = c.logM;
-      r.logT = ring_logT(c.logM, P.mmax, nt);
-      r.blue = c.blue;
-      r.rings = pack ? c.rings : c.rings_n;
-      const int64_t items = int64_t(count) * L.units, G = nt >> r.logT;
-      if (items > 0x7fffffff) return PS_ERR_INVALID;
-      r.count = int(items);
-      ctas += (items + G - 1) / G;
-      const size_t M = size_t(1) << c.logM;
-      smem = std::max(smem, size_t(G) * (M + M / 8 + (size_t(1) << r.logT)) * sizeof(double2));
+      if ((c.logM > 12) != (big == 1)) continue;
+      for (int p = nparts - 1; p >= 0; --p) {
+        const int count = part[p].pack ? c.count : c.count_n;
+        if (count == 0) continue;
+        if (L.n == RING_CLASSES) return PS_ERR_UNSUPPORTED;
+        RingClass& r = L.c[L.n++];
+        r.cta0 = int(ctas);
+        r.logM = c.logM;
+        r.logT = ring_logT(c.logM, P.mmax, nt);
+        r.blue = c.blue;
+        r.part = p;
+        r.rings = part[p].pack ? c.rings : c.rings_n;
+        const int64_t items = int64_t(count) * part[p].units, G = nt >> r.logT;
+        if (items > 0x7fffffff) return PS_ERR_INVALID;
+        r.count = int(items);
+        ctas += (items + G - 1) / G;
+        const size_t M = size_t(1) << c.logM;
+        smem = std::max(smem, size_t(G) * (M + M / 8 + (size_t(1) << r.logT)) * sizeof(double2));
+      }
     }
     if (L.n == 0) continue;
     if (ctas > 0x7fffffff) return PS_ERR_INVALID;
@@ -642,8 +661,12 @@ static int ring_launches(const Plan& P, const RingClassList* cls, int ncls, int6
   return PS_OK;
 }
 
-int launch_ring_synth_f64(const Plan& P, const RingClassList* cls, int ncls, const double2* phase, double* map,
-                          double2* minus, int64_t map_stride, int nf, int pack, cudaStream_t st) {
+static RingPart ring_part(const double2* phase, const double* map, int nf, int pack) {
+  return {pack ? (nf + 1) / 2 : nf, pack, nf, const_cast<double2*>(phase), const_cast<double*>(map)};
+}
+
+static int ring_synth(const Plan& P, const RingClassList* cls, int ncls, const RingPart* part, int nparts,
+                      double2* minus, int64_t map_stride, cudaStream_t st) {
   auto go = [&](const RingLaunch& L, int nt, int ctas, size_t smem) -> int {
     const auto kern = minus ? (nt == 512 ? ring_synth_f64<512, true> : ring_synth_f64<256, true>)
                             : (nt == 512 ? ring_synth_f64<512, false> : ring_synth_f64<256, false>);
@@ -651,15 +674,15 @@ int launch_ring_synth_f64(const Plan& P, const RingClassList* cls, int ncls, con
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
       return PS_ERR_CUDA;
     StatScope sc(PS_K_FFT_SYNTH, 0.0, 0.0, st);
-    kern<<<ctas, nt, smem, st>>>(L, phase, map, minus);
+    kern<<<ctas, nt, smem, st>>>(L, minus);
     PS_LAUNCH_CHECK();
     return PS_OK;
   };
-  return ring_launches(P, cls, ncls, map_stride, nf, pack, go);
+  return ring_launches(P, cls, ncls, map_stride, part, nparts, go);
 }
 
-int launch_ring_adjoint_f64(const Plan& P, const RingClassList* cls, int ncls, const double* map,
-                            const double2* minus, int64_t map_stride, double2* phase, int nf, int pack, cudaStream_t st) {
+static int ring_adjoint(const Plan& P, const RingClassList* cls, int ncls, const RingPart* part, int nparts,
+                        const double2* minus, int64_t map_stride, cudaStream_t st) {
   auto go = [&](const RingLaunch& L, int nt, int ctas, size_t smem) -> int {
     const auto kern = minus ? (nt == 512 ? ring_adjoint_f64<512, true> : ring_adjoint_f64<256, true>)
                             : (nt == 512 ? ring_adjoint_f64<512, false> : ring_adjoint_f64<256, false>);
@@ -667,11 +690,36 @@ int launch_ring_adjoint_f64(const Plan& P, const RingClassList* cls, int ncls, c
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
       return PS_ERR_CUDA;
     StatScope sc(PS_K_FFT_ADJOINT, 0.0, 0.0, st);
-    kern<<<ctas, nt, smem, st>>>(L, map, minus, phase);
+    kern<<<ctas, nt, smem, st>>>(L, minus);
     PS_LAUNCH_CHECK();
     return PS_OK;
   };
-  return ring_launches(P, cls, ncls, map_stride, nf, pack, go);
+  return ring_launches(P, cls, ncls, map_stride, part, nparts, go);
+}
+
+int launch_ring_synth_f64(const Plan& P, const RingClassList* cls, int ncls, const double2* phase, double* map,
+                          double2* minus, int64_t map_stride, int nf, int pack, cudaStream_t st) {
+  const RingPart part = ring_part(phase, map, nf, pack);
+  return ring_synth(P, cls, ncls, &part, 1, minus, map_stride, st);
+}
+
+int launch_ring_adjoint_f64(const Plan& P, const RingClassList* cls, int ncls, const double* map,
+                            const double2* minus, int64_t map_stride, double2* phase, int nf, int pack, cudaStream_t st) {
+  const RingPart part = ring_part(phase, map, nf, pack);
+  return ring_adjoint(P, cls, ncls, &part, 1, minus, map_stride, st);
+}
+
+// T at map and (Q, U) in the two components after it, of `batch` maps; phases of the two spins apart.
+int launch_ring_synth_fields_f64(const Plan& P, const RingClassList* cls, int ncls, const double2* phase0,
+                                 const double2* phase2, double* map, int64_t map_stride, int batch, cudaStream_t st) {
+  const RingPart part[2] = {ring_part(phase0, map, batch, 0), ring_part(phase2, map + P.npix, 2 * batch, 1)};
+  return ring_synth(P, cls, ncls, part, 2, nullptr, map_stride, st);
+}
+
+int launch_ring_adjoint_fields_f64(const Plan& P, const RingClassList* cls, int ncls, const double* map,
+                                   int64_t map_stride, double2* phase0, double2* phase2, int batch, cudaStream_t st) {
+  const RingPart part[2] = {ring_part(phase0, map, batch, 0), ring_part(phase2, map + P.npix, 2 * batch, 1)};
+  return ring_adjoint(P, cls, ncls, part, 2, nullptr, map_stride, st);
 }
 
 }  // namespace ps

@@ -26,6 +26,10 @@ int launch_ring_synth_f64(const Plan& P, const RingClassList* cls, int ncls, con
                           double2* minus, int64_t map_stride, int nf, int pack, cudaStream_t st);
 int launch_ring_adjoint_f64(const Plan& P, const RingClassList* cls, int ncls, const double* map,
                             const double2* minus, int64_t map_stride, double2* phase, int nf, int pack, cudaStream_t st);
+int launch_ring_synth_fields_f64(const Plan& P, const RingClassList* cls, int ncls, const double2* phase0,
+                                 const double2* phase2, double* map, int64_t map_stride, int batch, cudaStream_t st);
+int launch_ring_adjoint_fields_f64(const Plan& P, const RingClassList* cls, int ncls, const double* map,
+                                   int64_t map_stride, double2* phase0, double2* phase2, int batch, cudaStream_t st);
 int launch_ring_synth_f32(const Plan& P, const RingClassList* cls, int ncls, const float2* phase, double* map,
                           double2* minus, int64_t map_stride, int nf, int pack, cudaStream_t st);
 int launch_ring_adjoint_f32(const Plan& P, const RingClassList* cls, int ncls, const double* map,
@@ -832,6 +836,25 @@ static int adjoint(const ps_plan* plan, const double* map, const double* minus, 
                                          alm_stride, batch, spin, scale, stream);
 }
 
+// bytes of the FP64 phases of one field of each map
+static size_t phase_bytes(const ps::Plan& P, int batch) {
+  return align256(size_t(P.R) * (P.mmax + 1) * batch * sizeof(double2));
+}
+
+static int fields_check(const ps_plan* plan, const double* alm, int64_t& alm_stride, const double* map,
+                        int64_t& map_stride, int batch, const void* workspace, size_t workspace_bytes) {
+  if (!plan || batch < 0 || batch > (1 << 29)) return PS_ERR_INVALID;
+  if (plan->is_band || plan->p.prec != PS_PREC_FP64) return PS_ERR_UNSUPPORTED;
+  if (batch == 0) return PS_OK;
+  if (!alm || !map || !workspace) return PS_ERR_INVALID;
+  const ps::Plan& P = plan->p;
+  if (!P.d_seed[2]) return PS_ERR_INVALID;
+  if (workspace_bytes < 3 * phase_bytes(P, batch)) return PS_ERR_WORKSPACE;
+  if (alm_stride == 0) alm_stride = 3 * P.nalm;
+  if (map_stride == 0) map_stride = 3 * P.npix;
+  return alm_stride < 3 * P.nalm || map_stride < 3 * P.npix ? PS_ERR_INVALID : PS_OK;
+}
+
 extern "C" {
 
 int ps_synthesis(const ps_plan* plan, const double* alm, double* map, int batch, int spin, void* workspace,
@@ -860,6 +883,46 @@ int ps_adjoint_strided(const ps_plan* plan, const double* map, int64_t map_strid
                        cudaStream_t stream) {
   return adjoint(plan, map, nullptr, map_stride, alm, alm_stride, batch, spin, scale, workspace, workspace_bytes,
                  stream);
+}
+
+int ps_fields_workspace_bytes(const ps_plan* plan, int batch, size_t* bytes) {
+  if (!plan || !bytes || batch < 0) return PS_ERR_INVALID;
+  *bytes = 3 * phase_bytes(plan->p, batch);
+  return PS_OK;
+}
+
+int ps_synthesis_fields(const ps_plan* plan, const double* alm, int64_t alm_stride, double* map, int64_t map_stride,
+                        int batch, void* workspace, size_t workspace_bytes, cudaStream_t stream) {
+  const int rc0 = fields_check(plan, alm, alm_stride, map, map_stride, batch, workspace, workspace_bytes);
+  if (rc0 != PS_OK || batch == 0) return rc0;
+  const ps::Plan& P = plan->p;
+  const double2* a = reinterpret_cast<const double2*>(alm);
+  double2* phase0 = static_cast<double2*>(workspace);
+  double2* phase2 = reinterpret_cast<double2*>(static_cast<char*>(workspace) + phase_bytes(P, batch));
+  const int64_t row = P.mmax + 1;
+  int rc = ps::launch_legendre_synth_f64(P, a, alm_stride, phase0, 1, row, batch, 0, false, stream);
+  if (rc) return rc;
+  rc = ps::launch_legendre_synth_f64(P, a + P.nalm, alm_stride, phase2, 2, 2 * row, batch, 2, false, stream);
+  if (rc) return rc;
+  return ps::launch_ring_synth_fields_f64(P, plan->ring_cls.data(), int(plan->ring_cls.size()), phase0, phase2, map,
+                                          map_stride, batch, stream);
+}
+
+int ps_adjoint_fields(const ps_plan* plan, const double* map, int64_t map_stride, double* alm, int64_t alm_stride,
+                      int batch, double scale, void* workspace, size_t workspace_bytes, cudaStream_t stream) {
+  const int rc0 = fields_check(plan, alm, alm_stride, map, map_stride, batch, workspace, workspace_bytes);
+  if (rc0 != PS_OK || batch == 0) return rc0;
+  const ps::Plan& P = plan->p;
+  double2* a = reinterpret_cast<double2*>(alm);
+  double2* phase0 = static_cast<double2*>(workspace);
+  double2* phase2 = reinterpret_cast<double2*>(static_cast<char*>(workspace) + phase_bytes(P, batch));
+  const int64_t row = P.mmax + 1;
+  int rc = ps::launch_ring_adjoint_fields_f64(P, plan->ring_cls.data(), int(plan->ring_cls.size()), map, map_stride,
+                                              phase0, phase2, batch, stream);
+  if (rc) return rc;
+  rc = ps::launch_legendre_adjoint_f64(P, phase0, 1, row, a, alm_stride, batch, 0, scale, stream);
+  if (rc) return rc;
+  return ps::launch_legendre_adjoint_f64(P, phase2, 2, 2 * row, a + P.nalm, alm_stride, batch, 2, scale, stream);
 }
 
 int ps_adjoint_pm(const ps_plan* plan, const double* plus, const double* minus, double* gc, double* alm_plus,

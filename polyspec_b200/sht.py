@@ -187,6 +187,21 @@ class SHTPlan:
             self._ws = torch.empty(max(need, 256), dtype=torch.uint8, device=self.device)
         return self._ws, need
 
+    def _joint(self, B):
+        # T and (Q, U) in one call (ps_synthesis_fields): FP64 plans, while a spin's rings do not fill the device by
+        # themselves; more maps gain less and would hold the phases of both spins at once
+        return self.prec == "fp64" and B <= 4
+
+    def _joint_workspace(self, B):
+        need = self._ws_need.get(B)
+        if need is None:
+            n = ctypes.c_size_t()
+            _lib.call("ps_fields_workspace_bytes", self._h, B, ctypes.byref(n))
+            need = self._ws_need[B] = int(n.value)
+        if self._ws is None or self._ws.numel() < need:
+            self._ws = torch.empty(need, dtype=torch.uint8, device=self.device)
+        return self._ws, need
+
     @staticmethod
     def _stream():
         # the current stream's handle, without building a torch.cuda.Stream (4 us a call)
@@ -221,25 +236,33 @@ class SHTPlan:
             return t, t.stride(0)
         return t.contiguous(), nf * n
 
-    def _issue_synthesis(self, spin, B, alm, alm_stride, out, map_stride):
-        """Synthesis of B maps at the addresses and strides of ps_synthesis_strided."""
-        self._maybe_table(spin)
+    def _synthesis_call(self, spin, B, alm, alm_stride, out, map_stride):
+        """run(handle): synthesis of B maps at the addresses and strides of ps_synthesis_strided."""
         ws, nbytes = self.workspace(B, spin, 0)
 
         def run(h):
             _lib.call("ps_synthesis_strided", h, alm, alm_stride, out, map_stride, B, spin, ws.data_ptr(), nbytes,
                       self._stream())
+        return run
+
+    def _issue_synthesis(self, spin, B, alm, alm_stride, out, map_stride):
+        self._maybe_table(spin)
+        run = self._synthesis_call(spin, B, alm, alm_stride, out, map_stride)
         run(self._pick(("synthesis", spin, B), run))
         self.n_synthesis += B
 
-    def _issue_adjoint(self, spin, B, map, map_stride, out, alm_stride, scale):
-        """Adjoint of B maps at the addresses and strides of ps_adjoint_strided."""
-        self._maybe_table(spin)
+    def _adjoint_call(self, spin, B, map, map_stride, out, alm_stride, scale):
+        """run(handle): adjoint of B maps at the addresses and strides of ps_adjoint_strided."""
         ws, nbytes = self.workspace(B, spin, 1)
 
         def run(h):
             _lib.call("ps_adjoint_strided", h, map, map_stride, out, alm_stride, B, spin, float(scale), ws.data_ptr(),
                       nbytes, self._stream())
+        return run
+
+    def _issue_adjoint(self, spin, B, map, map_stride, out, alm_stride, scale):
+        self._maybe_table(spin)
+        run = self._adjoint_call(spin, B, map, map_stride, out, alm_stride, scale)
         run(self._pick(("adjoint", spin, B), run))
         self.n_adjoint += B
 
@@ -261,6 +284,15 @@ class SHTPlan:
         alm, stride = self._maps_in(alm, nf, self.nalm)
         if B > 0:
             a, o = alm.data_ptr(), out.data_ptr()
+            if nf == 3 and self._joint(B):
+                self._pick(("synthesis", 0, B), lambda h: self._synthesis_call(0, B, a, stride, o, 3 * self.npix)(h))
+                self._pick(("synthesis", 2, B), lambda h: self._synthesis_call(
+                    2, B, a + 16 * self.nalm, stride, o + 8 * self.npix, 3 * self.npix)(h))
+                ws, nbytes = self._joint_workspace(B)
+                _lib.call("ps_synthesis_fields", self._h, a, stride, o, 3 * self.npix, B, ws.data_ptr(), nbytes,
+                          self._stream())
+                self.n_synthesis += 2 * B
+                return
             self._issue_synthesis(0, B, a, stride, o, nf * self.npix)
             if nf == 3:
                 self._issue_synthesis(2, B, a + 16 * self.nalm, stride, o + 8 * self.npix, nf * self.npix)
@@ -351,6 +383,15 @@ class SHTPlan:
         maps, stride = self._maps_in(maps, nf, self.npix)
         if B > 0:
             m, o = maps.data_ptr(), out.data_ptr()
+            if nf == 3 and self._joint(B):
+                self._pick(("adjoint", 0, B), lambda h: self._adjoint_call(0, B, m, stride, o, 3 * self.nalm, scale)(h))
+                self._pick(("adjoint", 2, B), lambda h: self._adjoint_call(
+                    2, B, m + 8 * self.npix, stride, o + 16 * self.nalm, 3 * self.nalm, scale)(h))
+                ws, nbytes = self._joint_workspace(B)
+                _lib.call("ps_adjoint_fields", self._h, m, stride, o, 3 * self.nalm, B, float(scale), ws.data_ptr(),
+                          nbytes, self._stream())
+                self.n_adjoint += 2 * B
+                return
             self._issue_adjoint(0, B, m, stride, o, nf * self.nalm, scale)
             if nf == 3:
                 self._issue_adjoint(2, B, m + 8 * self.npix, stride, o + 16 * self.nalm, nf * self.nalm, scale)
