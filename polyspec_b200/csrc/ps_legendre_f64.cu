@@ -113,6 +113,7 @@ __global__ void __launch_bounds__(SYN_THREADS) synth0_f64(const RingInfo* __rest
                                                            const double2* __restrict__ alm, int64_t as,
                                                            double2* __restrict__ phase, int64_t ms, int64_t bs,
                                                            int R, int Rh, int lmax, int mmax, int B) {
+  next_may_start();
   const int m = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, b = blockIdx.z;
   const int wbase = (blockIdx.x * SYN_THREADS + (tid & ~31)) * RPT, r0 = wbase + lane;
   if (wbase >= Rh) return;
@@ -359,6 +360,7 @@ __global__ void __launch_bounds__(SYN_THREADS) synthS_f64(const RingInfo* __rest
       phase[o + 1] = GRAD ? make_double2(u.y, -u.x) : make_double2(-u.y, u.x);
     }
   }
+  end_after_previous();
 }
 
 // ---------------------------------------------------------------- adjoint
@@ -387,6 +389,7 @@ __global__ void __launch_bounds__(32 * NW) adj0_f64(const RingInfo* __restrict__
                                                     const double* __restrict__ lg, const double2* __restrict__ phase,
                                                     int64_t ms, int64_t bs, double2* __restrict__ alm, int64_t as,
                                                     int R, int Rh, int lmax, int mmax, int B, int bofs, double scale) {
+  next_may_start();
   const int m = blockIdx.y, b = bofs + blockIdx.z, tid = threadIdx.x, nt = blockDim.x;
   const int warp = tid >> 5, lane = tid & 31, nw = nt >> 5;
   __shared__ double2 s_red[2][NW][ADJ_LCH];
@@ -629,6 +632,7 @@ __global__ void __launch_bounds__(32 * NW) adjS_f64(const RingInfo* __restrict__
     }
     __syncthreads();
   }
+  end_after_previous();
 }
 
 // ---------------------------------------------------------------- launchers
@@ -643,9 +647,9 @@ static double leg_bytes(const Plan& P, int B, int spin) {
 }
 
 int launch_synth_mma_f64(const Plan& P, const double2* alm, int64_t as, double2* phase, int64_t ms, int64_t bs, int B,
-                         int spin, bool grad, cudaStream_t st);
+                         int spin, bool grad, bool beside, cudaStream_t st);
 int launch_adjoint_mma_f64(const Plan& P, const double2* phase, int64_t ms, int64_t bs, double2* alm, int64_t as, int B,
-                           int spin, double scale, cudaStream_t st);
+                           int spin, double scale, bool beside, cudaStream_t st);
 
 int launch_leg_tables_f64(const Plan& P, int spin, double* cd, double* gam, cudaStream_t st) {
   leg_tables_f64<<<(P.mmax + 64) / 64, 64, 0, st>>>(P.lmax, P.mmax, spin, cd, gam);
@@ -663,12 +667,12 @@ static void synth0_go(const Plan& P, const double2* alm, int64_t as, double2* ph
                                                 ms, bs, P.R, P.Rh, P.lmax, P.mmax, B);
 }
 template <int RPT, bool GRAD>
-static void synthS_go(const Plan& P, const double2* alm, int64_t as, double2* phase, int64_t ms, int64_t bs, int B,
-                      int spin, cudaStream_t st) {
+static int synthS_go(const Plan& P, const double2* alm, int64_t as, double2* phase, int64_t ms, int64_t bs, int B,
+                     int spin, bool beside, cudaStream_t st) {
   const dim3 grid((P.Rh + SYN_THREADS * RPT - 1) / (SYN_THREADS * RPT), P.mmax + 1, B);
-  synthS_f64<RPT, GRAD><<<grid, SYN_THREADS, 0, st>>>(P.d_rings, P.d_seed[spin],
-                                                reinterpret_cast<const double2*>(P.d_leg_cd[spin]), P.d_leg_g[spin],
-                                                alm, as, phase, ms, bs, P.R, P.Rh, P.lmax, P.mmax, B, P.nalm, spin);
+  return launch_leg(beside, synthS_f64<RPT, GRAD>, grid, SYN_THREADS, 0, st, P.d_rings, P.d_seed[spin],
+                    reinterpret_cast<const double2*>(P.d_leg_cd[spin]), P.d_leg_g[spin], alm, as, phase, ms, bs, P.R,
+                    P.Rh, P.lmax, P.mmax, B, P.nalm, spin);
 }
 
 // Batches run on the FP64 MMA, which takes maps four (spin 0) or two (spin s) at a time; fewer maps than most of a
@@ -684,21 +688,21 @@ static void synthS_go(const Plan& P, const double2* alm, int64_t as, double2* ph
 // 1661 / 1417 / 1353 us, Nside 512, lmax 1000 212 / 187 / 184 us, Nside 256, lmax 767 70 / 71 / 81 us; spin 2 (whose
 // eight sums per ring fill the registers) 4165 / 3880 / 3842 us at Nside 1024.
 int launch_legendre_synth_f64(const Plan& P, const double2* alm, int64_t as, double2* phase, int64_t ms, int64_t bs,
-                              int B, int spin, bool grad, cudaStream_t st) {
+                              int B, int spin, bool grad, bool beside, cudaStream_t st) {
   StatScope sc(PS_K_LEG_SYNTH, leg_flops(P, B, spin), leg_bytes(P, B, spin), st);
   if (spin > 0 && !P.d_seed[spin]) return PS_ERR_INVALID;
   const int t = P.tile[0][spin];
-  if (t && !grad ? t > 1 : B >= 3) return launch_synth_mma_f64(P, alm, as, phase, ms, bs, B, spin, grad, st);
+  if (t && !grad ? t > 1 : B >= 3) return launch_synth_mma_f64(P, alm, as, phase, ms, bs, B, spin, grad, beside, st);
   if (spin == 0) {
     if (P.Rh >= 1024) synth0_go<4>(P, alm, as, phase, ms, bs, B, st);
     else if (P.Rh > 128) synth0_go<2>(P, alm, as, phase, ms, bs, B, st);
     else synth0_go<1>(P, alm, as, phase, ms, bs, B, st);
   } else if (grad) {
-    if (P.Rh > 128) synthS_go<2, true>(P, alm, as, phase, ms, bs, B, spin, st);
-    else synthS_go<1, true>(P, alm, as, phase, ms, bs, B, spin, st);
+    return P.Rh > 128 ? synthS_go<2, true>(P, alm, as, phase, ms, bs, B, spin, beside, st)
+                      : synthS_go<1, true>(P, alm, as, phase, ms, bs, B, spin, beside, st);
   } else {
-    if (P.Rh > 128) synthS_go<2, false>(P, alm, as, phase, ms, bs, B, spin, st);
-    else synthS_go<1, false>(P, alm, as, phase, ms, bs, B, spin, st);
+    return P.Rh > 128 ? synthS_go<2, false>(P, alm, as, phase, ms, bs, B, spin, beside, st)
+                      : synthS_go<1, false>(P, alm, as, phase, ms, bs, B, spin, beside, st);
   }
   PS_LAUNCH_CHECK();
   return PS_OK;
@@ -714,13 +718,17 @@ static void adj0_go(const Plan& P, const double2* phase, int64_t ms, int64_t bs,
         scale);
 }
 template <int RPT, int NW>
-static void adjS_go(const Plan& P, const double2* phase, int64_t ms, int64_t bs, double2* alm, int64_t as, int B,
-                    int spin, double scale, cudaStream_t st) {
+static int adjS_go(const Plan& P, const double2* phase, int64_t ms, int64_t bs, double2* alm, int64_t as, int B,
+                   int spin, double scale, bool beside, cudaStream_t st) {
   const int warps = std::min(NW, (P.Rh + 32 * RPT - 1) / (32 * RPT));
-  for (int b0 = 0; b0 < B; b0 += MAX_GRID_Z)
-    adjS_f64<RPT, NW><<<dim3(1, P.mmax + 1, std::min(MAX_GRID_Z, B - b0)), 32 * warps, 0, st>>>(
-        P.d_rings, P.d_seed[spin], reinterpret_cast<const double2*>(P.d_leg_cd[spin]), P.d_leg_g[spin], phase, ms, bs,
-        alm, as, P.R, P.Rh, P.lmax, P.mmax, B, b0, P.nalm, spin, scale);
+  for (int b0 = 0; b0 < B; b0 += MAX_GRID_Z) {
+    const int rc =
+        launch_leg(beside && b0 == 0, adjS_f64<RPT, NW>, dim3(1, P.mmax + 1, std::min(MAX_GRID_Z, B - b0)), 32 * warps,
+                   0, st, P.d_rings, P.d_seed[spin], reinterpret_cast<const double2*>(P.d_leg_cd[spin]),
+                   P.d_leg_g[spin], phase, ms, bs, alm, as, P.R, P.Rh, P.lmax, P.mmax, B, b0, P.nalm, spin, scale);
+    if (rc != PS_OK) return rc;
+  }
+  return PS_OK;
 }
 
 // Rings per thread and warps per CTA.  Four rings halve the share of the warp sums and are used wherever a
@@ -735,12 +743,12 @@ static void adjS_go(const Plan& P, const double2* phase, int64_t ms, int64_t bs,
 // maps fill a tile): Nside 256, lmax 767, 2 maps 430 / 326, Nside 512, 24 maps 16359 / 9476; one map, half a tile,
 // 707 / 1054.  Tile 1 forces single maps of spin 0, tile 4 the MMA.
 int launch_legendre_adjoint_f64(const Plan& P, const double2* phase, int64_t ms, int64_t bs, double2* alm, int64_t as,
-                                int B, int spin, double scale, cudaStream_t st) {
+                                int B, int spin, double scale, bool beside, cudaStream_t st) {
   StatScope sc(PS_K_LEG_ADJOINT, leg_flops(P, B, spin), leg_bytes(P, B, spin), st);
   if (spin > 0 && !P.d_seed[spin]) return PS_ERR_INVALID;
   const int t = P.tile[1][spin];
   if (spin > 0 ? B >= 2 : t ? t > 1 : B >= 4)
-    return launch_adjoint_mma_f64(P, phase, ms, bs, alm, as, B, spin, scale, st);
+    return launch_adjoint_mma_f64(P, phase, ms, bs, alm, as, B, spin, scale, beside, st);
   const int64_t ctas = int64_t(P.mmax + 1) * B;
   if (spin == 0) {
     if (P.Rh > 256 && ctas < 1500) adj0_go<4, 8>(P, phase, ms, bs, alm, as, B, scale, st);
@@ -748,10 +756,10 @@ int launch_legendre_adjoint_f64(const Plan& P, const double2* phase, int64_t ms,
     else if (P.Rh > 64) adj0_go<2, 4>(P, phase, ms, bs, alm, as, B, scale, st);
     else adj0_go<1, 2>(P, phase, ms, bs, alm, as, B, scale, st);
   } else {
-    if (P.Rh > 256 && ctas >= 900) adjS_go<4, 4>(P, phase, ms, bs, alm, as, B, spin, scale, st);
-    else if (P.Rh > 256) adjS_go<2, 8>(P, phase, ms, bs, alm, as, B, spin, scale, st);
-    else if (P.Rh > 64) adjS_go<2, 4>(P, phase, ms, bs, alm, as, B, spin, scale, st);
-    else adjS_go<1, 2>(P, phase, ms, bs, alm, as, B, spin, scale, st);
+    if (P.Rh > 256 && ctas >= 900) return adjS_go<4, 4>(P, phase, ms, bs, alm, as, B, spin, scale, beside, st);
+    if (P.Rh > 256) return adjS_go<2, 8>(P, phase, ms, bs, alm, as, B, spin, scale, beside, st);
+    if (P.Rh > 64) return adjS_go<2, 4>(P, phase, ms, bs, alm, as, B, spin, scale, beside, st);
+    return adjS_go<1, 2>(P, phase, ms, bs, alm, as, B, spin, scale, beside, st);
   }
   PS_LAUNCH_CHECK();
   return PS_OK;

@@ -111,6 +111,7 @@ __global__ void __launch_bounds__(32 * SYN_WARPS) synth0_mma_f64(
     const RingInfo* __restrict__ rings, const double* __restrict__ mnorm, const double* __restrict__ lc,
     const double* __restrict__ lg, const double2* __restrict__ alm, int64_t as, double2* __restrict__ phase, int64_t ms,
     int64_t bs, int R, int Rh, int lmax, int mmax, int B, int per) {
+  next_may_start();
   constexpr int MAPS = 4 * NT, CH = 32;
   constexpr int AROW = 8 * NT + 2;  // B-operand rows l, l + 2, .. in distinct banks
   const int m = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -394,6 +395,7 @@ __global__ void __launch_bounds__(32 * SYN_WARPS) synthS_mma_f64(
       }
     }
   }
+  end_after_previous();
 }
 
 // ------------------------------------------------------------------ adjoint
@@ -419,6 +421,7 @@ __global__ void __launch_bounds__(32 * ADJ_MMA_WARPS, 3) adj_mma_f64(
     int64_t bs, double2* __restrict__ alm, int64_t as, int R, int Rh, int lmax, int mmax, int B, int bofs, int per,
     int64_t nalm,
     int spin, double scale) {
+  if constexpr (!SPIN) next_may_start();
   constexpr int CH = 16, MAPS = SPIN ? 2 * NT : 4 * NT, ITEMS = (MAPS + ADJ_MMA_WARPS - 1) / ADJ_MMA_WARPS;
   extern __shared__ __align__(16) unsigned char adj_smem[];
   AdjShared<SPIN, NT>& S = *reinterpret_cast<AdjShared<SPIN, NT>*>(adj_smem);
@@ -628,6 +631,7 @@ __global__ void __launch_bounds__(32 * ADJ_MMA_WARPS, 3) adj_mma_f64(
     }
     __syncthreads();
   }
+  if constexpr (SPIN) end_after_previous();
 }
 
 template <int NT>
@@ -641,17 +645,15 @@ int synth_go(const Plan& P, const double2* alm, int64_t as, double2* phase, int6
 }
 template <int NT, bool GRAD>
 int synthS_go(const Plan& P, const double2* alm, int64_t as, double2* phase, int64_t ms, int64_t bs, int B, int per,
-              int spin, cudaStream_t st) {
+              int spin, bool beside, cudaStream_t st) {
   const dim3 grid((P.Rh + 16 * SYN_WARPS - 1) / (16 * SYN_WARPS), P.mmax + 1, (B + per - 1) / per);
-  synthS_mma_f64<NT, GRAD><<<grid, 32 * SYN_WARPS, 0, st>>>(
-      P.d_rings, P.d_seed[spin], reinterpret_cast<const double2*>(P.d_leg_cd[spin]), P.d_leg_g[spin], alm, as, phase, ms,
-      bs, P.R, P.Rh, P.lmax, P.mmax, B, per, P.nalm, spin);
-  PS_LAUNCH_CHECK();
-  return PS_OK;
+  return launch_leg(beside, synthS_mma_f64<NT, GRAD>, grid, 32 * SYN_WARPS, 0, st, P.d_rings, P.d_seed[spin],
+                    reinterpret_cast<const double2*>(P.d_leg_cd[spin]), P.d_leg_g[spin], alm, as, phase, ms, bs, P.R,
+                    P.Rh, P.lmax, P.mmax, B, per, P.nalm, spin);
 }
 template <bool SPIN, int NT>
 int adj_go(const Plan& P, const double2* phase, int64_t ms, int64_t bs, double2* alm, int64_t as, int B, int per,
-           int spin, double scale, cudaStream_t st) {
+           int spin, double scale, bool beside, cudaStream_t st) {
   const size_t smem = sizeof(AdjShared<SPIN, NT>);
   if (cudaFuncSetAttribute(adj_mma_f64<SPIN, NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) !=
       cudaSuccess)
@@ -659,10 +661,11 @@ int adj_go(const Plan& P, const double2* phase, int64_t ms, int64_t bs, double2*
   const int step = per * 65535;  // grid limit
   for (int bofs = 0; bofs < B; bofs += step) {
     const int z = (std::min(step, B - bofs) + per - 1) / per;
-    adj_mma_f64<SPIN, NT><<<dim3(1, P.mmax + 1, z), 32 * ADJ_MMA_WARPS, smem, st>>>(
-        P.d_rings, P.d_mnorm0, P.d_seed[spin], P.d_leg_cd[spin], P.d_leg_g[spin], phase, ms, bs, alm, as, P.R, P.Rh,
-        P.lmax, P.mmax, B, bofs, per, P.nalm, spin, scale);
-    PS_LAUNCH_CHECK();
+    const int rc =
+        launch_leg(beside && bofs == 0, adj_mma_f64<SPIN, NT>, dim3(1, P.mmax + 1, z), 32 * ADJ_MMA_WARPS, smem, st,
+                   P.d_rings, P.d_mnorm0, P.d_seed[spin], P.d_leg_cd[spin], P.d_leg_g[spin], phase, ms, bs, alm, as,
+                   P.R, P.Rh, P.lmax, P.mmax, B, bofs, per, P.nalm, spin, scale);
+    if (rc != PS_OK) return rc;
   }
   return PS_OK;
 }
@@ -679,36 +682,36 @@ static int group_maps(int B, int most) {
 }
 
 int launch_synth_mma_f64(const Plan& P, const double2* alm, int64_t as, double2* phase, int64_t ms, int64_t bs, int B,
-                         int spin, bool grad, cudaStream_t st) {
+                         int spin, bool grad, bool beside, cudaStream_t st) {
   const int per = group_maps(B, 12);
   if (spin == 0)
     return per <= 4   ? synth_go<1>(P, alm, as, phase, ms, bs, B, per, st)
            : per <= 8 ? synth_go<2>(P, alm, as, phase, ms, bs, B, per, st)
                       : synth_go<3>(P, alm, as, phase, ms, bs, B, per, st);
   if (grad)
-    return per <= 4   ? synthS_go<1, true>(P, alm, as, phase, ms, bs, B, per, spin, st)
-           : per <= 8 ? synthS_go<2, true>(P, alm, as, phase, ms, bs, B, per, spin, st)
-                      : synthS_go<3, true>(P, alm, as, phase, ms, bs, B, per, spin, st);
+    return per <= 4   ? synthS_go<1, true>(P, alm, as, phase, ms, bs, B, per, spin, beside, st)
+           : per <= 8 ? synthS_go<2, true>(P, alm, as, phase, ms, bs, B, per, spin, beside, st)
+                      : synthS_go<3, true>(P, alm, as, phase, ms, bs, B, per, spin, beside, st);
   switch ((per + 1) / 2) {
-    case 1: return synthS_go<1, false>(P, alm, as, phase, ms, bs, B, per, spin, st);
-    case 2: return synthS_go<2, false>(P, alm, as, phase, ms, bs, B, per, spin, st);
-    case 3: return synthS_go<3, false>(P, alm, as, phase, ms, bs, B, per, spin, st);
-    case 4: return synthS_go<4, false>(P, alm, as, phase, ms, bs, B, per, spin, st);
-    case 5: return synthS_go<5, false>(P, alm, as, phase, ms, bs, B, per, spin, st);
-    default: return synthS_go<6, false>(P, alm, as, phase, ms, bs, B, per, spin, st);
+    case 1: return synthS_go<1, false>(P, alm, as, phase, ms, bs, B, per, spin, beside, st);
+    case 2: return synthS_go<2, false>(P, alm, as, phase, ms, bs, B, per, spin, beside, st);
+    case 3: return synthS_go<3, false>(P, alm, as, phase, ms, bs, B, per, spin, beside, st);
+    case 4: return synthS_go<4, false>(P, alm, as, phase, ms, bs, B, per, spin, beside, st);
+    case 5: return synthS_go<5, false>(P, alm, as, phase, ms, bs, B, per, spin, beside, st);
+    default: return synthS_go<6, false>(P, alm, as, phase, ms, bs, B, per, spin, beside, st);
   }
 }
 
 int launch_adjoint_mma_f64(const Plan& P, const double2* phase, int64_t ms, int64_t bs, double2* alm, int64_t as, int B,
-                           int spin, double scale, cudaStream_t st) {
+                           int spin, double scale, bool beside, cudaStream_t st) {
   const int per = group_maps(B, spin == 0 ? 12 : 6), nt = (per * (spin == 0 ? 2 : 4) + 7) / 8;
   if (spin == 0)
-    return nt == 1   ? adj_go<false, 1>(P, phase, ms, bs, alm, as, B, per, 0, scale, st)
-           : nt == 2 ? adj_go<false, 2>(P, phase, ms, bs, alm, as, B, per, 0, scale, st)
-                     : adj_go<false, 3>(P, phase, ms, bs, alm, as, B, per, 0, scale, st);
-  return nt == 1   ? adj_go<true, 1>(P, phase, ms, bs, alm, as, B, per, spin, scale, st)
-         : nt == 2 ? adj_go<true, 2>(P, phase, ms, bs, alm, as, B, per, spin, scale, st)
-                   : adj_go<true, 3>(P, phase, ms, bs, alm, as, B, per, spin, scale, st);
+    return nt == 1   ? adj_go<false, 1>(P, phase, ms, bs, alm, as, B, per, 0, scale, beside, st)
+           : nt == 2 ? adj_go<false, 2>(P, phase, ms, bs, alm, as, B, per, 0, scale, beside, st)
+                     : adj_go<false, 3>(P, phase, ms, bs, alm, as, B, per, 0, scale, beside, st);
+  return nt == 1   ? adj_go<true, 1>(P, phase, ms, bs, alm, as, B, per, spin, scale, beside, st)
+         : nt == 2 ? adj_go<true, 2>(P, phase, ms, bs, alm, as, B, per, spin, scale, beside, st)
+                   : adj_go<true, 3>(P, phase, ms, bs, alm, as, B, per, spin, scale, beside, st);
 }
 
 }  // namespace ps

@@ -16,10 +16,10 @@
 namespace ps {
 int launch_leg_tables_f64(const Plan& P, int spin, double* cd, double* gam, cudaStream_t st);
 int launch_legendre_synth_f64(const Plan& P, const double2* alm, int64_t as, double2* phase, int64_t ms, int64_t bs,
-                              int B, int spin, bool grad, cudaStream_t st);
+                              int B, int spin, bool grad, bool beside, cudaStream_t st);
 int launch_gc_to_pm(const double2* gc, double2* plus, double2* minus, int B, int64_t nalm, int spin, cudaStream_t st);
 int launch_legendre_adjoint_f64(const Plan& P, const double2* phase, int64_t ms, int64_t bs, double2* alm,
-                                int64_t as, int B, int spin, double scale, cudaStream_t st);
+                                int64_t as, int B, int spin, double scale, bool beside, cudaStream_t st);
 int launch_alm_to_T(const double2* alm, int64_t stride, const double* lscale, bool grad, double2* almT, int B, int ncomp,
                     int64_t nalm, cudaStream_t st);
 int launch_ring_synth_f64(const Plan& P, const RingClassList* cls, int ncls, const double2* phase, double* map,
@@ -686,7 +686,7 @@ int ps_legendre_synthesis(const ps_plan* plan, const double* alm, double* phase,
   }
   return ps::launch_legendre_synth_f64(P, reinterpret_cast<const double2*>(alm), ncomp * P.nalm,
                                        reinterpret_cast<double2*>(phase), int64_t(batch) * ncomp, ncomp, batch, spin,
-                                       false, stream);
+                                       false, false, stream);
 }
 
 int ps_legendre_adjoint(const ps_plan* plan, const double* phase, double* alm, int batch, int spin, double scale,
@@ -721,7 +721,7 @@ int ps_legendre_adjoint(const ps_plan* plan, const double* phase, double* alm, i
     return PS_OK;
   }
   return ps::launch_legendre_adjoint_f64(P, reinterpret_cast<const double2*>(phase), int64_t(batch) * ncomp, ncomp,
-                                         reinterpret_cast<double2*>(alm), ncomp * P.nalm, batch, spin, scale, stream);
+                                         reinterpret_cast<double2*>(alm), ncomp * P.nalm, batch, spin, scale, false, stream);
 }
 
 int ps_sht_workspace_bytes(const ps_plan* plan, int batch, int spin, int adjoint, size_t* bytes) {
@@ -778,7 +778,7 @@ static int synthesis(const ps_plan* plan, const double* alm, int64_t alm_stride,
   double2* phase = reinterpret_cast<double2*>(phase_ptr);
   // between the two stages the phases are [R][batch][mmax+1][ncomp]
   rc = ps::launch_legendre_synth_f64(P, reinterpret_cast<const double2*>(alm), alm_stride, phase, ncomp,
-                                     int64_t(P.mmax + 1) * ncomp, batch, spin, minus != nullptr, stream);
+                                     int64_t(P.mmax + 1) * ncomp, batch, spin, minus != nullptr, false, stream);
   if (rc) return rc;
   return ps::launch_ring_synth_f64(P, plan->ring_cls.data(), int(plan->ring_cls.size()), phase, map, mc,
                                    map_stride, nf, spin > 0, stream);
@@ -833,7 +833,7 @@ static int adjoint(const ps_plan* plan, const double* map, const double* minus, 
                                    phase, nf, spin > 0, stream);
   if (rc) return rc;
   return ps::launch_legendre_adjoint_f64(P, phase, ncomp, int64_t(P.mmax + 1) * ncomp, reinterpret_cast<double2*>(alm),
-                                         alm_stride, batch, spin, scale, stream);
+                                         alm_stride, batch, spin, scale, false, stream);
 }
 
 // bytes of the FP64 phases of one field of each map
@@ -900,9 +900,9 @@ int ps_synthesis_fields(const ps_plan* plan, const double* alm, int64_t alm_stri
   double2* phase0 = static_cast<double2*>(workspace);
   double2* phase2 = reinterpret_cast<double2*>(static_cast<char*>(workspace) + phase_bytes(P, batch));
   const int64_t row = P.mmax + 1;
-  int rc = ps::launch_legendre_synth_f64(P, a, alm_stride, phase0, 1, row, batch, 0, false, stream);
+  int rc = ps::launch_legendre_synth_f64(P, a, alm_stride, phase0, 1, row, batch, 0, false, false, stream);
   if (rc) return rc;
-  rc = ps::launch_legendre_synth_f64(P, a + P.nalm, alm_stride, phase2, 2, 2 * row, batch, 2, false, stream);
+  rc = ps::launch_legendre_synth_f64(P, a + P.nalm, alm_stride, phase2, 2, 2 * row, batch, 2, false, true, stream);
   if (rc) return rc;
   return ps::launch_ring_synth_fields_f64(P, plan->ring_cls.data(), int(plan->ring_cls.size()), phase0, phase2, map,
                                           map_stride, batch, stream);
@@ -920,9 +920,9 @@ int ps_adjoint_fields(const ps_plan* plan, const double* map, int64_t map_stride
   int rc = ps::launch_ring_adjoint_fields_f64(P, plan->ring_cls.data(), int(plan->ring_cls.size()), map, map_stride,
                                               phase0, phase2, batch, stream);
   if (rc) return rc;
-  rc = ps::launch_legendre_adjoint_f64(P, phase0, 1, row, a, alm_stride, batch, 0, scale, stream);
+  rc = ps::launch_legendre_adjoint_f64(P, phase0, 1, row, a, alm_stride, batch, 0, scale, false, stream);
   if (rc) return rc;
-  return ps::launch_legendre_adjoint_f64(P, phase2, 2, 2 * row, a + P.nalm, alm_stride, batch, 2, scale, stream);
+  return ps::launch_legendre_adjoint_f64(P, phase2, 2, 2 * row, a + P.nalm, alm_stride, batch, 2, scale, true, stream);
 }
 
 int ps_adjoint_pm(const ps_plan* plan, const double* plus, const double* minus, double* gc, double* alm_plus,

@@ -44,3 +44,31 @@ def test_refused_on_the_host():
     assert args(P._h, sa=3 * P.nalm - 1) == -1 and args(P._h, sm=3 * P.npix - 1) == -1 and args(P._h, b=-1) == -1
     assert args(Z._h) == -1
     assert args(M._h) == _lib.PS_ERR_UNSUPPORTED and args(P._h, nb=n - 1) not in (0, -1)
+
+
+@pytest.mark.parametrize("nside,lmax,batch", [(16, 47, 1), (128, 200, 1), (64, 100, 4)])
+def test_captured_and_back_to_back(nside, lmax, batch):
+    """Calls in a row share the workspace, on a stream and in a graph: each must see the one before it finished."""
+    from polyspec_b200.sht import SHTPlan
+    P = SHTPlan(nside, lmax, spins=(0, 2), autotune=False)
+    g = torch.Generator(device="cuda").manual_seed(nside)
+    x = [torch.randn((batch, 3, P.nalm), dtype=torch.complex128, device="cuda", generator=g) for _ in range(3)]
+    om = [torch.empty((batch, 3, P.npix), dtype=torch.float64, device="cuda") for _ in x]
+    oa = [torch.empty_like(a) for a in x]
+
+    def go():
+        for a, m, b in zip(x, om, oa):
+            P.synthesis_fields(a, m)
+            P.adjoint_fields(m, b)
+    go()
+    ref_m = [torch.cat([P.synthesis(a[:, 0], 0)[:, None], P.synthesis(a[:, 1:], 2)], 1) for a in x]
+    ref_a = [torch.cat([P.adjoint(m[:, 0], 0)[:, None], P.adjoint(m[:, 1:], 2)], 1) for m in ref_m]
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        go()
+    for run in (go, graph.replay):
+        for t in om + oa:
+            t.fill_(float("nan"))
+        for _ in range(20):
+            run()
+        assert all(torch.equal(a, b) for a, b in zip(om + oa, ref_m + ref_a))
