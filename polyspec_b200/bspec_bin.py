@@ -341,11 +341,11 @@ class BSpecBin:
             ptr2 = T['ptr2'][k0:]
             _lib.call("ps_bispec_pair_products", _vp(Hp1), nH, _vp(Hp1), nH, npix, _vp(ptr2), _vp(T['prods2']), nc,
                       _vp(X), _stream())
-            A2[k0:k0 + nc] = P.adjoint(X, 2, scale)
+            P.adjoint(X, 2, scale, out=A2[k0:k0 + nc])
             ptr1 = T['ptr1'][k0:]
             _lib.call("ps_bispec_pair_products", _vp(Hp1), nH, _vp(Hp2), nH, npix, _vp(ptr1), _vp(T['prods1']), nc,
                       _vp(X), _stream())
-            A1[k0:k0 + nc] = P.adjoint(X, 1, scale)
+            P.adjoint(X, 1, scale, out=A1[k0:k0 + nc])
             del X
         base.n_SHTs_forward += 2 * npair
         del Hp1, Hp2
@@ -380,6 +380,8 @@ class BSpecBin:
                 y = self.applySinv.batched(maps)
             else:
                 y = torch.stack([self.applySinv(m) for m in maps])
+            if len(y) == R:
+                return y
             if out is None:
                 out = torch.empty((R,) + tuple(y.shape[1:]), dtype=y.dtype, device=y.device)
             out[r0:r0 + len(y)] = y

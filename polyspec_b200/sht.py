@@ -365,12 +365,16 @@ class SHTPlan:
             B *= int(d)
         return lead, B, 1 if spin == 0 else 2
 
-    def adjoint(self, map, spin=0, scale=1.0):
+    def adjoint(self, map, spin=0, scale=1.0, out=None):
         spin = int(spin)
         lead, B, ncomp = self._check_map(map, spin)
         map, stride = self._maps_in(map, ncomp, self.npix)
         shape = tuple(lead) + ((2,) if spin > 0 else ()) + (self.nalm,)
-        out = torch.empty(shape, dtype=torch.complex128, device=map.device)
+        if out is None:
+            out = torch.empty(shape, dtype=torch.complex128, device=map.device)
+        elif (tuple(out.shape) != shape or out.dtype != torch.complex128 or out.device != map.device
+              or not out.is_contiguous() or out.is_conj()):
+            raise ValueError("out must be a contiguous complex128 tensor of shape %s" % (shape,))
         if B > 0:
             self._issue_adjoint(spin, B, map.data_ptr(), stride, out.data_ptr(), 0, scale)
         return out
