@@ -380,8 +380,6 @@ class BSpecBin:
                 y = self.applySinv.batched(maps)
             else:
                 y = torch.stack([self.applySinv(m) for m in maps])
-            if len(y) == R:
-                return y
             if out is None:
                 out = torch.empty((R,) + tuple(y.shape[1:]), dtype=y.dtype, device=y.device)
             out[r0:r0 + len(y)] = y

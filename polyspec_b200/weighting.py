@@ -256,7 +256,7 @@ class Weightings:
             maps = torch.stack([self.inpaint_map(m) for m in maps])
         beam = self.base.dev('beam_lm')
         lm = self.base.to_lm_batch(maps)
-        if lmax >= self.base.lmax and lm.shape[1] == 3:
+        if lmax >= self.base.lmax and lm.shape[1] == 3 and len(lm) > 0:
             # one kernel; as a product of matrices per (l, m) the library takes seven times as long (868 us against 123 us
             # for the rows of six bins at lmax 255)
             return lmops.matvec3(self.real3('inv_Cl_tot'), lm, post=beam.to(torch.float64))

@@ -31,6 +31,7 @@ def test_batched_equals_single(nside, lmax, batch, low, pol):
         ref = wts.applySinv_ideal(maps[b], lmax=top)
         assert got[b].shape == ref.shape
         assert float((got[b] - ref).abs().max() / ref.abs().max()) < 1e-12
+    assert tuple(wts.batched_applySinv_ideal(maps[:0], lmax=top).shape) == (0,) + tuple(got.shape[1:])
 
 
 def test_adjoint_into():
