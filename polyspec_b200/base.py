@@ -166,6 +166,8 @@ class PolySpec:
             filt = self.l_arr <= lmax
             if name == 'beam_lm':
                 arr = self.beam_lm[:, filt]
+                if not np.iscomplexobj(arr):
+                    arr = arr.astype(np.float64)  # kernels read it as such, whatever type the user's beam or spectra have
             elif name == 'inv_Cl_tot_lm_mat':
                 arr = self.inv_Cl_tot_lm_mat[:, :, filt].astype(np.complex128)
             elif name == 'm_weight':

@@ -107,23 +107,37 @@ class StepScalars:
         self.t = torch.zeros(4, dtype=torch.float64, device=device)
         self.t[0] = rz
 
+    def _check(self, nf, nlm, vectors, S=None, beam=None, w=None):
+        # the kernels take addresses alone
+        for shape, dtype, ts in (((nf, nlm), torch.complex128, vectors), ((nf, nf, nlm), torch.float64, (S,)),
+                                 ((nf, nlm), torch.float64, (beam,)), ((nlm,), torch.float64, (w,))):
+            for t in ts:
+                if t is not None and (t.dtype != dtype or t.shape != shape or not t.is_contiguous() or t.is_conj()
+                                      or t.is_neg() or t.device != self.t.device):
+                    raise ValueError("the CG step needs contiguous %s of shape %s on %s, not %s %s on %s"
+                                     % (dtype, shape, self.t.device, t.dtype, tuple(t.shape), t.device))
+
     def apply(self, S, beam, w, p, y):
         """y = beam y + S p in place; p^T y kept."""
+        self._check(*p.shape, (p, y), S=S, beam=beam, w=w)
         _lib.call("ps_cgd_apply", _vp(S), _vp(beam), _vp(w), _vp(p), _vp(y), p.shape[0], p.shape[1], _vp(self.t),
                   _vp(self.ws), self.nbytes, _stream())
 
     def update(self, Sigma, w, p, q, x, r, z):
         """x += alpha p, r -= alpha q; with Sigma z = Sigma r and the next r^T z."""
+        self._check(*p.shape, (p, q, x, r) if z is None else (p, q, x, r, z), S=Sigma, w=w)
         _lib.call("ps_cgd_update", _vp(Sigma), _vp(w), _vp(p), _vp(q), _vp(x), _vp(r), _vp(z), p.shape[0], p.shape[1],
                   _vp(self.t), _vp(self.ws), self.nbytes, _stream())
 
     def next_rz(self, w, r, z):
         """The next r^T z and beta."""
+        self._check(*r.shape, (r, z), w=w)
         _lib.call("ps_cgd_rz", _vp(w), _vp(r), _vp(z), r.shape[0], r.shape[1], _vp(self.t), _vp(self.ws), self.nbytes,
                   _stream())
 
     def direction(self, beam, z, p, beam_p):
         """p = z + beta p, beam_p = beam p."""
+        self._check(*p.shape, (z, p, beam_p), beam=beam)
         _lib.call("ps_cgd_direction", _vp(beam), _vp(z), _vp(p), _vp(beam_p), p.shape[0], p.shape[1], _vp(self.t),
                   _stream())
 

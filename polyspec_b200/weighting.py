@@ -256,10 +256,10 @@ class Weightings:
             maps = torch.stack([self.inpaint_map(m) for m in maps])
         beam = self.base.dev('beam_lm')
         lm = self.base.to_lm_batch(maps)
-        if lmax >= self.base.lmax and lm.shape[1] == 3 and len(lm) > 0:
+        if lmax >= self.base.lmax and lm.shape[1] == 3 and len(lm) > 0 and not beam.is_complex():
             # one kernel; as a product of matrices per (l, m) the library takes seven times as long (868 us against 123 us
             # for the rows of six bins at lmax 255)
-            return lmops.matvec3(self.real3('inv_Cl_tot'), lm, post=beam.to(torch.float64))
+            return lmops.matvec3(self.real3('inv_Cl_tot'), lm, post=beam)
         lfilt = torch.as_tensor(self.base.l_arr <= lmax, device=self.base.device)
         icov = self.base.dev('inv_Cl_tot_lm_mat')
         return beam[:, lfilt] * torch.einsum("abl,nbl->nal", icov[:, :, lfilt], lm[:, :, lfilt])
@@ -514,6 +514,10 @@ class CGD:
         self.p = z.contiguous()
         self.i = 0
         self.err = self.rz / self.rz0
+        # a complex beam multiplies outside the kernels, which read it as float64
+        self.fused = not self.base.dev('beam_lm').is_complex()
+        if not self.fused:
+            return
         # operands of the fused step (ps_cgd_*), which works on contiguous complex128 vectors of its own
         self.x, self.r = self.x.contiguous(), self.r.contiguous()
         W, base = weightings, self.base
@@ -572,6 +576,25 @@ class CGD:
             raise Exception("Unknown preconditioner %s specified!" % self.preconditioner)
 
     def step(self):
+        if self.fused:
+            self._step_fused()
+        else:
+            self._step()
+        self.i += 1
+
+    def _step(self):
+        Ap = self._apply_A(self.p)
+        alpha = self.rz / self.dot(self.p, Ap)
+        self.x += alpha * self.p
+        self.r -= alpha * Ap
+        z = self._apply_M(self.r)
+        next_rz = self.dot(self.r, z)
+        self.err = next_rz / self.rz0
+        beta = next_rz / self.rz
+        self.rz = next_rz
+        self.p = z + beta * self.p
+
+    def _step_fused(self):
         # A p = C^-1 p + B Y^dagger W N^-1 W Y B p
         Ap = self.base.to_lm(self.base.to_map(self.beam_p) * self.d_weight)
         sc = self.scal
@@ -589,7 +612,6 @@ class CGD:
             raise ZeroDivisionError("CGD step from a zero residual or direction")
         self.rz = rz
         self.err = self.rz / self.rz0
-        self.i += 1
 
     def run(self, nstep=10, thresh=1e-6):
         for i in range(nstep):
