@@ -376,6 +376,8 @@ int ps_cg_direction(double* p, const double* z, const double* beta, int batch, i
  * ps_cgd_update: alpha = scal[0] / scal[1]; x += alpha p, r -= alpha q; with Sigma also z = Sigma r and then as
  * ps_cgd_rz: scal[2] = t / scal[0], scal[0] = t, t = Sum w Re(r conj(z));
  * ps_cgd_direction: p = z + scal[2] p, beam_p = beam p.
+ * Where r^T z or p^T A p (scal[0], scal[1]) is zero there is no step: ps_cgd_update, ps_cgd_rz and ps_cgd_direction leave
+ * the vectors as they are and set scal[3] to 1 (0 otherwise).
  * The workspace (zeroed once) belongs to one solve on one stream. */
 int ps_cgd_workspace_bytes(size_t* bytes);
 int ps_cgd_apply(const double* S, const double* beam, const double* w, const double* p, double* y, int nf,

@@ -18,7 +18,12 @@ namespace ps {
 namespace {
 
 constexpr int CGD_THREADS = 256, CGD_MAX_BLOCKS = 1024;
-enum { RZ = 0, PQ = 1, BETA = 2 };  // scalars of the solve
+enum { RZ = 0, PQ = 1, BETA = 2, NO_STEP = 3 };  // scalars of the solve
+
+// r^T z or p^T A p is zero: there is no alpha or beta, and the vectors stay as they are.
+__device__ __forceinline__ bool no_step(const double* scal) {
+  return __ldcg(scal + RZ) == 0.0 || __ldcg(scal + PQ) == 0.0;
+}
 
 // Sum of the blocks' v by the last of them to arrive, on its thread 0; other threads get false.
 __device__ bool last_block_sum(double v, double* partial, unsigned* counter, double& total) {
@@ -86,6 +91,7 @@ __global__ void __launch_bounds__(CGD_THREADS) cgd_apply(const double* __restric
 
 // every block has read rz before the last one replaces it
 __device__ __forceinline__ void next_rz(double total, double* scal) {
+  scal[NO_STEP] = 0.0;
   scal[BETA] = total / scal[RZ];
   scal[RZ] = total;
 }
@@ -96,6 +102,10 @@ __global__ void __launch_bounds__(CGD_THREADS) cgd_update(const double* __restri
                                                           double2* __restrict__ x, double2* __restrict__ r,
                                                           double2* __restrict__ z, int64_t nalm, double* scal,
                                                           double* partial, unsigned* counter) {
+  if (no_step(scal)) {
+    if (SIGMA && blockIdx.x == 0 && threadIdx.x == 0) scal[NO_STEP] = 1.0;
+    return;
+  }
   const double alpha = __ldcg(scal + RZ) / __ldcg(scal + PQ);
   double dot = 0.0;
   for (int64_t i = int64_t(blockIdx.x) * CGD_THREADS + threadIdx.x; i < nalm; i += int64_t(gridDim.x) * CGD_THREADS) {
@@ -127,6 +137,10 @@ template <int NF>
 __global__ void __launch_bounds__(CGD_THREADS) cgd_rz(const double* __restrict__ w, const double2* __restrict__ r,
                                                       const double2* __restrict__ z, int64_t nalm, double* scal,
                                                       double* partial, unsigned* counter) {
+  if (no_step(scal)) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) scal[NO_STEP] = 1.0;
+    return;
+  }
   double dot = 0.0;
   for (int64_t i = int64_t(blockIdx.x) * CGD_THREADS + threadIdx.x; i < nalm; i += int64_t(gridDim.x) * CGD_THREADS) {
     double d = 0.0;
@@ -142,6 +156,7 @@ __global__ void __launch_bounds__(CGD_THREADS) cgd_direction(const double* __res
                                                              const double2* __restrict__ z, double2* __restrict__ p,
                                                              double2* __restrict__ bp, int64_t n,
                                                              const double* __restrict__ scal) {
+  if (scal[NO_STEP] != 0.0) return;
   const double beta = scal[BETA];
   for (int64_t i = int64_t(blockIdx.x) * CGD_THREADS + threadIdx.x; i < n; i += int64_t(gridDim.x) * CGD_THREADS) {
     const double2 v = cfma(beta, p[i], z[i]);
