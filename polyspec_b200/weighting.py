@@ -15,6 +15,7 @@ operators evaluated on the device.
 """
 import ctypes
 import os
+import types
 
 import numpy as np
 import torch
@@ -511,21 +512,30 @@ class CGD:
         z = self._apply_M(self.r)
         self.rz = self.dot(self.r, z)
         self.rz0 = float(self.dot(b0, self._apply_M(b0)))
-        self.p = z.contiguous()
+        self.p = z
         self.i = 0
         self.err = self.rz / self.rz0
-        # a complex beam multiplies outside the kernels, which read it as float64
-        self.fused = not self.base.dev('beam_lm').is_complex()
-        if not self.fused:
-            return
-        # operands of the fused step (ps_cgd_*), which works on contiguous complex128 vectors of its own
-        self.x, self.r = self.x.contiguous(), self.r.contiguous()
-        W, base = weightings, self.base
-        self.d_Cinv, self.d_Sigma = lmops.real3(W.d_inv_Cl), lmops.real3(W.d_Sigma)
-        self.d_beam = base.dev('beam_lm').expand(self.r.shape).contiguous()
-        self.d_weight = W.d_WNW / W.pixel_area
-        self.scal = lmops.StepScalars(self.rz, base.device)
-        self.beam_p = self._apply_beam(self.p).contiguous()
+        self._ops = None
+
+    @property
+    def p(self):
+        return self._p
+
+    @p.setter
+    def p(self, v):
+        self._p, self._beam_p = v, None
+
+    def _operands(self):
+        """What the kernels of the step (ps_cgd_*) read beside the vectors, or None for a complex beam, which
+        multiplies outside of them.  Made by the first step of a run and given back at its end: 0.7 GB for T, E, B
+        at Nside 1024, lmax 2048."""
+        beam = self.base.dev('beam_lm')
+        if beam.is_complex():
+            return None
+        W = self.weightings
+        return types.SimpleNamespace(
+            Cinv=lmops.real3(W.d_inv_Cl), Sigma=lmops.real3(W.d_Sigma), beam=beam.expand(self.r.shape).contiguous(),
+            weight=W.d_WNW / W.pixel_area, scal=lmops.StepScalars(self.rz, self.base.device), rz=self.rz)
 
     def dot(self, a, b):
         """m-weighted real inner product sum a b^* (1 + [m > 0]) (polyspec/weighting.py:255)."""
@@ -576,10 +586,12 @@ class CGD:
             raise Exception("Unknown preconditioner %s specified!" % self.preconditioner)
 
     def step(self):
-        if self.fused:
-            self._step_fused()
-        else:
+        if self._ops is None:
+            self._ops = self._operands()
+        if self._ops is None:
             self._step()
+        else:
+            self._step_fused(self._ops)
         self.i += 1
 
     def _step(self):
@@ -594,34 +606,46 @@ class CGD:
         self.rz = next_rz
         self.p = z + beta * self.p
 
-    def _step_fused(self):
+    def _step_fused(self, ops):
+        # the vectors and rz are the caller's to set between steps
+        def own(t):
+            return t.to(device=self.base.device, dtype=torch.complex128).resolve_conj().resolve_neg().contiguous()
+        if self._beam_p is None:
+            self._p = own(self._p).clone()  # written in place by the step
+            self._beam_p = self._p * ops.beam
         # A p = C^-1 p + B Y^dagger W N^-1 W Y B p
-        Ap = self.base.to_lm(self.base.to_map(self.beam_p) * self.d_weight)
-        sc = self.scal
-        sc.apply(self.d_Cinv, self.d_beam, self.w, self.p, Ap)
+        Ap = self.base.to_lm(self.base.to_map(self._beam_p) * ops.weight)
+        self.x, self.r = own(self.x), own(self.r)
+        p, sc = self._p, ops.scal
+        if self.rz != ops.rz:
+            sc.t[0] = self.rz
+        sc.apply(ops.Cinv, ops.beam, self.w, p, Ap)
         if self.preconditioner == 'harmonic':
             z = torch.empty_like(self.r)
-            sc.update(self.d_Sigma, self.w, self.p, Ap, self.x, self.r, z)
+            sc.update(ops.Sigma, self.w, p, Ap, self.x, self.r, z)
         else:
-            sc.update(None, self.w, self.p, Ap, self.x, self.r, None)
-            z = self._apply_M(self.r).contiguous()
+            sc.update(None, self.w, p, Ap, self.x, self.r, None)
+            z = own(self._apply_M(self.r))
             sc.next_rz(self.w, self.r, z)
-        sc.direction(self.d_beam, z, self.p, self.beam_p)
+        sc.direction(ops.beam, z, p, self._beam_p)
         rz, pq = sc.rz_pq()
         if self.rz == 0 or pq == 0:
             raise ZeroDivisionError("CGD step from a zero residual or direction")
-        self.rz = rz
+        self.rz = ops.rz = rz
         self.err = self.rz / self.rz0
 
     def run(self, nstep=10, thresh=1e-6):
-        for i in range(nstep):
-            self.step()
-            if self.verb:
-                print("CGD step %d: error = %.2e" % (self.i, self.err))
-            if self.err < thresh:
+        try:
+            for i in range(nstep):
+                self.step()
                 if self.verb:
-                    print("CGD terminating at step %d" % self.i)
-                break
+                    print("CGD step %d: error = %.2e" % (self.i, self.err))
+                if self.err < thresh:
+                    if self.verb:
+                        print("CGD terminating at step %d" % self.i)
+                    break
+        finally:
+            self._ops = self._beam_p = None
         if i == nstep - 1 and self.err > thresh:
             print("CGD did not converge to %.2e threshold after %d steps. Final error = %.2e" % (thresh, nstep, self.err))
 
