@@ -607,12 +607,17 @@ static int adjoint_chunk(const ps::Plan& P, int batch, int spin) {
   return batch < c ? batch : c;
 }
 
+// transposed alm of a mixed synthesis; the FP64 stages read alm where they lie
+static size_t almT_bytes(const ps::Plan& P, size_t nf) {
+  return P.prec == PS_PREC_FP64 ? 0 : align256(size_t(P.nalm) * nf * sizeof(double2));
+}
+
 static size_t sht_ws_bytes(const ps_plan* plan, int batch, int spin, int adjoint) {
   const ps::Plan& P = plan->p;
   const size_t ncomp = spin == 0 ? 1 : 2;
   const size_t nf = size_t(batch) * ncomp;
   const size_t phase = align256(size_t(P.R) * (P.mmax + 1) * nf * sizeof(double2));
-  if (!adjoint) return align256(size_t(P.nalm) * nf * sizeof(double2)) + phase;
+  if (!adjoint) return almT_bytes(P, nf) + phase;
   TabRef tr;
   // the FP64 and the table adjoint write alm directly
   if (P.prec == PS_PREC_FP64 || table_for(plan, spin, tr)) return phase;
@@ -753,7 +758,7 @@ static int synthesis(const ps_plan* plan, const double* alm, int64_t alm_stride,
   const int nf = batch * ncomp;
   char* ws = static_cast<char*>(workspace);
   double2* almT = reinterpret_cast<double2*>(ws);
-  char* phase_ptr = ws + align256(size_t(P.nalm) * nf * sizeof(double2));
+  char* phase_ptr = ws + almT_bytes(P, nf);
   int rc;
   if (P.prec == PS_PREC_MIXED) {
     if (nf == 1) {
