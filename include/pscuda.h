@@ -61,13 +61,17 @@ int ps_plan_info(const ps_plan* plan, int* nside, int* lmax, int64_t* npix, int6
  * device finishes its work) and optionally clears it.  No reference counterpart. */
 int ps_plan_error_flag(const ps_plan* plan, int* value, int reset);
 
-/* Tile setting of the Legendre stages (no reference counterpart): maps per CTA
- * for direction 0 (synthesis) or 1 (adjoint) and one spin; 0 restores the
- * library's choice by batch size.  Allowed: mixed synthesis spin 0 {8, 16, 32},
- * spin s {4, 8}; mixed adjoint spin 0 {1, 8}, spin s {1, 4}; FP64 synthesis
- * spin 0 {1, 4}, spin s {1, 2}; FP64 adjoint spin 0 {1, 4}, spin s {1}
- * (PS_ERR_UNSUPPORTED otherwise).  Used by the autotuner; it changes the plan,
- * so it must not run concurrently with transforms on the same plan. */
+/* Tile setting of the Legendre stages (no reference counterpart), for direction
+ * 0 (synthesis) or 1 (adjoint) and one spin; 0 restores the library's choice by
+ * plan and batch size.  Mixed plans, maps per CTA: synthesis spin 0 {8, 16, 32},
+ * spin s {4, 8}; adjoint spin 0 {1, 8}, spin s {1, 4}.  FP64 plans, 1 for the
+ * kernels that take single maps and more than 1 for those on the FP64 MMA:
+ * synthesis spin 0 {1, 4}, spin s {1, 2}; adjoint spin 0 {1, 4}; the adjoint of
+ * spin s takes {1} and has no choice (PS_ERR_UNSUPPORTED otherwise).  The two
+ * FP64 kernels sum in different orders (1e-15); with 0 a call gives the same
+ * bits each time, but a map's last bits may differ between batch sizes.
+ * The autotuner sets the mixed tiles; this changes the plan, so it must not run
+ * concurrently with transforms on the same plan. */
 int ps_plan_set_tile(ps_plan* plan, int direction, int spin, int tile);
 
 /* prec = PS_PREC_FP64: every stage in FP64.  prec = PS_PREC_MIXED: the

@@ -65,8 +65,8 @@ struct Plan {
   int n_bs_slots;
   int64_t bs_total;
   int num_sms;
-  // maps per CTA of the Legendre stages, [direction 0 synthesis / 1 adjoint][spin];
-  // 0 = the launcher's own choice (set by ps_plan_set_tile, e.g. from the autotuner)
+  // [direction 0 synthesis / 1 adjoint][spin], 0 = the launcher's own choice: maps per CTA of the mixed Legendre
+  // stages (the autotuner's), FP64: 1 single-map kernels, more FP64 MMA kernels (ps_plan_set_tile)
   int tile[2][4];
   // Legendre tables of a mixed-precision plan (ps_plan_build_table), per spin; null when
   // not built.  d_tab_off [mmax+2]: first table block of each order; d_tab_work: the

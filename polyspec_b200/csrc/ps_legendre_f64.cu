@@ -675,14 +675,28 @@ static int synthS_go(const Plan& P, const double2* alm, int64_t as, double2* pha
                     P.Rh, P.lmax, P.mmax, B, P.nalm, spin);
 }
 
-// Batches run on the FP64 MMA, which takes maps four (spin 0) or two (spin s) at a time; fewer maps than most of a
-// tile run one by one.  Measured, FMA / MMA kernels: spin 0, Nside 512, lmax 1000: 2 maps 357 / 389 us, 4 maps 475 /
-// 397, 24 maps 2880 / 1916; Nside 256, lmax 500, 3 maps 93 / 60.  Spin 2, Nside 512: 2 maps 811 / 805, 24 maps 9646 /
-// 7208; Nside 256, lmax 500, 3 maps 227 / 184 us (the FMA kernels then took four and two maps per CTA).
-// Tile 1 forces single maps, tile 4 (spin s: 2) the MMA.  grad (C = 0), spin 2: Nside 512, lmax 1000 one map 387 us (508
+// Which kernels a batch runs on: the FP64 MMA takes maps four (spin 0) or two (spin s) at a time, and has a longer
+// chain per launch; where the maps do not fill the chip the FMA kernels, a CTA for each map, are through first.  The
+// line lies where the times cross: (ring pairs) (orders) (maps) of 3 2^16 and three maps for spin 0, 3 2^15 and two maps for
+// spin s.  It is a rule, not a timing at run time, because the two order their sums differently (1e-15) and a call has
+// to give the same bits in every process.  Measured, whole transform, FMA / MMA kernels, us:
+//   spin 0: Nside 16, lmax 47: 32 maps 12.4 / 13.8; Nside 64, lmax 128: 8 maps 24.0 / 25.3, 12 27.3 / 27.4, 16 30.0 /
+//     27.8; Nside 128, lmax 256: 2 maps 32.7 / 37.0, 3 36.6 / 35.8, 24 177 / 131; Nside 512, lmax 1000: 2 maps 509 / 539,
+//     3 717 / 585; Nside 1024, lmax 2048: 2 maps 3042 / 3331, 3 4535 / 3528
+//   spin 2: Nside 16, lmax 47: 32 maps 18.3 / 23.7; Nside 32, lmax 95: 12 maps 24.3 / 30.1, 32 43.1 / 42.2; Nside 64, lmax
+//     128: 3 maps 24.1 / 25.7, 6 30.0 / 29.7, 24 78 / 63; Nside 128, lmax 256: 1 map 38.0 / 43.6, 2 52.7 / 49.0, 24 384 /
+//     285; Nside 512, lmax 1000: 1 map 638 / 1007, 2 1197 / 1089
+// Tile 1 forces the FMA kernels, tile 4 (spin s: 2) the MMA.  grad (C = 0), spin 2: Nside 512, lmax 1000 one map 387 us (508
 // with C), 2 maps 761 / 830, 3 maps 1130 / 845; Nside 256, lmax 500 one map 64 (82), 2 maps 124 / 127, 3 maps
-// 178 / 131: the same line, whatever the tile.
-//
+// 178 / 131 (Legendre stage alone): from three maps on, whatever the tile.
+static bool synth_on_mma(const Plan& P, int B, int spin, bool grad) {
+  if (grad) return B >= 3;
+  if (P.tile[0][spin]) return P.tile[0][spin] > 1;
+  const int64_t work = int64_t(P.Rh) * (P.mmax + 1) * B;
+  if (B > MAX_GRID_Z) return true;  // a grid layer per map
+  return spin == 0 ? B >= 3 && work >= 3 << 16 : B >= 2 && work >= 3 << 15;
+}
+
 // Rings per thread of single maps: the rings of a thread share each shared-memory broadcast, fewer keep more warps
 // in flight where a plan has few rings.  Measured, one map, spin 0, one / two / four rings: Nside 1024, lmax 2048
 // 1661 / 1417 / 1353 us, Nside 512, lmax 1000 212 / 187 / 184 us, Nside 256, lmax 767 70 / 71 / 81 us; spin 2 (whose
@@ -691,8 +705,8 @@ int launch_legendre_synth_f64(const Plan& P, const double2* alm, int64_t as, dou
                               int B, int spin, bool grad, bool beside, cudaStream_t st) {
   StatScope sc(PS_K_LEG_SYNTH, leg_flops(P, B, spin), leg_bytes(P, B, spin), st);
   if (spin > 0 && !P.d_seed[spin]) return PS_ERR_INVALID;
-  const int t = P.tile[0][spin];
-  if (t && !grad ? t > 1 : B >= 3) return launch_synth_mma_f64(P, alm, as, phase, ms, bs, B, spin, grad, beside, st);
+  if (synth_on_mma(P, B, spin, grad))
+    return launch_synth_mma_f64(P, alm, as, phase, ms, bs, B, spin, grad, beside, st);
   if (spin == 0) {
     if (P.Rh >= 1024) synth0_go<4>(P, alm, as, phase, ms, bs, B, st);
     else if (P.Rh > 128) synth0_go<2>(P, alm, as, phase, ms, bs, B, st);
@@ -731,23 +745,36 @@ static int adjS_go(const Plan& P, const double2* phase, int64_t ms, int64_t bs, 
   return PS_OK;
 }
 
+// Which kernels a batch runs on, as for the synthesis.  The MMA takes a CTA per order and twelve maps, the FMA
+// kernels one per order and map: with fewer orders than SMs the MMA needs many maps to be through first.  Measured, whole
+// transform, FMA / MMA kernels, us:
+//   spin 0: Nside 16, lmax 47: 32 maps 12.7 / 21.9; Nside 32, lmax 95: 32 maps 26.2 / 27.6; Nside 64, lmax 128: 1 map 20.6 /
+//     20.2, 4 21.5 / 20.5, 5 22.2 / 25.3, 12 29.3 / 34.2, 16 32.5 / 28.7; Nside 64, lmax 191: 3 maps 25.5 / 23.3, 4 27.1 /
+//     23.3, 24 72 / 48; Nside 128, lmax 256: 3 maps 37.7 / 41.9, 4 46.1 / 43.6, 5 52.3 / 57.2, 6 61.9 / 58.5, 24 201 / 127;
+//     Nside 128, lmax 383: 2 maps 48.9 / 56.3, 3 61.2 / 57.1; Nside 256, lmax 767: 2 maps 193 / 205, 3 287 / 218; Nside
+//     512, lmax 1000: 2 maps 581 / 571, 3 859 / 607
+//   spin 2 (the sums of two maps fill a tile), Legendre stage alone: Nside 256, lmax 767, 2 maps 430 / 326, Nside 512, 24
+//     maps 16359 / 9476; one map, half a tile, 707 / 1054
+// Tile 1 forces the FMA kernels of spin 0, tile 4 the MMA; spin s has no choice.
+static bool adjoint_on_mma(const Plan& P, int B, int spin) {
+  if (spin > 0) return B >= 2;
+  if (P.tile[1][0]) return P.tile[1][0] > 1;
+  const int64_t orders = P.mmax + 1, work = orders * P.Rh;
+  if (orders < P.num_sms) return work * B >= 1 << 18;
+  return B >= 4 || (B == 3 && work >= 90000);
+}
+
 // Rings per thread and warps per CTA.  Four rings halve the share of the warp sums and are used wherever a
 // plan has enough rings for one warp of them per scheduler; a CTA of four warps passes several times over l at
 // Rh > 512 but more CTAs share an SM and hide each other's barriers, eight warps keep more of the chip busy when
 // there are few (m, map) pairs.  Measured, four against eight warps of four rings, one map: Nside 1024, lmax 2048
 // 1898 / 1957 us (spin 0), Nside 512, lmax 1000 298 / 259 us; spin 2, <4, 4> against <2, 8>: 5280 / 5720 us,
 // 706 / 759 us and, Nside 256, lmax 767, 259 / 240 us.
-//
-// Batches run on the FP64 MMA.  Measured, FMA / MMA kernels: spin 0, Nside 512, lmax 1000, 4 maps 1011 / 593 us, 24
-// maps 6002 / 2597; Nside 256, lmax 767, 2 maps 171 / 192, lmax 500, 3 maps 124 / 125.  Spin 2 (the sums of two
-// maps fill a tile): Nside 256, lmax 767, 2 maps 430 / 326, Nside 512, 24 maps 16359 / 9476; one map, half a tile,
-// 707 / 1054.  Tile 1 forces single maps of spin 0, tile 4 the MMA.
 int launch_legendre_adjoint_f64(const Plan& P, const double2* phase, int64_t ms, int64_t bs, double2* alm, int64_t as,
                                 int B, int spin, double scale, bool beside, cudaStream_t st) {
   StatScope sc(PS_K_LEG_ADJOINT, leg_flops(P, B, spin), leg_bytes(P, B, spin), st);
   if (spin > 0 && !P.d_seed[spin]) return PS_ERR_INVALID;
-  const int t = P.tile[1][spin];
-  if (spin > 0 ? B >= 2 : t ? t > 1 : B >= 4)
+  if (adjoint_on_mma(P, B, spin))
     return launch_adjoint_mma_f64(P, phase, ms, bs, alm, as, B, spin, scale, beside, st);
   const int64_t ctas = int64_t(P.mmax + 1) * B;
   if (spin == 0) {

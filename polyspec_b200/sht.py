@@ -11,11 +11,17 @@ return CUDA tensors in the ducc0 layout used by the reference
 ``adjoint`` is ducc0's ``adjoint_synthesis`` times ``scale``.
 
 With ``autotune=True`` (default) the first call of each (direction, spin,
-batch bucket) times the candidate tile shapes of the Legendre kernels and, for
-``prec='mixed'``, the FP64 pipeline too (an FP64 plan is kept beside the mixed
-one) and keeps the fastest (polyspec_b200.autotune; choices cached in JSON).
-The tensor-core pipeline wins at large batches; for one or a few maps the FP64
-CUDA-core kernels are faster (and exact to FP64).
+batch bucket) of a ``prec='mixed'`` plan times the candidate tile shapes of its
+Legendre kernels and, up to eight maps, the FP64 pipeline (an FP64 plan is kept
+beside the mixed one) and keeps the fastest (polyspec_b200.autotune; choices
+cached in JSON).  The FP64 kernels win for small batches (and are exact to FP64),
+the tensor-core pipeline above 12 (spin s) to 16 maps (spin 0): Nside 256, lmax 511,
+spin 2, synthesis of 2 / 12 / 33 maps 0.24 / 0.79 / 2.14 ms in FP64 and 0.57 / 0.79 /
+1.68 ms mixed.
+
+FP64 results do not depend on timings: the same call gives the same bits in every
+process.  A map's last bits (1e-15) may depend on the size of the batch it comes in,
+since small and large batches run on kernels that order their sums differently.
 
 Legendre tables (``tables='auto'``, mixed precision only): the first transform
 of a spin builds the plan's FP32 Legendre table of that spin
