@@ -12,6 +12,7 @@
 #include <new>
 
 #include "ps_common.cuh"
+#include "ps_unit.h"
 
 namespace ps {
 int launch_leg_tables_f64(const Plan& P, int spin, double* cd, double* gam, cudaStream_t st);
@@ -94,6 +95,12 @@ void host_fft(std::vector<std::complex<double>>& a, const std::vector<double2>& 
       }
     }
   }
+}
+
+double2 unit(int64_t q, int64_t den) {  // e^{i pi q / den}
+  double2 w;
+  ps::unit_root(q, den, w.x, w.y);
+  return w;
 }
 
 int host_bitrev(int i, int logn) {
@@ -277,10 +284,7 @@ int ps_plan_create(int nside, int lmax, int mmax, int spin_mask, int prec, ps_pl
       ring_cls_rings.push_back(north);
     }
   std::vector<double2> tw(max_fft / 2);
-  for (int k = 0; k < max_fft / 2; ++k) {
-    const double ang = -2.0 * M_PI * double(k) / double(max_fft);
-    tw[k] = make_double2(std::cos(ang), std::sin(ang));
-  }
+  for (int k = 0; k < max_fft / 2; ++k) tw[k] = unit(-2 * k, max_fft);
   // ---- Bluestein spectra: b_n = e^{+i pi n^2 / N}, |n| < N, wrapped to M; FFT_M, bit-reversed order
   std::vector<double2> bs_spec;
   std::vector<int64_t> bs_off;
@@ -289,9 +293,8 @@ int ps_plan_create(int nside, int lmax, int mmax, int spin_mask, int prec, ps_pl
     int logM = 0; while ((1 << logM) < M) ++logM;
     std::vector<std::complex<double>> b(M, 0.0);
     for (int n = 0; n < N; ++n) {
-      const int64_t q = (int64_t(n) * n) % (2 * int64_t(N));
-      const double ang = M_PI * double(q) / double(N);
-      const std::complex<double> v(std::cos(ang), std::sin(ang));
+      const double2 w = unit(int64_t(n) * n, N);
+      const std::complex<double> v(w.x, w.y);
       b[n] = v;
       if (n > 0) b[M - n] = v;
     }
@@ -349,10 +352,7 @@ int ps_plan_create(int nside, int lmax, int mmax, int spin_mask, int prec, ps_pl
     std::vector<double2> levels;
     for (int64_t L = 8; L <= 2 * int64_t(std::max(max_fft, 4)); L *= 2)
       for (int64_t p = 1; p <= 4; p *= 2)
-        for (int64_t j = 0; j < L / 8; ++j) {
-          const double a = -2.0 * M_PI * double(p * j) / double(L);
-          levels.push_back(make_double2(std::cos(a), std::sin(a)));
-        }
+        for (int64_t j = 0; j < L / 8; ++j) levels.push_back(unit(-2 * p * j, L));
     P.d_twiddle = dev_upload(pl, levels, err);
     // Bluestein spectra as the middle pass reads them: [8][M/8], position 8 t + k at k M/8 + t
     std::vector<double2> spec(bs_spec.size());
@@ -361,11 +361,7 @@ int ps_plan_create(int nside, int lmax, int mmax, int spin_mask, int prec, ps_pl
       for (int64_t p = 0; p < M; ++p) spec[size_t(o + (p % 8) * (M / 8) + p / 8)] = bs_spec[size_t(o + p)];
     }
     P.d_bs_spec = dev_upload(pl, spec, err);
-    // ring rotations and Bluestein chirps from exact integer argument reduction
-    auto unit = [](int64_t q, int64_t den) {  // e^{i pi q / den}
-      const double a = M_PI * double(q % (2 * den)) / double(den);
-      return make_double2(std::cos(a), std::sin(a));
-    };
+    // ring rotations and Bluestein chirps
     std::vector<double2> root, chirp;
     std::vector<int64_t> chirp_off;
     root.reserve(size_t(2) * nside * (nside + 1));
@@ -373,10 +369,7 @@ int ps_plan_create(int nside, int lmax, int mmax, int spin_mask, int prec, ps_pl
       for (int64_t k = 0; k < 4 * i; ++k) root.push_back(unit(k, 4 * i));
     for (int N : bs_n) {
       chirp_off.push_back((int64_t)chirp.size());
-      for (int64_t j = 0; j < N; ++j) {
-        const double2 w = unit(j * j, N);
-        chirp.push_back(make_double2(w.x, -w.y));
-      }
+      for (int64_t j = 0; j < N; ++j) chirp.push_back(unit(-j * j, N));
     }
     P.d_root = dev_upload(pl, root, err);
     P.d_chirp = dev_upload(pl, chirp, err);
