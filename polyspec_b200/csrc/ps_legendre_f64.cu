@@ -37,6 +37,7 @@
 #include <type_traits>
 
 #include "ps_legendre_f64.cuh"
+#include "ps_legtab.h"
 #include "ps_stats.cuh"
 
 namespace ps {
@@ -45,26 +46,8 @@ constexpr int SYN_THREADS = 128;  // threads per synthesis CTA
 constexpr int ADJ_LCH = 64;       // l chunk of the adjoint between two CTA barriers
 
 // ---------------------------------------------------------------- recurrence tables
-// Three-term coefficients of the normalised functions:
-//   spin 0  lam_l = a_l x lam_{l-1} - (a_l / a_{l-1}) lam_{l-2},  a_l = sqrt((4l^2-1)/(l^2-m^2))
-//   spin s  f_{l+1} = (A x + D) f_l - C f_{l-1}  (g: -D),  l >= max(m, s)
-__device__ __forceinline__ double coef_a(int l, int m) {
-  const double ll = double(l) * l;
-  return sqrt((4.0 * ll - 1.0) / (ll - double(m) * m));
-}
-__device__ __forceinline__ void coef_spin(int l, int m, int s, double& A, double& D, double& C) {
-  auto rho = [&](double L) {
-    return sqrt(fmax(L * L - double(m) * m, 0.0) * fmax(L * L - double(s) * s, 0.0));
-  };
-  const double r1 = rho(l + 1.0), q = sqrt((2.0 * l + 3.0) * (2.0 * l + 1.0));
-  A = q * (l + 1.0) / r1;
-  D = q * double(m) * double(s) / (double(l) * r1);
-  C = sqrt((2.0 * l + 3.0) / (2.0 * l - 1.0)) * (l + 1.0) * rho(double(l)) / (double(l) * r1);
-}
-
-// One thread per order m: gam_{l0} = gam_{l0+1} = 1 at l0 = max(m, s), gam_{l+1} = C_l gam_{l-1} and
-// c_l = A_l gam_l / gam_{l+1} (d alike).  spin 0: cd is c [nalm]; spin s: (c, d) pairs.  Entries with
-// l < s are zero.  Runs once per plan (0.2 ms at lmax 2048).
+// One thread per order m, l by l (LegChain).  spin 0: cd is c [nalm]; spin s: (c, d) pairs.  Entries with l < s are
+// zero.  Runs once per plan.
 __global__ void leg_tables_f64(int lmax, int mmax, int s, double* __restrict__ cd, double* __restrict__ gam) {
   const int m = blockIdx.x * blockDim.x + threadIdx.x;
   if (m > mmax) return;
@@ -74,27 +57,17 @@ __global__ void leg_tables_f64(int lmax, int mmax, int s, double* __restrict__ c
     cd[2 * (o + l)] = cd[2 * (o + l) + 1] = 0.0;  // l < s only for spin s
     gam[o + l] = 0.0;
   }
-  double g0 = 1.0, gm = 1.0;  // gam_l, gam_{l-1}
-  double a0 = 0.0;
-  for (int l = l0; l <= lmax; ++l) {
+  LegChain t(m, s);
+  for (int l = l0; l <= lmax; ++l, t.step()) {
+    double c, d, g;
+    t.values(c, d, g);
     if (s == 0) {
-      const double a1 = coef_a(l + 1, m);
-      const double g1 = l == l0 ? 1.0 : a1 / a0 * gm;
-      cd[o + l] = a1 * g0 / g1;
-      gam[o + l] = g0;
-      a0 = a1;
-      gm = g0;
-      g0 = g1;
+      cd[o + l] = c;
     } else {
-      double A, D, C;
-      coef_spin(l, m, s, A, D, C);
-      const double g1 = l == l0 ? 1.0 : C * gm;
-      cd[2 * (o + l)] = A * g0 / g1;
-      cd[2 * (o + l) + 1] = D * g0 / g1;
-      gam[o + l] = g0;
-      gm = g0;
-      g0 = g1;
+      cd[2 * (o + l)] = c;
+      cd[2 * (o + l) + 1] = d;
     }
+    gam[o + l] = g;
   }
 }
 
