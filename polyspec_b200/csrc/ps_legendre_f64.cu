@@ -46,11 +46,17 @@ constexpr int SYN_THREADS = 128;  // threads per synthesis CTA
 constexpr int ADJ_LCH = 64;       // l chunk of the adjoint between two CTA barriers
 
 // ---------------------------------------------------------------- recurrence tables
-// One thread per order m, l by l (LegChain).  spin 0: cd is c [nalm]; spin s: (c, d) pairs.  Entries with l < s are
+// One thread per order m, l by l (LegChain), all spins of the plan side by side, since a chain's latency is what it takes
+// (four spins 43 us at lmax 47, 1.6 ms at 2048).  spin 0: cd is c [nalm]; spin s: (c, d) pairs.  Entries with l < s are
 // zero.  Runs once per plan.
-__global__ void leg_tables_f64(int lmax, int mmax, int s, double* __restrict__ cd, double* __restrict__ gam) {
-  const int m = blockIdx.x * blockDim.x + threadIdx.x;
-  if (m > mmax) return;
+struct LegTables {
+  double *cd[4], *gam[4];
+};
+__global__ void leg_tables_f64(int lmax, int mmax, LegTables t4) {
+  const int m = blockIdx.x * blockDim.x + threadIdx.x, s = blockIdx.y;
+  double* cd = t4.cd[s];
+  double* gam = t4.gam[s];
+  if (m > mmax || !cd) return;
   const int l0 = max(m, s);
   const int64_t o = alm_index(0, m, lmax);
   for (int l = m; l < min(l0, lmax + 1); ++l) {
@@ -624,8 +630,10 @@ int launch_synth_mma_f64(const Plan& P, const double2* alm, int64_t as, double2*
 int launch_adjoint_mma_f64(const Plan& P, const double2* phase, int64_t ms, int64_t bs, double2* alm, int64_t as, int B,
                            int spin, double scale, bool beside, cudaStream_t st);
 
-int launch_leg_tables_f64(const Plan& P, int spin, double* cd, double* gam, cudaStream_t st) {
-  leg_tables_f64<<<(P.mmax + 64) / 64, 64, 0, st>>>(P.lmax, P.mmax, spin, cd, gam);
+int launch_leg_tables_f64(const Plan& P, cudaStream_t st) {
+  LegTables t;
+  for (int s = 0; s < 4; ++s) t.cd[s] = P.d_leg_cd[s], t.gam[s] = P.d_leg_g[s];
+  leg_tables_f64<<<dim3((P.mmax + 64) / 64, 4), 64, 0, st>>>(P.lmax, P.mmax, t);
   PS_LAUNCH_CHECK();
   return PS_OK;
 }

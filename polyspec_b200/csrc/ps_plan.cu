@@ -15,7 +15,7 @@
 #include "ps_unit.h"
 
 namespace ps {
-int launch_leg_tables_f64(const Plan& P, int spin, double* cd, double* gam, cudaStream_t st);
+int launch_leg_tables_f64(const Plan& P, cudaStream_t st);
 int launch_legendre_synth_f64(const Plan& P, const double2* alm, int64_t as, double2* phase, int64_t ms, int64_t bs,
                               int B, int spin, bool grad, bool beside, cudaStream_t st);
 int launch_gc_to_pm(const double2* gc, double2* plus, double2* minus, int B, int64_t nalm, int spin, cudaStream_t st);
@@ -266,8 +266,8 @@ int ps_plan_create(int nside, int lmax, int mmax, int spin_mask, int prec, ps_pl
     const size_t elem = (prec == PS_PREC_FP64) ? sizeof(double2) : sizeof(float2);
     if (size_t(max_fft) * elem > size_t(optin)) { delete pl; return PS_ERR_UNSUPPORTED; }
   }
-  // rings of one work length, the power-of-two rings apart
-  std::vector<std::vector<int>> ring_cls_rings;
+  // rings of one work length, the power-of-two rings apart; their lists, all and north, one after the other
+  std::vector<int> ring_lists;
   for (auto kv = classes.rbegin(); kv != classes.rend(); ++kv)
     for (int blue = 1; blue >= 0; --blue) {
       std::vector<int> all, north;
@@ -280,8 +280,8 @@ int ps_plan_create(int nside, int lmax, int mmax, int spin_mask, int prec, ps_pl
       int logM = 0;
       while ((1 << logM) < kv->first) ++logM;
       pl->ring_cls.push_back({logM, blue, (int)all.size(), (int)north.size(), nullptr, nullptr});
-      ring_cls_rings.push_back(all);
-      ring_cls_rings.push_back(north);
+      ring_lists.insert(ring_lists.end(), all.begin(), all.end());
+      ring_lists.insert(ring_lists.end(), north.begin(), north.end());
     }
   std::vector<double2> tw(max_fft / 2);
   for (int k = 0; k < max_fft / 2; ++k) tw[k] = unit(-2 * k, max_fft);
@@ -386,9 +386,12 @@ int ps_plan_create(int nside, int lmax, int mmax, int spin_mask, int prec, ps_pl
     P.d_twiddle_f = dev_upload(pl, twf, err);
     P.d_bs_spec_f = dev_upload(pl, bsf, err);
   }
-  for (size_t c = 0; c < pl->ring_cls.size(); ++c) {
-    pl->ring_cls[c].rings = dev_upload(pl, ring_cls_rings[2 * c], err);
-    pl->ring_cls[c].rings_n = dev_upload(pl, ring_cls_rings[2 * c + 1], err);
+  // one upload (an allocation and a copy per list took a fifth of a small plan's creation)
+  const int* d_lists = dev_upload(pl, ring_lists, err);
+  for (ps::RingClassList& c : pl->ring_cls) {
+    c.rings = d_lists;
+    c.rings_n = d_lists + c.count;
+    d_lists += c.count + c.count_n;
   }
   {
     std::vector<int> zero(1, 0);
@@ -424,12 +427,18 @@ int ps_plan_create(int nside, int lmax, int mmax, int spin_mask, int prec, ps_pl
     P.d_chirp_off = dev_upload(pl, chirp_off, err);
   }
   if (prec == PS_PREC_FP64) {
-    for (int s = 0; s < 4 && err == PS_OK; ++s) {
+    int parts = 2;  // of nalm: c and gam of spin 0, (c, d) and gam of the others; pairs first, 16-byte aligned
+    for (int s = 1; s < 4; ++s) parts += P.d_seed[s] ? 3 : 0;
+    double* d = dev_alloc<double>(pl, size_t(P.nalm) * parts, err);
+    for (int s = 1; s < 4 && d; ++s)
+      if (P.d_seed[s]) { P.d_leg_cd[s] = d; d += 2 * P.nalm; }
+    for (int s = 0; s < 4 && d; ++s) {
       if (s > 0 && !P.d_seed[s]) continue;
-      P.d_leg_cd[s] = dev_alloc<double>(pl, size_t(P.nalm) * (s == 0 ? 1 : 2), err);
-      P.d_leg_g[s] = dev_alloc<double>(pl, size_t(P.nalm), err);
-      if (err == PS_OK) err = ps::launch_leg_tables_f64(P, s, P.d_leg_cd[s], P.d_leg_g[s], nullptr);
+      if (s == 0) { P.d_leg_cd[0] = d; d += P.nalm; }
+      P.d_leg_g[s] = d;
+      d += P.nalm;
     }
+    if (err == PS_OK) err = ps::launch_leg_tables_f64(P, nullptr);
     // the tables are read on the callers' streams
     if (err == PS_OK && cudaStreamSynchronize(nullptr) != cudaSuccess) err = PS_ERR_CUDA;
   }
