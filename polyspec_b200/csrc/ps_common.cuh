@@ -46,8 +46,10 @@ struct Plan {
   // c [nalm] (spin 0) or (c, d) [nalm][2], and gam [nalm]
   double* d_leg_cd[4];
   double* d_leg_g[4];
-  // FP64 plans: [max_fft/2] e^{-2 pi i k / max_fft}; Bluestein spectra; e^{i pi k / N}, k < N, of every ring
-  // length N = 4 i, i = 1 .. nside (at 2 i (i - 1)); the Bluestein chirps e^{-i pi j^2 / N}, j < N, of every slot
+  // FP64 plans: twiddles w^1, w^2 and w^4, w_j = e^{-2 pi i j / L}, j < L/8 each, for L = 8, 16, .. 2 max_fft, level after
+  // level; Bluestein spectra of every slot as [8][M/8], bit-reversed position 8 t + k at k M/8 + t; e^{i pi k / N}, k < N,
+  // of every ring length N = 4 i, i = 1 .. nside (at 2 i (i - 1)); the Bluestein chirps e^{-i pi j^2 / N}, j < N, of
+  // every slot
   double2* d_twiddle;
   double2* d_bs_spec;
   double2* d_root;

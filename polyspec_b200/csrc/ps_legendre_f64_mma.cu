@@ -4,12 +4,14 @@
 // loop), but it keeps that rate: FMAs with three distinct operands reach 60-75 % of it (register reads), and the
 // adjoint's sum over rings, which costs shuffles, selections and adds in ps_legendre_f64.cu, happens inside the
 // MMA.  What it needs is eight columns: four maps of spin 0 (re, im) or two of spin s (four sums each).  So this
-// file takes batches and ps_legendre_f64.cu single maps; the rule and both sides' times stand at its launchers.
+// file takes batches, and ps_legendre_f64.cu single maps and batches that do not fill the chip; the rule and both sides'
+// times stand at its launchers.
 //
-// A warp owns 32 ring pairs (spin-s synthesis: 16).  Every lane runs the recurrence of its ring for 16 l (spin 0) or
-// 8 l (spin s: f and (-1)^l g) and drops the values into the warp's shared tile, 16 rows of 32 rings, whose columns are
-// ordered so that one 16-byte read gives a lane the elements of two A operands, 8 rings x 4 l (synthesis) or 8 l x 4
-// rings (adjoint).  Rows 0-7 hold the l of parity 0 (f), rows 8-15 those of parity 1 ((-1)^l g):
+// A warp owns 32 ring pairs.  Every lane runs the recurrence of its ring for 16 l (spin 0) or 8 l (adjoint of spin s: f
+// and (-1)^l g) and drops the values into the warp's shared tile, 16 rows of 32 rings, whose columns are ordered so that
+// one 16-byte read gives a lane the elements of two A operands, 8 rings x 4 l (synthesis) or 8 l x 4 rings (adjoint).
+// Rows 0-7 hold the l of parity 0 (f), rows 8-15 those of parity 1 ((-1)^l g).  The spin-s synthesis owns 16 pairs, for
+// 16 l, f and g in half-warps (see there).
 //   synthesis spin 0: B = alm; E, O = even and odd sums, north = E + O, south = E - O.
 //   synthesis spin s: B = (a+, (-1)^l a-) for f and, the same columns exchanged, for (-1)^l g; the
 //                     accumulators are the north and south sums of ps_legendre_f64.cu.
@@ -19,8 +21,9 @@
 // Synthesis: accumulators of the warp's rings stay in registers over all l; the alm of 32 l are staged for the CTA's
 // four warps.  Adjoint: the B operand (phases) stays in registers over all l; per 16 l the warps' sums meet in
 // shared memory and are added up in a fixed order.  What bounds it is the latency of twelve warps an SM (the B
-// operand takes their registers): the MMA pipe is busy 41 % of the time.  Running the next tile's recurrence between
-// one tile's MMAs (two tiles a warp) was slower, 2806 us for 2667: it spills, and its FMAs queue behind the MMAs.
+// operand takes their registers): the MMA pipe is busy 47 % of the time (24 maps, Nside 512, lmax 1000; 48 spin-2 maps,
+// Nside 128: 41 %).  Running the next tile's recurrence between one tile's MMAs (two tiles a warp) was slower, 2806 us
+// for 2667: it spills, and its FMAs queue behind the MMAs.
 #include <algorithm>
 #include <climits>
 #include <type_traits>

@@ -5,7 +5,8 @@
 // plan holding the Legendre table of the spin this runs as: strided gather of the
 // input alm with the factor (layout [nalm][batch][ncomp]) -> table synthesis
 // (tensor cores) -> one ring kernel that synthesises each ring in shared memory,
-// weights its pixels and transforms it back (the maps never reach HBM) -> table adjoint writing the strided output with the factor.
+// weights its pixels and transforms it back (the maps never reach HBM) -> table
+// adjoint writing the strided output with the factor.
 // Without the table the entry returns PS_ERR_UNSUPPORTED and the caller composes
 // ps_synthesis, the weighting and ps_adjoint itself.
 #include <algorithm>
