@@ -102,6 +102,11 @@ double2 unit(int64_t q, int64_t den) {  // e^{i pi q / den}
   ps::unit_root(q, den, w.x, w.y);
   return w;
 }
+// the same for tables that are rounded to FP32: enough for them, and a few of their entries would round the other way
+double2 unit_f32(int64_t q, int64_t den) {
+  const double a = M_PI * double(q % (2 * den)) / double(den);
+  return make_double2(std::cos(a), std::sin(a));
+}
 
 int host_bitrev(int i, int logn) {
   int r = 0;
@@ -284,7 +289,8 @@ int ps_plan_create(int nside, int lmax, int mmax, int spin_mask, int prec, ps_pl
       ring_lists.insert(ring_lists.end(), north.begin(), north.end());
     }
   std::vector<double2> tw(max_fft / 2);
-  for (int k = 0; k < max_fft / 2; ++k) tw[k] = unit(-2 * k, max_fft);
+  const auto root_of = prec == PS_PREC_FP64 ? unit : unit_f32;
+  for (int k = 0; k < max_fft / 2; ++k) tw[k] = root_of(-2 * k, max_fft);
   // ---- Bluestein spectra: b_n = e^{+i pi n^2 / N}, |n| < N, wrapped to M; FFT_M, bit-reversed order
   std::vector<double2> bs_spec;
   std::vector<int64_t> bs_off;
@@ -293,7 +299,7 @@ int ps_plan_create(int nside, int lmax, int mmax, int spin_mask, int prec, ps_pl
     int logM = 0; while ((1 << logM) < M) ++logM;
     std::vector<std::complex<double>> b(M, 0.0);
     for (int n = 0; n < N; ++n) {
-      const double2 w = unit(int64_t(n) * n, N);
+      const double2 w = root_of(int64_t(n) * n, N);
       const std::complex<double> v(w.x, w.y);
       b[n] = v;
       if (n > 0) b[M - n] = v;
@@ -408,8 +414,8 @@ int ps_plan_create(int nside, int lmax, int mmax, int spin_mask, int prec, ps_pl
       const int64_t num = rings[rp].phi_num, den = rings[rp].phi_den;
       for (int m = 0; m <= mmax; ++m) {
         const int64_t q = (int64_t(m) * num) % (2 * den);
-        const double a = M_PI * double(q) / double(den);
-        rot[size_t(rp) * (mmax + 1) + m] = make_float2(float(std::cos(a)), float(std::sin(a)));
+        const double2 w = unit_f32(q, den);
+        rot[size_t(rp) * (mmax + 1) + m] = make_float2(float(w.x), float(w.y));
       }
     }
     std::vector<float2> chirp;
